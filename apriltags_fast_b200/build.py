@@ -52,7 +52,7 @@ def build(force: bool = False) -> str:
     if force or _newer(fam_c, [fam_bin, os.path.join(CSRC, "gen_families.py")]):
         _run([sys.executable, os.path.join(CSRC, "gen_families.py"), "csource", fam_c])
     fam_o = os.path.join(BUILD, "at_families_data.o")
-    if force or _newer(fam_o, [fam_c]):
+    if force or _newer(fam_o, [fam_c, os.path.join(ROOT, "include", "apriltag_fast.h")]):
         _run(["gcc", "-O1", "-fPIC", "-I", os.path.join(ROOT, "include"), "-c", fam_c, "-o", fam_o])
     objs.append(fam_o)
     # the upstream API shim (plain C over the native API)

@@ -21,6 +21,7 @@
 #define APRILTAG_FAST_H
 
 #include <stdbool.h>
+#include <stddef.h>
 #include <stdint.h>
 
 #ifdef __cplusplus
