@@ -100,16 +100,11 @@ enum {
     B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
     B_HYMIN, B_HYMAX, B_CSPAN, B_CY0, B_SPANOFF, B_PKFRAME, B_PGKEYS, B_PGSLOTS, B_PFRAMES, B_PBSUM, B_SEG,
-    B_QCL, B_CKEY, B_RNEED, B_RNT, B_RTLAB, B_RTPX, B_RTROOT, B_RTLIST, B_RTROW, B_RPRE, B_ROKEY, B_RIDX2, B_RSCR,
-    B_RFIN, B_RFINB, B_RBSLOT, B_RBINFO, B_ROUTROOT, B_RBM, B_RBSTART, B_RBWIDE, B_RDESC, B_RNBAND, B_RFSCR, B_RTCH, B_RLTOP, B_RLPX, B_RLBOT,
-    B_RLPX2,
+    B_QCL, B_CKEY, B_RNEED, B_RNT, B_RTLAB, B_RTPX, B_RTROOT, B_RTLIST, B_RTROW, B_RPRE, B_ROKEY, B_RIDX2,
+    B_RPAR, B_RSUM, B_RSTAMP, B_RTCH, B_RHIST,
     B_PREC, B_PPSLOT, B_PPCNT, B_PINFO, B_QSCR,
     B_CUB, B_ERR, B_NBUF
 };
-
-// the replay of the reference's union order keeps its arrays in shared
-// memory up to this size, else in a global scratch region per frame
-#define AT_REF_SMEM_MAX (200 * 1024)
 
 }  // namespace
 
@@ -135,7 +130,6 @@ struct at_internal {
     // sizes of the last run (frame 0), for at_detector_diag
     int64_t last_qw = 0, last_qh = 0, last_npts = 0, last_ncl = 0, last_nq = 0;
     int64_t launches = 0;  // kernels of this library launched so far
-    size_t ref_smem = 0;     // the shared memory the replay kernel is allowed (set per device)
     bool scan_smem = false;  // the point scan's shared memory allowance is set
     int64_t seg_slack = 64;  // row-table entries per cluster beyond its points (grows on a shortfall)
 
@@ -736,35 +730,20 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_RPRE].ensure((rows + n) * 4));
         CK(B[B_ROKEY].ensure(nd * 16));
         CK(B[B_RIDX2].ensure(nd * 4));
-        CK(B[B_RFIN].ensure(n * AT_REF_MAXT * 4));
-        CK(B[B_RFINB].ensure(n * AT_REF_MAXT * 4));
-        CK(B[B_RBSLOT].ensure(nodes * 2));
-        CK(B[B_RBINFO].ensure(nodes * 8));
-        CK(B[B_ROUTROOT].ensure(nodes * 4));
-        CK(B[B_RBM].ensure(rows * 4));
-        CK(B[B_RBSTART].ensure((rows + n) * 4));
-        CK(B[B_RBWIDE].ensure((rows + n) * 4));
-        CK(B[B_RDESC].ensure((rows + n) * 16));
-        CK(B[B_RNBAND].ensure(n * 4));
+        CK(B[B_RPAR].ensure(nodes * 8));
+        CK(B[B_RSUM].ensure(nodes * 4));
+        CK(B[B_RSTAMP].ensure(nodes * 4));
         CK(B[B_RTCH].ensure(nodes * 4));
-        CK(B[B_RLTOP].ensure(nodes * 4));
-        CK(B[B_RLPX].ensure(nodes * 4));
-        CK(B[B_RLBOT].ensure(nodes * 4));
-        CK(B[B_RLPX2].ensure(nodes * 4));
-        CK(cudaMemsetAsync(B[B_RTROOT].p, 0xff, n * AT_REF_MAXT * 4, st));
-        CK(cudaMemsetAsync(B[B_RFINB].p, 0xff, n * AT_REF_MAXT * 4, st));
-        const RefOrder ro{B[B_RNEED].as<uint32_t>(),   B[B_RNT].as<uint32_t>(),     B[B_RTLAB].as<uint32_t>(),
-                          B[B_RTPX].as<uint32_t>(),    B[B_RTROOT].as<uint32_t>(),  B[B_RTLIST].as<uint64_t>(),
-                          B[B_RTROW].as<uint32_t>(),   B[B_RPRE].as<uint32_t>(),    B[B_RFIN].as<uint32_t>(),
-                          B[B_RFINB].as<uint32_t>(),   B[B_RBSTART].as<uint32_t>(), B[B_RBWIDE].as<uint32_t>(),
-                          B[B_RDESC].as<uint4>(),      B[B_RNBAND].as<uint32_t>(),  B[B_RTCH].as<uint32_t>(),
-                          B[B_RLTOP].as<uint32_t>(),
-                          B[B_RLPX].as<uint32_t>(),
-                          B[B_RLBOT].as<uint32_t>(),   B[B_RLPX2].as<uint32_t>(),   B[B_RBSLOT].as<uint16_t>(),
-                          B[B_RBINFO].as<uint64_t>(),  B[B_ROUTROOT].as<uint32_t>(), B[B_RBM].as<uint32_t>()};
+        CK(B[B_RHIST].ensure(rows * AT_REF_MAXT * 4));
+        CK(cudaMemsetAsync(B[B_RHIST].p, 0, rows * AT_REF_MAXT * 4, st));
+        const RefOrder ro{B[B_RNEED].as<uint32_t>(),  B[B_RNT].as<uint32_t>(),    B[B_RTLAB].as<uint32_t>(),
+                          B[B_RTPX].as<uint32_t>(),   B[B_RTROOT].as<uint32_t>(), B[B_RTLIST].as<uint64_t>(),
+                          B[B_RTROW].as<uint32_t>(),  B[B_RPRE].as<uint32_t>(),   B[B_RPAR].as<uint64_t>(),
+                          B[B_RSUM].as<uint32_t>(),   B[B_RSTAMP].as<uint32_t>(), B[B_RTCH].as<uint32_t>(),
+                          B[B_RHIST].as<uint32_t>()};
         int64_t capr = 1;
         for (auto &f : fd) capr = f.qw - 1 > capr ? f.qw - 1 : capr;
-        if (nodes >= ((int64_t)1 << 31)) {  // the replay marks symbols with the top bit of a node id
+        if (nodes >= ((int64_t)1 << 31)) {
             set_error(in, 2, "batch too large for the order replay (node ids above 2^31)");
             return false;
         }
@@ -772,30 +751,10 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
             set_error(in, 2, "quad image too wide for the order replay (" + std::to_string(capr + 1) + " px)");
             return false;
         }
-        // the frontier pass and the wide-row replay work in global scratch
-        // when their arrays do not fit the shared memory
-        RefPlan plan{capr, capr > REF_PCAP_MIN ? capr : REF_PCAP_MIN, nullptr, 0, nullptr, 0};
-        if (ref_frontier_bytes(capr, true) > AT_REF_SMEM_MAX) {
-            plan.front_bytes = ref_frontier_bytes(capr, false);
-            CK(B[B_RFSCR].ensure(plan.front_bytes * n));
-            plan.front_scratch = B[B_RFSCR].as<uint8_t>();
-        }
-        if (capr > REF_SMALLR && ref_band_bytes(capr, true) > AT_REF_SMEM_MAX) {
-            plan.band_bytes = ref_replay_bytes(capr);
-            CK(B[B_RSCR].ensure(plan.band_bytes * n * REF_BAND_BLOCKS));
-            plan.band_scratch = B[B_RSCR].as<uint8_t>();
-        }
-        if (in->ref_smem == 0) {
-            if (!ref_replay_set_smem(AT_REF_SMEM_MAX)) {
-                set_error(in, 1, "cudaFuncSetAttribute for the order replay failed");
-                return false;
-            }
-            in->ref_smem = AT_REF_SMEM_MAX;
-        }
-        launch_ref_order(L, dfr, thr, runs, B[B_ROWRUNS].as<uint32_t>(), in->nfam, B[B_QSTART].as<int64_t>(),
-                         B[B_DETS].as<GpuDetection>(), B[B_DETOK].as<uint32_t>(), B[B_QCL].as<uint32_t>(), ckey, nb,
-                         plan, ro, B[B_ERR].as<uint32_t>());
-        in->launches += ref_order_launches(plan);
+        in->launches += launch_ref_order(L, dfr, thr, runs, B[B_ROWRUNS].as<uint32_t>(), in->nfam,
+                                         B[B_QSTART].as<int64_t>(), B[B_DETS].as<GpuDetection>(),
+                                         B[B_DETOK].as<uint32_t>(), B[B_QCL].as<uint32_t>(), ckey, nb, ro,
+                                         B[B_ERR].as<uint32_t>());
         launch_finalize(st, (int)n, B[B_QSTART].as<int64_t>(), in->nfam, B[B_DETS].as<GpuDetection>(),
                         B[B_DETOK].as<uint32_t>(), B[B_DIDX].as<uint32_t>(), B[B_DRM].as<uint8_t>(),
                         B[B_OUT].as<GpuDetection>(), B[B_OUTOFF].as<int64_t>(), B[B_OUTN].as<int64_t>(), dfr, ro,

@@ -126,59 +126,31 @@ void launch_decode(cudaStream_t s, const FrameDesc *frames, const GpuParams &prm
                    const DecodeScratch &scr, GpuDetection *dets, uint32_t *det_ok);
 // The reference's order of the quads whose detections share an id
 // (at_order.cu). Per frame: whether it has such detections (need), the
-// target components (GPU labels, pixel counts, and after the replay their
-// roots in the reference's packed node numbering); per node, the frame's
-// target runs compacted by row (tlist); per row, their count (trow); per
-// row plus one per frame, the runs above the row (rpre).
+// target components (GPU labels, pixel counts, and at last their roots in
+// the reference's packed node numbering); per node, the frame's target runs
+// compacted by row (tlist); per row, their count (trow); per row plus one
+// per frame, the runs above the row (rpre).
 #define AT_REF_MAXT 192
-#define REF_BAND 16         // rows per band of the replay, at most
-#define REF_PCAP 4160       // target runs of a row, at most (quad images up to 4161 px wide)
-#define REF_PCAP_MIN 2048   // target runs per band, at most, when every row has fewer
-#define REF_SMALLR 256      // the replay's narrow class: rows of at most this many target runs
-#define REF_BAND_BLOCKS 32  // replay blocks per frame when the replay works in a global scratch
+#define REF_PCAP 4160       // runs of a row, at most (quad images up to 4161 px wide)
 struct RefOrder {
     uint32_t *need, *nt;
     uint32_t *tlabel, *tpx, *troot;
     uint64_t *tlist;
     uint32_t *trow;
     uint32_t *rpre;
-    uint32_t *fin, *finb;     // per target: its root (node or symbol) and the band where it was found
-    // per band (rows + one per frame each): first row (and the end after the
-    // last band), the widest row, the band's summary (at_order.cu); per
-    // frame: the band count
-    uint32_t *bstart, *bwide;
-    uint4 *desc;
-    uint32_t *nband;
-    // per node (at the rows of the band edges, at_order.cu):
-    uint32_t *tch;            //   each target run: the target runs above it touches (first | last << 16)
-    uint32_t *ltop, *lpx;     //   top row: each run's band component, their pixels
-    uint32_t *lbot, *lpx2;    //   bottom row: each run's band component, the others' pixels
-    uint16_t *bslot;          //   row above a band: each target run's slot
-    uint64_t *binfo;          //   row above a band: each slot, pixels | first run << 32 | target << 48
-    uint32_t *outroot;        //   row above a band: each slot's root after the band above
-    uint32_t *bm;             // per row: slots at the row above a band
+    // per node: its edge in the forest of unions (time << 32 | parent), the
+    // pixels below it, a mark; per target run (in tlist's order): the first
+    // and last run of the row above that it touches
+    uint64_t *par;
+    uint32_t *sum, *stamp, *tch;
+    // per target (AT_REF_MAXT a frame) and row: pixels gained (zeroed by the caller)
+    uint32_t *hist;
 };
-// The sizes the order replay runs at: capr, the most runs in a row of the
-// batch; pcap, the most target runs of a band; global scratch regions (a
-// frame's, a block's) for the frontier pass and the wide-row replay when
-// their arrays exceed the shared memory (else null).
-struct RefPlan {
-    int64_t capr, pcap;
-    uint8_t *front_scratch;
-    size_t front_bytes;
-    uint8_t *band_scratch;
-    size_t band_bytes;
-};
-size_t ref_replay_bytes(int64_t capr);
-size_t ref_band_bytes(int64_t capr, bool staged);
-size_t ref_local_bytes(int64_t pcap);
-size_t ref_frontier_bytes(int64_t capr, bool staged);
-bool ref_replay_set_smem(size_t bytes);
-int ref_order_launches(const RefPlan &P);
-void launch_ref_order(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
-                      const uint32_t *row_nruns, int nfam, const int64_t *qstart, const GpuDetection *dets,
-                      const uint32_t *det_ok, const uint32_t *qcl, const uint64_t *ckey, int nb,
-                      const RefPlan &P, const RefOrder &ref, uint32_t *err);
+// returns the kernels launched
+int launch_ref_order(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
+                     const uint32_t *row_nruns, int nfam, const int64_t *qstart, const GpuDetection *dets,
+                     const uint32_t *det_ok, const uint32_t *qcl, const uint64_t *ckey, int nb, const RefOrder &ref,
+                     uint32_t *err);
 // okey: 2 u64 + 1 u32 per detection slot (the order keys, a second index)
 void launch_finalize(cudaStream_t s, int nframes, const int64_t *frame_qstart, int nfam, const GpuDetection *dets,
                      const uint32_t *det_ok, uint32_t *idx, uint8_t *removed, GpuDetection *out,
