@@ -118,9 +118,9 @@ struct at_internal {
     bool fam_dirty = true;
 
     int device = 0;
-    cudaStream_t stream = nullptr, side = nullptr, side2 = nullptr, side3 = nullptr;
+    cudaStream_t stream = nullptr;
     cudaEvent_t ev[12];
-    cudaEvent_t fork = nullptr, join = nullptr, join2 = nullptr, join3 = nullptr;  // ordering only, no timing
+    FitStreams fit = {};  // the fit's own streams
     DBuf buf[B_NBUF];
     HBuf h_frames, h_small, h_out;
     std::vector<at_detection> dets;
@@ -666,7 +666,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_QOK].ensure(ncl * 4));
         CK(B[B_QSCAN].ensure((ncl + 1) * 4));
         CK(B[B_QSCR].ensure(scan_u32_scratch(ncl) * 4));
-        CK(B[B_FLIST].ensure(ncl * 4 * 5));
+        CK(B[B_FLIST].ensure(ncl * 4 * 6));
         CK(B[B_FCNT].ensure(64));
         FitScratch scr{B[B_SKEYS].as<uint64_t>(), B[B_SSKEY].as<uint64_t>(), B[B_SSVAL].as<uint32_t>(),
                        B[B_SW].as<double>(),      B[B_SFX].as<double>(),    B[B_SFY].as<double>(),
@@ -675,9 +675,11 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
                        B[B_SERRS].as<double>(),   B[B_SFILT].as<double>(),  B[B_SMXE].as<double>(),
                        B[B_SMXI].as<int32_t>(),   B[B_FLIST].as<uint32_t>(), B[B_FCNT].as<uint32_t>()};
         uint32_t *qok = B[B_QOK].as<uint32_t>(), *qscan = B[B_QSCAN].as<uint32_t>();
-        launch_fit_quads(st, in->side, in->side2, in->side3, in->fork, in->join, in->join2, in->join3, dfr, prm, qim, spts, B[B_CSTART].as<uint32_t>(), B[B_CFRAME].as<int32_t>(), ncl,
-                         (int64_t)npts, scr, B[B_QUADS].as<GpuQuad>(), qok, B[B_ERR].as<uint32_t>());
-        in->launches += 8;
+        int64_t max_px = 0;
+        for (auto &f : fd) max_px = f.max_px > max_px ? f.max_px : max_px;
+        in->launches += launch_fit_quads(st, in->fit, dfr, prm, qim, spts, B[B_CSTART].as<uint32_t>(),
+                                         B[B_CFRAME].as<int32_t>(), ncl, (int64_t)npts, max_px, scr,
+                                         B[B_QUADS].as<GpuQuad>(), qok, B[B_ERR].as<uint32_t>());
         CK(cudaGetLastError());
         launch_scan_u32(st, qok, ncl, qscan, B[B_QSCR].as<uint32_t>());
         in->launches += 3;
@@ -856,13 +858,9 @@ at_detector *at_detector_create(void) {
         abort();
     }
     for (int k = 0; k < 12; k++) cudaEventCreate(&in->ev[k]);
-    cudaStreamCreateWithFlags(&in->side, cudaStreamNonBlocking);
-    cudaStreamCreateWithFlags(&in->side2, cudaStreamNonBlocking);
-    cudaStreamCreateWithFlags(&in->side3, cudaStreamNonBlocking);
-    cudaEventCreateWithFlags(&in->fork, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&in->join, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&in->join2, cudaEventDisableTiming);
-    cudaEventCreateWithFlags(&in->join3, cudaEventDisableTiming);
+    for (cudaStream_t &q : in->fit.side) cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking);
+    cudaEventCreateWithFlags(&in->fit.fork, cudaEventDisableTiming);
+    for (cudaEvent_t &e : in->fit.join) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     return td;
 }
 
@@ -895,13 +893,9 @@ void at_detector_destroy(at_detector *td) {
             if (e) cudaEventDestroy(e);
         delete in->chain;
     }
-    cudaEventDestroy(in->fork);
-    cudaEventDestroy(in->join);
-    cudaEventDestroy(in->join2);
-    cudaEventDestroy(in->join3);
-    cudaStreamDestroy(in->side);
-    cudaStreamDestroy(in->side2);
-    cudaStreamDestroy(in->side3);
+    cudaEventDestroy(in->fit.fork);
+    for (cudaEvent_t e : in->fit.join) cudaEventDestroy(e);
+    for (cudaStream_t q : in->fit.side) cudaStreamDestroy(q);
     cudaStreamDestroy(in->stream);
     delete in;
     free(td);

@@ -1333,58 +1333,65 @@ __device__ __forceinline__ void leaf_network(uint64_t *k, int n) {
 }
 
 
-// Sort (key, val) pairs ascending by key (keys distinct): a merge sort of
-// log2(n) levels; at each level every thread writes a contiguous chunk of
-// the output, starting at the merge-path split of its first element (a
-// binary search). kb/vb are scratch of n entries; the result is in ka/va.
-__device__ void block_merge_sort(uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_t *vb, int n) {
-    uint64_t *sk = ka, *dk = kb;
-    uint32_t *sv = va, *dv = vb;
-    const int ipt = (n + (int)blockDim.x - 1) / (int)blockDim.x;
-    for (int w = 1; w < n; w <<= 1) {
-        const int o0 = (int)threadIdx.x * ipt, o1 = min(n, o0 + ipt);
-        int o = o0;
-        while (o < o1) {
-            const int lo = (o / (2 * w)) * (2 * w);
-            const int la = min(w, n - lo), lb = max(0, min(w, n - lo - la));
-            const uint64_t *A = sk + lo, *B = sk + lo + la;
-            const int k = o - lo, seg_end = min(o1, lo + la + lb);
-            int l = max(0, k - lb), h = min(k, la);
-            while (l < h) {
-                const int m = (l + h) >> 1;
-                if (A[m] < B[k - m - 1])
-                    l = m + 1;
-                else
-                    h = m;
+// The six moment terms of a point (fast/quads.c:968-1035): w =
+// sqrt(gx^2 + gy^2) + 1 on the quad image (1 at its border), fx = x / 2 +
+// 1 / 2, the reference's products. g2: the squared gradient at pt.
+__device__ __forceinline__ int32_t point_grad2(const uint8_t *im, int qw, int qh, uint64_t pt) {
+    const int32_t px = (int32_t)(pt & 0xffff), py = (int32_t)(pt >> 16 & 0xffff);
+    const int32_t ix = (px >> 1) + (px & 1), iy = (py >> 1) + (py & 1);
+    if (ix <= 0 || ix + 1 >= qw || iy <= 0 || iy + 1 >= qh) return 0;
+    const int64_t cc = (int64_t)iy * qw + ix;
+    const int32_t gx = (int32_t)im[cc + 1] - im[cc - 1];
+    const int32_t gy = (int32_t)im[cc + qw] - im[cc - qw];
+    return gx * gx + gy * gy;
+}
+__device__ __forceinline__ void moment_terms(uint64_t pt, int32_t g2, double m[6]) {
+    const int32_t px = (int32_t)(pt & 0xffff), py = (int32_t)(pt >> 16 & 0xffff);
+    const double w = __dadd_rn(__dsqrt_rn((double)g2), 1.0);
+    const double fx = __dadd_rn(__dmul_rn((double)px, 0.5), 0.5);
+    const double fy = __dadd_rn(__dmul_rn((double)py, 0.5), 0.5);
+    const double wx = __dmul_rn(w, fx), wy = __dmul_rn(w, fy);
+    m[0] = wx;
+    m[1] = wy;
+    m[2] = __dmul_rn(wx, fx);
+    m[3] = __dmul_rn(wx, fy);
+    m[4] = __dmul_rn(wy, fy);
+    m[5] = w;
+}
+
+// The prefix sums of src[0, n) in place, after `run`, one lane: a chain of
+// dependent additions (8.3 cycles each); the next 8 terms are loaded before
+// the additions of these 8, and the stores follow them, so the chain does
+// not wait for shared memory.
+__device__ __forceinline__ void prefix_chain(double *src, int n, double &run) {
+    int t = 0;
+    if (n >= 8) {
+        double v[8], x[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = src[u];
+        for (; t + 16 <= n; t += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; u++) x[u] = src[t + 8 + u];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                run = __dadd_rn(run, v[u]);
+                v[u] = run;
             }
-            int i = l, j = k - l;
-            for (; o < seg_end; o++) {
-                const bool take_a = j >= lb || (i < la && A[i] < B[j]);
-                if (take_a) {
-                    dk[o] = A[i];
-                    dv[o] = sv[lo + i];
-                    i++;
-                } else {
-                    dk[o] = B[j];
-                    dv[o] = sv[lo + la + j];
-                    j++;
-                }
-            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) src[t + u] = v[u];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = x[u];
         }
-        __syncthreads();
-        uint64_t *tk = sk;
-        sk = dk;
-        dk = tk;
-        uint32_t *tv = sv;
-        sv = dv;
-        dv = tv;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            run = __dadd_rn(run, v[u]);
+            src[t + u] = run;
+        }
+        t += 8;
     }
-    if (sk != ka) {
-        for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            ka[t] = sk[t];
-            va[t] = sv[t];
-        }
-        __syncthreads();
+    for (; t < n; t++) {
+        run = __dadd_rn(run, src[t]);
+        src[t] = run;
     }
 }
 
@@ -1497,78 +1504,69 @@ __device__ __forceinline__ void line_of(MSum s, double lp[4], double *mse) {
 }
 
 
-// A double as a 64-bit integer in the same order (negative values
-// reversed below the positive ones); no NaN reaches it.
-__device__ __forceinline__ uint64_t dorder_key(double d) {
-    const uint64_t b = (uint64_t)__double_as_longlong(d);
-    return (b >> 63) ? ~b : b | 0x8000000000000000ull;
-}
-__device__ __forceinline__ double dorder_val(uint64_t k) {
-    return __longlong_as_double((long long)((k >> 63) ? k & 0x7fffffffffffffffull : ~k));
+// The largest of a warp's e[first], e[first + stride], ... (below n) after
+// (pv, pi) in the order (value descending, index ascending); -inf if none.
+__device__ __forceinline__ void warp_next_desc(const double *e, int n, int first, int stride, double &pv, int &pi) {
+    double v = -__longlong_as_double(0x7ff0000000000000ll);
+    int at = 0x7fffffff;
+    for (int i = first; i < n; i += stride) {
+        const double x = e[i];
+        if ((x < pv || (x == pv && i > pi)) && x > v) {
+            v = x;
+            at = i;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
+        const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
+        if (v2 > v || (v2 == v && a2 < at)) {
+            v = v2;
+            at = a2;
+        }
+    }
+    pv = v;
+    pi = at;
 }
 
-// The (r+1)-th largest of e[0, n) (r < n), by the whole block: a radix
-// select over dorder_key, 8 bits a pass from the top. hist holds 256
-// counters; *selp and *selr are the prefix found and the rank left.
-// Warp 0 finds each pass's digit: lane l counts digits 255-8l .. 248-8l.
-__device__ double block_select_desc(const double *e, int64_t n, uint32_t r, uint32_t *hist, uint64_t *selp,
-                                    uint32_t *selr) {
-    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31;
-    if (tid == 0) {
-        *selp = 0;
-        *selr = r;
+// The (r + 1)-th largest of e[0, n) (r < n, r <= AT_MAX_NMAXIMA), by the
+// whole block: each warp's r + 1 largest (they hold the block's), then those
+// of the warps' lists by warp 0. cand: (r + 1) values per warp. A radix
+// select over the 64 bits (8 passes, three barriers each) took 20k cycles
+// for 700 points and 140k for 21000; this takes r + 1 short rounds.
+__device__ double block_select_desc(const double *e, int n, int r, double *cand, double *res) {
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    const double inf = __longlong_as_double(0x7ff0000000000000ll);
+    double pv = inf;
+    int pi = -1;
+    __syncthreads();
+    for (int t = 0; t <= r; t++) {
+        warp_next_desc(e, n, threadIdx.x, blockDim.x, pv, pi);
+        if (lane == 0) cand[w * (r + 1) + t] = pv;
     }
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        for (int b = tid; b < 256; b += nt) hist[b] = 0;
-        __syncthreads();
-        const uint64_t prefix = *selp, mask = shift == 56 ? 0ull : ~0ull << (shift + 8);
-        for (int64_t i = tid; i < n; i += nt) {
-            const uint64_t key = dorder_key(e[i]);
-            if ((key & mask) == prefix) atomicAdd(hist + ((key >> shift) & 255u), 1u);
-        }
-        __syncthreads();
-        if (tid < 32) {
-            const uint32_t rr = *selr;
-            uint32_t c[8], sum = 0;
-#pragma unroll
-            for (int j = 0; j < 8; j++) {
-                c[j] = hist[255 - 8 * lane - j];
-                sum += c[j];
-            }
-            uint32_t inc = sum;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            const uint32_t excl = inc - sum;
-            if (excl <= rr && rr < inc) {
-                uint32_t acc = excl;
-                int bin = 255 - 8 * lane;
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    if (rr >= acc + c[j]) {
-                        acc += c[j];
-                        continue;
-                    }
-                    bin = 255 - 8 * lane - j;
-                    break;
-                }
-                *selr = rr - acc;
-                *selp = prefix | (uint64_t)bin << shift;
-            }
-        }
-        __syncthreads();
+    __syncthreads();
+    if (w == 0) {
+        pv = inf;
+        pi = -1;
+        for (int t = 0; t <= r; t++) warp_next_desc(cand, nw * (r + 1), lane, 32, pv, pi);
+        if (lane == 0) *res = pv;
     }
-    return dorder_val(*selp);
+    __syncthreads();
+    return *res;
 }
 
-// Two size classes of clusters, one kernel template: 128 threads for
-// clusters of at most FIT_SMALL points (everything staged in shared
-// memory), FIT_LARGE_NT threads for the larger ones (dynamic shared memory; sorts
-// beyond FIT_LARGE_SORT points fall back to global scratch).
+// Three size classes of clusters, one kernel template: 128 threads for
+// clusters of at most FIT_SMALL points, FIT_LARGE_NT threads, two blocks an
+// SM, up to FIT_LARGE_SORT, FIT_HUGE_NT threads, one block an SM, above. The
+// last sorts in shared memory up to FIT_HUGE_SORT points and in global
+// scratch beyond (the same radix sort). Clusters above 6144 points come only
+// from quad images above about 1080p (a cluster has at most 4 (qw + qh)
+// points); a merge sort in global memory, with the blocks of the class
+// below, took 1.4M cycles for 9000 points and 3.9M for 21000.
 #define FIT_SMALL 1024
 #define FIT_LARGE_SORT 6144
+#define FIT_HUGE_SORT 13312
+#define FIT_HUGE_NT 512
 #define FIT_CHUNK_SMALL 256
 #define FIT_CHUNK_LARGE 512
 #define FIT_LARGE_NT 256  // threads of the largest class's blocks (two blocks an SM)
@@ -1688,6 +1686,26 @@ extern "C" int at_fit_prof_copy(void *dst, int n) {
 #define DEC_PROF(k)
 #endif
 
+// The 4-subsets {m0 < m1 < m2 < m3} of {0..15} in colex order (by m3, then
+// m2, m1, m0), one per entry as nibbles m0 | m1 << 4 | m2 << 8 | m3 << 12:
+// the first C(n, 4) entries are the 4-subsets of {0..n-1}.
+struct Quad4Table {
+    uint16_t v[1820];
+};
+constexpr Quad4Table make_quad4() {
+    Quad4Table t{};
+    int k = 0;
+    for (int d = 3; d < 16; d++)
+        for (int c = 2; c < d; c++)
+            for (int b = 1; b < c; b++)
+                for (int a = 0; a < b; a++) t.v[k++] = (uint16_t)(a | b << 4 | c << 8 | d << 12);
+    return t;
+}
+__device__ const Quad4Table g_quad4 = make_quad4();
+static_assert(AT_MAX_NMAXIMA <= 16, "the 4-subset table covers 16 maxima");
+
+__host__ __device__ constexpr int binom4(int n) { return n < 4 ? 0 : n * (n - 1) * (n - 2) * (n - 3) / 24; }
+
 template <int NT>
 __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit_quads(const FrameDesc *frames, GpuParams prm, const uint8_t *qim,
                                                    const uint64_t *pts, const uint32_t *cstart,
@@ -1711,10 +1729,9 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
     __shared__ double s_perr[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA], s_pmse[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA],
         s_pnx[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA], s_pny[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA];
     __shared__ double s_be[NT / 32], s_lines[4][4], s_lmse[4], s_best;
-    __shared__ int64_t s_bo[NT / 32];
+    __shared__ int s_bo[NT / 32];
     __shared__ uint32_t s_next;
-    __shared__ uint64_t s_selp;
-    __shared__ uint32_t s_selr;
+    __shared__ double s_cand[(NT / 32) * (AT_MAX_NMAXIMA + 1)];
     const int tid = threadIdx.x;
     const uint32_t ncl = *count;
 
@@ -1839,103 +1856,78 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // place), packed into 64 bits as head's slope bits, 0xffff - head's
         // index, and the place.
         FIT_PROF(3)
-        uint64_t *sk = scr.skey + s0;
-        uint32_t *sv = scr.sval + s0;
-        if (in_smem) {
-            // Lay the points out in (head index descending, place) order:
-            // leaves in reverse order, and in each leaf its blocks by head
-            // index descending, each block in network order. A stable sort
-            // by the head's slope bits then gives the (head, place) order.
-            // Each warp finds the leaves that start in its 32 points at a
-            // time, queues them in its slice of the (still unused) radix
-            // histograms, and arranges them 32 leaves at a time.
-            auto arrange = [&](uint32_t lf) {
-                const int lo = (int)(lf >> 8), len = (int)(lf & 255);
-                // everything indexed by constants: registers only
-                uint64_t k5[5];
+        // the sort's two pairs of buffers, in shared memory or global scratch
+        uint32_t *ka = in_smem ? s_ka : reinterpret_cast<uint32_t *>(scr.skey + s0), *kb = in_smem ? s_kb : ka + sz;
+        uint16_t *va = in_smem ? s_val : reinterpret_cast<uint16_t *>(scr.sval + s0), *vb = in_smem ? s_vb : va + sz;
+        // Lay the points out in (head index descending, place) order:
+        // leaves in reverse order, and in each leaf its blocks by head
+        // index descending, each block in network order. A stable sort
+        // by the head's slope bits then gives the (head, place) order.
+        // Each warp finds the leaves that start in its 32 points at a
+        // time, queues them in its slice of the (still unused) radix
+        // histograms, and arranges them 32 leaves at a time.
+        auto arrange = [&](uint32_t lf) {
+            const int lo = (int)(lf >> 8), len = (int)(lf & 255);
+            // everything indexed by constants: registers only
+            uint64_t k5[5];
 #pragma unroll
-                for (int t = 0; t < 5; t++) k5[t] = t < len ? keys[lo + t] : ~0ull;
-                leaf_network(k5, len);
-                uint32_t hid[5], hkey[5];
-                int bs[5];
-                uint64_t head = k5[0];
-                int start = 0;
+            for (int t = 0; t < 5; t++) k5[t] = t < len ? keys[lo + t] : ~0ull;
+            leaf_network(k5, len);
+            uint32_t hid[5], hkey[5];
+            int bs[5];
+            uint64_t head = k5[0];
+            int start = 0;
 #pragma unroll
-                for (int t = 0; t < 5; t++) {
-                    if (t > 0 && k5[t] > head) {
-                        head = k5[t];
-                        start = t;
-                    }
-                    hid[t] = ~(uint32_t)head;
-                    hkey[t] = (uint32_t)(head >> 32);
-                    bs[t] = start;
+            for (int t = 0; t < 5; t++) {
+                if (t > 0 && k5[t] > head) {
+                    head = k5[t];
+                    start = t;
                 }
-                const int base = (int)sz - lo - len;
+                hid[t] = ~(uint32_t)head;
+                hkey[t] = (uint32_t)(head >> 32);
+                bs[t] = start;
+            }
+            const int base = (int)sz - lo - len;
 #pragma unroll
-                for (int t = 0; t < 5; t++) {
-                    if (t >= len) continue;
-                    int before = 0;  // points of blocks with a larger head index
+            for (int t = 0; t < 5; t++) {
+                if (t >= len) continue;
+                int before = 0;  // points of blocks with a larger head index
 #pragma unroll
-                    for (int t2 = 0; t2 < 5; t2++) before += t2 < len && hid[t2] > hid[t];
-                    const int pos = base + before + (t - bs[t]);
-                    s_ka[pos] = hkey[t];
-                    s_val[pos] = (uint16_t)~(uint32_t)k5[t];
-                }
-            };
-            {
-                const int lane = tid & 31;
-                uint32_t *lq = s_hist + (tid >> 5) * 256;
-                int qn = 0;
-                for (int64_t p0 = (int64_t)(tid >> 5) * 32; p0 < sz; p0 += NT) {
-                    const int64_t p = p0 + lane;
-                    int llo = -1, llen = 0;
-                    if (p < sz) leaf_of32((int)sz, (int)p, llo, llen);
-                    const bool lead = llo == (int)p;
-                    const uint32_t lf = (uint32_t)llo << 8 | (uint32_t)llen;
-                    const uint32_t bal = __ballot_sync(0xffffffffu, lead);
-                    if (lead) lq[qn + __popc(bal & ((1u << lane) - 1u))] = lf;
-                    qn += __popc(bal);
+                for (int t2 = 0; t2 < 5; t2++) before += t2 < len && hid[t2] > hid[t];
+                const int pos = base + before + (t - bs[t]);
+                ka[pos] = hkey[t];
+                va[pos] = (uint16_t)~(uint32_t)k5[t];
+            }
+        };
+        {
+            const int lane = tid & 31;
+            uint32_t *lq = s_hist + (tid >> 5) * 256;
+            int qn = 0;
+            for (int64_t p0 = (int64_t)(tid >> 5) * 32; p0 < sz; p0 += NT) {
+                const int64_t p = p0 + lane;
+                int llo = -1, llen = 0;
+                if (p < sz) leaf_of32((int)sz, (int)p, llo, llen);
+                const bool lead = llo == (int)p;
+                const uint32_t lf = (uint32_t)llo << 8 | (uint32_t)llen;
+                const uint32_t bal = __ballot_sync(0xffffffffu, lead);
+                if (lead) lq[qn + __popc(bal & ((1u << lane) - 1u))] = lf;
+                qn += __popc(bal);
+                __syncwarp();
+                if (qn >= 32) {
+                    qn -= 32;
+                    arrange(lq[qn + lane]);
                     __syncwarp();
-                    if (qn >= 32) {
-                        qn -= 32;
-                        arrange(lq[qn + lane]);
-                        __syncwarp();
-                    }
-                }
-                if (lane < qn) arrange(lq[lane]);
-            }
-            __syncthreads();
-            FIT_PROF(4)
-            block_radix_sort32(s_ka, s_val, s_kb, s_vb, (int)sz, s_hist);
-        } else {
-            for (int64_t p = tid; p < sz; p += NT) {
-                uint32_t lf = leaf_of(sz, p);
-                int64_t lo = lf >> 8, len = lf & 255;
-                if (p != lo) continue;
-                uint64_t k5[5];
-                for (int t = 0; t < len; t++) k5[t] = keys[lo + t];
-                leaf_network(k5, (int)len);
-                uint64_t head = 0;
-                for (int t = 0; t < len; t++) {
-                    if (t == 0 || k5[t] > head) head = k5[t];
-                    uint32_t hidx = ~(uint32_t)head;
-                    sk[lo + t] = (head & 0xffffffff00000000ull) | (uint64_t)(0xffffu - hidx) << 3 | (uint64_t)t;
-                    sv[lo + t] = ~(uint32_t)k5[t];
                 }
             }
-            __syncthreads();
-            FIT_PROF(4)
-            // the merge's second buffer: two scratch arrays
-            uint64_t *kb = reinterpret_cast<uint64_t *>(scr.w + s0);
-            uint32_t *vb = reinterpret_cast<uint32_t *>(scr.fx + s0);
-            block_merge_sort(sk, sv, kb, vb, (int)sz);
+            if (lane < qn) arrange(lq[lane]);
         }
+        __syncthreads();
+        FIT_PROF(4)
+        block_radix_sort32(ka, va, kb, vb, (int)sz, s_hist);
         FIT_PROF(5)
 
         // cumulative weighted moments in angle order (fast/quads.c:968-1035):
-        // w = sqrt(gx^2 + gy^2) + 1 on the quad image (1 at its border),
-        // fx = x/2 + 1/2. Chunks of points get their six terms (w fx, w fy,
-        // w fx fx, w fx fy, w fy fy, w; the reference's products) staged in
+        // Chunks of points get their six terms (moment_terms) staged in
         // shared memory, two buffers deep: while lane q < 6 of warp 0 runs
         // prefix sum q over chunk c in point order, the other warps stage
         // chunk c + 1.
@@ -1943,39 +1935,30 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         double *M[6] = {scr.mx + s0, scr.my + s0, scr.mxx + s0, scr.mxy + s0, scr.myy + s0, scr.mw + s0};
         double run = 0.0;
         const int cs = chunk + 2;  // row stride of the staged terms
+        // (two points a thread at a time, so that their gathers overlap)
         auto stage = [&](int64_t k0, double *buf, int first, int stride) {
-            const int64_t kn = dmin((int64_t)chunk, sz - k0);
-            for (int64_t t = first; t < kn; t += stride) {
-                const uint32_t src = in_smem ? (uint32_t)s_val[k0 + t] : sv[k0 + t];
-                const uint64_t pt = P[src];
-                const int32_t px = (int32_t)(pt & 0xffff), py = (int32_t)(pt >> 16 & 0xffff);
-                const int32_t ix = (px >> 1) + (px & 1), iy = (py >> 1) + (py & 1);
-                int32_t g2 = 0;
-                if (ix > 0 && ix + 1 < f.qw && iy > 0 && iy + 1 < f.qh) {
-                    const int64_t cc = (int64_t)iy * f.qw + ix;
-                    const int32_t gx = (int32_t)im[cc + 1] - im[cc - 1];
-                    const int32_t gy = (int32_t)im[cc + f.qw] - im[cc - f.qw];
-                    g2 = gx * gx + gy * gy;
+            const int kn = (int)dmin((int64_t)chunk, sz - k0);
+            for (int t = first; t < kn; t += 2 * stride) {
+                const int t2 = t + stride < kn ? t + stride : t;
+                const uint64_t p1 = P[va[k0 + t]], p2 = P[va[k0 + t2]];
+                const int32_t g1 = point_grad2(im, f.qw, f.qh, p1), g2 = point_grad2(im, f.qw, f.qh, p2);
+                double m1[6], m2[6];
+                moment_terms(p1, g1, m1);
+                moment_terms(p2, g2, m2);
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    buf[q * cs + t] = m1[q];
+                    buf[q * cs + t2] = m2[q];
                 }
-                const double w = __dadd_rn(__dsqrt_rn((double)g2), 1.0);
-                const double fx = __dadd_rn(__dmul_rn((double)px, 0.5), 0.5);
-                const double fy = __dadd_rn(__dmul_rn((double)py, 0.5), 0.5);
-                const double wx = __dmul_rn(w, fx), wy = __dmul_rn(w, fy);
-                buf[0 * cs + t] = wx;
-                buf[1 * cs + t] = wy;
-                buf[2 * cs + t] = __dmul_rn(wx, fx);
-                buf[3 * cs + t] = __dmul_rn(wx, fy);
-                buf[4 * cs + t] = __dmul_rn(wy, fy);
-                buf[5 * cs + t] = w;
             }
         };
         // the prefix sums are taken in place in shared memory; the other
         // warps copy a finished chunk out before staging into its buffer
         auto copy_out = [&](int64_t k0, const double *buf, int first, int stride) {
-            const int64_t kn = dmin((int64_t)chunk, sz - k0);
-            for (int64_t t = first; t < 6 * kn; t += stride) {
-                const int64_t q = t / kn, i = t - q * kn;
-                M[q][k0 + i] = buf[q * cs + i];
+            const int kn = (int)dmin((int64_t)chunk, sz - k0);
+            for (int i = first; i < kn; i += stride) {
+#pragma unroll
+                for (int q = 0; q < 6; q++) M[q][k0 + i] = buf[q * cs + i];
             }
         };
         stage(0, s_w, tid, NT);
@@ -1984,29 +1967,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         for (int64_t k0 = 0; k0 < sz; k0 += chunk, ch++) {
             double *cur = s_w + (ch & 1) * 6 * cs, *oth = s_w + ((ch + 1) & 1) * 6 * cs;
             if (tid < 32) {
-                if (tid < 6) {
-                    const int64_t kn = dmin((int64_t)chunk, sz - k0);
-                    double *src = cur + tid * cs;
-                    int64_t t = 0;
-                    // 16 loads, the 16 dependent additions, then 16 stores:
-                    // stores between the additions would lengthen the chain
-                    for (; t + 16 <= kn; t += 16) {
-                        double v[16];
-#pragma unroll
-                        for (int u = 0; u < 16; u++) v[u] = src[t + u];
-#pragma unroll
-                        for (int u = 0; u < 16; u++) {
-                            run = __dadd_rn(run, v[u]);
-                            v[u] = run;
-                        }
-#pragma unroll
-                        for (int u = 0; u < 16; u++) src[t + u] = v[u];
-                    }
-                    for (; t < kn; t++) {
-                        run = __dadd_rn(run, src[t]);
-                        src[t] = run;
-                    }
-                }
+                if (tid < 6) prefix_chain(cur + tid * cs, (int)dmin((int64_t)chunk, sz - k0), run);
             } else {
                 if (ch > 0) copy_out(k0 - chunk, oth, tid - 32, NT - 32);
                 asm volatile("bar.sync 1, %0;" ::"r"(NT - 32));
@@ -2068,17 +2029,13 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         if (nm < 4) continue;
         if (nm > prm.max_nmaxima) {
             // The reference keeps the maxima whose error is above the
-            // (max_nmaxima+1)-th largest (its quickselect, quads.c:827-862).
-            // e_i exceeds that order statistic exactly when at most
-            // max_nmaxima errors are >= e_i: a parallel count, then an
-            // order-keeping compaction.
-            // The order statistic by a radix select over the errors'
-            // order-preserving 64-bit images, 8 bits a pass: e_i is kept
-            // exactly when e_i > T, T the (max_nmaxima+1)-th largest.
-            const int64_t k = prm.max_nmaxima;
-            double *e = in_smem && nm <= sort_cap ? reinterpret_cast<double *>(s_key) : filt;
+            // (max_nmaxima+1)-th largest (its quickselect, quads.c:827-862)
+            // (block_select_desc): e_i is kept exactly when e_i > T, T the
+            // (max_nmaxima+1)-th largest.
+            const int k = prm.max_nmaxima;
+            double *e = nm <= sort_cap ? reinterpret_cast<double *>(s_key) : filt;
             for (int64_t i = tid; i < nm; i += NT) e[i] = mxe[i];
-            const double T = block_select_desc(e, nm, (uint32_t)k, s_hist, &s_selp, &s_selr);
+            const double T = block_select_desc(e, (int)nm, k, s_cand, &s_best);
             int64_t kept_run = 0;
             for (int64_t i0 = 0; i0 < nm; i0 += NT) {
                 int64_t i = i0 + tid;
@@ -2116,35 +2073,35 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // the 4 maxima with the smallest total error (quads.c:931-958): the
         // reference keeps the first strictly smaller error in (m0, m1, m2, m3)
         // order, i.e. the smallest error and, among equal ones, the first in
-        // that order. Each thread scans some (m0, m1, m2) triples; then a
-        // block-wide minimum of (error, order).
+        // that order. Each thread scans some of the 4-subsets (g_quad4); then
+        // a block-wide minimum of (error, order).
         {
             const double inf = __longlong_as_double(0x7ff0000000000000ll);
             double be = inf;
-            int64_t bo = INT64_MAX;
-            for (int64_t t = tid; t < nm * nm * nm; t += NT) {
-                const int64_t m0 = t / (nm * nm), m1 = (t / nm) % nm, m2 = t % nm;
-                if (!(m0 < m1 && m1 < m2 && m2 < nm - 1)) continue;
-                const int64_t p01 = m0 * nm + m1, p12 = m1 * nm + m2;
+            int bo = 0x10000;
+            const int n = (int)nm, nsub = binom4(n);
+            for (int t = tid; t < nsub; t += NT) {
+                const int v = g_quad4.v[t];
+                const int m0 = v & 15, m1 = v >> 4 & 15, m2 = v >> 8 & 15, m3 = v >> 12;
+                const int p01 = m0 * n + m1, p12 = m1 * n + m2;
                 if (s_pmse[p01] > prm.max_mse || s_pmse[p12] > prm.max_mse) continue;
                 const double dot = s_pnx[p01] * s_pnx[p12] + s_pny[p01] * s_pny[p12];
                 if (fabs(dot) > prm.max_dot) continue;
+                const int p23 = m2 * n + m3, p30 = m3 * n + m0;
                 const double e012 = s_perr[p01] + s_perr[p12];
-                for (int64_t m3 = m2 + 1; m3 < nm; m3++) {
-                    const int64_t p23 = m2 * nm + m3, p30 = m3 * nm + m0;
-                    const double e23 = s_pmse[p23] > prm.max_mse ? inf : s_perr[p23];
-                    const double e30 = s_pmse[p30] > prm.max_mse ? inf : s_perr[p30];
-                    const double e = e012 + e23 + e30;
-                    if (e < be) {  // within a thread: ascending order already
-                        be = e;
-                        bo = t * nm + m3;
-                    }
+                const double e23 = s_pmse[p23] > prm.max_mse ? inf : s_perr[p23];
+                const double e30 = s_pmse[p30] > prm.max_mse ? inf : s_perr[p30];
+                const double e = e012 + e23 + e30;
+                const int ord = m0 << 12 | m1 << 8 | m2 << 4 | m3;
+                if (e < be || (e == be && ord < bo)) {
+                    be = e;
+                    bo = ord;
                 }
             }
             // block minimum of (be, bo)
             for (int o = 16; o > 0; o >>= 1) {
                 double e2 = __shfl_xor_sync(0xffffffffu, be, o);
-                int64_t o2 = __shfl_xor_sync(0xffffffffu, bo, o);
+                const int o2 = __shfl_xor_sync(0xffffffffu, bo, o);
                 if (e2 < be || (e2 == be && o2 < bo)) {
                     be = e2;
                     bo = o2;
@@ -2169,10 +2126,9 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             bo = s_bo[0];
             // the 4 line fits (quads.c:1069-1075), one per thread
             if (be != inf && tid < 4) {
-                const int64_t t = bo / nm, m3 = bo % nm;
-                const int64_t mi[4] = {t / (nm * nm), (t / nm) % nm, t % nm, m3};
                 double mse;
-                line_of(seg_moments(mo, sz, mxi[mi[tid]], mxi[mi[(tid + 1) & 3]]), s_lines[tid], &mse);
+                const int ma = bo >> (12 - 4 * tid) & 15, mb = bo >> (12 - 4 * ((tid + 1) & 3)) & 15;
+                line_of(seg_moments(mo, sz, mxi[ma], mxi[mb]), s_lines[tid], &mse);
                 s_lmse[tid] = mse;
             }
             __syncthreads();
@@ -2249,13 +2205,14 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
 
 // ---------------------------------------------------------------------------
 // The fit's size classes: clusters of at most 128, 256, 512 points (a warp
-// each), at most 1024 (a block of 128), and larger (a block of 512). Each
+// each), at most 1024 (a block of 128), at most 6144 (a block of 256), and
+// larger (a block of 512). Each
 // class gets a list of its clusters; clusters outside [min_cluster_pixels,
 // max_px] of their frame get none (fast/quads.c:1180-1190). Every cluster's
 // quad flag starts at 0.
-#define FIT_NCLASS 5
+#define FIT_NCLASS 6
 __device__ __forceinline__ int fit_class(int64_t sz) {
-    return sz <= 128 ? 0 : sz <= 256 ? 1 : sz <= 512 ? 2 : sz <= 1024 ? 3 : 4;
+    return sz <= 128 ? 0 : sz <= 256 ? 1 : sz <= 512 ? 2 : sz <= FIT_SMALL ? 3 : sz <= FIT_LARGE_SORT ? 4 : 5;
 }
 
 __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, const int32_t *cframe,
@@ -2325,26 +2282,6 @@ __global__ void __launch_bounds__(1024) k_fit_order(const uint32_t *cstart, int6
 // block barriers. The same steps as k_fit_quads; the angle sort is a bitonic
 // sort in registers, the prefix moments stay in shared memory.
 #define FIT_WPB 2
-
-// The 4-subsets {m0 < m1 < m2 < m3} of {0..15} in colex order (by m3, then
-// m2, m1, m0), one per entry as nibbles m0 | m1 << 4 | m2 << 8 | m3 << 12:
-// the first C(n, 4) entries are the 4-subsets of {0..n-1}.
-struct Quad4Table {
-    uint16_t v[1820];
-};
-constexpr Quad4Table make_quad4() {
-    Quad4Table t{};
-    int k = 0;
-    for (int d = 3; d < 16; d++)
-        for (int c = 2; c < d; c++)
-            for (int b = 1; b < c; b++)
-                for (int a = 0; a < b; a++) t.v[k++] = (uint16_t)(a | b << 4 | c << 8 | d << 12);
-    return t;
-}
-__device__ const Quad4Table g_quad4 = make_quad4();
-static_assert(AT_MAX_NMAXIMA <= 16, "the 4-subset table covers 16 maxima");
-
-__host__ __device__ constexpr int binom4(int n) { return n < 4 ? 0 : n * (n - 1) * (n - 2) * (n - 3) / 24; }
 
 // per warp: six prefix arrays, then region x0 (angle keys; errors; the
 // maxima) and region x1 (dot terms; filtered errors; the pair fits)
@@ -4003,11 +3940,11 @@ static void launch_fit_warp(cudaStream_t s, const FrameDesc *frames, const GpuPa
         scr.counts + q, scr.counts + FIT_NCLASS + q, quads, quad_ok, mm, scr);
 }
 
-void launch_fit_quads(cudaStream_t s, cudaStream_t side, cudaStream_t side2, cudaStream_t side3, cudaEvent_t fork,
-                      cudaEvent_t join, cudaEvent_t join2, cudaEvent_t join3, const FrameDesc *frames, const GpuParams &prm, const uint8_t *qim,
-                      const uint64_t *pts, const uint32_t *cstart, const int32_t *cframe, int64_t nclusters,
-                      int64_t npoints, const FitScratch &scr, GpuQuad *quads, uint32_t *quad_ok, uint32_t *err) {
-    if (nclusters <= 0) return;
+int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frames, const GpuParams &prm,
+                      const uint8_t *qim, const uint64_t *pts, const uint32_t *cstart, const int32_t *cframe,
+                      int64_t nclusters, int64_t npoints, int64_t max_px, const FitScratch &scr, GpuQuad *quads,
+                      uint32_t *quad_ok, uint32_t *err) {
+    if (nclusters <= 0) return 0;
     const size_t small = fit_smem_bytes(FIT_SMALL, FIT_CHUNK_SMALL, 128 / 32),
                  large = fit_smem_bytes(FIT_LARGE_SORT, FIT_CHUNK_LARGE, FIT_LARGE_NT / 32);
     cudaFuncSetAttribute(k_fit_quads<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small);
@@ -4019,36 +3956,46 @@ void launch_fit_quads(cudaStream_t s, cudaStream_t side, cudaStream_t side2, cud
     k_fit_classify<<<flat_blocks(nclusters, 256), 256, 0, s>>>(frames, cstart, cframe, nclusters, npoints,
                                                                 prm.min_cluster_pixels, quad_ok, scr.lists,
                                                                 scr.counts);
-    // four streams, one per group of classes: the large clusters (a block
-    // of FIT_LARGE_NT each, two an SM); 513-1024 points (a block of 128);
-    // 257-512 (a warp each); up to 256 (a warp each). Only the two block
-    // classes are put largest first, each on its own stream, so the warp
-    // classes start at once (unsorted, the 513-1024 class measured slower:
-    // 175 vs 159 us, a long cluster last).
-    cudaEventRecord(fork, s);
-    cudaStreamWaitEvent(side, fork, 0);
-    cudaStreamWaitEvent(side2, fork, 0);
-    cudaStreamWaitEvent(side3, fork, 0);
-    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, side>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 4);
-    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, side2>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 3);
+    // five streams, one per group of classes: above 6144 points (a block of
+    // FIT_HUGE_NT each; only when a frame allows such clusters at all); the
+    // other large clusters (a block of FIT_LARGE_NT each, two an SM);
+    // 513-1024 points (a block of 128); 257-512 (a warp each); up to 256 (a
+    // warp each). Only the block classes are put largest first, each on its
+    // own stream, so the warp classes start at once (unsorted, the 513-1024
+    // class measured slower: 175 vs 159 us, a long cluster last).
+    const bool huge = max_px > FIT_LARGE_SORT;
+    auto list = [&](int q) { return scr.lists + q * nclusters; };
+    cudaEventRecord(S.fork, s);
+    for (int k = 0; k < (huge ? 4 : 3); k++) cudaStreamWaitEvent(S.side[k], S.fork, 0);
+    if (huge) {
+        const size_t hsm = fit_smem_bytes(FIT_HUGE_SORT, FIT_CHUNK_LARGE, FIT_HUGE_NT / 32);
+        cudaFuncSetAttribute(k_fit_quads<FIT_HUGE_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
+        k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[3]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 5);
+        k_fit_quads<FIT_HUGE_NT><<<(unsigned)(nclusters < 148 ? nclusters : 148), FIT_HUGE_NT, hsm, S.side[3]>>>(
+            frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(5),
+            scr.counts + 5, scr.counts + FIT_NCLASS + 5, FIT_HUGE_SORT, FIT_CHUNK_LARGE);
+        cudaEventRecord(S.join[3], S.side[3]);
+    }
+    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[0]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 4);
+    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[1]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 3);
     // two blocks an SM: one cluster's serial steps overlap the other's
     const unsigned nbig = (unsigned)(nclusters < 2 * 148 ? nclusters : 2 * 148);
-    k_fit_quads<FIT_LARGE_NT><<<nbig, FIT_LARGE_NT, large, side>>>(frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
-                                                 quads, quad_ok, err, scr.lists + 4 * nclusters, scr.counts + 4,
-                                                 scr.counts + FIT_NCLASS + 4, FIT_LARGE_SORT, FIT_CHUNK_LARGE);
-    cudaEventRecord(join, side);
+    k_fit_quads<FIT_LARGE_NT><<<nbig, FIT_LARGE_NT, large, S.side[0]>>>(
+        frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(4), scr.counts + 4,
+        scr.counts + FIT_NCLASS + 4, FIT_LARGE_SORT, FIT_CHUNK_LARGE);
+    cudaEventRecord(S.join[0], S.side[0]);
     const unsigned mid = (unsigned)(nclusters < 148 * 4 ? nclusters : 148 * 4);
-    k_fit_quads<128><<<mid, 128, small, side2>>>(frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
-                                                 quads, quad_ok, err, scr.lists + 3 * nclusters, scr.counts + 3,
-                                                 scr.counts + FIT_NCLASS + 3, FIT_SMALL, FIT_CHUNK_SMALL);
-    cudaEventRecord(join2, side2);
-    launch_fit_warp<16>(side3, frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 2, quads, quad_ok, mm);
-    cudaEventRecord(join3, side3);
+    k_fit_quads<128><<<mid, 128, small, S.side[1]>>>(frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
+                                                     quads, quad_ok, err, list(3), scr.counts + 3,
+                                                     scr.counts + FIT_NCLASS + 3, FIT_SMALL, FIT_CHUNK_SMALL);
+    cudaEventRecord(S.join[1], S.side[1]);
+    launch_fit_warp<16>(S.side[2], frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 2, quads, quad_ok,
+                        mm);
+    cudaEventRecord(S.join[2], S.side[2]);
     launch_fit_warp<4>(s, frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 0, quads, quad_ok, mm);
     launch_fit_warp<8>(s, frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 1, quads, quad_ok, mm);
-    cudaStreamWaitEvent(s, join, 0);
-    cudaStreamWaitEvent(s, join2, 0);
-    cudaStreamWaitEvent(s, join3, 0);
+    for (int k = 0; k < (huge ? 4 : 3); k++) cudaStreamWaitEvent(s, S.join[k], 0);
+    return huge ? 10 : 8;
 }
 
 void launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,

@@ -101,10 +101,17 @@ void launch_point_place(const Launch &L, const FrameDesc *frames, const PointRow
 void launch_cluster_starts(cudaStream_t s, const uint64_t *key, const uint32_t *head, const uint32_t *head_scan,
                            int64_t n, int nb, const FrameDesc *frames, int nframes, uint32_t *cstart, int32_t *cframe,
                            uint64_t *ckey);
-void launch_fit_quads(cudaStream_t s, cudaStream_t side, cudaStream_t side2, cudaStream_t side3, cudaEvent_t fork,
-                      cudaEvent_t join, cudaEvent_t join2, cudaEvent_t join3, const FrameDesc *frames, const GpuParams &prm, const uint8_t *qim,
-                      const uint64_t *pts, const uint32_t *cstart, const int32_t *cframe, int64_t nclusters,
-                      int64_t npoints, const FitScratch &scr, GpuQuad *quads, uint32_t *quad_ok, uint32_t *err);
+// The streams of the fit's size classes, their start and ends (events
+// without timing). max_px: the largest FrameDesc.max_px of the batch.
+// Returns the kernels launched.
+struct FitStreams {
+    cudaStream_t side[4];
+    cudaEvent_t fork, join[4];
+};
+int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frames, const GpuParams &prm,
+                     const uint8_t *qim, const uint64_t *pts, const uint32_t *cstart, const int32_t *cframe,
+                     int64_t nclusters, int64_t npoints, int64_t max_px, const FitScratch &scr, GpuQuad *quads,
+                     uint32_t *quad_ok, uint32_t *err);
 // also each gathered quad's cluster index (qcl)
 void launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,
                          GpuQuad *out, uint32_t *nq, uint32_t *qcl);
