@@ -1567,6 +1567,7 @@ __device__ double block_select_desc(const double *e, int n, int r, double *cand,
 #define FIT_LARGE_SORT 6144
 #define FIT_HUGE_SORT 13312
 #define FIT_HUGE_NT 512
+#define FIT_COUNT_MAX 256
 #define FIT_CHUNK_SMALL 256
 #define FIT_CHUNK_LARGE 512
 #define FIT_LARGE_NT 256  // threads of the largest class's blocks (two blocks an SM)
@@ -2003,59 +2004,88 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         }
         __syncthreads();
         FIT_PROF(7)
-        // local maxima with wrap-around, compacted in index order
+        // local maxima with wrap-around, compacted in index order: each
+        // warp counts those of its own stretch, then writes them after the
+        // warps' before it (two reads of filt, but only two barriers)
         int32_t *mxi = scr.mxi + s0;
         double *mxe = scr.mxe + s0;
-        int64_t nm_run = 0;
-        for (int64_t i0 = 0; i0 < sz; i0 += NT) {
-            int64_t i = i0 + tid;
-            uint32_t is_max = 0;
-            double e = 0.0;
-            if (i < sz) {
+        int nm;
+        {
+            const int n = (int)sz, lane = tid & 31, w = tid >> 5;
+            const int per = ((n + NT / 32 - 1) / (NT / 32) + 31) & ~31, i0 = w * per, i1 = min(i0 + per, n);
+            auto is_max = [&](int i, double &e) {
                 e = filt[i];
-                double l = filt[i == 0 ? sz - 1 : i - 1], r = filt[i + 1 == sz ? 0 : i + 1];
-                is_max = e > l && e > r;
+                return e > filt[i == 0 ? n - 1 : i - 1] && e > filt[i + 1 == n ? 0 : i + 1];
+            };
+            int cnt = 0;
+            double e;
+            for (int i = i0 + lane; i < i1; i += 32) cnt += is_max(i, e);
+            cnt = __reduce_add_sync(0xffffffffu, cnt);
+            if (lane == 0) s_scan[w] = (uint32_t)cnt;
+            __syncthreads();
+            int at = 0;
+            nm = 0;
+            for (int v = 0; v < NT / 32; v++) {
+                if (v == w) at = nm;
+                nm += (int)s_scan[v];
             }
-            uint32_t total;
-            uint32_t off = block_excl_scan(is_max, &total, s_scan);
-            if (is_max) {
-                mxi[nm_run + off] = (int32_t)i;
-                mxe[nm_run + off] = e;
+            for (int j0 = i0; j0 < i1; j0 += 32) {
+                const int i = j0 + lane;
+                const bool mx = i < i1 && is_max(i, e);
+                const uint32_t bal = __ballot_sync(0xffffffffu, mx);
+                if (mx) {
+                    const int o = at + __popc(bal & ((1u << lane) - 1u));
+                    mxi[o] = i;
+                    mxe[o] = e;
+                }
+                at += __popc(bal);
             }
-            nm_run += total;
+            __syncthreads();
         }
-        __syncthreads();
-        int64_t nm = nm_run;
         if (nm < 4) continue;
         if (nm > prm.max_nmaxima) {
             // The reference keeps the maxima whose error is above the
-            // (max_nmaxima+1)-th largest (its quickselect, quads.c:827-862)
-            // (block_select_desc): e_i is kept exactly when e_i > T, T the
-            // (max_nmaxima+1)-th largest.
+            // (max_nmaxima+1)-th largest T (its quickselect, quads.c:827-862):
+            // e_i > T exactly when at most max_nmaxima errors are >= e_i. Up
+            // to FIT_COUNT_MAX maxima each thread counts for its own; more
+            // find T first (block_select_desc).
             const int k = prm.max_nmaxima;
             double *e = nm <= sort_cap ? reinterpret_cast<double *>(s_key) : filt;
-            for (int64_t i = tid; i < nm; i += NT) e[i] = mxe[i];
-            const double T = block_select_desc(e, (int)nm, k, s_cand, &s_best);
-            int64_t kept_run = 0;
-            for (int64_t i0 = 0; i0 < nm; i0 += NT) {
-                int64_t i = i0 + tid;
-                uint32_t keep = 0;
-                if (i < nm) keep = e[i] > T;
-                uint32_t total;
-                uint32_t off = block_excl_scan(keep, &total, s_scan);
-                int32_t mi = i < nm ? mxi[i] : 0;
+            for (int i = tid; i < nm; i += NT) e[i] = mxe[i];
+            const bool count = nm <= FIT_COUNT_MAX;
+            double T = 0.0;
+            if (count)
                 __syncthreads();
-                if (keep) mxi[kept_run + off] = mi;
-                kept_run += total;
+            else
+                T = block_select_desc(e, nm, k, s_cand, &s_best);
+            int kept = 0;
+            for (int i0 = 0; i0 < nm; i0 += NT) {
+                const int i = i0 + tid;
+                uint32_t keep = 0;
+                if (i < nm) {
+                    if (count) {
+                        int ge = 0;
+                        for (int j = 0; j < nm; j++) ge += e[j] >= e[i];
+                        keep = ge <= k;
+                    } else {
+                        keep = e[i] > T;
+                    }
+                }
+                uint32_t total;
+                const uint32_t off = block_excl_scan(keep, &total, s_scan);
+                const int32_t mi = i < nm ? mxi[i] : 0;
+                __syncthreads();
+                if (keep) mxi[kept + off] = mi;
+                kept += (int)total;
             }
             __syncthreads();
-            nm = kept_run;
+            nm = kept;
         }
         FIT_PROF(8)
         // line fits of pairs of maxima: (a, b), a < b, and the closing pair
         // (b, a) wrapping around for b >= a + 3
-        for (int64_t t = tid; t < nm * nm; t += NT) {
-            int64_t p = t / nm, q = t - p * nm;
+        for (int t = tid; t < nm * nm; t += NT) {
+            const int p = t / nm, q = t - p * nm;
             bool used = p < q || p >= q + 3;
             if (!used) continue;
             int64_t i0 = mxi[p], i1 = mxi[q];
@@ -2079,7 +2109,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             const double inf = __longlong_as_double(0x7ff0000000000000ll);
             double be = inf;
             int bo = 0x10000;
-            const int n = (int)nm, nsub = binom4(n);
+            const int n = nm, nsub = binom4(n);
             for (int t = tid; t < nsub; t += NT) {
                 const int v = g_quad4.v[t];
                 const int m0 = v & 15, m1 = v >> 4 & 15, m2 = v >> 8 & 15, m3 = v >> 12;
