@@ -95,7 +95,7 @@ struct HBuf {
 
 enum {
     B_FRAMES, B_IMG, B_QIM, B_THR, B_TMPA, B_TMPB, B_TMAX, B_TMIN, B_LAB,
-    B_RSTART, B_REND, B_RV, B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF,
+    B_RSTART, B_REND, B_RV, B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS,
     B_KEY, B_VAL, B_KEY2, B_VAL2, B_HEAD, B_HSCAN, B_CSTART, B_CFRAME,
     B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
@@ -130,6 +130,7 @@ struct at_internal {
     // sizes of the last run (frame 0), for at_detector_diag
     int64_t last_qw = 0, last_qh = 0, last_npts = 0, last_ncl = 0, last_nq = 0;
     int64_t launches = 0;  // kernels of this library launched so far
+    bool segment_smem = false;  // the segmentation's shared memory allowance is set
     bool scan_smem = false;  // the point scan's shared memory allowance is set
     int64_t seg_slack = 64;  // row-table entries per cluster beyond its points (grows on a shortfall)
 
@@ -377,7 +378,9 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     // frame layout
     std::vector<FrameDesc> fd(n);
     std::vector<char> copied(n, 0);  // frames copied into the input arena
-    int64_t img = 0, qpx = 0, nodes = 0, rows = 0, tiles = 0;
+    int64_t img = 0, qpx = 0, nodes = 0, rows = 0, tiles = 0, words = 0;
+    int64_t max_bands = 1;  // of a frame, for the segmentation
+    size_t band_smem = 0;
     uint32_t all = in->nfam >= 32 ? 0xffffffffu : ((1u << in->nfam) - 1u);
     for (int64_t i = 0; i < n; i++) {
         FrameDesc &f = fd[i];
@@ -416,6 +419,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         f.node_off = nodes;
         f.row0 = rows;
         f.tile_off = tiles;
+        f.word_off = words;
         f.fam_mask = fr.family_mask ? (fr.family_mask & all) : all;
         frame_families(td, in, f.fam_mask, &f);
         f.max_px = (int32_t)(2 * (2 * f.qw + 2 * f.qh));
@@ -423,6 +427,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         nodes += (int64_t)f.qw * f.qh + f.qh;
         rows += f.qh;
         tiles += (int64_t)(f.qw / 4) * (f.qh / 4);
+        words += (int64_t)((f.qw + 31) / 32) * f.qh;
+        segment_plan(f.qw, f.qh, &max_bands, &band_smem);
     }
     for (int64_t i = 0; i < n; i++) res[i] = at_frame_result{0, 0, 0};
     in->dets.clear();
@@ -448,7 +454,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     CK(B[B_FRAMES].ensure(n * sizeof(FrameDesc)));
     CK(B[B_IMG].ensure(img + 1));
     CK(B[B_QIM].ensure(qpx));
-    CK(B[B_THR].ensure(qpx));
+    CK(B[B_THR].ensure(qpx + 4));  // rows are read by 4-byte words
     CK(B[B_TMPA].ensure(qpx));
     CK(B[B_TMPB].ensure(qpx));
     CK(B[B_TMAX].ensure(tiles + 1));
@@ -517,10 +523,16 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     RunArrays runs{B[B_RSTART].as<uint16_t>(), B[B_REND].as<uint16_t>(), B[B_RV].as<uint8_t>(),
                    B[B_PARENT].as<uint32_t>(), B[B_PX].as<uint32_t>(), B[B_MINID].as<uint32_t>()};
     uint32_t *lab = B[B_LAB].as<uint32_t>();
-    int64_t max_qh = 0;
-    for (auto &f : fd) max_qh = f.qh > max_qh ? f.qh : max_qh;
-    in->launches += launch_segment(L, dfr, thr, runs, B[B_ROWRUNS].as<uint32_t>(), lab, td->qtp.min_cluster_pixels,
-                                   max_qh);
+    CK(B[B_WORDS].ensure(words * sizeof(RowWord)));
+    if (!in->segment_smem) {
+        if (!segment_set_smem()) {
+            set_error(in, 1, "cudaFuncSetAttribute for the segmentation failed");
+            return false;
+        }
+        in->segment_smem = true;
+    }
+    in->launches += launch_segment(L, dfr, max_bands, band_smem, thr, runs, B[B_ROWRUNS].as<uint32_t>(),
+                                   B[B_WORDS].as<RowWord>(), lab, td->qtp.min_cluster_pixels);
     CK(cudaEventRecord(in->ev[4], st));
     CK(cudaGetLastError());
 

@@ -4,6 +4,7 @@
 #include <stdint.h>
 
 #include "at_gpu.h"
+#include "at_kernels.h"
 
 __device__ __forceinline__ int64_t dmin(int64_t a, int64_t b) { return a < b ? a : b; }
 __device__ __forceinline__ int64_t dmax(int64_t a, int64_t b) { return a > b ? a : b; }
@@ -75,6 +76,21 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) 
     }
     *total = __shfl_sync(0xffffffffu, incl, 31);
     return incl - v;
+}
+
+// Words of row masks (RowWord): the columns of word i that runs cover (all
+// but the last column of the image), the run that covers column b of a word
+// (of its row; the column is in a run), and a node's component root (two
+// steps at most, once k_root_sums has run).
+__device__ __forceinline__ uint32_t run_columns(int i, int qw) {
+    const int n = qw - 1 - 32 * i;
+    return n >= 32 ? ~0u : n <= 0 ? 0u : (1u << n) - 1u;
+}
+__device__ __forceinline__ uint32_t run_at(const RowWord &w, int b) {
+    return w.before + __popc(w.starts & ((2u << b) - 1u)) - 1u;
+}
+__device__ __forceinline__ uint32_t root_of(const RunArrays &runs, int64_t node) {
+    return runs.parent[runs.parent[node]];
 }
 
 // Open-addressing table of cluster keys (label pairs).

@@ -33,10 +33,18 @@ struct FrameDesc {
     int64_t node_off;      // first union-find node id of the frame
     int64_t row0;          // global index of quad row 0
     int64_t tile_off;      // into the tile arenas ((qw/4) * (qh/4))
+    int64_t word_off;      // into the row words (ceil(qw / 32) a row)
     uint32_t fam_mask;     // families decoded for this frame
     int32_t max_px;        // 2 * (2 qw + 2 qh)
     int32_t tag_width;     // min_tag_width of the frame's families (fast/detector.c:67-81)
     int32_t normal_border, reversed_border;  // whether any of them has a normal / reversed border
+};
+
+// 32 columns of a threshold row as bits: the white (255) and black (0)
+// pixels, the columns where a run of either starts (runs leave out the last
+// column of the image), and the row's runs before the word.
+struct alignas(16) RowWord {
+    uint32_t white, black, starts, before;
 };
 
 // Detector parameters that the kernels need (host copies them per call).

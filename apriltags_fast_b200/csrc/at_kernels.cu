@@ -446,611 +446,6 @@ __global__ void k_morph(const FrameDesc *frames, const uint8_t *in, uint8_t *out
 }
 
 // ---------------------------------------------------------------------------
-// 4-5. Runs and connected components over runs.
-//
-// 5. Connected components over runs (fast/unionfind.c:89-196): the same
-// pairs of runs join as in the reference; lock-free union that links the
-// larger root under the smaller, so every component's root is its smallest
-// node id (the label the cluster order is defined by).
-
-__device__ __forceinline__ uint32_t uf_find(uint32_t *par, uint32_t x) {
-    volatile uint32_t *p = par;
-    uint32_t px = p[x];
-    while (px != x) {
-        uint32_t ppx = p[px];
-        if (ppx == px) return px;
-        p[x] = ppx;  // path halving: only ever an ancestor
-        x = ppx;
-        px = p[x];
-    }
-    return x;
-}
-
-// Roots are linked in the order of a bijective hash of their ids: one fixed
-// total order, so concurrent links can never form a cycle, and a random one,
-// so trees stay shallow (linking by id would chain the pieces of a row).
-// The label of a component, its smallest node id, is tracked apart.
-__device__ __forceinline__ uint32_t uf_rank(uint32_t x) {
-    uint32_t h = x * 0x9e3779b1u;
-    return h ^ (h >> 16);
-}
-
-__device__ __forceinline__ void uf_unite(uint32_t *par, uint32_t a, uint32_t b) {
-    for (;;) {
-        a = uf_find(par, a);
-        b = uf_find(par, b);
-        if (a == b) return;
-        if (uf_rank(a) < uf_rank(b)) {
-            uint32_t t = a;
-            a = b;
-            b = t;
-        }
-        if (atomicCAS(par + a, a, b) == a) return;
-    }
-}
-
-// The runs of row y of slots [base, base + n) that touch run (a0, a1, v),
-// in order, by binary search for the first with end + 1 >= a0.
-#define FOR_TOUCHING(SE, V, base, n, a0, a1, v, k, BODY)                                 \
-    {                                                                                     \
-        int64_t lo_ = 0, hi_ = (n);                                                       \
-        while (lo_ < hi_) {                                                               \
-            int64_t mid_ = (lo_ + hi_) >> 1;                                              \
-            if ((int64_t)((SE)[(base) + mid_] >> 16) + 1 < (a0))                          \
-                lo_ = mid_ + 1;                                                           \
-            else                                                                          \
-                hi_ = mid_;                                                               \
-        }                                                                                 \
-        for (int64_t k = lo_; k < (n) && (int64_t)((SE)[(base) + k] & 0xffff) <= (a1) + 1; k++) { \
-            if ((V)[(base) + k] != (v)) continue;                                         \
-            if (runs_touch((a0), (a1), (SE)[(base) + k] & 0xffff, (SE)[(base) + k] >> 16, (v))) BODY \
-        }                                                                                 \
-    }
-
-// The flat form of the same union-find: one block per row, one thread per
-// run, links in global memory (hash-ordered, so trees stay shallow), then
-// one pass that sums each component's pixels and smallest node at its root.
-#define ROW_STAGE 4096
-
-__global__ void __launch_bounds__(256) k_row_runs(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
-                                                  uint32_t *row_nruns) {
-    // a warp per row: runs of equal value over columns [0, qw - 2], 32
-    // columns at a time (ballots of run starts), 127 runs not stored
-    const FrameDesc f = frames[blockIdx.y];
-    const int lane = threadIdx.x & 31;
-    const uint32_t lt = (1u << lane) - 1u;
-    const int64_t wpb = blockDim.x >> 5;
-    for (int64_t y = blockIdx.x * wpb + (threadIdx.x >> 5); y < f.qh; y += gridDim.x * wpb) {
-        const uint8_t *row = thr + f.q_off + y * f.qw;
-        const int64_t base = f.node_off + y * f.qw;
-        const int64_t xmax = f.qw - 2;
-        int64_t count = 0, open = -1;
-        for (int64_t x0 = 0; x0 <= xmax; x0 += 32) {
-            int64_t x = x0 + lane;
-            bool valid = x <= xmax;
-            uint8_t v = valid ? row[x] : 0;
-            bool start = valid && (x == 0 || row[x - 1] != v);
-            uint32_t S = __ballot_sync(0xffffffffu, start);
-            uint32_t N = __ballot_sync(0xffffffffu, start && v != 127);
-            if (start) {
-                uint32_t below = S & lt;
-                int64_t prev_slot;
-                if (below) {
-                    int pl = 31 - __clz(below);
-                    prev_slot = (N >> pl & 1u) ? count + __popc(N & ((1u << pl) - 1u)) : -1;
-                } else {
-                    prev_slot = open;
-                }
-                if (prev_slot >= 0) runs.end[base + prev_slot] = (uint16_t)(x - 1);
-                if (v != 127) {
-                    int64_t sl = base + count + __popc(N & lt);
-                    runs.start[sl] = (uint16_t)x;
-                    runs.v[sl] = v;
-                    runs.parent[sl] = (uint32_t)sl;
-                    runs.px[sl] = 0;
-                    runs.minid[sl] = 0xffffffffu;
-                }
-            }
-            if (S) {
-                int ls = 31 - __clz(S);
-                open = (N >> ls & 1u) ? count + __popc(N & ((1u << ls) - 1u)) : -1;
-            }
-            count += __popc(N);
-        }
-        if (lane == 0) {
-            if (open >= 0) runs.end[base + open] = (uint16_t)xmax;
-            row_nruns[f.row0 + y] = (uint32_t)count;
-            int64_t vn = f.node_off + (int64_t)f.qw * f.qh + y;
-            runs.parent[vn] = (uint32_t)vn;
-            runs.px[vn] = 0;
-            runs.minid[vn] = 0xffffffffu;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) k_row_union(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
-                                                   const uint32_t *row_nruns) {
-    __shared__ uint32_t s_se[ROW_STAGE];
-    __shared__ uint8_t s_v[ROW_STAGE];
-    const FrameDesc f = frames[blockIdx.y];
-    for (int64_t y = 1 + blockIdx.x; y < f.qh; y += gridDim.x) {
-        const int64_t cur = f.node_off + y * f.qw, prev = cur - f.qw;
-        const int64_t ncur = row_nruns[f.row0 + y], nprev = row_nruns[f.row0 + y - 1];
-        const bool staged = nprev <= ROW_STAGE;
-        __syncthreads();
-        if (staged)
-            for (int64_t t = threadIdx.x; t < nprev; t += blockDim.x) {
-                s_se[t] = (uint32_t)runs.start[prev + t] | (uint32_t)runs.end[prev + t] << 16;
-                s_v[t] = runs.v[prev + t];
-            }
-        __syncthreads();
-        for (int64_t i = threadIdx.x; i < ncur; i += blockDim.x) {
-            int64_t a0 = runs.start[cur + i], a1 = runs.end[cur + i];
-            uint8_t v = runs.v[cur + i];
-            if (staged) {
-                FOR_TOUCHING(s_se, s_v, 0, nprev, a0, a1, v, kk,
-                             { uf_unite(runs.parent, (uint32_t)(cur + i), (uint32_t)(prev + kk)); })
-            } else {
-                int64_t lo = 0, hi = nprev;
-                while (lo < hi) {
-                    int64_t mid = (lo + hi) >> 1;
-                    if ((int64_t)runs.end[prev + mid] + 1 < a0)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                for (int64_t kk = lo; kk < nprev && (int64_t)runs.start[prev + kk] <= a1 + 1; kk++) {
-                    if (runs.v[prev + kk] != v) continue;
-                    if (runs_touch(a0, a1, runs.start[prev + kk], runs.end[prev + kk], v))
-                        uf_unite(runs.parent, (uint32_t)(cur + i), (uint32_t)(prev + kk));
-                }
-            }
-        }
-        if (threadIdx.x == 0 && ncur > 0) {
-            int64_t last = cur + ncur - 1;
-            const uint8_t *above = thr + f.q_off + (y - 1) * f.qw;
-            if (runs.end[last] == f.qw - 2 && runs.v[last] == 255 && above[f.qw - 1] == 255 && above[f.qw - 2] != 255)
-                uf_unite(runs.parent, (uint32_t)last, (uint32_t)(f.node_off + (int64_t)f.qw * f.qh + y - 1));
-        }
-    }
-}
-
-// The same unions in bands: a block takes UB_ROWS rows of a frame and does
-// the unions between those rows in shared memory over band-local ids (the
-// larger id hooked under the smaller, lock-free, so a local root is its
-// set's smallest node of the band); every node then points at its local
-// root in global memory. k_band_join then joins the bands in global memory
-// (each band's first row with the row above, hash-ordered links between
-// roots as in uf_unite) and adds the last-column links of every row. The
-// same pairs are joined as by k_row_union, so the partition is the same. A
-// band with more than UB_CAP runs joins its rows in global memory instead.
-#define UB_ROWS 8
-#define UB_CAP 3072
-#define UB_PAIRS 3072  // touching pairs listed per band, at most
-
-__device__ __forceinline__ uint32_t lu_find(volatile uint32_t *par, uint32_t x) {
-    uint32_t p = par[x];
-    while (p != x) {
-        const uint32_t pp = par[p];
-        if (pp != p) par[x] = pp;  // path halving: only ever an ancestor
-        x = p;
-        p = par[x];
-    }
-    return x;
-}
-
-__device__ __forceinline__ void lu_unite(uint32_t *par, uint32_t a, uint32_t b) {
-    volatile uint32_t *vp = par;
-    for (;;) {
-        a = lu_find(vp, a);
-        b = lu_find(vp, b);
-        if (a == b) return;
-        if (a < b) {
-            const uint32_t t = a;
-            a = b;
-            b = t;
-        }
-        if (atomicCAS(par + a, a, b) == a) return;
-    }
-}
-
-__global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, RunArrays runs,
-                                                    const uint32_t *row_nruns) {
-    __shared__ uint32_t s_se[UB_CAP];
-    __shared__ uint32_t s_par[UB_CAP];
-    __shared__ uint8_t s_v[UB_CAP];
-    __shared__ uint8_t s_row[UB_CAP];
-    __shared__ uint32_t s_roff[UB_ROWS + 1];
-    __shared__ uint32_t s_pair[UB_PAIRS];  // touching pairs: run | run above << 16
-    __shared__ uint32_t s_npair;
-    static_assert(UB_ROWS <= 32, "one warp scans the band's row counts");
-    static_assert(UB_CAP <= 65536, "band-local run ids fit 16 bits");
-    const FrameDesc f = frames[blockIdx.y];
-    const int tid = threadIdx.x;
-    const int nband = (f.qh + UB_ROWS - 1) / UB_ROWS;
-    for (int b = blockIdx.x; b < nband; b += gridDim.x) {
-        const int y0 = b * UB_ROWS, nr = min(UB_ROWS, f.qh - y0);
-        __syncthreads();
-        if (tid < 32) {
-            const uint32_t c = tid < nr ? row_nruns[f.row0 + y0 + tid] : 0u;
-            uint32_t total;
-            const uint32_t off = warp_excl_scan(c, &total);
-            if (tid < nr) s_roff[tid] = off;
-            if (tid == 0) s_roff[nr] = total;
-        }
-        __syncthreads();
-        const uint32_t L = s_roff[nr];
-        if (L > UB_CAP) {
-            // too many runs to stage: the band's unions in global memory
-            for (int r = 1; r < nr; r++) {
-                const int64_t cur = f.node_off + (int64_t)(y0 + r) * f.qw, prev = cur - f.qw;
-                const int64_t ncur = s_roff[r + 1] - s_roff[r], nprev = s_roff[r] - s_roff[r - 1];
-                for (int64_t i = tid; i < ncur; i += blockDim.x) {
-                    const int64_t a0 = runs.start[cur + i], a1 = runs.end[cur + i];
-                    const uint8_t v = runs.v[cur + i];
-                    int64_t lo = 0, hi = nprev;
-                    while (lo < hi) {
-                        const int64_t mid = (lo + hi) >> 1;
-                        if ((int64_t)runs.end[prev + mid] + 1 < a0)
-                            lo = mid + 1;
-                        else
-                            hi = mid;
-                    }
-                    for (int64_t k = lo; k < nprev && (int64_t)runs.start[prev + k] <= a1 + 1; k++)
-                        if (runs.v[prev + k] == v && runs_touch(a0, a1, runs.start[prev + k], runs.end[prev + k], v))
-                            uf_unite(runs.parent, (uint32_t)(cur + i), (uint32_t)(prev + k));
-                }
-            }
-            continue;
-        }
-        // stage the band's runs (local id l = s_roff[row] + index)
-        for (uint32_t l = tid; l < L; l += blockDim.x) {
-            int r = 0;
-            while (s_roff[r + 1] <= l) r++;
-            const int64_t node = f.node_off + (int64_t)(y0 + r) * f.qw + (l - s_roff[r]);
-            s_se[l] = (uint32_t)runs.start[node] | (uint32_t)runs.end[node] << 16;
-            s_v[l] = runs.v[node];
-            s_par[l] = l;
-            s_row[l] = (uint8_t)r;
-        }
-        __syncthreads();
-        // the unions of rows 1.. of the band with the row above, in shared
-        // memory: the touching pairs listed first (a thread per run), then
-        // one union per pair, the pairs spread evenly over the threads (a
-        // run touching many runs above no longer holds its warp); a band
-        // with more pairs than the list holds unites them where found
-        if (tid == 0) s_npair = 0;
-        __syncthreads();
-        for (uint32_t l = s_roff[1] + tid; l < L; l += blockDim.x) {
-            const int r = s_row[l];
-            const uint32_t pb = s_roff[r - 1], pe = s_roff[r];
-            const int a0 = (int)(s_se[l] & 0xffffu), a1 = (int)(s_se[l] >> 16);
-            const uint8_t v = s_v[l];
-            uint32_t lo = pb, hi = pe;
-            while (lo < hi) {  // the first run above whose end reaches a0 - 1
-                const uint32_t mid = (lo + hi) >> 1;
-                if ((int)(s_se[mid] >> 16) + 1 < a0)
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            for (uint32_t k = lo; k < pe && (int)(s_se[k] & 0xffffu) <= a1 + 1; k++)
-                if (s_v[k] == v && runs_touch(a0, a1, s_se[k] & 0xffffu, s_se[k] >> 16, v)) {
-                    const uint32_t p = atomicAdd(&s_npair, 1u);
-                    if (p < UB_PAIRS)
-                        s_pair[p] = l | k << 16;
-                    else
-                        lu_unite(s_par, l, k);
-                }
-        }
-        __syncthreads();
-        const uint32_t np = min(s_npair, (uint32_t)UB_PAIRS);
-        for (uint32_t p = tid; p < np; p += blockDim.x) lu_unite(s_par, s_pair[p] & 0xffffu, s_pair[p] >> 16);
-        __syncthreads();
-        // every node points at its local root (read-only walks)
-        for (uint32_t l = tid; l < L; l += blockDim.x) {
-            uint32_t x = l;
-            while (s_par[x] != x) x = s_par[x];
-            const int r = s_row[l], rr = s_row[x];
-            const int64_t node = f.node_off + (int64_t)(y0 + r) * f.qw + (l - s_roff[r]);
-            const int64_t root = f.node_off + (int64_t)(y0 + rr) * f.qw + (x - s_roff[rr]);
-            runs.parent[node] = (uint32_t)root;
-        }
-    }
-}
-
-// The joins between bands (each band's first row with the row above) and
-// the last-column links of every row (fast/unionfind.c:89-97), in global
-// memory: a block per band boundary row, then a thread per row for the
-// last column.
-#define BJ_CAP 4096  // runs of the two rows staged at once
-__global__ void __launch_bounds__(256) k_band_join(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
-                                                   const uint32_t *row_nruns) {
-    __shared__ uint32_t s_se[BJ_CAP];
-    __shared__ uint8_t s_v[BJ_CAP];
-    const FrameDesc f = frames[blockIdx.y];
-    const int tid = threadIdx.x;
-    const int nband = (f.qh + UB_ROWS - 1) / UB_ROWS;
-    for (int b = 1 + blockIdx.x; b < nband; b += gridDim.x) {
-        const int64_t y = (int64_t)b * UB_ROWS;
-        const int64_t cur = f.node_off + y * f.qw, prev = cur - f.qw;
-        const uint32_t ncur = row_nruns[f.row0 + y], nprev = row_nruns[f.row0 + y - 1];
-        const uint32_t L = ncur + nprev;  // staged: the row above [0, nprev), this row [nprev, L)
-        const bool staged = L <= BJ_CAP;
-        __syncthreads();
-        if (staged)
-            for (uint32_t l = tid; l < L; l += blockDim.x) {
-                const int64_t node = l < nprev ? prev + l : cur + (l - nprev);
-                s_se[l] = (uint32_t)runs.start[node] | (uint32_t)runs.end[node] << 16;
-                s_v[l] = runs.v[node];
-            }
-        __syncthreads();
-        auto se_at = [&](uint32_t l) -> uint32_t {
-            if (staged) return s_se[l];
-            const int64_t node = l < nprev ? prev + l : cur + (l - nprev);
-            return (uint32_t)runs.start[node] | (uint32_t)runs.end[node] << 16;
-        };
-        auto v_at = [&](uint32_t l) -> uint8_t {
-            if (staged) return s_v[l];
-            return runs.v[l < nprev ? prev + l : cur + (l - nprev)];
-        };
-        // each run of either row: the runs of the other row covering its
-        // start column and the column before (see k_band_union)
-        for (uint32_t l = tid; l < L; l += blockDim.x) {
-            const uint32_t se = se_at(l);
-            const int a0 = (int)(se & 0xffffu), a1 = (int)(se >> 16);
-            const uint8_t v = v_at(l);
-            const uint32_t ob = l < nprev ? nprev : 0, oe = l < nprev ? L : nprev;
-            uint32_t lo = ob, hi = oe;
-            while (lo < hi) {
-                const uint32_t mid = (lo + hi) >> 1;
-                if ((int)(se_at(mid) & 0xffffu) <= a0)
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            if (lo == ob) continue;
-            const int64_t node = l < nprev ? prev + l : cur + (l - nprev);
-            // runs_touch as the reference calls it: this row's run, then the
-            // run above (it is not symmetric at column 0)
-            const bool upper = l < nprev;
-            for (uint32_t k = lo - 1, t = 0; t < 2; t++) {
-                const uint32_t sk = se_at(k);
-                const int b0 = (int)(sk & 0xffffu), b1 = (int)(sk >> 16);
-                if (v_at(k) == v && (upper ? runs_touch(b0, b1, a0, a1, v) : runs_touch(a0, a1, b0, b1, v)))
-                    uf_unite(runs.parent, (uint32_t)node, (uint32_t)(k < nprev ? prev + k : cur + (k - nprev)));
-                if ((int)(sk & 0xffffu) != a0 || k == ob) break;
-                k--;  // the run covering a0 - 1
-            }
-        }
-    }
-    for (int64_t y = 1 + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; y < f.qh;
-         y += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t ncur = row_nruns[f.row0 + y];
-        if (ncur == 0) continue;
-        const int64_t last = f.node_off + y * f.qw + ncur - 1;
-        const uint8_t *above = thr + f.q_off + (y - 1) * f.qw;
-        if (runs.end[last] == f.qw - 2 && runs.v[last] == 255 && above[f.qw - 1] == 255 && above[f.qw - 2] != 255)
-            uf_unite(runs.parent, (uint32_t)last, (uint32_t)(f.node_off + (int64_t)f.qw * f.qh + y - 1));
-    }
-}
-
-// The root of x without writes (after the unions: a path-halving write that
-// read its value before another thread stored a root would undo it).
-__device__ __forceinline__ uint32_t uf_root(const uint32_t *par, uint32_t x) {
-    const volatile uint32_t *p = par;
-    uint32_t px = p[x];
-    while (px != x) {
-        x = px;
-        px = p[x];
-    }
-    return x;
-}
-
-// Each node adds its pixels and offers its id to its root (one atomic per
-// distinct root of a warp), and from here on points at its root.
-__global__ void __launch_bounds__(256) k_row_sums(const FrameDesc *frames, RunArrays runs, const uint32_t *row_nruns) {
-    const FrameDesc f = frames[blockIdx.y];
-    const int lane = threadIdx.x & 31;
-    for (int64_t y = blockIdx.x; y < f.qh; y += gridDim.x) {
-        const int64_t base = f.node_off + y * f.qw;
-        const int64_t n = row_nruns[f.row0 + y];
-        for (int64_t i0 = 0; i0 <= n; i0 += blockDim.x) {
-            const int64_t i = i0 + threadIdx.x;
-            const bool valid = i <= n;
-            const uint32_t live = __ballot_sync(0xffffffffu, valid);
-            if (!valid) continue;
-            const int64_t node = i < n ? base + i : f.node_off + (int64_t)f.qw * f.qh + y;
-            const uint32_t r = uf_root(runs.parent, (uint32_t)node);
-            // no unions run any more: pointing straight at the root is safe
-            // for the walks of other threads, and the labels read it once
-            if (r != (uint32_t)node) runs.parent[node] = r;
-            const uint32_t px = i < n ? (uint32_t)(runs.end[node] - runs.start[node] + 1) : 1u;
-            const uint32_t peers = __match_any_sync(live, r);
-            const uint32_t sum = __reduce_add_sync(peers, px), mn = __reduce_min_sync(peers, (uint32_t)node);
-            if (lane == __ffs(peers) - 1) {
-                atomicAdd(runs.px + r, sum);
-                atomicMin(runs.minid + r, mn);
-            }
-        }
-    }
-}
-
-// Per pixel: its component's label if the component has at least
-// min_cluster_pixels pixels, else AT_NOK (no run: 127, or too small). A
-// block per row: each run's label once (every node points at its root after
-// k_row_sums), spread over the run's pixels by a max-scan of the run starts;
-// the last column is the row's extra node.
-#define LAB_THREADS 256
-__global__ void __launch_bounds__(LAB_THREADS) k_labels(const FrameDesc *frames, const RunArrays runs,
-                                                        const uint32_t *row_nruns, uint32_t *lab, int32_t min_px) {
-    __shared__ uint32_t s_run[ROW_STAGE];
-    __shared__ uint32_t s_rlab[ROW_STAGE];
-    __shared__ uint16_t s_end[ROW_STAGE];
-    __shared__ uint32_t s_wmax[LAB_THREADS / 32];
-    const FrameDesc f = frames[blockIdx.y];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int qw = (int)f.qw, W = qw - 1;
-    for (int y = blockIdx.x; y < (int)f.qh; y += gridDim.x) {
-        const int64_t base = f.node_off + (int64_t)y * qw;
-        const int nr = (int)row_nruns[f.row0 + y];
-        uint32_t *out = lab + f.q_off + (int64_t)y * qw;
-        if (tid == 0) {
-            const uint32_t r = runs.parent[f.node_off + (int64_t)qw * f.qh + y];
-            out[W] = (int64_t)runs.px[r] >= min_px ? runs.minid[r] : AT_NOK;
-        }
-        if (W > ROW_STAGE) {
-            // rows too wide to stage: a binary search per pixel
-            for (int x = tid; x < W; x += LAB_THREADS) {
-                int lo = 0, hi = nr;
-                while (lo < hi) {  // the first run with start > x
-                    const int mid = (lo + hi) >> 1;
-                    if ((int)runs.start[base + mid] <= x)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                uint32_t l = AT_NOK;
-                if (lo > 0 && (int)runs.end[base + lo - 1] >= x) {
-                    const uint32_t r = runs.parent[base + lo - 1];
-                    if ((int64_t)runs.px[r] >= min_px) l = runs.minid[r];
-                }
-                out[x] = l;
-            }
-            continue;
-        }
-        __syncthreads();
-        for (int x = tid; x < W; x += LAB_THREADS) s_run[x] = 0;
-        __syncthreads();
-        for (int i = tid; i < nr; i += LAB_THREADS) {
-            s_run[runs.start[base + i]] = (uint32_t)i + 1;
-            s_end[i] = runs.end[base + i];
-            const uint32_t r = runs.parent[base + i];
-            s_rlab[i] = (int64_t)runs.px[r] >= min_px ? runs.minid[r] : AT_NOK;
-        }
-        __syncthreads();
-        // thread t owns pixels [t * seg, t * seg + seg): the largest run
-        // number started at or before each of them
-        const int seg = (W + LAB_THREADS - 1) / LAB_THREADS;
-        const int x0 = tid * seg, x1 = x0 + seg < W ? x0 + seg : W;
-        uint32_t m = 0;
-        for (int x = x0; x < x1; x++) m = max(m, s_run[x]);
-        uint32_t incl = m;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl = max(incl, t);
-        }
-        if (lane == 31) s_wmax[wid] = incl;
-        uint32_t run = __shfl_up_sync(0xffffffffu, incl, 1);
-        if (lane == 0) run = 0;
-        __syncthreads();
-        for (int w = 0; w < wid; w++) run = max(run, s_wmax[w]);
-        for (int x = x0; x < x1; x++) {
-            run = max(run, s_run[x]);
-            s_run[x] = run && x <= (int)s_end[run - 1] ? s_rlab[run - 1] : AT_NOK;
-        }
-        __syncthreads();
-        for (int x = tid; x < W; x += LAB_THREADS) out[x] = s_run[x];
-    }
-}
-
-// The same labels with a warp per row (8 rows a block, for batches large
-// enough to fill the GPU that way): the run starting at each column staged
-// in the warp's slice of shared memory, then 128 columns at a time, 4 a
-// lane: a max-scan gives each column its run (carried across chunks), the
-// label is read through the run's root (the L1 cache holds the few roots of
-// a row; a lane's 4 pixels usually share one run), and a pixel that no
-// stored run covers is a 127 of the threshold image. Rows wider than
-// LW_CAP columns search the runs per pixel instead.
-#define LW_CAP 2048
-__global__ void __launch_bounds__(256) k_labels_w(const FrameDesc *frames, const uint8_t *thr, const RunArrays runs,
-                                                  const uint32_t *row_nruns, uint32_t *lab, int32_t min_px) {
-    __shared__ __align__(16) uint16_t s_run[8][LW_CAP + 8];
-    const FrameDesc f = frames[blockIdx.y];
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int qw = (int)f.qw, W = qw - 1;
-    uint16_t *sr = s_run[w];
-    for (int y = (int)blockIdx.x * 8 + w; y < (int)f.qh; y += (int)gridDim.x * 8) {
-        const int64_t base = f.node_off + (int64_t)y * qw;
-        const int nr = (int)row_nruns[f.row0 + y];
-        uint32_t *out = lab + f.q_off + (int64_t)y * qw;
-        const uint8_t *row = thr + f.q_off + (int64_t)y * qw;
-        auto label_of = [&](int i) -> uint32_t {
-            const uint32_t r = runs.parent[base + i];
-            return (int64_t)runs.px[r] >= min_px ? runs.minid[r] : AT_NOK;
-        };
-        if (lane == 0) {
-            const uint32_t r = runs.parent[f.node_off + (int64_t)qw * f.qh + y];
-            out[W] = (int64_t)runs.px[r] >= min_px ? runs.minid[r] : AT_NOK;
-        }
-        if (W > LW_CAP) {
-            for (int x = lane; x < W; x += 32) {
-                int lo = 0, hi = nr;
-                while (lo < hi) {  // the first run with start > x
-                    const int mid = (lo + hi) >> 1;
-                    if ((int)runs.start[base + mid] <= x)
-                        lo = mid + 1;
-                    else
-                        hi = mid;
-                }
-                out[x] = lo > 0 && (int)runs.end[base + lo - 1] >= x ? label_of(lo - 1) : AT_NOK;
-            }
-            continue;
-        }
-        const int Wp = (W + 3) & ~3;
-        for (int x = lane; x < Wp; x += 32) sr[x] = 0;
-        __syncwarp();
-        for (int i = lane; i < nr; i += 32) sr[runs.start[base + i]] = (uint16_t)(i + 1);
-        __syncwarp();
-        // 16-byte stores when the row and the label array allow
-        const bool v4 = ((((uintptr_t)out) | ((uintptr_t)row)) & 15) == 0;
-        uint32_t carry = 0;
-        for (int x0 = 0; x0 < W; x0 += 128) {
-            const int x = x0 + 4 * lane;
-            const uint2 pr = x < Wp ? *reinterpret_cast<const uint2 *>(sr + x) : make_uint2(0, 0);
-            uint32_t m[4] = {pr.x & 0xffffu, pr.x >> 16, pr.y & 0xffffu, pr.y >> 16};
-            m[1] = max(m[1], m[0]);
-            m[2] = max(m[2], m[1]);
-            m[3] = max(m[3], m[2]);
-            uint32_t incl = m[3];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl = max(incl, t);
-            }
-            uint32_t excl = __shfl_up_sync(0xffffffffu, incl, 1);
-            if (lane == 0) excl = 0;
-            excl = max(excl, carry);
-            carry = max(carry, __shfl_sync(0xffffffffu, incl, 31));
-            uint32_t l4[4];
-            uint32_t prev_run = 0, prev_lab = AT_NOK;
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t v = max(m[k], excl);
-                uint32_t l = AT_NOK;
-                if (x + k < W && v) {
-                    if (v != prev_run) {
-                        prev_run = v;
-                        prev_lab = label_of((int)v - 1);
-                    }
-                    l = row[x + k] != 127 ? prev_lab : AT_NOK;
-                }
-                l4[k] = l;
-            }
-            if (v4 && x + 4 <= W) {
-                *reinterpret_cast<uint4 *>(out + x) = make_uint4(l4[0], l4[1], l4[2], l4[3]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (x + k < W) out[x + k] = l4[k];
-            }
-        }
-        __syncwarp();
-    }
-}
-
-// ---------------------------------------------------------------------------
 // 6. Boundary points (fast/clusters.c:144-252). Pixel (x, y), y in
 // 1..qh-2, against (1,0), (0,1), (-1,1), (1,1): a point where one pixel is
 // 0 and the other 255 and both labels are not AT_NOK. The (-1,1) point is
@@ -3897,25 +3292,6 @@ int64_t decimate_threshold_blocks(int64_t qw, int64_t qh) {
 void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uint8_t *tmp) {
     k_morph<<<frame_grid(L), 256, 0, L.stream>>>(frames, thr, tmp, 1);
     k_morph<<<frame_grid(L), 256, 0, L.stream>>>(frames, tmp, thr, 0);
-}
-
-int launch_segment(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs, uint32_t *row_nruns,
-                   uint32_t *lab, int32_t min_px, int64_t max_qh) {
-    dim3 rg((unsigned)(max_qh < 148 * 16 ? max_qh : 148 * 16), (unsigned)L.nframes);
-    const int64_t rb = (max_qh + 7) / 8;
-    k_row_runs<<<dim3((unsigned)(rb < 148 * 8 ? rb : 148 * 8), (unsigned)L.nframes), 256, 0, L.stream>>>(frames, thr,
-                                                                                                        runs, row_nruns);
-    const int64_t nb = (max_qh + UB_ROWS - 1) / UB_ROWS;
-    k_band_union<<<dim3((unsigned)(nb < 148 * 4 ? nb : 148 * 4), (unsigned)L.nframes), 256, 0, L.stream>>>(
-        frames, runs, row_nruns);
-    k_band_join<<<dim3((unsigned)(nb < 148 * 4 ? nb : 148 * 4), (unsigned)L.nframes), 256, 0, L.stream>>>(
-        frames, thr, runs, row_nruns);
-    k_row_sums<<<rg, 256, 0, L.stream>>>(frames, runs, row_nruns);
-    if (warp_rows(L))
-        k_labels_w<<<row_warp_grid(L), 256, 0, L.stream>>>(frames, thr, runs, row_nruns, lab, min_px);
-    else
-        k_labels<<<rg, LAB_THREADS, 0, L.stream>>>(frames, runs, row_nruns, lab, min_px);
-    return 5;
 }
 
 void launch_point_count(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,

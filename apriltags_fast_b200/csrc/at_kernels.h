@@ -9,7 +9,7 @@
 struct RunArrays {
     uint16_t *start, *end;
     uint8_t *v;
-    uint32_t *parent;  // union-find parent
+    uint32_t *parent;  // union-find parent (in the end: a run's band root, a band root's component root)
     uint32_t *px;      // at a root: its component's pixel count
     uint32_t *minid;   // at a root: its component's smallest node id (the label)
 };
@@ -50,8 +50,12 @@ void launch_decimate_threshold(const Launch &L, const FrameDesc *frames, int64_t
                                uint8_t *thr, int32_t diff);
 int64_t decimate_threshold_blocks(int64_t qw, int64_t qh);
 void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uint8_t *tmp);
-int launch_segment(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs, uint32_t *row_nruns,
-                   uint32_t *lab, int32_t min_px, int64_t max_qh);
+// Runs, components and labels (at_segment.cu). segment_plan: the most bands
+// of a frame and the shared memory of a band, over the batch's frames.
+bool segment_set_smem();
+void segment_plan(int qw, int qh, int64_t *max_bands, size_t *smem);
+int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,
+                   RunArrays runs, uint32_t *row_nruns, RowWord *words, uint32_t *lab, int32_t min_px);
 void launch_point_count(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
                         uint64_t *row_npts);
 void launch_point_emit(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,

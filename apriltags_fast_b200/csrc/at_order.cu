@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) k_ref_targets(const FrameDesc *frames, in
         }
         const uint32_t label = s_key[i] - 1;
         tl[t] = label;
-        tp[t] = runs.px[runs.parent[label]];  // every node points at its root after the unions
+        tp[t] = runs.px[root_of(runs, label)];
     }
     __syncthreads();
     const bool need = s_need && !s_over;
@@ -218,7 +218,7 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
         for (int64_t j0 = 0; j0 < n; j0 += 32) {
             const int64_t j = j0 + lane;
             uint32_t t = REF_NONE;
-            if (j < n) t = ref_lookup(s_key, s_idx, runs.minid[runs.parent[base + j]]);
+            if (j < n) t = ref_lookup(s_key, s_idx, runs.minid[root_of(runs, base + j)]);
             const uint32_t bal = __ballot_sync(0xffffffffu, t != REF_NONE);
             if (t != REF_NONE) {
                 const uint64_t e = (uint64_t)runs.start[base + j] | (uint64_t)runs.end[base + j] << 16 |

@@ -1,0 +1,68 @@
+"""Runs, components and points from the row masks (csrc/at_segment.cu,
+csrc/at_cluster.cu) against the oracle at the widths and heights where words
+(32 columns) and bands (8, 4 and 2 rows; one above 8192 columns) begin and
+end, on images of random blobs: the labels of all pixels, the points and the
+clusters are equal."""
+import numpy as np
+import pytest
+
+import apriltags_fast_b200 as AT
+from oracle import oracle as O
+from tests import helpers as H
+from tests.test_gpu_parity import oracle_pixel_labels
+
+pytestmark = pytest.mark.gpu
+
+
+def _blobs(w, h, cell, seed):
+    """Random cells of cell x cell pixels, dark, light or flat, with noise."""
+    rng = np.random.default_rng(seed)
+    g = rng.choice([30, 220, 220, 30, 125], size=(h // cell + 1, w // cell + 1))
+    img = np.kron(g, np.ones((cell, cell), int))[:h, :w]
+    return np.clip(img + rng.normal(0, 3, (h, w)), 0, 255).astype(np.uint8)
+
+
+def _check(imgs, min_px, dec=1.0):
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=dec, min_cluster_pixels=min_px)
+    fams = [H.oracle_family("tag36h11")]
+    prm = O.default_params(quad_decimate=dec, min_cluster_pixels=min_px)
+    for img in imgs:
+        det.detect(img)
+        r = O.detect(img, fams, [2], prm, order=O.ORDER_CANON)
+        assert np.array_equal(det.diag("threshold"), r.thresh)
+        assert np.array_equal(det.diag("labels"), oracle_pixel_labels(r, min_px))
+        assert np.array_equal(det.diag("points"), r.pts)
+        assert np.array_equal(det.diag("clusters"), r.cstart[:-1])
+
+
+@pytest.mark.parametrize("w,h", [(31, 40), (32, 33), (33, 16), (34, 17), (64, 8), (65, 9), (97, 47), (1023, 24),
+                                 (1025, 23), (2048, 17), (2049, 18), (4097, 11), (4161, 12)])
+def test_word_and_band_edges(w, h):
+    _check([_blobs(w, h, cell, 7 * w + cell) for cell in (1, 2, 3, 5)], 24)
+
+
+@pytest.mark.parametrize("min_px", [2, 5, 200])
+def test_component_gate(min_px):
+    _check([_blobs(203, 99, 1, 5), _blobs(203, 99, 3, 6)], min_px)
+
+
+@pytest.mark.parametrize("w", [8200, 16390])
+def test_wide_frames(w):
+    """Bands of one row (with and without unions in shared memory): labels
+    of blank frames (detected as empty) and of a frame with one edge, which
+    is wider than the order of same-id detections allows and so refused; at
+    a higher decimation the quad image is narrow again."""
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    fams = [H.oracle_family("tag36h11")]
+    blank = np.full((64, w), 90, np.uint8)
+    edge = blank[:40].copy()
+    edge[8:32, w // 2:] = 250
+    for img, refused in ((blank, False), (edge, True)):
+        if refused:
+            with pytest.raises(RuntimeError, match="too wide"):
+                det.detect(img)
+        else:
+            assert det.detect(img) == [] and det.nquads == 0
+        r = O.detect(img, fams, [2], O.default_params(quad_decimate=1.0), order=O.ORDER_CANON)
+        assert np.array_equal(det.diag("labels"), oracle_pixel_labels(r, 24))
+    _check([_blobs(w, 48, 7, w)], 24, 3.0 if w < 12000 else 4.0)
