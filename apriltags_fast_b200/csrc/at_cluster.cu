@@ -3,15 +3,16 @@
 //
 // The reference groups the boundary points by the pair of components they
 // lie between, each cluster's points in emission order (y, x, neighbour),
-// and orders the clusters. Here each point is made once, from the
-// threshold image and the labels, as a 4-byte record in its row's region;
-// the records are then placed, each at its place in its cluster:
+// and orders the clusters. Here each point is made once, from the row
+// masks and the run labels, as a 4-byte record in its row's region; the
+// records are then placed, each at its place in its cluster:
 //
-//   k_point_scan     a warp per row: the row's points, their label pairs
-//                    gathered in the warp's table (shared memory), the
-//                    records in emission order; at the row's end each pair
-//                    of the row into the frame's pair table (point count,
-//                    first and last row) and the row's pair list.
+//   k_point_scan     a warp per row, a word of 32 columns a lane: the row's
+//                    points, their label pairs gathered in the warp's table
+//                    (shared memory), the records in emission order; at the
+//                    row's end each pair of the row into the frame's pair
+//                    table (point count, first and last row) and the row's
+//                    pair list.
 //   k_cluster_collect (at_kernels.cu): the distinct pairs.
 //   -- the host reads the pair and point counts (its only wait here) --
 //   k_pair_frame, k_pair_scatter, k_pair_rank: the distinct pairs in order.
@@ -34,15 +35,6 @@
 #include "at_gpu.h"
 #include "at_kernels.h"
 
-// The cluster key and the packed value of point j (neighbour (1,0), (0,1),
-// (-1,1), (1,1)) of pixel x of row y (la, lb: labels of rows y, y + 1).
-__device__ __forceinline__ uint64_t point_key(const uint32_t *la, const uint32_t *lb, int64_t x, int j, int nb) {
-    const int dx = j == 0 || j == 3 ? 1 : j == 2 ? -1 : 0;
-    const uint32_t l0 = la[x], l1 = j == 0 ? la[x + dx] : lb[x + dx];
-    const uint64_t hi = l0 > l1 ? l0 : l1, lo = l0 > l1 ? l1 : l0;
-    return hi << nb | lo;
-}
-
 // Rows 1 .. qh-2 of each frame, a warp per row.
 #define ROW_WARPS_BEGIN                                                                              \
     const FrameDesc f = frames[blockIdx.y];                                                          \
@@ -52,161 +44,191 @@ __device__ __forceinline__ uint64_t point_key(const uint32_t *la, const uint32_t
 #define ROW_WARPS_END }
 
 // A warp's table of the pairs of its row: open addressing over 2 nd_cap
-// slots (key, index), and per index (the order pairs first appear in the
-// row) the key, the slot and the number of points.
-struct RowPairs {
-    uint64_t *tkey, *ikey;
-    uint32_t *icnt;
-    uint16_t *tpos, *islot;
-};
-__host__ __device__ inline size_t row_pairs_bytes(int nd_cap) { return (size_t)34 * nd_cap; }
-__device__ inline RowPairs row_pairs(uint8_t *base, int nd_cap) {
-    RowPairs W;
-    W.tkey = reinterpret_cast<uint64_t *>(base);
-    W.ikey = W.tkey + 2 * nd_cap;
-    W.icnt = reinterpret_cast<uint32_t *>(W.ikey + nd_cap);
-    W.tpos = reinterpret_cast<uint16_t *>(W.icnt + nd_cap);
-    W.islot = W.tpos + 2 * nd_cap;
-    return W;
-}
+// slots (larger label << 32 | smaller, points), then the records of up to
+// 1024 columns before they are copied out, and the pairs' count.
+#define SCAN_BUF 1024
+__host__ __device__ inline size_t row_pairs_bytes(int nd_cap) { return (size_t)24 * nd_cap + 4 * SCAN_BUF + 16; }
 
-// Point records: pair index in the row | neighbour j << 11 | (pixel is 0)
-// << 13 | x << 14.
-#define PREC_ID 0x7ffu
+// Point records: the pair's slot in the row's table | neighbour j << 12 |
+// (pixel is 0) << 14 | x << 15.
+#define PREC_ID 0xfffu
 
-// Every boundary point, once: its pair into the warp's row table, its
-// record (emission order) into the row's region; at the row's end each of
-// the row's pairs into the frame's pair table (count, first and last row)
-// and, with its points in the row, into the row's pair list. Any capacity
-// exceeded (pairs of a row, records of a row, probes of the pair table)
-// sets *full and the batch takes the sorting path instead.
-__global__ void __launch_bounds__(256, 5) k_point_scan(const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
+// Every boundary point, once. The points of 32 columns are bit operations
+// on the masks of the row and the row below (the masks hold labelled pixels
+// only; fast/clusters.c:144-252, as point_mask per pixel). Then a lane goes
+// through its word's points in emission order (x, then neighbour): the
+// labels by run number, the pair looked up in the row's table when it
+// differs from the last one, the record into the warp's buffer. At the
+// row's end each pair goes into the frame's pair table (count, first and
+// last row) and, with its points in the row, into the row's pair list. Any
+// capacity exceeded (pairs of a row, records of a row, probes of the pair
+// table) sets *full and the batch takes the sorting path instead.
+//
+// Bound by instruction issue: about 25 instructions a point, where a lane
+// per pixel with labels per pixel took some 90 a pixel group and 4 bytes a
+// pixel of labels written and read.
+__global__ void __launch_bounds__(256) k_point_scan(const FrameDesc *frames, const RowWord *words, const uint32_t *lab,
                                                     int nb, PairTable T, PointRows P, uint32_t *full,
                                                     unsigned long long *npoints) {
     extern __shared__ __align__(16) uint8_t s_mem[];
     const int nd_cap = P.nd_cap, rt = 2 * nd_cap;
-    RowPairs W = row_pairs(s_mem + (threadIdx.x >> 5) * row_pairs_bytes(nd_cap), nd_cap);
-    for (int i = threadIdx.x & 31; i < rt; i += 32) W.tkey[i] = CH_EMPTY;
+    uint64_t *tkey = reinterpret_cast<uint64_t *>(s_mem + (threadIdx.x >> 5) * row_pairs_bytes(nd_cap));
+    uint32_t *tcnt = reinterpret_cast<uint32_t *>(tkey + rt), *buf = tcnt + rt, *npair = buf + SCAN_BUF;
+    for (int i = threadIdx.x & 31; i < rt; i += 32) {
+        tkey[i] = CH_EMPTY;
+        tcnt[i] = 0;
+    }
+    if ((threadIdx.x & 31) == 0) *npair = 0;
     __syncwarp();
     const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
     uint64_t pts = 0;
     ROW_WARPS_BEGIN
-    const uint8_t *a = thr + f.q_off + y * f.qw, *b = a + f.qw;
-    const uint32_t *la = lab + f.q_off + y * f.qw, *lb = la + f.qw;
-    uint32_t *rec = P.rec + 2 * (f.q_off + y * f.qw);
-    const uint32_t rcap = (uint32_t)(2 * f.qw);
-    uint32_t nd = 0, nrec = 0;
-    for (int64_t x0 = 0; x0 < f.qw; x0 += 32) {
-        const int64_t x = x0 + lane;
-        const uint32_t m = x < f.qw ? point_mask(a, b, la, lb, x, f.qw) : 0u;
-        if (!__any_sync(0xffffffffu, m != 0)) continue;
+    const int qw = f.qw, nw = (qw + 31) / 32;
+    const RowWord *wa = words + f.word_off + y * nw, *wb = wa + nw;
+    const uint32_t *la_of = lab + f.node_off + y * qw, *lb_of = la_of + qw;
+    const uint32_t *lcol = lab + f.node_off + (int64_t)qw * f.qh + y;  // last column: this row, the next
+    uint32_t *rec = P.rec + 2 * (f.q_off + y * qw);
+    const uint32_t rcap = (uint32_t)(2 * qw);
+    uint32_t nrec = 0;
+    for (int i0 = 0; i0 < nw; i0 += 32) {
+        const int i = i0 + lane;
+        // the lane's word of both rows and the words beside it
+        RowWord a = {0, 0, 0, 0}, b = a, an = a, bn = a, bp = a;
+        uint32_t pWa = 0, pKa = 0;
+        if (i < nw) {
+            a = wa[i];
+            b = wb[i];
+            if (i + 1 < nw) {
+                an = wa[i + 1];
+                bn = wb[i + 1];
+            }
+            if (i > 0) {
+                bp = wb[i - 1];
+                pWa = wa[i - 1].white >> 31;
+                pKa = wa[i - 1].black >> 31;
+            }
+        }
+        const uint32_t Wa1 = a.white >> 1 | an.white << 31, Ka1 = a.black >> 1 | an.black << 31;
+        const uint32_t Wb1 = b.white >> 1 | bn.white << 31, Kb1 = b.black >> 1 | bn.black << 31;
+        const uint32_t Wbm = b.white << 1 | bp.white >> 31, Kbm = b.black << 1 | bp.black >> 31;
+        const uint32_t Wam = a.white << 1 | pWa, Kam = a.black << 1 | pKa;
+        const uint32_t xm = i < nw ? run_columns(i, qw) : 0u, x1 = i == 0 ? xm & ~1u : xm;  // column 0: only (1, 0)
+        const uint32_t left11 = ((Wam & b.black) | (Kam & b.white)) & (i == 0 ? ~3u : ~0u);
+        const uint32_t c10 = ((a.white & Ka1) | (a.black & Wa1)) & xm;
+        const uint32_t c01 = ((a.white & b.black) | (a.black & b.white)) & x1;
+        const uint32_t cm1 = ((a.white & Kbm) | (a.black & Wbm)) & x1 & ~left11;
+        const uint32_t c11 = ((a.white & Kb1) | (a.black & Wb1)) & x1;
         uint32_t total;
-        const uint32_t o = warp_excl_scan(__popc(m), &total);
+        const uint32_t off = warp_excl_scan(__popc(c10) + __popc(c01) + __popc(cm1) + __popc(c11), &total);
+        if (total == 0) continue;
         if (nrec + total > rcap) {
             if (lane == 0) atomicOr(full, 1u);
             return;
         }
-        uint32_t id4[4];
-#pragma unroll
-        for (int j = 0; j < 4; j++) {
-            const bool has = (m >> j & 1u) != 0;
-            const uint64_t k = has ? point_key(la, lb, x, j, nb) : CH_EMPTY;
-            // the pair's index in the row, if the row has met it already
-            uint32_t id = 0xffffffffu;
-            if (has) {
-                uint32_t h = ch_hash(k) & (uint32_t)(rt - 1);
-                for (int p = 0; p < rt; p++) {
-                    const uint64_t cur = W.tkey[h];
-                    if (cur == k) {
-                        id = W.tpos[h];
-                        break;
-                    }
-                    if (cur == CH_EMPTY) break;
-                    h = (h + 1) & (uint32_t)(rt - 1);
-                }
+        uint32_t *dst = total <= SCAN_BUF ? buf + off : rec + nrec + off;
+        uint32_t any = c10 | c01 | cm1 | c11, jm = 0, rx = 0, la = 0, pla = 0, plb = 0, id = 0, cnt = 0;
+        int c = 0;
+        while (jm | any) {
+            if (jm == 0) {  // the next pixel with points
+                c = __ffs(any) - 1;
+                any &= any - 1;
+                jm = (c10 >> c & 1u) | (c01 >> c & 1u) << 1 | (cm1 >> c & 1u) << 2 | (c11 >> c & 1u) << 3;
+                la = la_of[run_at(a, c)];
+                rx = (uint32_t)(32 * i + c) << 15 | (a.black >> c & 1u) << 14;
             }
-            const bool miss = has && id == 0xffffffffu;
-            if (__any_sync(0xffffffffu, miss)) {
-                // pairs new to the row: each one's leader adds it
-                __syncwarp();
-                const uint64_t km = miss ? k : CH_EMPTY;
-                const uint32_t peers = __match_any_sync(0xffffffffu, km);
-                const int leader = __ffs(peers) - 1;
-                const bool lead = miss && lane == leader;
-                uint32_t h = 0;
-                bool added = false;
-                if (lead) {
-                    h = ch_hash(k) & (uint32_t)(rt - 1);
-                    for (int p = 0; p < rt; p++) {
-                        const unsigned long long old =
-                            atomicCAS(reinterpret_cast<unsigned long long *>(W.tkey + h), CH_EMPTY, k);
-                        if (old == CH_EMPTY) {
-                            added = true;
+            const uint32_t j = (uint32_t)__ffs(jm) - 1u;
+            jm &= jm - 1;
+            // the neighbour's label: this row or the next, column c + d
+            const int d = j == 0 || j == 3 ? 1 : j == 2 ? -1 : 0, cc = c + d;
+            uint32_t st = j == 0 ? a.starts : b.starts, be = j == 0 ? a.before : b.before;
+            if (cc > 31) {
+                st = j == 0 ? an.starts : bn.starts;
+                be = j == 0 ? an.before : bn.before;
+            } else if (cc < 0) {
+                st = bp.starts;
+                be = bp.before;
+            }
+            const uint32_t *lp = (j == 0 ? la_of : lb_of) + (be + __popc(st & ((2u << (cc & 31)) - 1u)) - 1u);
+            if (d > 0 && 32 * i + cc == qw - 1) lp = lcol + (j == 0 ? 0 : 1);
+            const uint32_t lb = *lp;
+            if (la != pla || lb != plb || cnt == 0) {
+                if (cnt) atomicAdd(tcnt + id, cnt);
+                cnt = 0;
+                pla = la;
+                plb = lb;
+                const uint32_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
+                const uint64_t k = (uint64_t)hi << 32 | lo;
+                uint32_t h = hi * 0x9e3779b1u + lo * 0x85ebca6bu;
+                h = (h ^ h >> 16) & (uint32_t)(rt - 1);
+                for (int p = 0; p < rt; p++) {  // a table without room has set *full below
+                    uint64_t cur = *(volatile uint64_t *)(tkey + h);
+                    if (cur == CH_EMPTY) {
+                        cur = atomicCAS(reinterpret_cast<unsigned long long *>(tkey + h), CH_EMPTY, k);
+                        if (cur == CH_EMPTY) {
+                            if (atomicAdd(npair, 1u) >= (uint32_t)nd_cap) atomicOr(full, 1u);
                             break;
                         }
-                        h = (h + 1) & (uint32_t)(rt - 1);
                     }
+                    if (cur == k) break;
+                    h = (h + 1) & (uint32_t)(rt - 1);
                 }
-                const uint32_t nadd = __ballot_sync(0xffffffffu, added);
-                if (nd + __popc(nadd) > (uint32_t)nd_cap) {
-                    if (lane == 0) atomicOr(full, 1u);
-                    return;
-                }
-                uint32_t nid = 0;
-                if (added) {
-                    nid = nd + __popc(nadd & lt);
-                    W.tpos[h] = (uint16_t)nid;
-                    W.ikey[nid] = k;
-                    W.islot[nid] = (uint16_t)h;
-                    W.icnt[nid] = 0;
-                }
-                nd += __popc(nadd);
-                nid = __shfl_sync(0xffffffffu, nid, leader);
-                if (miss) id = nid;
-                __syncwarp();
+                id = h;
             }
-            if (has) atomicAdd(W.icnt + id, 1u);
-            id4[j] = id;
-            __syncwarp();
+            cnt++;
+            *dst++ = id | j << 12 | rx;
         }
-        // this lane's points, in emission order (x, then neighbour)
-        if (m) {
-            const uint32_t g = a[x] == 0 ? 1u : 0u;
-            uint32_t t = nrec + o;
-#pragma unroll
-            for (int j = 0; j < 4; j++)
-                if (m >> j & 1u) rec[t++] = id4[j] | (uint32_t)j << 11 | g << 13 | (uint32_t)x << 14;
-        }
+        if (cnt) atomicAdd(tcnt + id, cnt);
+        __syncwarp();
+        if (total <= SCAN_BUF)
+            for (uint32_t t = lane; t < total; t += 32) rec[nrec + t] = buf[t];
+        if (*(volatile uint32_t *)npair > (uint32_t)nd_cap) return;  // *full is set
+        __syncwarp();
         nrec += total;
     }
-    __syncwarp();
     // the row's pairs into the frame's pair table; the table cleared
     uint32_t *ps = P.pslot + (f.row0 + y) * nd_cap, *pc = P.pcnt + (f.row0 + y) * nd_cap;
-    for (uint32_t i = lane; i < nd; i += 32) {
-        const uint64_t k = W.ikey[i];
-        uint32_t slot = ch_hash(k) & T.mask;
-        int p = 0;
-        for (; p < CH_PROBES; p++) {
-            uint64_t cur = *(volatile uint64_t *)(T.keys + slot);
-            if (cur == CH_EMPTY) {
-                const unsigned long long old = atomicCAS(reinterpret_cast<unsigned long long *>(T.keys + slot), CH_EMPTY, k);
-                cur = old == CH_EMPTY ? k : old;
+    uint16_t *pi = P.pid + (f.row0 + y) * nd_cap;
+    uint32_t nd = 0;
+    if (nrec)
+        for (int s = lane; s < rt; s += 32) {
+            const uint64_t kk = tkey[s];
+            const bool occ = kk != CH_EMPTY;
+            const uint32_t bal = __ballot_sync(0xffffffffu, occ);
+            if (occ) {
+                const uint32_t at = nd + __popc(bal & lt), n = tcnt[s];
+                const uint64_t k = (kk >> 32) << nb | (kk & 0xffffffffu);
+                uint32_t slot = ch_hash(k) & T.mask;
+                int p = 0;
+                for (; p < CH_PROBES; p++) {
+                    uint64_t cur = *(volatile uint64_t *)(T.keys + slot);
+                    if (cur == CH_EMPTY) {
+                        const unsigned long long old =
+                            atomicCAS(reinterpret_cast<unsigned long long *>(T.keys + slot), CH_EMPTY, k);
+                        cur = old == CH_EMPTY ? k : old;
+                    }
+                    if (cur == k) break;
+                    slot = (slot + 1) & T.mask;
+                }
+                if (p == CH_PROBES) {
+                    atomicOr(full, 1u);
+                } else {
+                    atomicAdd(T.count + slot, n);
+                    atomicMin(T.ymin + slot, (uint32_t)y);
+                    atomicMax(T.ymax + slot, (uint32_t)y);
+                }
+                ps[at] = slot;
+                pc[at] = n;
+                pi[at] = (uint16_t)s;
+                tkey[s] = CH_EMPTY;
+                tcnt[s] = 0;
             }
-            if (cur == k) break;
-            slot = (slot + 1) & T.mask;
+            nd += __popc(bal);
+            __syncwarp();
         }
-        if (p == CH_PROBES) {
-            atomicOr(full, 1u);
-        } else {
-            atomicAdd(T.count + slot, W.icnt[i]);
-            atomicMin(T.ymin + slot, (uint32_t)y);
-            atomicMax(T.ymax + slot, (uint32_t)y);
-        }
-        ps[i] = slot;
-        pc[i] = W.icnt[i];
-        W.tkey[W.islot[i]] = CH_EMPTY;
+    if (lane == 0) {
+        P.info[f.row0 + y] = make_uint2(nrec, nd);
+        *npair = 0;
     }
-    if (lane == 0) P.info[f.row0 + y] = make_uint2(nrec, nd);
     pts += nrec;
     __syncwarp();
     ROW_WARPS_END
@@ -441,14 +463,15 @@ __global__ void __launch_bounds__(256) k_point_place(const FrameDesc *frames, Po
                                                      uint64_t *out, int64_t npts, uint32_t *err) {
     extern __shared__ __align__(16) uint32_t s_base[];
     if (spanoff[ncl] > cap) return;
-    uint32_t *base = s_base + (threadIdx.x >> 5) * P.nd_cap;
+    uint32_t *base = s_base + (threadIdx.x >> 5) * 2 * P.nd_cap;  // by the pair's slot in the row's table
     const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
     ROW_WARPS_BEGIN
     const uint2 inf = P.info[f.row0 + y];
     const uint32_t *ps = P.pslot + (f.row0 + y) * P.nd_cap;
+    const uint16_t *pi = P.pid + (f.row0 + y) * P.nd_cap;
     for (uint32_t i = lane; i < inf.y; i += 32) {
         const uint32_t c = rank_of_slot[ps[i]];
-        base[i] = seg[spanoff[c] + ((uint32_t)y - cy0[c])];
+        base[pi[i]] = seg[spanoff[c] + ((uint32_t)y - cy0[c])];
     }
     __syncwarp();
     const uint32_t *rec = P.rec + 2 * (f.q_off + y * f.qw);
@@ -462,9 +485,9 @@ __global__ void __launch_bounds__(256) k_point_place(const FrameDesc *frames, Po
         __syncwarp();
         if (valid && lane == __ffs(peers) - 1) base[id] += __popc(peers);
         if (valid) {
-            const uint32_t j = (rc >> 11) & 3u, x = rc >> 14;
+            const uint32_t j = (rc >> 12) & 3u, x = rc >> 15;
             const int dx = j == 0 || j == 3 ? 1 : j == 2 ? -1 : 0, dy = j == 0 ? 0 : 1;
-            const int g = (rc >> 13 & 1u) ? 255 : -255;
+            const int g = (rc >> 14 & 1u) ? 255 : -255;
             const uint64_t px = (uint64_t)(2 * (int64_t)x + dx), py = (uint64_t)(2 * y + dy);
             const uint64_t gx = (uint16_t)(int16_t)(dx * g), gy = (uint16_t)(int16_t)(dy * g);
             if (at < npts)  // always, unless the counts disagree: then an error, not a stray write
@@ -498,15 +521,15 @@ static inline int scan_warps(int nd_cap) {
 
 bool point_scan_set_smem() {
     return cudaFuncSetAttribute(k_point_scan, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024) == cudaSuccess &&
-           cudaFuncSetAttribute(k_point_place, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) == cudaSuccess;
+           cudaFuncSetAttribute(k_point_place, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) == cudaSuccess;
 }
 
-void launch_point_scan(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab, int nb,
+void launch_point_scan(const Launch &L, const FrameDesc *frames, const RowWord *words, const uint32_t *lab, int nb,
                        const PairTable &T, const PointRows &P, uint32_t *full, unsigned long long *npoints) {
     const int w = scan_warps(P.nd_cap);
     const int64_t b = (L.max_qh + w - 1) / w;
     const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 * 8 ? b : 148 * 8), (unsigned)L.nframes);
-    k_point_scan<<<grid, 32 * w, w * row_pairs_bytes(P.nd_cap), L.stream>>>(frames, thr, lab, nb, T, P, full, npoints);
+    k_point_scan<<<grid, 32 * w, w * row_pairs_bytes(P.nd_cap), L.stream>>>(frames, words, lab, nb, T, P, full, npoints);
 }
 
 void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, int nb,
@@ -552,6 +575,6 @@ void launch_point_place(const Launch &L, const FrameDesc *frames, const PointRow
     k_seg_zero<<<flat_grid(cap, 256), 256, 0, L.stream>>>(spanoff, ncl, seg, cap, err);
     k_seg_fill<<<row_warps(L), 256, 0, L.stream>>>(frames, P, rank_of_slot, spanoff, cy0, ncl, seg, cap);
     k_seg_scan<<<flat_grid(ncl * 32, 256), 256, 0, L.stream>>>(cstart, spanoff, cspan, ncl, seg, cap);
-    k_point_place<<<row_warps(L), 256, 8 * P.nd_cap * 4, L.stream>>>(frames, P, rank_of_slot, spanoff, cy0, ncl, seg,
+    k_point_place<<<row_warps(L), 256, 16 * P.nd_cap * 4, L.stream>>>(frames, P, rank_of_slot, spanoff, cy0, ncl, seg,
                                                                     cap, out, npts, err);
 }

@@ -95,14 +95,14 @@ struct HBuf {
 
 enum {
     B_FRAMES, B_IMG, B_QIM, B_THR, B_TMPA, B_TMPB, B_TMAX, B_TMIN, B_LAB,
-    B_RSTART, B_REND, B_RV, B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS,
+    B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS, B_RUNLAB,
     B_KEY, B_VAL, B_KEY2, B_VAL2, B_HEAD, B_HSCAN, B_CSTART, B_CFRAME,
     B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
     B_HYMIN, B_HYMAX, B_CSPAN, B_CY0, B_SPANOFF, B_PKFRAME, B_PGKEYS, B_PGSLOTS, B_PFRAMES, B_PBSUM, B_SEG,
     B_QCL, B_CKEY, B_RNEED, B_RNT, B_RTLAB, B_RTPX, B_RTROOT, B_RTLIST, B_RTROW, B_RPRE, B_ROKEY, B_RIDX2,
-    B_RPAR, B_RSUM, B_RSTAMP, B_RTCH, B_RHIST,
-    B_PREC, B_PPSLOT, B_PPCNT, B_PINFO, B_QSCR,
+    B_RPAR, B_RLEN, B_RSUM, B_RSTAMP, B_RTCH, B_RHIST,
+    B_PREC, B_PPSLOT, B_PPCNT, B_PPID, B_PINFO, B_QSCR,
     B_CUB, B_ERR, B_NBUF
 };
 
@@ -129,6 +129,7 @@ struct at_internal {
     std::string msg;
     // sizes of the last run (frame 0), for at_detector_diag
     int64_t last_qw = 0, last_qh = 0, last_npts = 0, last_ncl = 0, last_nq = 0;
+    bool labelled = false;   // the last run got as far as its run labels
     int64_t launches = 0;  // kernels of this library launched so far
     bool segment_smem = false;  // the segmentation's shared memory allowance is set
     bool scan_smem = false;  // the point scan's shared memory allowance is set
@@ -432,6 +433,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     }
     for (int64_t i = 0; i < n; i++) res[i] = at_frame_result{0, 0, 0};
     in->dets.clear();
+    in->labelled = false;
     in->last_qw = n > 0 ? fd[0].qw : 0;
     in->last_qh = n > 0 ? fd[0].qh : 0;
     in->last_npts = in->last_ncl = in->last_nq = 0;
@@ -459,10 +461,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     CK(B[B_TMPB].ensure(qpx));
     CK(B[B_TMAX].ensure(tiles + 1));
     CK(B[B_TMIN].ensure(tiles + 1));
-    CK(B[B_LAB].ensure(qpx * 4));
-    CK(B[B_RSTART].ensure(nodes * 2));
-    CK(B[B_REND].ensure(nodes * 2));
-    CK(B[B_RV].ensure(nodes));
+    CK(B[B_RUNLAB].ensure(nodes * 4));
     CK(B[B_PARENT].ensure(nodes * 4));
     CK(B[B_PX].ensure(nodes * 4));
     CK(B[B_ROWRUNS].ensure(rows * 4));
@@ -520,9 +519,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     }
     CK(cudaEventRecord(in->ev[3], st));
     CK(B[B_MINID].ensure(nodes * 4));
-    RunArrays runs{B[B_RSTART].as<uint16_t>(), B[B_REND].as<uint16_t>(), B[B_RV].as<uint8_t>(),
-                   B[B_PARENT].as<uint32_t>(), B[B_PX].as<uint32_t>(), B[B_MINID].as<uint32_t>()};
-    uint32_t *lab = B[B_LAB].as<uint32_t>();
+    const RunArrays runs{B[B_PARENT].as<uint32_t>(), B[B_PX].as<uint32_t>(), B[B_MINID].as<uint32_t>(),
+                         B[B_RUNLAB].as<uint32_t>()};
     CK(B[B_WORDS].ensure(words * sizeof(RowWord)));
     if (!in->segment_smem) {
         if (!segment_set_smem()) {
@@ -532,7 +530,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         in->segment_smem = true;
     }
     in->launches += launch_segment(L, dfr, max_bands, band_smem, thr, runs, B[B_ROWRUNS].as<uint32_t>(),
-                                   B[B_WORDS].as<RowWord>(), lab, td->qtp.min_cluster_pixels);
+                                   B[B_WORDS].as<RowWord>(), td->qtp.min_cluster_pixels);
+    in->labelled = true;
     CK(cudaEventRecord(in->ev[4], st));
     CK(cudaGetLastError());
 
@@ -566,6 +565,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     CK(B[B_PREC].ensure(qpx * 8));
     CK(B[B_PPSLOT].ensure(rows * nd_cap * 4));
     CK(B[B_PPCNT].ensure(rows * nd_cap * 4));
+    CK(B[B_PPID].ensure(rows * nd_cap * 2));
     CK(B[B_PINFO].ensure(rows * 8));
     if (!in->scan_smem) {
         if (!point_scan_set_smem()) {
@@ -575,8 +575,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         in->scan_smem = true;
     }
     const PointRows prow{B[B_PREC].as<uint32_t>(), B[B_PPSLOT].as<uint32_t>(), B[B_PPCNT].as<uint32_t>(),
-                         B[B_PINFO].as<uint2>(), nd_cap};
-    launch_point_scan(L, dfr, thr, lab, nb, pt, prow, misc, reinterpret_cast<unsigned long long *>(misc + 2));
+                         B[B_PPID].as<uint16_t>(), B[B_PINFO].as<uint2>(), nd_cap};
+    launch_point_scan(L, dfr, B[B_WORDS].as<RowWord>(), runs.lab, nb, pt, prow, misc, reinterpret_cast<unsigned long long *>(misc + 2));
     CK(B[B_HOKEYS].ensure((size_t)hsize * 8));
     CK(B[B_HOSLOTS].ensure((size_t)hsize * 4));
     launch_cluster_collect(st, pt.keys, hsize, B[B_HOKEYS].as<uint64_t>(), B[B_HOSLOTS].as<uint32_t>(), misc + 1);
@@ -622,6 +622,10 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         // the pair table overflowed: points in emission order, sorted by pair
         uint64_t *row_npts = B[B_ROWPTS].as<uint64_t>(), *row_off = B[B_ROWOFF].as<uint64_t>();
         CK(cudaMemsetAsync(row_npts + rows, 0, 8, st));
+        CK(B[B_LAB].ensure(qpx * 4));
+        uint32_t *lab = B[B_LAB].as<uint32_t>();
+        launch_labels(L, dfr, runs, B[B_WORDS].as<RowWord>(), lab);
+        in->launches += 1;
         launch_point_count(L, dfr, thr, lab, row_npts);
         in->launches += 1;
         if (!cub_call(in, [&](void *t, size_t &b) {
@@ -745,6 +749,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_ROKEY].ensure(nd * 16));
         CK(B[B_RIDX2].ensure(nd * 4));
         CK(B[B_RPAR].ensure(nodes * 8));
+        CK(B[B_RLEN].ensure(nodes * 2));
         CK(B[B_RSUM].ensure(nodes * 4));
         CK(B[B_RSTAMP].ensure(nodes * 4));
         CK(B[B_RTCH].ensure(nodes * 4));
@@ -754,7 +759,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
                           B[B_RTPX].as<uint32_t>(),   B[B_RTROOT].as<uint32_t>(), B[B_RTLIST].as<uint64_t>(),
                           B[B_RTROW].as<uint32_t>(),  B[B_RPRE].as<uint32_t>(),   B[B_RPAR].as<uint64_t>(),
                           B[B_RSUM].as<uint32_t>(),   B[B_RSTAMP].as<uint32_t>(), B[B_RTCH].as<uint32_t>(),
-                          B[B_RHIST].as<uint32_t>()};
+                          B[B_RLEN].as<uint16_t>(),   B[B_RHIST].as<uint32_t>()};
         int64_t capr = 1;
         for (auto &f : fd) capr = f.qw - 1 > capr ? f.qw - 1 : capr;
         if (nodes >= ((int64_t)1 << 31)) {
@@ -765,7 +770,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
             set_error(in, 2, "quad image too wide for the order replay (" + std::to_string(capr + 1) + " px)");
             return false;
         }
-        in->launches += launch_ref_order(L, dfr, thr, runs, B[B_ROWRUNS].as<uint32_t>(), in->nfam,
+        in->launches += launch_ref_order(L, dfr, B[B_WORDS].as<RowWord>(), runs, B[B_ROWRUNS].as<uint32_t>(), in->nfam,
                                          B[B_QSTART].as<int64_t>(), B[B_DETS].as<GpuDetection>(),
                                          B[B_DETOK].as<uint32_t>(), B[B_QCL].as<uint32_t>(), ckey, nb, ro,
                                          B[B_ERR].as<uint32_t>());
@@ -1106,7 +1111,19 @@ int64_t at_detector_diag(const at_detector *td, int what, void *dst, int64_t cap
     switch (what) {
     case AT_DIAG_QUAD_IMAGE: src = B[B_QIM].p, bytes = in->last_qw * in->last_qh; break;
     case AT_DIAG_THRESHOLD: src = B[B_THR].p, bytes = in->last_qw * in->last_qh; break;
-    case AT_DIAG_LABELS: src = B[B_LAB].p, bytes = 4 * in->last_qw * in->last_qh; break;
+    case AT_DIAG_LABELS: {
+        bytes = 4 * in->last_qw * in->last_qh;
+        if (!in->labelled || !B[B_WORDS].p || bytes == 0 || !dst) break;
+        // per pixel only here (frame 0's offsets are all 0)
+        if (cudaSetDevice(in->device) != cudaSuccess || in->buf[B_LAB].ensure(bytes) != cudaSuccess) return -1;
+        const RunArrays runs{B[B_PARENT].as<uint32_t>(), B[B_PX].as<uint32_t>(), B[B_MINID].as<uint32_t>(),
+                             B[B_RUNLAB].as<uint32_t>()};
+        launch_labels(Launch{in->stream, 1, 0, in->last_qh}, B[B_FRAMES].as<FrameDesc>(), runs,
+                      B[B_WORDS].as<RowWord>(), B[B_LAB].as<uint32_t>());
+        if (cudaStreamSynchronize(in->stream) != cudaSuccess) return -1;
+        src = B[B_LAB].p;
+        break;
+    }
     case AT_DIAG_POINTS: src = B[B_VAL2].p, bytes = 8 * in->last_npts; break;
     case AT_DIAG_CLUSTERS: src = B[B_CSTART].p, bytes = 4 * in->last_ncl; break;
     case AT_DIAG_QUADS: src = B[B_QUADSC].p, bytes = (int64_t)sizeof(GpuQuad) * in->last_nq; break;

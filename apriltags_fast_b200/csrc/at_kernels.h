@@ -5,13 +5,12 @@
 
 #include "at_gpu.h"
 
-// Run table and union-find nodes, indexed by node id.
+// Union-find nodes, indexed by node id.
 struct RunArrays {
-    uint16_t *start, *end;
-    uint8_t *v;
     uint32_t *parent;  // union-find parent (in the end: a run's band root, a band root's component root)
     uint32_t *px;      // at a root: its component's pixel count
     uint32_t *minid;   // at a root: its component's smallest node id (the label)
+    uint32_t *lab;     // each node's label, or AT_NOK
 };
 
 // Per-point scratch of the quad fit, indexed by point position.
@@ -55,7 +54,9 @@ void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uin
 bool segment_set_smem();
 void segment_plan(int qw, int qh, int64_t *max_bands, size_t *smem);
 int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,
-                   RunArrays runs, uint32_t *row_nruns, RowWord *words, uint32_t *lab, int32_t min_px);
+                   RunArrays runs, uint32_t *row_nruns, RowWord *words, int32_t min_px);
+// the labels per pixel (the sorting fallback of the clusters, diagnostics)
+void launch_labels(const Launch &L, const FrameDesc *frames, RunArrays runs, const RowWord *words, uint32_t *lab);
 void launch_point_count(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
                         uint64_t *row_npts);
 void launch_point_emit(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
@@ -79,18 +80,19 @@ struct PairScratch {
     uint32_t *gslots, *bsum_a, *bsum_b;
 };
 // The points of each row (rows 1 .. qh-2): records in emission order at
-// rec + 2 (q_off + y qw), at most 2 qw a row (pair index in the row |
-// neighbour << 11 | pixel is 0 << 13 | x << 14); the row's distinct pairs
-// (slot in the pair table, points) at (row0 + y) nd_cap; info[row0 + y] =
-// (records, pairs).
+// rec + 2 (q_off + y qw), at most 2 qw a row (the pair's place in the row's
+// table | neighbour << 12 | pixel is 0 << 14 | x << 15); the row's distinct
+// pairs (slot in the pair table, points, place in the row's table) at (row0 +
+// y) nd_cap; info[row0 + y] = (records, pairs).
 struct PointRows {
     uint32_t *rec;
     uint32_t *pslot, *pcnt;
+    uint16_t *pid;
     uint2 *info;
     int32_t nd_cap;
 };
 bool point_scan_set_smem();
-void launch_point_scan(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab, int nb,
+void launch_point_scan(const Launch &L, const FrameDesc *frames, const RowWord *words, const uint32_t *lab, int nb,
                        const PairTable &T, const PointRows &P, uint32_t *full, unsigned long long *npoints);
 void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, int nb,
                        const FrameDesc *frames, int nframes, const PairTable &T, const PairScratch &P,
@@ -154,11 +156,12 @@ struct RefOrder {
     // and last run of the row above that it touches
     uint64_t *par;
     uint32_t *sum, *stamp, *tch;
+    uint16_t *len;            // per target run: its pixels
     // per target (AT_REF_MAXT a frame) and row: pixels gained (zeroed by the caller)
     uint32_t *hist;
 };
 // returns the kernels launched
-int launch_ref_order(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
+int launch_ref_order(const Launch &L, const FrameDesc *frames, const RowWord *words, RunArrays runs,
                      const uint32_t *row_nruns, int nfam, const int64_t *qstart, const GpuDetection *dets,
                      const uint32_t *det_ok, const uint32_t *qcl, const uint64_t *ckey, int nb, const RefOrder &ref,
                      uint32_t *err);

@@ -189,7 +189,7 @@ __device__ __forceinline__ void ref_node_init(const RefOrder &ref, uint32_t node
     ref.stamp[node] = 0;
 }
 
-__global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
+__global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const RowWord *words, RunArrays runs,
                                                   const uint32_t *row_nruns, RefOrder ref) {
     __shared__ uint32_t s_key[REF_HASH];
     __shared__ uint8_t s_idx[REF_HASH];
@@ -211,34 +211,56 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const int64_t wpb = blockDim.x >> 5;
+    const int qw = fd.qw, nw = (qw + 31) / 32;
     for (int64_t y = blockIdx.x * wpb + (threadIdx.x >> 5); y < fd.qh; y += gridDim.x * wpb) {
-        const int64_t base = fd.node_off + y * fd.qw;
-        const int64_t n = row_nruns[fd.row0 + y];
-        uint32_t cnt = 0, last_t = REF_NONE;
-        for (int64_t j0 = 0; j0 < n; j0 += 32) {
-            const int64_t j = j0 + lane;
-            uint32_t t = REF_NONE;
-            if (j < n) t = ref_lookup(s_key, s_idx, runs.minid[root_of(runs, base + j)]);
-            const uint32_t bal = __ballot_sync(0xffffffffu, t != REF_NONE);
-            if (t != REF_NONE) {
-                const uint64_t e = (uint64_t)runs.start[base + j] | (uint64_t)runs.end[base + j] << 16 |
-                                   (uint64_t)j << 32 | (uint64_t)runs.v[base + j] << 48 | (uint64_t)t << 56;
-                ref.tlist[base + cnt + __popc(bal & ((1u << lane) - 1u))] = e;
-                ref_node_init(ref, (uint32_t)(base + j), (uint32_t)(e >> 16 & 0xffff) - (uint32_t)(e & 0xffff) + 1);
+        const int64_t base = fd.node_off + y * qw;
+        const RowWord *row = words + fd.word_off + y * nw;
+        uint32_t cnt = 0;
+        for (int i0 = 0; i0 < nw; i0 += 32) {
+            // a word a lane: its target runs, then (after the lanes before) their entries
+            const int i = i0 + lane;
+            RowWord w = {0, 0, 0, 0};
+            uint32_t tm = 0;
+            if (i < nw) {
+                w = row[i];
+                uint32_t k = w.before;
+                for (uint32_t m = w.starts; m; m &= m - 1, k++)
+                    if (((w.white | w.black) & m & (0u - m)) &&
+                        ref_lookup(s_key, s_idx, runs.lab[base + k]) != REF_NONE)
+                        tm |= m & (0u - m);
             }
-            if (j == n - 1) last_t = t;
-            cnt += __popc(bal);
+            uint32_t total;
+            uint32_t at = cnt + warp_excl_scan(__popc(tm), &total);
+            for (uint32_t m = tm; m; m &= m - 1, at++) {
+                const int c = __ffs(m) - 1;
+                const uint32_t k = run_at(w, c), t = ref_lookup(s_key, s_idx, runs.lab[base + k]);
+                const bool white = w.white >> c & 1u;
+                // the run's end: the first later column of another value or the last run column
+                int e = 32 * i + c + 1;
+                for (int j = i; j < nw; j++) {
+                    const uint32_t colour = (white ? row[j].white : row[j].black) & run_columns(j, qw);
+                    const uint32_t stop = ~colour & (j == i ? ~0u << c : ~0u);
+                    e = 32 * j + (stop ? __ffs(stop) - 1 : 32);
+                    if (stop) break;
+                }
+                const uint32_t start = (uint32_t)(32 * i + c), end = (uint32_t)(e - 1);
+                ref.tlist[base + at] = (uint64_t)start | (uint64_t)end << 16 | (uint64_t)k << 32 |
+                                       (uint64_t)(white ? 255 : 0) << 48 | (uint64_t)t << 56;
+                ref_node_init(ref, (uint32_t)(base + k), end - start + 1);
+                ref.len[base + k] = (uint16_t)(end - start + 1);
+            }
+            cnt += total;
         }
-        last_t = __shfl_sync(0xffffffffu, last_t, (int)((n - 1) & 31));
         if (lane == 0) {
+            // the last-column link (the masks hold labelled pixels only; a
+            // target's are, and so is what it touches)
             bool link = false;
-            if (y >= 1 && n > 0 && last_t != REF_NONE) {
-                const int64_t last = base + n - 1;
-                const uint8_t *above = thr + fd.q_off + (y - 1) * fd.qw;
-                link = runs.end[last] == fd.qw - 2 && runs.v[last] == 255 && above[fd.qw - 1] == 255 &&
-                       above[fd.qw - 2] != 255;
+            if (y >= 1) {
+                auto white = [&](const RowWord *r, int x) { return r[x >> 5].white >> (x & 31) & 1u; };
+                link = white(row, qw - 2) && white(row - nw, qw - 1) && !white(row - nw, qw - 2) &&
+                       ref_lookup(s_key, s_idx, runs.lab[base + row_nruns[fd.row0 + y] - 1]) != REF_NONE;
             }
-            if (link) ref_node_init(ref, (uint32_t)(fd.node_off + (int64_t)fd.qw * fd.qh + y - 1), 1u);
+            if (link) ref_node_init(ref, (uint32_t)(fd.node_off + (int64_t)qw * fd.qh + y - 1), 1u);
             ref.trow[fd.row0 + y] = cnt | (link ? 0x80000000u : 0u);
         }
     }
@@ -400,8 +422,7 @@ __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_sums(const FrameDesc *f
 // before its own row).
 #define REF_ROOT_THREADS 128
 
-__global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *frames, RunArrays runs, RefOrder ref,
-                                                               uint32_t *err) {
+__global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *frames, RefOrder ref, uint32_t *err) {
     __shared__ uint32_t s_scan[32];
     __shared__ uint32_t s_ev, s_before, s_evj;
     __shared__ uint32_t s_win, s_winz;
@@ -434,8 +455,7 @@ __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *
         int ymax = fd.qh - 1, y0 = (int)((x - off) / qw);
         bool part = false;
         uint32_t lim = REF_INF, gen = 0;
-        auto len = [&](uint32_t u) { return (uint32_t)(runs.end[u] - runs.start[u]) + 1; };
-        uint32_t lx = len(x);
+        uint32_t lx = ref.len[x];
         scan_gain(y0, ymax);
         for (int guard = 0; guard < (1 << 16); guard++) {
             // the first row (y0 - 1: x alone) that leaves more than Z / 2:
@@ -575,7 +595,7 @@ __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *
             // branches start in its own row at the earliest, and join by row r)
             x = win;
             y0 = (int)((x - off) / qw);
-            lx = len(x);
+            lx = ref.len[x];
             for (int y = y0 + tid; y <= r; y += REF_ROOT_THREADS) gain[y] = 0;
             __syncthreads();
             for (int y = y0 + (tid >> 5); y <= r; y += REF_ROOT_THREADS / 32) {
@@ -612,7 +632,7 @@ __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *
 // ---------------------------------------------------------------------------
 // Launchers.
 
-int launch_ref_order(const Launch &L, const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
+int launch_ref_order(const Launch &L, const FrameDesc *frames, const RowWord *words, RunArrays runs,
                      const uint32_t *row_nruns, int nfam, const int64_t *qstart, const GpuDetection *dets,
                      const uint32_t *det_ok, const uint32_t *qcl, const uint64_t *ckey, int nb, const RefOrder &ref,
                      uint32_t *err) {
@@ -620,10 +640,10 @@ int launch_ref_order(const Launch &L, const FrameDesc *frames, const uint8_t *th
                                                    ref, err);
     const int64_t b = (L.max_qh + 7) / 8;
     const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 ? b : 148), (unsigned)L.nframes);
-    k_ref_mark<<<grid, 256, 0, L.stream>>>(frames, thr, runs, row_nruns, ref);
+    k_ref_mark<<<grid, 256, 0, L.stream>>>(frames, words, runs, row_nruns, ref);
     const dim3 rows((unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16), (unsigned)L.nframes);
     k_ref_link<<<rows, REF_ROW_THREADS, 0, L.stream>>>(frames, ref);
     k_ref_sums<<<rows, REF_ROW_THREADS, 0, L.stream>>>(frames, ref);
-    k_ref_root<<<dim3(AT_REF_MAXT, (unsigned)L.nframes), REF_ROOT_THREADS, 0, L.stream>>>(frames, runs, ref, err);
+    k_ref_root<<<dim3(AT_REF_MAXT, (unsigned)L.nframes), REF_ROOT_THREADS, 0, L.stream>>>(frames, ref, err);
     return 5;
 }
