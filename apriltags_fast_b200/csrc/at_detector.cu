@@ -95,7 +95,7 @@ struct HBuf {
 
 enum {
     B_FRAMES, B_IMG, B_QIM, B_THR, B_TMPA, B_TMPB, B_TMAX, B_TMIN, B_LAB,
-    B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS, B_RUNLAB,
+    B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS, B_RUNLAB, B_BANDN,
     B_KEY, B_VAL, B_KEY2, B_VAL2, B_HEAD, B_HSCAN, B_CSTART, B_CFRAME,
     B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
@@ -465,6 +465,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     CK(B[B_PARENT].ensure(nodes * 4));
     CK(B[B_PX].ensure(nodes * 4));
     CK(B[B_ROWRUNS].ensure(rows * 4));
+    CK(B[B_BANDN].ensure(rows * 4));
     CK(B[B_ROWPTS].ensure((rows + 1) * 8));
     CK(B[B_ROWOFF].ensure((rows + 1) * 8));
     CK(B[B_ERR].ensure(4));
@@ -530,7 +531,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         in->segment_smem = true;
     }
     in->launches += launch_segment(L, dfr, max_bands, band_smem, thr, runs, B[B_ROWRUNS].as<uint32_t>(),
-                                   B[B_WORDS].as<RowWord>(), td->qtp.min_cluster_pixels);
+                                   B[B_BANDN].as<uint32_t>(), B[B_WORDS].as<RowWord>(), td->qtp.min_cluster_pixels);
     in->labelled = true;
     CK(cudaEventRecord(in->ev[4], st));
     CK(cudaGetLastError());

@@ -54,7 +54,7 @@ void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uin
 bool segment_set_smem();
 void segment_plan(int qw, int qh, int64_t *max_bands, size_t *smem);
 int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,
-                   RunArrays runs, uint32_t *row_nruns, RowWord *words, int32_t min_px);
+                   RunArrays runs, uint32_t *row_nruns, uint32_t *band_roots, RowWord *words, int32_t min_px);
 // the labels per pixel (the sorting fallback of the clusters, diagnostics)
 void launch_labels(const Launch &L, const FrameDesc *frames, RunArrays runs, const RowWord *words, uint32_t *lab);
 void launch_point_count(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,

@@ -313,11 +313,14 @@ __device__ __forceinline__ uint32_t ref_col(uint64_t e) { return (uint32_t)(e >>
 // A block per row: each target run's touching runs in the row above (they
 // are target runs too), kept for k_ref_root in tch[rbase + j] (first | last
 // << 16 of the row above's list, 0xffffffff: none; the runs of its value
-// between them touch it as well), and the unions with them. Bound by the
-// latency of the searches and climbs (L2), so a block per row: the rows of
-// one frame alone have too few runs for a warp per row.
+// between them touch it as well), and the unions with them, listed first
+// and then one per thread (a union climbs to two tops through L2; from the
+// runs' own loops the warps waited for their slowest lane). A block per row:
+// the rows of one frame alone have too few runs for a warp per row.
 #define REF_ROW_THREADS 128
+#define REF_LIST 2048  // unions listed at once (more are made where they are found)
 __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_link(const FrameDesc *frames, RefOrder ref) {
+    __shared__ uint32_t s_list[REF_LIST], s_n;
     const int f = blockIdx.y;
     if (!ref.need[f]) return;
     const FrameDesc fd = frames[f];
@@ -325,11 +328,13 @@ __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_link(const FrameDesc *f
         const uint32_t tr = ref.trow[fd.row0 + y];
         const uint32_t n = tr & 0x7fffffffu, na = ref.trow[fd.row0 + y - 1] & 0x7fffffffu;
         const int64_t rb = fd.node_off + y * fd.qw, ra = rb - fd.qw;
+        __syncthreads();
+        if (threadIdx.x == 0) s_n = 0;
+        __syncthreads();
         for (uint32_t j = threadIdx.x; j < n; j += blockDim.x) {
             const uint64_t e = ref.tlist[rb + j];
             const int64_t a0 = e & 0xffff, a1 = e >> 16 & 0xffff;
             const uint8_t v = (uint8_t)(e >> 48);
-            const uint32_t i = (uint32_t)rb + ref_col(e);
             uint32_t lo = 0, hi = na;
             while (lo < hi) {  // the first run above whose end reaches a0 - 1
                 const uint32_t mid = (lo + hi) >> 1;
@@ -345,13 +350,23 @@ __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_link(const FrameDesc *f
                 if ((uint8_t)(b >> 48) != v || !runs_touch(a0, a1, b & 0xffff, b >> 16 & 0xffff, v)) continue;
                 if (first == 0xffffu) first = k;
                 last = k;
-                ref_insert(ref, i, (uint32_t)ra + ref_col(b), i);
+                const uint32_t at = atomicAdd(&s_n, 1u);
+                if (at < REF_LIST)
+                    s_list[at] = ref_col(e) | ref_col(b) << 16;
+                else
+                    ref_insert(ref, (uint32_t)rb + ref_col(e), (uint32_t)ra + ref_col(b), (uint32_t)rb + ref_col(e));
             }
             ref.tch[rb + j] = first == 0xffffu ? 0xffffffffu : first | last << 16;
-            if (j == n - 1 && (tr >> 31))
-                ref_insert(ref, i, (uint32_t)(fd.node_off + (int64_t)fd.qw * fd.qh + y - 1),
-                           (uint32_t)(rb + fd.qw - 1));
         }
+        __syncthreads();
+        const uint32_t np = min(s_n, (uint32_t)REF_LIST);
+        for (uint32_t p = threadIdx.x; p < np; p += blockDim.x) {
+            const uint32_t i = (uint32_t)rb + (s_list[p] & 0xffffu);
+            ref_insert(ref, i, (uint32_t)ra + (s_list[p] >> 16), i);
+        }
+        if (threadIdx.x == 0 && (tr >> 31))
+            ref_insert(ref, (uint32_t)rb + ref_col(ref.tlist[rb + n - 1]),
+                       (uint32_t)(fd.node_off + (int64_t)fd.qw * fd.qh + y - 1), (uint32_t)(rb + fd.qw - 1));
     }
 }
 

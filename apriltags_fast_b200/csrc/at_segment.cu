@@ -17,8 +17,8 @@
 //
 //   k_band_union   a block per band of rows: masks, run numbers, the unions
 //                  inside the band in shared memory; every run then points
-//                  at its band root, which holds the band component's pixels
-//                  and its smallest run.
+//                  at its band root (its set's smallest run), which holds
+//                  the band component's pixels.
 //   k_band_join    the unions across band edges and of the last column, in
 //                  global memory.
 //   k_root_sums    each band root adds its pixels to its component's root
@@ -74,6 +74,8 @@ __device__ __forceinline__ void uf_unite(uint32_t *par, uint32_t a, uint32_t b) 
 // within 32 KB). Images over 16384 wide get bands of one row, whose runs are
 // their own band roots.
 #define BAND_IDS 16384
+#define BAND_SEEN 512
+#define BAND_LIST 4096  // touching pairs listed at once (more are united where they are found)
 __host__ __device__ inline int band_shift(int qw) {
     int s = 5;
     while ((1 << s) < qw) s++;
@@ -85,7 +87,8 @@ __host__ __device__ inline int band_rows(int qw) {
 }
 __host__ __device__ inline size_t band_smem(int qw) {
     const int s = band_shift(qw), r = band_rows(qw);
-    return (size_t)r * ((qw + 31) / 32) * 16 + ((1 << s) > BAND_IDS ? 0 : (size_t)r * 2 << s);
+    const size_t ids = (1 << s) > BAND_IDS ? 0 : (size_t)r << s;
+    return (size_t)r * ((qw + 31) / 32) * 16 + 2 * ids + (2 * ids > 4 * BAND_LIST ? 2 * ids : 4 * BAND_LIST);
 }
 
 // The 4 bits 0, 8, 16, 24 of x as bits 0 to 3.
@@ -183,17 +186,26 @@ __device__ __forceinline__ uint32_t pair_count(const PairMasks &p) {
     return __popc(p.meet) + __popc(p.left) + __popc(p.right);
 }
 
-// Pairs listed at once (more are united where they are found). A union per
-// thread from the list: unions straight from the words' loops kept their
-// warps waiting for their slowest lane (the band joins of one 640 x 480
-// frame took 200 us that way).
-#define BAND_LIST 4096
+// Calls add(x, val) for the active lanes (every lane calls it): once with
+// the sum for the lanes that share the first active lane's x, then for the
+// others each. Components are few and large or many and small; finding all
+// groups (match_any, a reduction per group) took 10 times as long.
+template <class F>
+__device__ __forceinline__ void by_root(uint32_t x, uint32_t val, bool act, F add) {
+    const uint32_t am = __ballot_sync(0xffffffffu, act);
+    if (!am) return;
+    const uint32_t x0 = __shfl_sync(0xffffffffu, x, __ffs(am) - 1);
+    const bool same = act && x == x0;
+    const uint32_t sum = __reduce_add_sync(0xffffffffu, same ? val : 0u);
+    if ((int)(threadIdx.x & 31) == __ffs(am) - 1) add(x0, sum);
+    if (act && !same) add(x, val);
+}
 
-// Unions over band-local ids in shared memory, lock-free. Roots are linked
-// in the order of a bijective hash of their 14 bits (as uf_rank does): with
-// the larger id always under the smaller, the pieces of a row chained up and
-// the unions took 32k cycles a band instead of 6k.
-__device__ __forceinline__ uint32_t lu_rank(uint32_t x) { return x * 0x9e35u & (BAND_IDS - 1); }
+// Unions over band-local ids in shared memory, lock-free, the larger id
+// hooked under the smaller, so a root is its set's smallest node and the
+// large sets' roots stay where they are (in the order of a hash the root of
+// the largest set moves and every union that meets it waits for the others:
+// 42k cycles a band instead of 32k).
 __device__ __forceinline__ uint32_t lu_find(volatile uint16_t *par, uint32_t x) {
     uint32_t p = par[x];
     while (p != x) {
@@ -209,7 +221,7 @@ __device__ __forceinline__ void lu_unite(uint16_t *par, uint32_t a, uint32_t b) 
         a = lu_find(par, a);
         b = lu_find(par, b);
         if (a == b) return;
-        if (lu_rank(a) < lu_rank(b)) {
+        if (a < b) {
             const uint32_t t = a;
             a = b;
             b = t;
@@ -219,15 +231,18 @@ __device__ __forceinline__ void lu_unite(uint16_t *par, uint32_t a, uint32_t b) 
 }
 
 __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
-                                                    uint32_t *row_nruns, RowWord *words) {
+                                                    uint32_t *row_nruns, uint32_t *band_roots, RowWord *words) {
     extern __shared__ __align__(16) uint8_t s_band[];
-    __shared__ uint32_t s_list[BAND_LIST], s_n;
+    __shared__ uint32_t s_n, s_m;
     const FrameDesc f = frames[blockIdx.y];
     const int tid = threadIdx.x, lane = tid & 31;
     const int qw = f.qw, nw = (qw + 31) / 32, sh = band_shift(qw), R = band_rows(qw);
     const bool solo = (1 << sh) > BAND_IDS;
     RowWord *s_word = reinterpret_cast<RowWord *>(s_band);
     uint16_t *s_par = reinterpret_cast<uint16_t *>(s_word + R * nw);
+    uint32_t *s_list = reinterpret_cast<uint32_t *>(s_par + (solo ? 0 : R << sh));
+    const uint32_t list_cap = max((uint32_t)BAND_LIST, solo ? 0u : (uint32_t)(R << sh) / 2);
+    uint32_t *s_px = s_list;  // after the unions: two 16-bit counts a word (a band has at most 16384 pixels)
     const int nband = (f.qh + R - 1) / R;
     for (int b = blockIdx.x; b < nband; b += gridDim.x) {
         const int y0 = b * R, nr = min(R, f.qh - y0);
@@ -242,7 +257,7 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
             w.starts = w.before = 0;
             s_word[it] = w;
         }
-        if (tid == 0) s_n = 0;
+        if (tid == 0) s_n = s_m = 0;
         __syncthreads();
         // run starts and the runs before each word, a warp per row; each run
         // its own set (the rows' nodes are written in order)
@@ -267,9 +282,10 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
             }
             const int64_t base = node0 + (int64_t)r * qw;
             for (uint32_t k = lane; k < n; k += 32) {
-                runs.px[base + k] = 0;
-                runs.minid[base + k] = 0xffffffffu;
-                if (!solo) s_par[(r << sh) + k] = (uint16_t)((r << sh) + k);
+                if (!solo)
+                    s_par[(r << sh) + k] = (uint16_t)((r << sh) + k);
+                else
+                    runs.px[base + k] = 0;
             }
             if (lane == 0) {
                 row_nruns[f.row0 + y0 + r] = n;
@@ -279,8 +295,28 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
                 runs.minid[vn] = (uint32_t)vn;
             }
         }
+        // every run to its root so far (a thread walks on from what others
+        // found); at last the pixel counts, in the list's place, cleared
+        auto flatten = [&](bool last) {
+            if (solo) return;
+            for (int r = tid >> 5; r < nr; r += blockDim.x >> 5) {
+                const RowWord &lw = s_word[r * nw + nw - 1];
+                const uint32_t n = lw.before + __popc(lw.starts);
+                for (uint32_t k = lane; k < n; k += 32) {
+                    const uint32_t l = (uint32_t)(r << sh) + k;
+                    const volatile uint16_t *par = s_par;
+                    uint32_t x = l;
+                    for (uint32_t p = par[x]; p != x; p = par[x]) x = p;
+                    s_par[l] = (uint16_t)x;
+                    if (last) reinterpret_cast<uint16_t *>(s_px)[l] = 0;
+                }
+            }
+        };
         __syncthreads();
         for (int it = tid; it < nr * nw; it += blockDim.x) out[it] = s_word[it];
+        // the touching pairs; any run above that a run touches is its first
+        // parent (one plain store wins: the trees go up row by row, so no
+        // cycle), which leaves few unions to make
         for (int it0 = nw; it0 < nr * nw; it0 += blockDim.x) {
             const int it = it0 + tid, r = it / nw, i = it - r * nw;
             const RowWord *cur = s_word + r * nw, *abv = cur - nw;
@@ -291,20 +327,45 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
                 for_pairs(cur, abv, i, pm, [&](uint32_t c, uint32_t a) {
                     c += (uint32_t)r << sh;
                     a += (uint32_t)(r - 1) << sh;
-                    if (at < BAND_LIST)
-                        s_list[at] = c | a << 16;
-                    else
-                        lu_unite(s_par, c, a);
+                    s_par[c] = (uint16_t)a;
+                    if (at < list_cap) s_list[at] = c | a << 16;
                     at++;
                 });
         }
         __syncthreads();
-        const uint32_t np = min(s_n, (uint32_t)BAND_LIST);
-        for (uint32_t p = tid; p < np; p += blockDim.x) lu_unite(s_par, s_list[p] & 0xffffu, s_list[p] >> 16);
+        flatten(false);  // most pairs are then one step from one root
         __syncthreads();
-        // the words' pieces of runs, one of each word at a time: their pixels
-        // and smallest run to their band root (one atomic per distinct root
-        // of a warp)
+        // the pairs of different roots, as root pairs, to the list's front;
+        // then a union per thread
+        const uint32_t np = min(s_n, list_cap);
+        for (uint32_t p0 = 0; p0 < np; p0 += blockDim.x) {
+            uint32_t c = 0, a = 0;
+            if (p0 + tid < np) {
+                const uint32_t e = s_list[p0 + tid];
+                c = s_par[e & 0xffffu];
+                a = s_par[e >> 16];
+            }
+            __syncthreads();
+            const uint32_t at = list_places(c != a ? 1u : 0u, &s_m);
+            if (c != a) s_list[at] = c | a << 16;  // at or before the places read
+            __syncthreads();
+        }
+        const uint32_t nu = s_m;
+        for (uint32_t p = tid; p < nu; p += blockDim.x) lu_unite(s_par, s_list[p] & 0xffffu, s_list[p] >> 16);
+        if (s_n > list_cap) {  // the pairs that the list did not hold: all of them again
+            for (int it = nw + tid; it < nr * nw; it += blockDim.x) {
+                const int r = it / nw, i = it - r * nw;
+                const RowWord *cur = s_word + r * nw, *abv = cur - nw;
+                for_pairs(cur, abv, i, pair_masks(cur, abv, i, nw, qw), [&](uint32_t c, uint32_t a) {
+                    lu_unite(s_par, c + ((uint32_t)r << sh), a + ((uint32_t)(r - 1) << sh));
+                });
+            }
+        }
+        __syncthreads();
+        flatten(true);
+        if (tid == 0) s_n = 0;
+        __syncthreads();
+        // the pixels of the words' pieces of runs to their band roots
         for (int it0 = 0; it0 < nr * nw; it0 += blockDim.x) {
             const int it = it0 + tid, r = it / nw, i = it - r * nw;
             RowWord w = {0, 0, 0, 0};
@@ -314,41 +375,43 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
                 m = (w.white | w.black) & run_columns(i, qw);
             }
             const uint32_t stop = w.starts | ~m;
-            uint32_t live = __ballot_sync(0xffffffffu, m != 0);
-            while (m) {
-                const int c = __ffs(m) - 1;
-                const uint32_t past = c < 31 ? stop & (~0u << (c + 1)) : 0u;
-                const int e = past ? __ffs(past) - 1 : 32;
-                m = e < 32 ? m & (~0u << e) : 0u;
-                const uint32_t k = run_at(w, c);
-                uint32_t x = (uint32_t)(r << sh) + k;
-                if (!solo) {
-                    const volatile uint16_t *par = s_par;
-                    for (uint32_t p = par[x]; p != x; p = par[x]) x = p;
+            while (__any_sync(0xffffffffu, m != 0)) {
+                const bool act = m != 0;
+                uint32_t x = 0, z = 0;
+                if (act) {
+                    const int c = __ffs(m) - 1;
+                    const uint32_t past = c < 31 ? stop & (~0u << (c + 1)) : 0u;
+                    const int e = past ? __ffs(past) - 1 : 32;
+                    m = e < 32 ? m & (~0u << e) : 0u;
+                    x = (uint32_t)(r << sh) + run_at(w, c);
+                    z = (uint32_t)(e - c);
+                    if (!solo) x = s_par[x];
                 }
-                const uint32_t node = (uint32_t)(node0 + (int64_t)r * qw) + k;
-                const uint32_t peers = __match_any_sync(live, x);
-                const uint32_t sum = __reduce_add_sync(peers, (uint32_t)(e - c)), mn = __reduce_min_sync(peers, node);
-                if (lane == __ffs(peers) - 1) {
-                    const int64_t root = node0 + (int64_t)(x >> sh) * qw + (x & ((1u << sh) - 1u));
-                    atomicAdd(runs.px + root, sum);  // not 0: a band root
-                    atomicMin(runs.minid + root, mn);
-                }
-                live = __ballot_sync(live, m != 0);
+                by_root(x, z, act, [&](uint32_t to, uint32_t sum) {
+                    if (solo)
+                        atomicAdd(runs.px + node0 + to, sum);
+                    else
+                        atomicAdd(s_px + (to >> 1), sum << (16 * (to & 1)));
+                });
             }
-            __syncwarp();
         }
+        __syncthreads();
         for (int r = tid >> 5; r < nr; r += blockDim.x >> 5) {
             const RowWord &lw = s_word[r * nw + nw - 1];
             const uint32_t n = lw.before + __popc(lw.starts);
             const int64_t base = node0 + (int64_t)r * qw;
             for (uint32_t k = lane; k < n; k += 32) {
-                uint32_t x = (uint32_t)(r << sh) + k;
-                if (!solo)
-                    for (uint32_t p = s_par[x]; p != x; p = s_par[x]) x = p;
+                const uint32_t l = (uint32_t)(r << sh) + k, x = solo ? l : s_par[l];
                 runs.parent[base + k] = (uint32_t)(node0 + (int64_t)(x >> sh) * qw + (x & ((1u << sh) - 1u)));
+                if (!solo) runs.px[base + k] = x == l ? reinterpret_cast<uint16_t *>(s_px)[l] : 0u;  // not 0: a band root
+                if (x == l) {
+                    runs.minid[base + k] = (uint32_t)(base + k);
+                    runs.lab[node0 + atomicAdd(&s_n, 1u)] = (uint32_t)(base + k);  // the band's roots, listed
+                }
             }
         }
+        __syncthreads();
+        if (tid == 0) band_roots[f.row0 + y0] = s_n;
     }
 }
 
@@ -356,7 +419,11 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
 // of every row (fast/unionfind.c:89-97).
 __global__ void __launch_bounds__(256) k_band_join(const FrameDesc *frames, RunArrays runs, const uint32_t *row_nruns,
                                                    const RowWord *words) {
+    // a union per thread from the list: unions straight from the words' loops
+    // kept their warps waiting for their slowest lane (200 us for one
+    // 640 x 480 frame)
     __shared__ uint32_t s_list[BAND_LIST], s_n;
+    __shared__ unsigned long long s_seen[BAND_SEEN];
     const FrameDesc f = frames[blockIdx.y];
     const int tid = threadIdx.x, qw = f.qw, nw = (qw + 31) / 32, R = band_rows(qw > 0 ? qw : 1);
     const int nband = (f.qh + R - 1) / R;
@@ -382,9 +449,17 @@ __global__ void __launch_bounds__(256) k_band_join(const FrameDesc *frames, RunA
                 });
         }
         __syncthreads();
+        // most pairs repeat another's two band roots: a lossy table of the
+        // last pair met per place lets most of them through once only
+        for (int t = tid; t < BAND_SEEN; t += blockDim.x) s_seen[t] = 0;
+        __syncthreads();
         const uint32_t np = min(s_n, (uint32_t)BAND_LIST);
-        for (uint32_t p = tid; p < np; p += blockDim.x)
-            uf_unite(runs.parent, base + (s_list[p] & 0xffffu), above + (s_list[p] >> 16));
+        for (uint32_t p = tid; p < np; p += blockDim.x) {
+            const uint32_t c = runs.parent[base + (s_list[p] & 0xffffu)], a = runs.parent[above + (s_list[p] >> 16)];
+            const unsigned long long k = (unsigned long long)c << 32 | a;  // never 0: c is below the frame's first row
+            if (atomicExch(s_seen + ((c * 0x9e3779b1u ^ a * 0x85ebca6bu) >> 23), k) == k) continue;
+            uf_unite(runs.parent, c, a);
+        }
     }
     // the last run of row y reaches column qw - 2, white; above it only the
     // last column is white
@@ -409,38 +484,32 @@ __device__ __forceinline__ uint32_t uf_root(const uint32_t *par, uint32_t x) {
     return x;
 }
 
-// Each band root (and last-column node) adds its pixels and offers its
-// smallest run to its component's root (one atomic per distinct root of a
-// warp), and from here on points at it.
-__global__ void __launch_bounds__(256) k_root_sums(const FrameDesc *frames, RunArrays runs, const uint32_t *row_nruns) {
+// Each band root (and last-column node) adds its pixels and offers its id
+// to its component's root, and from here on points at it.
+__global__ void __launch_bounds__(128) k_root_sums(const FrameDesc *frames, RunArrays runs, const uint32_t *band_roots) {
     const FrameDesc f = frames[blockIdx.y];
-    const int lane = threadIdx.x & 31;
-    for (int64_t y = blockIdx.x; y < f.qh; y += gridDim.x) {
-        const int64_t base = f.node_off + y * f.qw;
-        const int64_t n = row_nruns[f.row0 + y];
-        for (int64_t i0 = 0; i0 <= n; i0 += blockDim.x) {
-            const int64_t i = i0 + threadIdx.x;
-            const int64_t node = i < n ? base + i : f.node_off + (int64_t)f.qw * f.qh + y;
-            // a component's root is a band root too, and its count may grow
-            // meanwhile, but it adds to no other
-            const uint32_t px = i <= n ? runs.px[node] : 0u;
-            uint32_t r = 0;
+    const int R = band_rows(f.qw > 0 ? f.qw : 1), nband = (f.qh + R - 1) / R;
+    for (int b = blockIdx.x; b < nband; b += gridDim.x) {
+        const int y0 = b * R, nr = min(R, f.qh - y0);
+        const uint32_t n = band_roots[f.row0 + y0];
+        const uint32_t *list = runs.lab + f.node_off + (int64_t)y0 * f.qw;
+        for (uint32_t i0 = 0; i0 < n + nr; i0 += blockDim.x) {
+            const uint32_t i = i0 + threadIdx.x;
+            uint32_t node = 0, px = 0, r = 0;
             bool add = false;
-            if (px) {
-                r = uf_root(runs.parent, (uint32_t)node);
-                add = r != (uint32_t)node;
+            if (i < n + nr) {
+                node = i < n ? list[i] : (uint32_t)(f.node_off + (int64_t)f.qw * f.qh + y0 + (i - n));
+                // a component's root is a band root too, and its count may
+                // grow meanwhile, but it adds to no other
+                px = runs.px[node];
+                r = uf_root(runs.parent, node);
+                add = r != node;
             }
-            const uint32_t live = __ballot_sync(0xffffffffu, add);
-            if (!add) continue;
             // no unions run any more: pointing straight at the root is safe
             // for the walks of other threads
-            runs.parent[node] = r;
-            const uint32_t peers = __match_any_sync(live, r);
-            const uint32_t sum = __reduce_add_sync(peers, px), mn = __reduce_min_sync(peers, runs.minid[node]);
-            if (lane == __ffs(peers) - 1) {
-                atomicAdd(runs.px + r, sum);
-                atomicMin(runs.minid + r, mn);
-            }
+            if (add) runs.parent[node] = r;
+            by_root(r, px, add, [&](uint32_t to, uint32_t sum) { atomicAdd(runs.px + to, sum); });
+            if (add && node < *(volatile uint32_t *)(runs.minid + r)) atomicMin(runs.minid + r, node);
         }
     }
 }
@@ -515,17 +584,16 @@ __global__ void __launch_bounds__(256) k_labels(const FrameDesc *frames, RunArra
 bool segment_set_smem() {
     // the most a band takes: 8 rows of 2048 columns or one of 16384, or the
     // words alone of a row of 65536
-    return cudaFuncSetAttribute(k_band_union, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024) == cudaSuccess;
+    return cudaFuncSetAttribute(k_band_union, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024) == cudaSuccess;
 }
 
 int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,
-                   RunArrays runs, uint32_t *row_nruns, RowWord *words, int32_t min_px) {
+                   RunArrays runs, uint32_t *row_nruns, uint32_t *band_roots, RowWord *words, int32_t min_px) {
     const unsigned n = (unsigned)L.nframes;
     const unsigned nb = (unsigned)(max_bands < 148 * 8 ? max_bands : 148 * 8);
-    k_band_union<<<dim3(nb, n), 256, smem, L.stream>>>(frames, thr, runs, row_nruns, words);
+    k_band_union<<<dim3(nb, n), 256, smem, L.stream>>>(frames, thr, runs, row_nruns, band_roots, words);
     k_band_join<<<dim3(nb, n), 256, 0, L.stream>>>(frames, runs, row_nruns, words);
-    const unsigned rows = (unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16);
-    k_root_sums<<<dim3(rows < 1 ? 1 : rows, n), 256, 0, L.stream>>>(frames, runs, row_nruns);
+    k_root_sums<<<dim3(nb, n), 128, 0, L.stream>>>(frames, runs, band_roots);
     const int64_t b = (L.max_qh + 7) / 8;
     k_run_labels<<<dim3((unsigned)(b < 1 ? 1 : b < 148 * 8 ? b : 148 * 8), n), 256, 0, L.stream>>>(
         frames, runs, row_nruns, words, min_px);
