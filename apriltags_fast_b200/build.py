@@ -45,7 +45,7 @@ def _newer(target, deps):
 
 def build(force: bool = False) -> str:
     os.makedirs(BUILD, exist_ok=True)
-    headers = [os.path.join(CSRC, h) for h in ("at_gpu.h", "at_kernels.h", "at_device.cuh")] + [
+    headers = [os.path.join(CSRC, h) for h in ("at_gpu.h", "at_kernels.h", "at_launch.h", "at_device.cuh")] + [
         os.path.join(ROOT, "include", "apriltag_fast.h")]
     objs = []
     fam_c = os.path.join(BUILD, "at_families_data.c")

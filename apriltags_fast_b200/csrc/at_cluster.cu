@@ -34,6 +34,7 @@
 #include "at_device.cuh"
 #include "at_gpu.h"
 #include "at_kernels.h"
+#include "at_launch.h"
 
 // Rows 1 .. qh-2 of each frame, a warp per row.
 #define ROW_WARPS_BEGIN                                                                              \
@@ -70,6 +71,7 @@ __host__ __device__ inline size_t row_pairs_bytes(int nd_cap) { return (size_t)2
 __global__ void __launch_bounds__(256) k_point_scan(const FrameDesc *frames, const RowWord *words, const uint32_t *lab,
                                                     int nb, PairTable T, PointRows P, uint32_t *full,
                                                     unsigned long long *npoints) {
+    kernel_begin();
     extern __shared__ __align__(16) uint8_t s_mem[];
     const int nd_cap = P.nd_cap, rt = 2 * nd_cap;
     uint64_t *tkey = reinterpret_cast<uint64_t *>(s_mem + (threadIdx.x >> 5) * row_pairs_bytes(nd_cap));
@@ -250,6 +252,7 @@ __device__ __forceinline__ int frame_of_node(const FrameDesc *frames, int nframe
 // Each distinct pair's frame; pairs per frame.
 __global__ void k_pair_frame(const uint64_t *okeys, int64_t ncl, int nb, const FrameDesc *frames, int nframes,
                              uint32_t *kframe, uint32_t *fcount) {
+    kernel_begin();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < ncl; r += (int64_t)gridDim.x * blockDim.x) {
         const int fr = frame_of_node(frames, nframes, (int64_t)(okeys[r] >> nb));
         kframe[r] = (uint32_t)fr;
@@ -260,6 +263,7 @@ __global__ void k_pair_frame(const uint64_t *okeys, int64_t ncl, int nb, const F
 // One block: each frame's first pair (foff, nframes + 1 entries).
 __global__ void __launch_bounds__(1024) k_pair_frame_offsets(const uint32_t *fcount, int nframes, uint32_t *foff,
                                                              uint32_t *fcur) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     uint32_t base = 0;
     for (int f0 = 0; f0 < nframes; f0 += blockDim.x) {
@@ -278,6 +282,7 @@ __global__ void __launch_bounds__(1024) k_pair_frame_offsets(const uint32_t *fco
 
 __global__ void k_pair_scatter(const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, const uint32_t *kframe,
                                const uint32_t *foff, uint32_t *fcur, uint64_t *gkeys, uint32_t *gslots) {
+    kernel_begin();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < ncl; r += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t fr = kframe[r];
         const uint32_t p = foff[fr] + atomicAdd(fcur + fr, 1u);
@@ -291,6 +296,7 @@ __global__ void k_pair_scatter(const uint64_t *okeys, const uint32_t *oslots, in
 __global__ void __launch_bounds__(256) k_pair_rank(const uint64_t *gkeys, const uint32_t *gslots, int64_t ncl,
                                                    const uint32_t *foff, int nframes, uint64_t *skeys,
                                                    uint32_t *sslots) {
+    kernel_begin();
     const int lane = threadIdx.x & 31;
     for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < ncl;
          p += ((int64_t)gridDim.x * blockDim.x) >> 5) {
@@ -319,6 +325,7 @@ __global__ void __launch_bounds__(256) k_pair_rank(const uint64_t *gkeys, const 
 __global__ void k_cluster_span(const uint64_t *skeys, const uint32_t *sslots, int64_t ncl, PairTable T, int nb,
                                const FrameDesc *frames, int nframes, uint32_t *rank_of_slot, uint32_t *ccount,
                                uint32_t *cspan, uint32_t *cy0, int32_t *cframe) {
+    kernel_begin();
     for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < ncl; c += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t s = sslots[c];
         rank_of_slot[s] = (uint32_t)c;
@@ -337,6 +344,7 @@ __global__ void k_cluster_span(const uint64_t *skeys, const uint32_t *sslots, in
 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan2_sums(const uint32_t *a, const uint32_t *b, int64_t n,
                                                              uint32_t *sa, uint32_t *sb) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     const int64_t i0 = (int64_t)blockIdx.x * SCAN_ITEMS + 4 * threadIdx.x;
     uint32_t va = 0, vb = 0;
@@ -355,6 +363,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan2_sums(const uint32_t *a, 
 }
 
 __global__ void __launch_bounds__(1024) k_scan2_top(uint32_t *sa, uint32_t *sb, int64_t nblocks) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     uint32_t ba = 0, bb = 0;
     for (int64_t i0 = 0; i0 < nblocks; i0 += blockDim.x) {
@@ -378,6 +387,7 @@ __global__ void __launch_bounds__(1024) k_scan2_top(uint32_t *sa, uint32_t *sb, 
 __global__ void __launch_bounds__(SCAN_THREADS) k_scan2_apply(const uint32_t *a, const uint32_t *b, int64_t n,
                                                               const uint32_t *sa, const uint32_t *sb,
                                                               int64_t nblocks, uint32_t *out_a, uint32_t *out_b) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     const int64_t i0 = (int64_t)blockIdx.x * SCAN_ITEMS + 4 * threadIdx.x;
     uint32_t xa[4], xb[4], va = 0, vb = 0;
@@ -406,6 +416,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan2_apply(const uint32_t *a,
 // a shortfall sets AT_ERR_SEGCAP and the host runs the batch again with
 // room enough; the point kernels then skip their work).
 __global__ void k_seg_zero(const uint32_t *spanoff, int64_t ncl, uint32_t *seg, int64_t cap, uint32_t *err) {
+    kernel_begin();
     const int64_t total = spanoff[ncl];
     if (total > cap) {
         if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(err, AT_ERR_SEGCAP);
@@ -419,6 +430,7 @@ __global__ void k_seg_zero(const uint32_t *spanoff, int64_t ncl, uint32_t *seg, 
 // first point in row cy0[c] + r.
 __global__ void __launch_bounds__(256) k_seg_scan(const uint32_t *cstart, const uint32_t *spanoff,
                                                   const uint32_t *cspan, int64_t ncl, uint32_t *seg, int64_t cap) {
+    kernel_begin();
     if (spanoff[ncl] > cap) return;
     const int lane = threadIdx.x & 31;
     for (int64_t c = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < ncl;
@@ -442,6 +454,7 @@ __global__ void __launch_bounds__(256) k_seg_scan(const uint32_t *cstart, const 
 __global__ void __launch_bounds__(256) k_seg_fill(const FrameDesc *frames, PointRows P, const uint32_t *rank_of_slot,
                                                   const uint32_t *spanoff, const uint32_t *cy0, int64_t ncl,
                                                   uint32_t *seg, int64_t cap) {
+    kernel_begin();
     if (spanoff[ncl] > cap) return;
     ROW_WARPS_BEGIN
     const uint32_t nd = P.info[f.row0 + y].y;
@@ -461,6 +474,7 @@ __global__ void __launch_bounds__(256) k_point_place(const FrameDesc *frames, Po
                                                      const uint32_t *rank_of_slot, const uint32_t *spanoff,
                                                      const uint32_t *cy0, int64_t ncl, const uint32_t *seg, int64_t cap,
                                                      uint64_t *out, int64_t npts, uint32_t *err) {
+    kernel_begin();
     extern __shared__ __align__(16) uint32_t s_base[];
     if (spanoff[ncl] > cap) return;
     uint32_t *base = s_base + (threadIdx.x >> 5) * 2 * P.nd_cap;  // by the pair's slot in the row's table
@@ -529,7 +543,7 @@ void launch_point_scan(const Launch &L, const FrameDesc *frames, const RowWord *
     const int w = scan_warps(P.nd_cap);
     const int64_t b = (L.max_qh + w - 1) / w;
     const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 * 8 ? b : 148 * 8), (unsigned)L.nframes);
-    k_point_scan<<<grid, 32 * w, w * row_pairs_bytes(P.nd_cap), L.stream>>>(frames, words, lab, nb, T, P, full, npoints);
+    launch(k_point_scan, grid, 32 * w, w * row_pairs_bytes(P.nd_cap), L.stream, frames, words, lab, nb, T, P, full, npoints);
 }
 
 void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, int nb,
@@ -538,17 +552,17 @@ void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *os
                        uint32_t *cy0, int32_t *cframe, uint32_t *cstart, uint32_t *spanoff) {
     if (ncl <= 0) return;
     cudaMemsetAsync(P.fcount, 0, (size_t)nframes * 4, s);
-    k_pair_frame<<<flat_grid(ncl, 256), 256, 0, s>>>(okeys, ncl, nb, frames, nframes, P.kframe, P.fcount);
-    k_pair_frame_offsets<<<1, 1024, 0, s>>>(P.fcount, nframes, P.foff, P.fcur);
-    k_pair_scatter<<<flat_grid(ncl, 256), 256, 0, s>>>(okeys, oslots, ncl, P.kframe, P.foff, P.fcur, P.gkeys,
+    launch(k_pair_frame, flat_grid(ncl, 256), 256, 0, s, okeys, ncl, nb, frames, nframes, P.kframe, P.fcount);
+    launch(k_pair_frame_offsets, 1, 1024, 0, s, P.fcount, nframes, P.foff, P.fcur);
+    launch(k_pair_scatter, flat_grid(ncl, 256), 256, 0, s, okeys, oslots, ncl, P.kframe, P.foff, P.fcur, P.gkeys,
                                                        P.gslots);
-    k_pair_rank<<<flat_grid(ncl * 32, 256), 256, 0, s>>>(P.gkeys, P.gslots, ncl, P.foff, nframes, skeys, sslots);
-    k_cluster_span<<<flat_grid(ncl, 256), 256, 0, s>>>(skeys, sslots, ncl, T, nb, frames, nframes, rank_of_slot,
+    launch(k_pair_rank, flat_grid(ncl * 32, 256), 256, 0, s, P.gkeys, P.gslots, ncl, P.foff, nframes, skeys, sslots);
+    launch(k_cluster_span, flat_grid(ncl, 256), 256, 0, s, skeys, sslots, ncl, T, nb, frames, nframes, rank_of_slot,
                                                        ccount, cspan, cy0, cframe);
     const int64_t nblk = (ncl + SCAN_ITEMS - 1) / SCAN_ITEMS;
-    k_scan2_sums<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(ccount, cspan, ncl, P.bsum_a, P.bsum_b);
-    k_scan2_top<<<1, 1024, 0, s>>>(P.bsum_a, P.bsum_b, nblk);
-    k_scan2_apply<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(ccount, cspan, ncl, P.bsum_a, P.bsum_b, nblk, cstart,
+    launch(k_scan2_sums, (unsigned)nblk, SCAN_THREADS, 0, s, ccount, cspan, ncl, P.bsum_a, P.bsum_b);
+    launch(k_scan2_top, 1, 1024, 0, s, P.bsum_a, P.bsum_b, nblk);
+    launch(k_scan2_apply, (unsigned)nblk, SCAN_THREADS, 0, s, ccount, cspan, ncl, P.bsum_a, P.bsum_b, nblk, cstart,
                                                           spanoff);
 }
 
@@ -563,18 +577,18 @@ void launch_scan_u32(cudaStream_t s, const uint32_t *a, int64_t n, uint32_t *out
     if (n <= 0) return;
     const int64_t nblk = (n + SCAN_ITEMS - 1) / SCAN_ITEMS;
     uint32_t *sa = scratch, *sb = scratch + nblk + 1, *ob = scratch + 2 * (nblk + 1);
-    k_scan2_sums<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(a, a, n, sa, sb);
-    k_scan2_top<<<1, 1024, 0, s>>>(sa, sb, nblk);
-    k_scan2_apply<<<(unsigned)nblk, SCAN_THREADS, 0, s>>>(a, a, n, sa, sb, nblk, out, ob);
+    launch(k_scan2_sums, (unsigned)nblk, SCAN_THREADS, 0, s, a, a, n, sa, sb);
+    launch(k_scan2_top, 1, 1024, 0, s, sa, sb, nblk);
+    launch(k_scan2_apply, (unsigned)nblk, SCAN_THREADS, 0, s, a, a, n, sa, sb, nblk, out, ob);
 }
 
 void launch_point_place(const Launch &L, const FrameDesc *frames, const PointRows &P, const uint32_t *rank_of_slot,
                         const uint32_t *cstart, const uint32_t *spanoff, const uint32_t *cspan, const uint32_t *cy0,
                         int64_t ncl, uint32_t *seg, int64_t cap, uint64_t *out, int64_t npts, uint32_t *err) {
     if (ncl <= 0) return;
-    k_seg_zero<<<flat_grid(cap, 256), 256, 0, L.stream>>>(spanoff, ncl, seg, cap, err);
-    k_seg_fill<<<row_warps(L), 256, 0, L.stream>>>(frames, P, rank_of_slot, spanoff, cy0, ncl, seg, cap);
-    k_seg_scan<<<flat_grid(ncl * 32, 256), 256, 0, L.stream>>>(cstart, spanoff, cspan, ncl, seg, cap);
-    k_point_place<<<row_warps(L), 256, 16 * P.nd_cap * 4, L.stream>>>(frames, P, rank_of_slot, spanoff, cy0, ncl, seg,
+    launch(k_seg_zero, flat_grid(cap, 256), 256, 0, L.stream, spanoff, ncl, seg, cap, err);
+    launch(k_seg_fill, row_warps(L), 256, 0, L.stream, frames, P, rank_of_slot, spanoff, cy0, ncl, seg, cap);
+    launch(k_seg_scan, flat_grid(ncl * 32, 256), 256, 0, L.stream, cstart, spanoff, cspan, ncl, seg, cap);
+    launch(k_point_place, row_warps(L), 256, 16 * P.nd_cap * 4, L.stream, frames, P, rank_of_slot, spanoff, cy0, ncl, seg,
                                                                     cap, out, npts, err);
 }

@@ -12,6 +12,7 @@
 #include "at_gpu.h"
 #include "at_device.cuh"
 #include "at_kernels.h"
+#include "at_launch.h"
 
 // ---------------------------------------------------------------------------
 // Small helpers.
@@ -34,6 +35,7 @@ __device__ __forceinline__ int64_t c_int(double x) {
 // output pixel.
 
 __global__ void k_decimate(const FrameDesc *frames, const uint8_t *img, uint8_t *qim, float factor) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const uint8_t *src = f.img;
     const int64_t stride = f.stride;
@@ -108,6 +110,7 @@ __global__ void k_decimate(const FrameDesc *frames, const uint8_t *img, uint8_t 
 // wide variant (images of 65536 pixels or more) filters one more output.
 
 __global__ void k_blur_pass(const FrameDesc *frames, const uint8_t *in, uint8_t *out, BlurTaps taps, int dir) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int qw = (int)f.qw, qh = (int)f.qh;
     const bool wide = (int64_t)qw * qh >= 65536;
@@ -134,6 +137,7 @@ __global__ void k_blur_pass(const FrameDesc *frames, const uint8_t *in, uint8_t 
 
 // sharpen: im = clamp(2 * orig - blurred) (fast/image.c:484-489); else copy
 __global__ void k_blur_finish(const FrameDesc *frames, const uint8_t *blurred, uint8_t *qim, int sharpen) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int64_t n = (int64_t)f.qw * f.qh;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
@@ -153,6 +157,7 @@ __global__ void k_blur_finish(const FrameDesc *frames, const uint8_t *blurred, u
 // neighbourhood (cells outside the grid left out).
 
 __global__ void k_tile_minmax(const FrameDesc *frames, const uint8_t *qim, uint8_t *tmax, uint8_t *tmin) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int64_t tw = f.qw / 4, th = f.qh / 4, n = tw * th;
     // 4-byte loads when every tile row is 4-byte aligned, else byte loads
@@ -206,6 +211,7 @@ __device__ __forceinline__ uint32_t box2(int x, int xv, uint32_t a, uint32_t b, 
 
 __global__ void __launch_bounds__(DT_THREADS) k_decimate_threshold(const FrameDesc *frames, uint8_t *qim, uint8_t *thr,
                                                                    int32_t diff) {
+    kernel_begin();
     __shared__ __align__(16) uint8_t s_q[4 * DT_ROWS][4 * DT_COLS];
     __shared__ uint8_t s_tmax[DT_ROWS + 2][DT_COLS + 4], s_tmin[DT_ROWS + 2][DT_COLS + 4];
     __shared__ uint16_t s_cell[DT_ROWS][DT_COLS];  // threshold | flat << 8
@@ -374,6 +380,7 @@ __global__ void __launch_bounds__(DT_THREADS) k_decimate_threshold(const FrameDe
 // (fast/threshold.c:85-91, 144-148): the partial tiles there clamp.
 __global__ void k_threshold(const FrameDesc *frames, const uint8_t *qim, const uint8_t *tmax, const uint8_t *tmin,
                             uint8_t *thr, int32_t diff) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int qw = (int)f.qw, qh = (int)f.qh;
     const int tw = qw / 4, th = qh / 4, cw = (qw + 3) / 4, ch = (qh + 3) / 4;
@@ -424,6 +431,7 @@ __global__ void k_threshold(const FrameDesc *frames, const uint8_t *qim, const u
 // Deglitch (fast/threshold.c:173-193): 3x3 dilate into tmp (its border
 // zero), then 3x3 erode back; the image border keeps its values.
 __global__ void k_morph(const FrameDesc *frames, const uint8_t *in, uint8_t *out, int dilate) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int qw = (int)f.qw, qh = (int)f.qh;
     for (int y = blockIdx.x; y < qh; y += gridDim.x) {
@@ -456,6 +464,7 @@ __global__ void k_morph(const FrameDesc *frames, const uint8_t *in, uint8_t *out
 // Block-per-row forms of the point passes (a block scan per 256 columns),
 // for batches too small to fill the GPU with a warp per row.
 __global__ void k_point_count_block(const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab, uint64_t *row_npts) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     const FrameDesc f = frames[blockIdx.y];
     for (int64_t y = blockIdx.x; y < f.qh; y += gridDim.x) {
@@ -473,6 +482,7 @@ __global__ void k_point_count_block(const FrameDesc *frames, const uint8_t *thr,
 
 __global__ void k_point_emit_block(const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
                              const uint64_t *row_pt_off, uint64_t *pt_key, uint64_t *pt_val, int nb) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     const FrameDesc f = frames[blockIdx.y];
     for (int64_t y = 1 + blockIdx.x; y + 1 < f.qh; y += gridDim.x) {
@@ -509,6 +519,7 @@ __global__ void k_point_emit_block(const FrameDesc *frames, const uint8_t *thr, 
 
 __global__ void __launch_bounds__(256) k_point_count(const FrameDesc *frames, const uint8_t *thr,
                                                      const uint32_t *lab, uint64_t *row_npts) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int lane = threadIdx.x & 31;
     const int64_t wpb = blockDim.x >> 5;
@@ -530,6 +541,7 @@ __global__ void __launch_bounds__(256) k_point_count(const FrameDesc *frames, co
 __global__ void __launch_bounds__(256) k_point_emit(const FrameDesc *frames, const uint8_t *thr,
                                                     const uint32_t *lab, const uint64_t *row_pt_off,
                                                     uint64_t *pt_key, uint64_t *pt_val, int nb) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int lane = threadIdx.x & 31;
     const int64_t wpb = blockDim.x >> 5;
@@ -569,6 +581,7 @@ __global__ void __launch_bounds__(256) k_point_emit(const FrameDesc *frames, con
 // The occupied slots, in no particular order: (pair, slot).
 __global__ void k_cluster_collect(const uint64_t *tkeys, uint32_t size, uint64_t *okeys, uint32_t *oslots,
                                   uint32_t *count) {
+    kernel_begin();
     const int lane = threadIdx.x & 31;
     for (uint32_t s0 = blockIdx.x * blockDim.x; s0 < size; s0 += gridDim.x * blockDim.x) {
         const uint32_t s = s0 + threadIdx.x;
@@ -591,6 +604,7 @@ __global__ void k_cluster_collect(const uint64_t *tkeys, uint32_t size, uint64_t
 // key, each run of equal keys is a cluster (points in emission order).
 
 __global__ void k_cluster_heads(const uint64_t *key, int64_t n, uint32_t *head) {
+    kernel_begin();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         head[i] = i == 0 || key[i] != key[i - 1];
 }
@@ -598,6 +612,7 @@ __global__ void k_cluster_heads(const uint64_t *key, int64_t n, uint32_t *head) 
 __global__ void k_cluster_starts(const uint64_t *key, const uint32_t *head, const uint32_t *head_scan, int64_t n,
                                  int nb, const FrameDesc *frames, int nframes, uint32_t *cstart, int32_t *cframe,
                                  uint64_t *ckey) {
+    kernel_begin();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         if (!head[i]) continue;
         uint32_t c = head_scan[i];
@@ -1109,6 +1124,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
                                                    FitScratch scr, GpuQuad *quads, uint32_t *quad_ok, uint32_t *err,
                                                    const uint32_t *list, const uint32_t *count, uint32_t *next,
                                                    int sort_cap, int chunk) {
+    kernel_begin();
     extern __shared__ __align__(16) unsigned char fit_smem[];
     const size_t xb = fit_x_bytes(sort_cap, chunk);
     uint64_t *s_key = reinterpret_cast<uint64_t *>(fit_smem);  // X: angle keys
@@ -1643,6 +1659,7 @@ __device__ __forceinline__ int fit_class(int64_t sz) {
 __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, const int32_t *cframe,
                                int64_t nclusters, int64_t npoints, int32_t min_px, uint32_t *quad_ok,
                                uint32_t *lists, uint32_t *counts) {
+    kernel_begin();
     const int lane = threadIdx.x & 31;
     for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nclusters; c0 += (int64_t)gridDim.x * blockDim.x) {
         const int64_t c = c0 + threadIdx.x;
@@ -1670,6 +1687,7 @@ __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, 
 #define FIT_ORDER_CAP 8192
 __global__ void __launch_bounds__(1024) k_fit_order(const uint32_t *cstart, int64_t nclusters, int64_t npoints,
                                                    uint32_t *lists, const uint32_t *counts, int first_class) {
+    kernel_begin();
     extern __shared__ __align__(16) uint64_t s_ord[];
     const int q = first_class + blockIdx.x;
     const uint32_t n = counts[q];
@@ -1801,6 +1819,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                                                           const uint32_t *list, const uint32_t *count,
                                                           uint32_t *next, GpuQuad *quads, uint32_t *quad_ok, int mm,
                                                           FitScratch scr) {
+    kernel_begin();
     constexpr int CAP = 32 * R;
     constexpr bool GP = R >= 16;  // prefix arrays in global scratch
     extern __shared__ __align__(16) unsigned char fw_smem[];
@@ -2605,6 +2624,7 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_refine(const FrameDesc *fram
                                                               const uint8_t *img, const uint8_t *qim,
                                                               const GpuQuad *quads, const uint32_t *nq, float *corners,
                                                               uint32_t *det_ok) {
+    kernel_begin();
     const int64_t nquads = *nq;
     __shared__ float s_p[4][2];
     __shared__ double s_lines[4][4];
@@ -2747,6 +2767,7 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_refine(const FrameDesc *fram
 #define QH_WARPS 4
 __global__ void __launch_bounds__(QH_WARPS * 32) k_quad_homography(const float *corners, const uint32_t *nq, double *hs,
                                                                      uint32_t *hok) {
+    kernel_begin();
     const int64_t nquads = *nq;
     __shared__ float s_p[QH_WARPS][4][2];
     __shared__ double s_hm[QH_WARPS][72];
@@ -2770,6 +2791,7 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_decode(const FrameDesc *fram
                                                               const uint8_t *qim, const GpuQuad *quads,
                                                               const uint32_t *nq, const double *hs, const uint32_t *hok,
                                                               GpuDetection *dets, uint32_t *det_ok) {
+    kernel_begin();
     const int64_t nquads = *nq;
     __shared__ double s_H[9];
     __shared__ double s_gx[8 * AT_MAX_TW], s_gy[8 * AT_MAX_TW], s_gv[8 * AT_MAX_TW];
@@ -3045,6 +3067,7 @@ __global__ void k_finalize(int nframes, const int64_t *frame_qstart, int nfam, c
                            const int64_t *out_off, int64_t *out_n, const FrameDesc *frames, RefOrder ref,
                            const uint32_t *qcl, const uint64_t *ckey, int nb, uint64_t *okey, uint32_t *idx2,
                            uint32_t *err) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     const int f = blockIdx.x;
     if (f >= nframes) return;
@@ -3163,6 +3186,7 @@ __global__ void k_finalize(int nframes, const int64_t *frame_qstart, int nfam, c
 // The quads in cluster order (so grouped by frame), and their count.
 __global__ void k_gather_quads(const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,
                                GpuQuad *out, uint32_t *nq, uint32_t *qcl) {
+    kernel_begin();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         if (ok[i]) {
             out[scan[i]] = quads[i];
@@ -3175,6 +3199,7 @@ __global__ void k_gather_quads(const GpuQuad *quads, const uint32_t *ok, const u
 // Per frame: its first quad and its first detection slot (nfam per quad).
 __global__ void k_frame_bounds(const GpuQuad *quads, const uint32_t *nq, int nframes, int nfam, int64_t *qstart,
                                int64_t *out_off) {
+    kernel_begin();
     const int64_t n = *nq;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f <= nframes; f += gridDim.x * blockDim.x) {
         int64_t lo = 0, hi = n;
@@ -3197,6 +3222,7 @@ __global__ void k_frame_bounds(const GpuQuad *quads, const uint32_t *nq, int nfr
 // k_output_copy: a warp per detection, its 21 words in one coalesced write.
 __global__ void __launch_bounds__(256) k_output_meta(int nframes, const int64_t *qstart, const int64_t *out_n,
                                                      int64_t *first, int64_t *meta) {
+    kernel_begin();
     __shared__ uint32_t sh[32];
     int64_t base = 0;
     for (int f0 = 0; f0 < nframes; f0 += blockDim.x) {
@@ -3221,6 +3247,7 @@ __global__ void __launch_bounds__(256) k_output_meta(int nframes, const int64_t 
 
 __global__ void k_output_copy(int nframes, const GpuDetection *out, const int64_t *out_off, const int64_t *first,
                               GpuDetection *host) {
+    kernel_begin();
     constexpr int W = (int)(sizeof(GpuDetection) / 8);
     const int lane = threadIdx.x & 31;
     const int64_t total = first[nframes];
@@ -3260,27 +3287,27 @@ static inline unsigned flat_blocks(int64_t n, int threads) {
 }
 
 void launch_decimate(const Launch &L, const FrameDesc *frames, const uint8_t *img, uint8_t *qim, float factor) {
-    k_decimate<<<frame_grid(L), 256, 0, L.stream>>>(frames, img, qim, factor);
+    launch(k_decimate, frame_grid(L), 256, 0, L.stream, frames, img, qim, factor);
 }
 
 void launch_blur(const Launch &L, const FrameDesc *frames, uint8_t *qim, uint8_t *tmp_a, uint8_t *tmp_b,
                  const BlurTaps &taps, bool sharpen) {
-    k_blur_pass<<<frame_grid(L), 256, 0, L.stream>>>(frames, qim, tmp_a, taps, 0);
-    k_blur_pass<<<frame_grid(L), 256, 0, L.stream>>>(frames, tmp_a, tmp_b, taps, 1);
-    k_blur_finish<<<frame_grid(L), 256, 0, L.stream>>>(frames, tmp_b, qim, sharpen ? 1 : 0);
+    launch(k_blur_pass, frame_grid(L), 256, 0, L.stream, frames, qim, tmp_a, taps, 0);
+    launch(k_blur_pass, frame_grid(L), 256, 0, L.stream, frames, tmp_a, tmp_b, taps, 1);
+    launch(k_blur_finish, frame_grid(L), 256, 0, L.stream, frames, tmp_b, qim, sharpen ? 1 : 0);
 }
 
 void launch_threshold(const Launch &L, const FrameDesc *frames, const uint8_t *qim, uint8_t *tmax, uint8_t *tmin,
                       uint8_t *thr, int32_t diff) {
-    k_tile_minmax<<<frame_grid(L), 256, 0, L.stream>>>(frames, qim, tmax, tmin);
-    k_threshold<<<frame_grid(L), 256, 0, L.stream>>>(frames, qim, tmax, tmin, thr, diff);
+    launch(k_tile_minmax, frame_grid(L), 256, 0, L.stream, frames, qim, tmax, tmin);
+    launch(k_threshold, frame_grid(L), 256, 0, L.stream, frames, qim, tmax, tmin, thr, diff);
 }
 
 void launch_decimate_threshold(const Launch &L, const FrameDesc *frames, int64_t max_cells, uint8_t *qim, uint8_t *thr,
                                int32_t diff) {
     // blocks per frame: enough regions for the frame with the most cells
     // (each block finds its region from its frame's width; extra ones exit)
-    k_decimate_threshold<<<dim3((unsigned)max_cells, (unsigned)L.nframes), DT_THREADS, 0, L.stream>>>(frames, qim, thr,
+    launch(k_decimate_threshold, dim3((unsigned)max_cells, (unsigned)L.nframes), DT_THREADS, 0, L.stream, frames, qim, thr,
                                                                                                      diff);
 }
 
@@ -3290,39 +3317,39 @@ int64_t decimate_threshold_blocks(int64_t qw, int64_t qh) {
 }
 
 void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uint8_t *tmp) {
-    k_morph<<<frame_grid(L), 256, 0, L.stream>>>(frames, thr, tmp, 1);
-    k_morph<<<frame_grid(L), 256, 0, L.stream>>>(frames, tmp, thr, 0);
+    launch(k_morph, frame_grid(L), 256, 0, L.stream, frames, thr, tmp, 1);
+    launch(k_morph, frame_grid(L), 256, 0, L.stream, frames, tmp, thr, 0);
 }
 
 void launch_point_count(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
                         uint64_t *row_npts) {
     if (warp_rows(L))
-        k_point_count<<<row_warp_grid(L), 256, 0, L.stream>>>(frames, thr, lab, row_npts);
+        launch(k_point_count, row_warp_grid(L), 256, 0, L.stream, frames, thr, lab, row_npts);
     else
-        k_point_count_block<<<frame_grid(L), 256, 0, L.stream>>>(frames, thr, lab, row_npts);
+        launch(k_point_count_block, frame_grid(L), 256, 0, L.stream, frames, thr, lab, row_npts);
 }
 
 void launch_point_emit(const Launch &L, const FrameDesc *frames, const uint8_t *thr, const uint32_t *lab,
                        const uint64_t *row_pt_off, uint64_t *pt_key, uint64_t *pt_val, int nb) {
     if (warp_rows(L))
-        k_point_emit<<<row_warp_grid(L), 256, 0, L.stream>>>(frames, thr, lab, row_pt_off, pt_key, pt_val, nb);
+        launch(k_point_emit, row_warp_grid(L), 256, 0, L.stream, frames, thr, lab, row_pt_off, pt_key, pt_val, nb);
     else
-        k_point_emit_block<<<frame_grid(L), 256, 0, L.stream>>>(frames, thr, lab, row_pt_off, pt_key, pt_val, nb);
+        launch(k_point_emit_block, frame_grid(L), 256, 0, L.stream, frames, thr, lab, row_pt_off, pt_key, pt_val, nb);
 }
 
 void launch_cluster_collect(cudaStream_t s, const uint64_t *tkeys, uint32_t size, uint64_t *okeys, uint32_t *oslots,
                             uint32_t *count) {
-    k_cluster_collect<<<flat_blocks(size, 256), 256, 0, s>>>(tkeys, size, okeys, oslots, count);
+    launch(k_cluster_collect, flat_blocks(size, 256), 256, 0, s, tkeys, size, okeys, oslots, count);
 }
 
 void launch_cluster_heads(cudaStream_t s, const uint64_t *key, int64_t n, uint32_t *head) {
-    k_cluster_heads<<<flat_blocks(n, 256), 256, 0, s>>>(key, n, head);
+    launch(k_cluster_heads, flat_blocks(n, 256), 256, 0, s, key, n, head);
 }
 
 void launch_cluster_starts(cudaStream_t s, const uint64_t *key, const uint32_t *head, const uint32_t *head_scan,
                            int64_t n, int nb, const FrameDesc *frames, int nframes, uint32_t *cstart, int32_t *cframe,
                            uint64_t *ckey) {
-    k_cluster_starts<<<flat_blocks(n, 256), 256, 0, s>>>(key, head, head_scan, n, nb, frames, nframes, cstart, cframe,
+    launch(k_cluster_starts, flat_blocks(n, 256), 256, 0, s, key, head, head_scan, n, nb, frames, nframes, cstart, cframe,
                                                          ckey);
 }
 
@@ -3341,7 +3368,7 @@ static void launch_fit_warp(cudaStream_t s, const FrameDesc *frames, const GpuPa
         per_sm = 1;
     const int64_t full = 148 * (int64_t)per_sm;
     const int64_t wb = (nclusters + FIT_WPB - 1) / FIT_WPB;
-    k_fit_warp<R><<<(unsigned)(wb < full ? wb : full), FIT_WPB * 32, wsm, s>>>(
+    launch(k_fit_warp<R>, (unsigned)(wb < full ? wb : full), FIT_WPB * 32, wsm, s, 
         frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr.lists + (int64_t)q * nclusters,
         scr.counts + q, scr.counts + FIT_NCLASS + q, quads, quad_ok, mm, scr);
 }
@@ -3359,7 +3386,7 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
     const int mm = prm.max_nmaxima > 4 ? prm.max_nmaxima : 4;
     // the size classes' lists, the two block classes' largest first
     cudaMemsetAsync(scr.counts, 0, 2 * FIT_NCLASS * sizeof(uint32_t), s);
-    k_fit_classify<<<flat_blocks(nclusters, 256), 256, 0, s>>>(frames, cstart, cframe, nclusters, npoints,
+    launch(k_fit_classify, flat_blocks(nclusters, 256), 256, 0, s, frames, cstart, cframe, nclusters, npoints,
                                                                 prm.min_cluster_pixels, quad_ok, scr.lists,
                                                                 scr.counts);
     // five streams, one per group of classes: above 6144 points (a block of
@@ -3376,22 +3403,22 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
     if (huge) {
         const size_t hsm = fit_smem_bytes(FIT_HUGE_SORT, FIT_CHUNK_LARGE, FIT_HUGE_NT / 32);
         cudaFuncSetAttribute(k_fit_quads<FIT_HUGE_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
-        k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[3]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 5);
-        k_fit_quads<FIT_HUGE_NT><<<(unsigned)(nclusters < 148 ? nclusters : 148), FIT_HUGE_NT, hsm, S.side[3]>>>(
+        launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[3], cstart, nclusters, npoints, scr.lists, scr.counts, 5);
+        launch(k_fit_quads<FIT_HUGE_NT>, (unsigned)(nclusters < 148 ? nclusters : 148), FIT_HUGE_NT, hsm, S.side[3], 
             frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(5),
             scr.counts + 5, scr.counts + FIT_NCLASS + 5, FIT_HUGE_SORT, FIT_CHUNK_LARGE);
         cudaEventRecord(S.join[3], S.side[3]);
     }
-    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[0]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 4);
-    k_fit_order<<<1, 1024, FIT_ORDER_CAP * 8, S.side[1]>>>(cstart, nclusters, npoints, scr.lists, scr.counts, 3);
+    launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[0], cstart, nclusters, npoints, scr.lists, scr.counts, 4);
+    launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[1], cstart, nclusters, npoints, scr.lists, scr.counts, 3);
     // two blocks an SM: one cluster's serial steps overlap the other's
     const unsigned nbig = (unsigned)(nclusters < 2 * 148 ? nclusters : 2 * 148);
-    k_fit_quads<FIT_LARGE_NT><<<nbig, FIT_LARGE_NT, large, S.side[0]>>>(
+    launch(k_fit_quads<FIT_LARGE_NT>, nbig, FIT_LARGE_NT, large, S.side[0], 
         frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(4), scr.counts + 4,
         scr.counts + FIT_NCLASS + 4, FIT_LARGE_SORT, FIT_CHUNK_LARGE);
     cudaEventRecord(S.join[0], S.side[0]);
     const unsigned mid = (unsigned)(nclusters < 148 * 4 ? nclusters : 148 * 4);
-    k_fit_quads<128><<<mid, 128, small, S.side[1]>>>(frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
+    launch(k_fit_quads<128>, mid, 128, small, S.side[1], frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
                                                      quads, quad_ok, err, list(3), scr.counts + 3,
                                                      scr.counts + FIT_NCLASS + 3, FIT_SMALL, FIT_CHUNK_SMALL);
     cudaEventRecord(S.join[1], S.side[1]);
@@ -3407,20 +3434,20 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
 void launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,
                          GpuQuad *out, uint32_t *nq, uint32_t *qcl) {
     if (n <= 0) return;
-    k_gather_quads<<<flat_blocks(n, 256), 256, 0, s>>>(quads, ok, scan, n, out, nq, qcl);
+    launch(k_gather_quads, flat_blocks(n, 256), 256, 0, s, quads, ok, scan, n, out, nq, qcl);
 }
 
 void launch_frame_bounds(cudaStream_t s, const GpuQuad *quads, const uint32_t *nq, int nframes, int nfam,
                          int64_t *qstart, int64_t *out_off) {
-    k_frame_bounds<<<flat_blocks(nframes + 1, 256), 256, 0, s>>>(quads, nq, nframes, nfam, qstart, out_off);
+    launch(k_frame_bounds, flat_blocks(nframes + 1, 256), 256, 0, s, quads, nq, nframes, nfam, qstart, out_off);
 }
 
 void launch_output(cudaStream_t s, int nframes, const int64_t *qstart, const GpuDetection *out,
                    const int64_t *out_off, const int64_t *out_n, int64_t *first, GpuDetection *host,
                    int64_t *meta, int64_t max_dets) {
-    k_output_meta<<<1, 256, 0, s>>>(nframes, qstart, out_n, first, meta);
+    launch(k_output_meta, 1, 256, 0, s, nframes, qstart, out_n, first, meta);
     const int64_t blocks = (max_dets + 7) / 8;
-    k_output_copy<<<(unsigned)(blocks < 1 ? 1 : blocks < 148 * 4 ? blocks : 148 * 4), 256, 0, s>>>(nframes, out, out_off,
+    launch(k_output_copy, (unsigned)(blocks < 1 ? 1 : blocks < 148 * 4 ? blocks : 148 * 4), 256, 0, s, nframes, out, out_off,
                                                                                                 first, host);
 }
 
@@ -3430,11 +3457,11 @@ void launch_decode(cudaStream_t s, const FrameDesc *frames, const GpuParams &prm
     // grids for at most max_quads quads; the kernels read the count (scr.nq)
     if (max_quads <= 0) return;
     const unsigned blocks = (unsigned)(max_quads < 148 * 64 ? max_quads : 148 * 64);
-    k_refine<<<blocks, AT_DEC_THREADS, 0, s>>>(frames, prm, img, qim, quads, scr.nq, scr.corners, det_ok);
+    launch(k_refine, blocks, AT_DEC_THREADS, 0, s, frames, prm, img, qim, quads, scr.nq, scr.corners, det_ok);
     const int64_t hb = (max_quads + QH_WARPS - 1) / QH_WARPS;
-    k_quad_homography<<<(unsigned)(hb < 148 * 16 ? hb : 148 * 16), QH_WARPS * 32, 0, s>>>(scr.corners, scr.nq,
+    launch(k_quad_homography, (unsigned)(hb < 148 * 16 ? hb : 148 * 16), QH_WARPS * 32, 0, s, scr.corners, scr.nq,
                                                                                         scr.h, scr.hok);
-    k_decode<<<blocks, AT_DEC_THREADS, 0, s>>>(frames, prm, fams, img, qim, quads, scr.nq, scr.h, scr.hok, dets,
+    launch(k_decode, blocks, AT_DEC_THREADS, 0, s, frames, prm, fams, img, qim, quads, scr.nq, scr.h, scr.hok, dets,
                                                det_ok);
 }
 
@@ -3443,6 +3470,6 @@ void launch_finalize(cudaStream_t s, int nframes, const int64_t *frame_qstart, i
                      const int64_t *out_off, int64_t *out_n, const FrameDesc *frames, const RefOrder &ref,
                      const uint32_t *qcl, const uint64_t *ckey, int nb, uint64_t *okey, uint32_t *idx2,
                      uint32_t *err) {
-    k_finalize<<<nframes, 256, 0, s>>>(nframes, frame_qstart, nfam, dets, det_ok, idx, removed, out, out_off, out_n,
+    launch(k_finalize, nframes, 256, 0, s, nframes, frame_qstart, nfam, dets, det_ok, idx, removed, out, out_off, out_n,
                                        frames, ref, qcl, ckey, nb, okey, idx2, err);
 }

@@ -66,6 +66,7 @@
 #include "at_device.cuh"
 #include "at_gpu.h"
 #include "at_kernels.h"
+#include "at_launch.h"
 
 #define REF_HASH 1024          // open-addressing table of target labels (k_ref_targets, k_ref_mark)
 #define REF_NONE 0xffu         // no target
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(256) k_ref_targets(const FrameDesc *frames, in
                                                      const uint32_t *qcl, const uint64_t *ckey, int nb,
                                                      RunArrays runs, const uint32_t *row_nruns, RefOrder ref,
                                                      uint32_t *err) {
+    kernel_begin();
     __shared__ uint32_t s_once[2048], s_twice[2048];
     __shared__ uint32_t s_key[REF_HASH];
     __shared__ uint32_t s_n, s_need, s_over;
@@ -191,6 +193,7 @@ __device__ __forceinline__ void ref_node_init(const RefOrder &ref, uint32_t node
 
 __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const RowWord *words, RunArrays runs,
                                                   const uint32_t *row_nruns, RefOrder ref) {
+    kernel_begin();
     __shared__ uint32_t s_key[REF_HASH];
     __shared__ uint8_t s_idx[REF_HASH];
     const int f = blockIdx.y;
@@ -320,6 +323,7 @@ __device__ __forceinline__ uint32_t ref_col(uint64_t e) { return (uint32_t)(e >>
 #define REF_ROW_THREADS 128
 #define REF_LIST 2048  // unions listed at once (more are made where they are found)
 __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_link(const FrameDesc *frames, RefOrder ref) {
+    kernel_begin();
     __shared__ uint32_t s_list[REF_LIST], s_n;
     const int f = blockIdx.y;
     if (!ref.need[f]) return;
@@ -384,6 +388,7 @@ __device__ __forceinline__ uint64_t ref_true_parent(const RefOrder &ref, uint32_
 // target's gain in the row where its branch joins the top (hist). Lanes of
 // a warp that add to one place add once.
 __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_sums(const FrameDesc *frames, RefOrder ref) {
+    kernel_begin();
     const int f = blockIdx.y;
     if (!ref.need[f]) return;
     const FrameDesc fd = frames[f];
@@ -431,7 +436,7 @@ __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_sums(const FrameDesc *f
 // ---------------------------------------------------------------------------
 // The root of each target, a block per target: from the whole component
 // back to the run that the reference's unions leave as its root (see the top
-// of the file). x: the top of the current set; Z its pixels; ymax the last
+// of the file). (48 blocks a frame take them in turn.) x: the top of the current set; Z its pixels; ymax the last
 // row that it holds whole; with `part`, also the events before node `lim` of
 // the row after. gain[y]: the pixels x's set gained up to row y (x alone
 // before its own row).
@@ -442,14 +447,16 @@ __global__ void __launch_bounds__(REF_ROW_THREADS) k_ref_sums(const FrameDesc *f
 #define REF_ROOT_THREADS 1024
 
 __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *frames, RefOrder ref, uint32_t *err) {
+    kernel_begin();
     __shared__ uint32_t s_scan[32];
     __shared__ uint32_t s_ev, s_before, s_evj;
     __shared__ uint32_t s_win, s_winz;
     const int f = blockIdx.y;
-    const uint32_t t = blockIdx.x;
-    if (!ref.need[f] || t >= ref.nt[f]) return;
+    if (!ref.need[f]) return;
     const FrameDesc fd = frames[f];
     const int tid = threadIdx.x, lane = tid & 31;
+    for (uint32_t t = blockIdx.x; t < ref.nt[f]; t += gridDim.x) {
+    __syncthreads();
     const uint32_t off = (uint32_t)fd.node_off, qw = (uint32_t)fd.qw;
     const uint32_t vbase = off + (uint32_t)((int64_t)fd.qw * fd.qh);
     uint32_t *gain = ref.hist + fd.row0 * AT_REF_MAXT + (int64_t)t * fd.qh;
@@ -655,6 +662,7 @@ __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *
         }
         ref.troot[(int64_t)f * AT_REF_MAXT + t] = root;
     }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -664,14 +672,14 @@ int launch_ref_order(const Launch &L, const FrameDesc *frames, const RowWord *wo
                      const uint32_t *row_nruns, int nfam, const int64_t *qstart, const GpuDetection *dets,
                      const uint32_t *det_ok, const uint32_t *qcl, const uint64_t *ckey, int nb, const RefOrder &ref,
                      uint32_t *err) {
-    k_ref_targets<<<L.nframes, 256, 0, L.stream>>>(frames, nfam, qstart, dets, det_ok, qcl, ckey, nb, runs, row_nruns,
+    launch(k_ref_targets, L.nframes, 256, 0, L.stream, frames, nfam, qstart, dets, det_ok, qcl, ckey, nb, runs, row_nruns,
                                                    ref, err);
     const int64_t b = (L.max_qh + 7) / 8;
     const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 ? b : 148), (unsigned)L.nframes);
-    k_ref_mark<<<grid, 256, 0, L.stream>>>(frames, words, runs, row_nruns, ref);
+    launch(k_ref_mark, grid, 256, 0, L.stream, frames, words, runs, row_nruns, ref);
     const dim3 rows((unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16), (unsigned)L.nframes);
-    k_ref_link<<<rows, REF_ROW_THREADS, 0, L.stream>>>(frames, ref);
-    k_ref_sums<<<rows, REF_ROW_THREADS, 0, L.stream>>>(frames, ref);
-    k_ref_root<<<dim3(AT_REF_MAXT, (unsigned)L.nframes), REF_ROOT_THREADS, 0, L.stream>>>(frames, ref, err);
+    launch(k_ref_link, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
+    launch(k_ref_sums, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
+    launch(k_ref_root, dim3(48, (unsigned)L.nframes), REF_ROOT_THREADS, 0, L.stream, frames, ref, err);
     return 5;
 }

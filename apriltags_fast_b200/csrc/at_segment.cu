@@ -32,6 +32,7 @@
 #include "at_device.cuh"
 #include "at_gpu.h"
 #include "at_kernels.h"
+#include "at_launch.h"
 
 __device__ __forceinline__ uint32_t uf_find(uint32_t *par, uint32_t x) {
     volatile uint32_t *p = par;
@@ -232,6 +233,7 @@ __device__ __forceinline__ void lu_unite(uint16_t *par, uint32_t a, uint32_t b) 
 
 __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, const uint8_t *thr, RunArrays runs,
                                                     uint32_t *row_nruns, uint32_t *band_roots, RowWord *words) {
+    kernel_begin();
     extern __shared__ __align__(16) uint8_t s_band[];
     __shared__ uint32_t s_n, s_m;
     const FrameDesc f = frames[blockIdx.y];
@@ -419,6 +421,7 @@ __global__ void __launch_bounds__(256) k_band_union(const FrameDesc *frames, con
 // of every row (fast/unionfind.c:89-97).
 __global__ void __launch_bounds__(256) k_band_join(const FrameDesc *frames, RunArrays runs, const uint32_t *row_nruns,
                                                    const RowWord *words) {
+    kernel_begin();
     // a union per thread from the list: unions straight from the words' loops
     // kept their warps waiting for their slowest lane (200 us for one
     // 640 x 480 frame)
@@ -487,6 +490,7 @@ __device__ __forceinline__ uint32_t uf_root(const uint32_t *par, uint32_t x) {
 // Each band root (and last-column node) adds its pixels and offers its id
 // to its component's root, and from here on points at it.
 __global__ void __launch_bounds__(128) k_root_sums(const FrameDesc *frames, RunArrays runs, const uint32_t *band_roots) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int R = band_rows(f.qw > 0 ? f.qw : 1), nband = (f.qh + R - 1) / R;
     for (int b = blockIdx.x; b < nband; b += gridDim.x) {
@@ -521,6 +525,7 @@ __global__ void __launch_bounds__(128) k_root_sums(const FrameDesc *frames, RunA
 // order, then a word a lane.
 __global__ void __launch_bounds__(256) k_run_labels(const FrameDesc *frames, RunArrays runs, const uint32_t *row_nruns,
                                                     RowWord *words, int32_t min_px) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int lane = threadIdx.x & 31, wpb = blockDim.x >> 5;
     const int qw = f.qw, nw = (qw + 31) / 32;
@@ -564,6 +569,7 @@ __global__ void __launch_bounds__(256) k_run_labels(const FrameDesc *frames, Run
 // node), from k_run_labels.
 __global__ void __launch_bounds__(256) k_labels(const FrameDesc *frames, RunArrays runs, const RowWord *words,
                                                 uint32_t *lab) {
+    kernel_begin();
     const FrameDesc f = frames[blockIdx.y];
     const int qw = f.qw, nw = (qw + 31) / 32;
     for (int y = blockIdx.x; y < f.qh; y += gridDim.x)
@@ -591,18 +597,18 @@ int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, 
                    RunArrays runs, uint32_t *row_nruns, uint32_t *band_roots, RowWord *words, int32_t min_px) {
     const unsigned n = (unsigned)L.nframes;
     const unsigned nb = (unsigned)(max_bands < 148 * 8 ? max_bands : 148 * 8);
-    k_band_union<<<dim3(nb, n), 256, smem, L.stream>>>(frames, thr, runs, row_nruns, band_roots, words);
-    k_band_join<<<dim3(nb, n), 256, 0, L.stream>>>(frames, runs, row_nruns, words);
-    k_root_sums<<<dim3(nb, n), 128, 0, L.stream>>>(frames, runs, band_roots);
+    launch(k_band_union, dim3(nb, n), 256, smem, L.stream, frames, thr, runs, row_nruns, band_roots, words);
+    launch(k_band_join, dim3(nb, n), 256, 0, L.stream, frames, runs, row_nruns, words);
+    launch(k_root_sums, dim3(nb, n), 128, 0, L.stream, frames, runs, band_roots);
     const int64_t b = (L.max_qh + 7) / 8;
-    k_run_labels<<<dim3((unsigned)(b < 1 ? 1 : b < 148 * 8 ? b : 148 * 8), n), 256, 0, L.stream>>>(
+    launch(k_run_labels, dim3((unsigned)(b < 1 ? 1 : b < 148 * 8 ? b : 148 * 8), n), 256, 0, L.stream, 
         frames, runs, row_nruns, words, min_px);
     return 4;
 }
 
 void launch_labels(const Launch &L, const FrameDesc *frames, RunArrays runs, const RowWord *words, uint32_t *lab) {
     const unsigned rows = (unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16);
-    k_labels<<<dim3(rows < 1 ? 1 : rows, (unsigned)L.nframes), 256, 0, L.stream>>>(frames, runs, words, lab);
+    launch(k_labels, dim3(rows < 1 ? 1 : rows, (unsigned)L.nframes), 256, 0, L.stream, frames, runs, words, lab);
 }
 
 void segment_plan(int qw, int qh, int64_t *max_bands, size_t *smem) {
