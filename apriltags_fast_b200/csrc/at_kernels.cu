@@ -813,43 +813,28 @@ struct Moments {
     const double *mx, *my, *mxx, *mxy, *myy, *mw;
 };
 
+__device__ __forceinline__ MSum moments_at(const Moments &a, int64_t i) {
+    return {a.mx[i], a.my[i], a.mxx[i], a.mxy[i], a.myy[i], a.mw[i]};
+}
+
 // Moments of sorted points i0..i1, wrapping past the end, summed in the
-// reference's forms (fast/quads.c:539-569, 658-700, 885-921).
-__device__ __forceinline__ MSum seg_moments(const Moments &a, int64_t sz, int64_t i0, int64_t i1) {
-    MSum s;
-    if (i0 <= i1) {
-        s.x = a.mx[i1];
-        s.y = a.my[i1];
-        s.xx = a.mxx[i1];
-        s.xy = a.mxy[i1];
-        s.yy = a.myy[i1];
-        s.w = a.mw[i1];
-        if (i0 > 0) {
-            s.x = s.x - a.mx[i0 - 1];
-            s.y = s.y - a.my[i0 - 1];
-            s.xx = s.xx - a.mxx[i0 - 1];
-            s.xy = s.xy - a.mxy[i0 - 1];
-            s.yy = s.yy - a.myy[i0 - 1];
-            s.w = s.w - a.mw[i0 - 1];
-        }
-    } else {
-        s.x = (a.mx[sz - 1] - a.mx[i0 - 1]) + a.mx[i1];
-        s.y = (a.my[sz - 1] - a.my[i0 - 1]) + a.my[i1];
-        s.xx = (a.mxx[sz - 1] - a.mxx[i0 - 1]) + a.mxx[i1];
-        s.xy = (a.mxy[sz - 1] - a.mxy[i0 - 1]) + a.mxy[i1];
-        s.yy = (a.myy[sz - 1] - a.myy[i0 - 1]) + a.myy[i1];
-        s.w = (a.mw[sz - 1] - a.mw[i0 - 1]) + a.mw[i1];
-    }
-    return s;
+// reference's forms (fast/quads.c:539-569, 658-700, 885-921); `all`: the
+// moments of all points. One path for all cases, as code size is time here.
+__device__ __forceinline__ MSum seg_moments(const Moments &a, const MSum &all, int64_t i0, int64_t i1) {
+    const MSum q = moments_at(a, i1);
+    MSum p = moments_at(a, i0 > 0 ? i0 - 1 : 0);
+    if (i0 <= 0) p = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};  // q - 0 is q
+    if (i0 <= i1) return {q.x - p.x, q.y - p.y, q.xx - p.xx, q.xy - p.xy, q.yy - p.yy, q.w - p.w};
+    return {(all.x - p.x) + q.x,    (all.y - p.y) + q.y,    (all.xx - p.xx) + q.xx,
+            (all.xy - p.xy) + q.xy, (all.yy - p.yy) + q.yy, (all.w - p.w) + q.w};
 }
 
 // The moments of the window of 2 ksz + 1 points centred on i, wrapping
 // around the ends (fast/quads.c:797-808).
-__device__ __forceinline__ MSum window_moments(const Moments &a, int64_t sz, int64_t ksz, int64_t i) {
-    const int64_t i0 = i - ksz, i1 = i + ksz;
-    if (i0 < 0) return seg_moments(a, sz, i0 + sz, i1);
-    if (i1 < sz) return seg_moments(a, sz, i0, i1);
-    return seg_moments(a, sz, i0, i1 - sz);
+template <typename I>
+__device__ __forceinline__ MSum window_moments(const Moments &a, const MSum &all, I sz, I ksz, I i) {
+    const I i0 = i - ksz, i1 = i + ksz;
+    return seg_moments(a, all, i0 < 0 ? i0 + sz : i0, i1 >= sz ? i1 - sz : i1);
 }
 
 // The smoothed error at i (fast/quads.c:809-826): the 7-tap filter over
@@ -872,24 +857,40 @@ __device__ __forceinline__ double smooth_at(const double *e, I n, I i, const dou
     return acc;
 }
 
+// a / b rounded to nearest, from r = 1 / b rounded to nearest (Markstein's
+// division by a fused multiply-add: the second quotient is faithful, the
+// third correct; a, b and the quotient far from the ends of the range, as
+// sums of weights >= 1 and of coordinates in [1/2, 65536) are). Five
+// divisions by one weight take one reciprocal.
+__device__ __forceinline__ double div_by(double a, double b, double r) {
+    double q = __dmul_rn(a, r);
+    q = __fma_rn(__fma_rn(-b, q, a), r, q);
+    return __fma_rn(__fma_rn(-b, q, a), r, q);
+}
+
+// Centroid and covariance of the moments (fast/quads.c:570-600, 604-653).
+struct MCov {
+    double ex, ey, xx, xy, yy;
+};
+__device__ __forceinline__ MCov moments_cov(const MSum &s) {
+    const double r = __drcp_rn(s.w);
+    const double ex = div_by(s.x, s.w, r), ey = div_by(s.y, s.w, r);
+    return {ex, ey, div_by(s.xx, s.w, r) - ex * ex, div_by(s.xy, s.w, r) - ex * ey, div_by(s.yy, s.w, r) - ey * ey};
+}
+
 // The error of a window of nn points (fast/quads.c:604-653).
-__device__ __forceinline__ double window_error(MSum s, double nn) {
-    double ex = s.x / s.w, ey = s.y / s.w;
-    double cxx = s.xx / s.w - ex * ex;
-    double cxy = s.xy / s.w - ex * ey;
-    double cyy = s.yy / s.w - ey * ey;
-    double d = cxx - cyy;
-    double root = (double)__fsqrt_rn((float)(d * d + 4.0 * (cxy * cxy)));
-    return nn * (0.5 * (cxx + cyy - root));
+__device__ __forceinline__ double window_error(const MSum &s, double nn) {
+    const MCov c = moments_cov(s);
+    const double d = c.xx - c.yy;
+    const double root = (double)__fsqrt_rn((float)(d * d + 4.0 * (c.xy * c.xy)));
+    return nn * (0.5 * (c.xx + c.yy - root));
 }
 
 // The line of the moments: centroid, unit normal, smaller eigenvalue
 // (fast/quads.c:570-600, 756-783).
-__device__ __forceinline__ void line_of(MSum s, double lp[4], double *mse) {
-    double ex = s.x / s.w, ey = s.y / s.w;
-    double cxx = s.xx / s.w - ex * ex;
-    double cxy = s.xy / s.w - ex * ey;
-    double cyy = s.yy / s.w - ey * ey;
+__device__ __forceinline__ void line_of(const MSum &s, double lp[4], double *mse) {
+    const MCov c = moments_cov(s);
+    const double ex = c.ex, ey = c.ey, cxx = c.xx, cxy = c.xy, cyy = c.yy;
     double root = (double)__fsqrt_rn((float)((cxx - cyy) * (cxx - cyy) + 4.0 * cxy * cxy));
     double eig_small = 0.5 * (cxx + cyy - root);
     double eig = 0.5 * (cxx + cyy + root);
@@ -1390,6 +1391,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         if (ch > 0) copy_out((ch - 1) * chunk, s_w + ((ch - 1) & 1) * 6 * cs, tid, NT);
         __syncthreads();
         const Moments mo = {M[0], M[1], M[2], M[3], M[4], M[5]};
+        const MSum all = moments_at(mo, sz - 1);
         FIT_PROF(6)
 
         // corner search (fast/quads.c:788-959)
@@ -1401,7 +1403,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // store (a store could alias the next loads)
         for (int64_t i = tid; i < sz; i += 2 * NT) {
             const int64_t i2 = i + NT < sz ? i + NT : i;
-            const MSum sa = window_moments(mo, sz, ksz, i), sb = window_moments(mo, sz, ksz, i2);
+            const MSum sa = window_moments(mo, all, sz, ksz, i), sb = window_moments(mo, all, sz, ksz, i2);
             const double ea = window_error(sa, nn), eb = window_error(sb, nn);
             errs[i] = ea;
             errs[i2] = eb;
@@ -1500,7 +1502,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             bool used = p < q || p >= q + 3;
             if (!used) continue;
             int64_t i0 = mxi[p], i1 = mxi[q];
-            MSum s = seg_moments(mo, sz, i0, i1);
+            MSum s = seg_moments(mo, all, i0, i1);
             double n = (double)(i0 <= i1 ? i1 - i0 + 1 : sz - i0 + i1 + 1);
             double lp[4], mse;
             line_of(s, lp, &mse);
@@ -1569,7 +1571,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             if (be != inf && tid < 4) {
                 double mse;
                 const int ma = bo >> (12 - 4 * tid) & 15, mb = bo >> (12 - 4 * ((tid + 1) & 3)) & 15;
-                line_of(seg_moments(mo, sz, mxi[ma], mxi[mb]), s_lines[tid], &mse);
+                line_of(seg_moments(mo, all, mxi[ma], mxi[mb]), s_lines[tid], &mse);
                 s_lmse[tid] = mse;
             }
             __syncthreads();
@@ -1734,7 +1736,7 @@ __host__ __device__ constexpr size_t fit_warp_x1(int cap, int mm) {
 // gp: the prefix arrays in global scratch (the largest warp class, where
 // 48 B per point of shared memory would leave few warps per SM)
 __host__ __device__ constexpr size_t fit_warp_smem(int cap, int mm, bool gp = false) {
-    return (size_t)(gp ? 8 : 56) * cap + fit_warp_x1(cap, mm);
+    return (size_t)8 * cap + (gp ? 0 : 48 * (cap + 1)) + fit_warp_x1(cap, mm);
 }
 
 
@@ -1822,12 +1824,13 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
     kernel_begin();
     constexpr int CAP = 32 * R;
     constexpr bool GP = R >= 16;  // prefix arrays in global scratch
+    constexpr int RS = CAP + 1;   // row stride of the prefix arrays (six rows on distinct banks)
     extern __shared__ __align__(16) unsigned char fw_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
     unsigned char *base = fw_smem + fit_warp_smem(CAP, mm, GP) * wid;
-    double *pm = reinterpret_cast<double *>(base);  // prefix array q at pm + q * CAP (not GP)
-    unsigned char *x0 = base + (GP ? 0 : 48 * CAP), *x1 = x0 + 8 * CAP;
+    double *pm = reinterpret_cast<double *>(base);  // prefix array q at pm + q * RS (not GP)
+    unsigned char *x0 = base + (GP ? 0 : 48 * RS), *x1 = x0 + 8 * CAP;
     uint64_t *s_akey = reinterpret_cast<uint64_t *>(x0);
     double *s_err = reinterpret_cast<double *>(x0);
     double *s_mxe = reinterpret_cast<double *>(x0);
@@ -1928,7 +1931,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             // packs the slope bits of its block head, 0xffff - the head's index,
             // t, and (below the order, since the rest is distinct) the index of
             // its point. The keys live in the last prefix array until the moments.
-            uint64_t *s_skey = reinterpret_cast<uint64_t *>(pm + 5 * CAP);
+            uint64_t *s_skey = reinterpret_cast<uint64_t *>(pm + 5 * RS);
             int np = 32;
             while (np < n) np <<= 1;
             for (int i = lane; i < np; i += 32) {
@@ -2017,64 +2020,84 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         FITW_PROF(5)
 
         // cumulative weighted moments in angle order (fast/quads.c:968-1035):
-        // every lane stages the six terms of its positions, then lane q < 6
-        // turns array q into its prefix sums in place
-        double *M0 = GP ? scr.mx + s0 : pm, *M1 = GP ? scr.my + s0 : pm + CAP, *M2 = GP ? scr.mxx + s0 : pm + 2 * CAP,
-               *M3 = GP ? scr.mxy + s0 : pm + 3 * CAP, *M4 = GP ? scr.myy + s0 : pm + 4 * CAP,
-               *M5 = GP ? scr.mw + s0 : pm + 5 * CAP;
+        // the six terms of each position (moment_terms), then lane q < 6
+        // turns row q into its prefix sums
+        double *M0 = GP ? scr.mx + s0 : pm, *M1 = GP ? scr.my + s0 : pm + RS, *M2 = GP ? scr.mxx + s0 : pm + 2 * RS,
+               *M3 = GP ? scr.mxy + s0 : pm + 3 * RS, *M4 = GP ? scr.myy + s0 : pm + 4 * RS,
+               *M5 = GP ? scr.mw + s0 : pm + 5 * RS;
         const uint8_t *im = qim + f.q_off;
-        for (int k = lane; k < n; k += 32) {
-            uint32_t src;
-            if constexpr (R <= 8)
-                src = (uint32_t)(reinterpret_cast<const uint64_t *>(pm + 5 * CAP)[k] & 0x1fffu);
-            else
-                src = s_order[k];
-            const uint64_t p = P[src];
-            const int32_t px = (int32_t)(p & 0xffff), py = (int32_t)(p >> 16 & 0xffff);
-            const int32_t ix = (px >> 1) + (px & 1), iy = (py >> 1) + (py & 1);
-            int32_t g2 = 0;
-            if (ix > 0 && ix + 1 < f.qw && iy > 0 && iy + 1 < f.qh) {
-                const int64_t cc = (int64_t)iy * f.qw + ix;
-                const int32_t gx = (int32_t)im[cc + 1] - im[cc - 1];
-                const int32_t gy = (int32_t)im[cc + f.qw] - im[cc - f.qw];
-                g2 = gx * gx + gy * gy;
-            }
-            const double w = __dadd_rn(__dsqrt_rn((double)g2), 1.0);
-            const double fx = __dadd_rn(__dmul_rn((double)px, 0.5), 0.5);
-            const double fy = __dadd_rn(__dmul_rn((double)py, 0.5), 0.5);
-            const double wx = __dmul_rn(w, fx), wy = __dmul_rn(w, fy);
-            M0[k] = wx;
-            M1[k] = wy;
-            M2[k] = __dmul_rn(wx, fx);
-            M3[k] = __dmul_rn(wx, fy);
-            M4[k] = __dmul_rn(wy, fy);
-            M5[k] = w;
-        }
-        __syncwarp();
-        if (lane < 6) {
-            double *o = lane == 0 ? M0 : lane == 1 ? M1 : lane == 2 ? M2 : lane == 3 ? M3 : lane == 4 ? M4 : M5;
+        if constexpr (GP) {
+            // the prefix arrays are in global memory: chunks of 64 points in
+            // shared memory (x0), two a lane; a chunk's gathers are under way
+            // while the chain of the one before runs (point values two chunks
+            // ahead, pixels one). With the terms and the chain in global
+            // memory the moments took 77k cycles for 360 points.
+            double *buf = reinterpret_cast<double *>(x0);
+            constexpr int BS = 66;  // row stride: the six rows on distinct banks
+            static_assert(6 * BS <= CAP, "the chunk's terms fit x0");
+            auto point = [&](int k) { return k < n ? P[s_order[k]] : 0ull; };
+            uint64_t pa = point(lane), pb = point(32 + lane), na = point(64 + lane), nb2 = point(96 + lane);
+            int32_t ga = point_grad2(im, f.qw, f.qh, pa), gb = point_grad2(im, f.qw, f.qh, pb);
             double run = 0.0;
-            int t = 0;
-            for (; t + 16 <= n; t += 16) {
-                double v[16];
+            for (int k0 = 0; k0 < n; k0 += 64) {
+                double m[6];
+                moment_terms(pa, ga, m);
 #pragma unroll
-                for (int u = 0; u < 16; u++) v[u] = o[t + u];
+                for (int q = 0; q < 6; q++) buf[q * BS + lane] = m[q];
+                moment_terms(pb, gb, m);
 #pragma unroll
-                for (int u = 0; u < 16; u++) {
-                    run = __dadd_rn(run, v[u]);
-                    v[u] = run;
-                }
+                for (int q = 0; q < 6; q++) buf[q * BS + 32 + lane] = m[q];
+                pa = na;
+                pb = nb2;
+                na = point(k0 + 128 + lane);
+                nb2 = point(k0 + 160 + lane);
+                ga = point_grad2(im, f.qw, f.qh, pa);
+                gb = point_grad2(im, f.qw, f.qh, pb);
+                __syncwarp();
+                if (lane < 6) prefix_chain(buf + lane * BS, min(64, n - k0), run);
+                __syncwarp();
+                double *out[6] = {M0, M1, M2, M3, M4, M5};
 #pragma unroll
-                for (int u = 0; u < 16; u++) o[t + u] = v[u];
+                for (int h = 0; h < 64; h += 32)
+                    if (k0 + h + lane < n) {
+#pragma unroll
+                        for (int q = 0; q < 6; q++) out[q][k0 + h + lane] = buf[q * BS + h + lane];
+                    }
+                __syncwarp();
             }
-            for (; t < n; t++) {
-                run = __dadd_rn(run, o[t]);
-                o[t] = run;
+        } else {
+            for (int k = lane; k < n; k += 64) {
+                const int k2 = k + 32 < n ? k + 32 : k;
+                uint32_t src, src2;
+                if constexpr (R <= 8) {
+                    const uint64_t *key = reinterpret_cast<const uint64_t *>(M5);
+                    src = (uint32_t)(key[k] & 0x1fffu);
+                    src2 = (uint32_t)(key[k2] & 0x1fffu);
+                } else {
+                    src = s_order[k];
+                    src2 = s_order[k2];
+                }
+                const uint64_t p1 = P[src], p2 = P[src2];
+                const int32_t g1 = point_grad2(im, f.qw, f.qh, p1), g2 = point_grad2(im, f.qw, f.qh, p2);
+                double m1[6], m2[6];
+                moment_terms(p1, g1, m1);
+                moment_terms(p2, g2, m2);
+#pragma unroll
+                for (int q = 0; q < 6; q++) {
+                    pm[q * RS + k] = m1[q];
+                    pm[q * RS + k2] = m2[q];
+                }
+            }
+            __syncwarp();
+            if (lane < 6) {
+                double run = 0.0;
+                prefix_chain(pm + lane * RS, n, run);
             }
         }
         __syncwarp();
         FITW_PROF(6)
         const Moments mo = {M0, M1, M2, M3, M4, M5};
+        const MSum all = moments_at(mo, n - 1);
 
         // corner search (fast/quads.c:788-959)
         const int ksz = min(20, n / 12);
@@ -2082,7 +2105,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         const double nn = (double)(2 * ksz + 1);
         for (int i = lane; i < n; i += 64) {
             const int i2 = i + 32 < n ? i + 32 : i;
-            const MSum sa = window_moments(mo, n, ksz, i), sb = window_moments(mo, n, ksz, i2);
+            const MSum sa = window_moments(mo, all, n, ksz, i), sb = window_moments(mo, all, n, ksz, i2);
             const double ea = window_error(sa, nn), eb = window_error(sb, nn);
             s_err[i] = ea;
             s_err[i2] = eb;
@@ -2145,7 +2168,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             const int p = t / nm, q = t - p * nm;
             if (!(p < q || p >= q + 3)) continue;
             const int i0 = s_mxi[p], i1 = s_mxi[q];
-            const MSum s = seg_moments(mo, n, i0, i1);
+            const MSum s = seg_moments(mo, all, i0, i1);
             const double cnt = (double)(i0 <= i1 ? i1 - i0 + 1 : n - i0 + i1 + 1);
             double lp[4], mse;
             line_of(s, lp, &mse);
@@ -2193,7 +2216,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         double ln[4] = {0.0, 0.0, 0.0, 0.0}, lmse = 0.0;
         if (lane < 4) {
             const int ma = bo >> (12 - 4 * lane) & 15, mb = bo >> (12 - 4 * ((lane + 1) & 3)) & 15;
-            line_of(seg_moments(mo, n, s_mxi[ma], s_mxi[mb]), ln, &lmse);
+            line_of(seg_moments(mo, all, s_mxi[ma], s_mxi[mb]), ln, &lmse);
         }
         double lines[4][4], lm[4];
 #pragma unroll
