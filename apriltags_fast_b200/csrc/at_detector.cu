@@ -683,8 +683,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_QOK].ensure(ncl * 4));
         CK(B[B_QSCAN].ensure((ncl + 1) * 4));
         CK(B[B_QSCR].ensure(scan_u32_scratch(ncl) * 4));
-        CK(B[B_FLIST].ensure(ncl * 4 * 6));
-        CK(B[B_FCNT].ensure(64));
+        CK(B[B_FLIST].ensure(ncl * 4 * FIT_NBUCKET));
+        CK(B[B_FCNT].ensure(2 * FIT_NBUCKET * 4));
         FitScratch scr{B[B_SKEYS].as<uint64_t>(), B[B_SSKEY].as<uint64_t>(), B[B_SSVAL].as<uint32_t>(),
                        B[B_SW].as<double>(),      B[B_SFX].as<double>(),    B[B_SFY].as<double>(),
                        B[B_SMX].as<double>(),     B[B_SMY].as<double>(),    B[B_SMXX].as<double>(),
@@ -876,7 +876,11 @@ at_detector *at_detector_create(void) {
         abort();
     }
     for (int k = 0; k < 12; k++) cudaEventCreate(&in->ev[k]);
-    for (cudaStream_t &q : in->fit.side) cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking);
+    // the fit's streams: larger clusters first (launch_fit_quads)
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    const int prio[4] = {std::max(greatest, least - 2), std::max(greatest, least - 1), least, greatest};
+    for (int k = 0; k < 4; k++) cudaStreamCreateWithPriority(&in->fit.side[k], cudaStreamNonBlocking, prio[k]);
     cudaEventCreateWithFlags(&in->fit.fork, cudaEventDisableTiming);
     for (cudaEvent_t &e : in->fit.join) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     return td;

@@ -1098,6 +1098,60 @@ extern "C" int at_fit_prof_copy(void *dst, int n) {
 #define DEC_PROF(k)
 #endif
 
+// ---------------------------------------------------------------------------
+// The fit's size classes: clusters of at most 128, 256, 512 points (a warp
+// each), at most 1024 (a block of 128), at most 6144 (a block of 256), and
+// larger (a block of 512). A class's clusters are listed by size in a few
+// buckets, and its blocks take those of the largest bucket first, so that a
+// long cluster does not start last (unsorted, the 513-1024 class took 175
+// instead of 159 us; sorting the lists took a kernel of 27 us before each
+// block class). Clusters outside [min_cluster_pixels, max_px] of their frame
+// get no list (fast/quads.c:1180-1190). Every cluster's quad flag starts at 0.
+__device__ __forceinline__ int fit_bucket(int64_t sz) {
+    if (sz <= 512) return sz <= 128 ? 0 : sz <= 256 ? 1 : 2;
+    if (sz <= FIT_SMALL) return sz <= 640 ? 3 : sz <= 768 ? 4 : sz <= 896 ? 5 : 6;
+    if (sz <= FIT_LARGE_SORT) return sz <= 1536 ? 7 : sz <= 2048 ? 8 : sz <= 3072 ? 9 : sz <= 4096 ? 10 : 11;
+    return sz <= 9216 ? 12 : sz <= FIT_HUGE_SORT ? 13 : sz <= 20480 ? 14 : 15;
+}
+
+// The next cluster of buckets top .. bottom (0xffffffff: none left): counts
+// holds each bucket's length, then per bucket (used at `top`) the clusters
+// taken.
+__device__ __forceinline__ uint32_t fit_next(const FitScratch &scr, int64_t nclusters, int top, int bottom) {
+    uint32_t i = atomicAdd(scr.counts + FIT_NBUCKET + top, 1u);
+    for (int q = top; q >= bottom; q--) {
+        const uint32_t n = scr.counts[q];
+        if (i < n) return scr.lists[(int64_t)q * nclusters + i];
+        i -= n;
+    }
+    return 0xffffffffu;
+}
+
+__global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, const int32_t *cframe,
+                               int64_t nclusters, int64_t npoints, int32_t min_px, uint32_t *quad_ok,
+                               uint32_t *lists, uint32_t *counts) {
+    kernel_begin();
+    const int lane = threadIdx.x & 31;
+    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nclusters; c0 += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t c = c0 + threadIdx.x;
+        int k = -1;
+        if (c < nclusters) {
+            quad_ok[c] = 0;
+            const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - cstart[c];
+            if (sz >= min_px && sz <= frames[cframe[c]].max_px) k = fit_bucket(sz);
+        }
+        // (a frame's clusters are few sizes apart: a turn per bucket met)
+        for (uint32_t met = __reduce_or_sync(0xffffffffu, k < 0 ? 0u : 1u << k); met; met &= met - 1) {
+            const int q = __ffs(met) - 1;
+            const uint32_t bal = __ballot_sync(0xffffffffu, k == q);
+            uint32_t at = 0;
+            if (lane == __ffs(bal) - 1) at = atomicAdd(counts + q, (uint32_t)__popc(bal));
+            at = __shfl_sync(0xffffffffu, at, __ffs(bal) - 1);
+            if (k == q) lists[(int64_t)q * nclusters + at + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)c;
+        }
+    }
+}
+
 // The 4-subsets {m0 < m1 < m2 < m3} of {0..15} in colex order (by m3, then
 // m2, m1, m0), one per entry as nibbles m0 | m1 << 4 | m2 << 8 | m3 << 12:
 // the first C(n, 4) entries are the 4-subsets of {0..n-1}.
@@ -1123,8 +1177,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
                                                    const uint64_t *pts, const uint32_t *cstart,
                                                    const int32_t *cframe, int64_t nclusters, int64_t npoints,
                                                    FitScratch scr, GpuQuad *quads, uint32_t *quad_ok, uint32_t *err,
-                                                   const uint32_t *list, const uint32_t *count, uint32_t *next,
-                                                   int sort_cap, int chunk) {
+                                                   int top, int bottom, int sort_cap, int chunk) {
     kernel_begin();
     extern __shared__ __align__(16) unsigned char fit_smem[];
     const size_t xb = fit_x_bytes(sort_cap, chunk);
@@ -1146,15 +1199,14 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
     __shared__ uint32_t s_next;
     __shared__ double s_cand[(NT / 32) * (AT_MAX_NMAXIMA + 1)];
     const int tid = threadIdx.x;
-    const uint32_t ncl = *count;
 
-    // the class's clusters, largest first, each to the next free block
+    // the class's clusters, its largest sizes first, each to the next free block
     for (;;) {
         __syncthreads();
-        if (tid == 0) s_next = atomicAdd(next, 1u);
+        if (tid == 0) s_next = fit_next(scr, nclusters, top, bottom);
         __syncthreads();
-        if (s_next >= ncl) break;
-        const int64_t c = list[s_next];
+        if (s_next == 0xffffffffu) break;
+        const int64_t c = s_next;
         const int64_t s0 = cstart[c];
         const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - s0;
         const FrameDesc f = frames[cframe[c]];
@@ -1647,82 +1699,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
 }
 
 // ---------------------------------------------------------------------------
-// The fit's size classes: clusters of at most 128, 256, 512 points (a warp
-// each), at most 1024 (a block of 128), at most 6144 (a block of 256), and
-// larger (a block of 512). Each
-// class gets a list of its clusters; clusters outside [min_cluster_pixels,
-// max_px] of their frame get none (fast/quads.c:1180-1190). Every cluster's
-// quad flag starts at 0.
-#define FIT_NCLASS 6
-__device__ __forceinline__ int fit_class(int64_t sz) {
-    return sz <= 128 ? 0 : sz <= 256 ? 1 : sz <= 512 ? 2 : sz <= FIT_SMALL ? 3 : sz <= FIT_LARGE_SORT ? 4 : 5;
-}
-
-__global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, const int32_t *cframe,
-                               int64_t nclusters, int64_t npoints, int32_t min_px, uint32_t *quad_ok,
-                               uint32_t *lists, uint32_t *counts) {
-    kernel_begin();
-    const int lane = threadIdx.x & 31;
-    for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nclusters; c0 += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t c = c0 + threadIdx.x;
-        int k = -1;
-        if (c < nclusters) {
-            quad_ok[c] = 0;
-            const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - cstart[c];
-            if (sz >= min_px && sz <= frames[cframe[c]].max_px) k = fit_class(sz);
-        }
-#pragma unroll
-        for (int q = 0; q < FIT_NCLASS; q++) {
-            const uint32_t bal = __ballot_sync(0xffffffffu, k == q);
-            if (!bal) continue;
-            uint32_t at = 0;
-            if (lane == __ffs(bal) - 1) at = atomicAdd(counts + q, (uint32_t)__popc(bal));
-            at = __shfl_sync(0xffffffffu, at, __ffs(bal) - 1);
-            if (k == q) lists[(int64_t)q * nclusters + at + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)c;
-        }
-    }
-}
-
-// One block per list: the list by size, largest first (then by cluster),
-// when it has at most FIT_ORDER_CAP clusters; a bitonic sort in shared
-// memory.
-#define FIT_ORDER_CAP 8192
-__global__ void __launch_bounds__(1024) k_fit_order(const uint32_t *cstart, int64_t nclusters, int64_t npoints,
-                                                   uint32_t *lists, const uint32_t *counts, int first_class) {
-    kernel_begin();
-    extern __shared__ __align__(16) uint64_t s_ord[];
-    const int q = first_class + blockIdx.x;
-    const uint32_t n = counts[q];
-    if (n < 2 || n > FIT_ORDER_CAP) return;
-    uint32_t *list = lists + (int64_t)q * nclusters;
-    uint32_t np = 2;
-    while (np < n) np <<= 1;
-    for (uint32_t i = threadIdx.x; i < np; i += blockDim.x) {
-        uint64_t key = ~0ull;
-        if (i < n) {
-            const uint32_t c = list[i];
-            const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - cstart[c];
-            key = (uint64_t)(0xffffffffu - (uint32_t)sz) << 32 | c;
-        }
-        s_ord[i] = key;
-    }
-    __syncthreads();
-    for (uint32_t kk = 2; kk <= np; kk <<= 1)
-        for (uint32_t j = kk >> 1; j > 0; j >>= 1) {
-            for (uint32_t t = threadIdx.x; t < np / 2; t += blockDim.x) {
-                const uint32_t i = ((t & ~(j - 1)) << 1) | (t & (j - 1)), l = i + j;
-                const uint64_t a = s_ord[i], b = s_ord[l];
-                if (((i & kk) == 0) == (a > b)) {
-                    s_ord[i] = b;
-                    s_ord[l] = a;
-                }
-            }
-            __syncthreads();
-        }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) list[i] = (uint32_t)s_ord[i];
-}
-
-// ---------------------------------------------------------------------------
 // Clusters of at most 32 * R points: one warp each, FIT_WPB per block, no
 // block barriers. The same steps as k_fit_quads; the angle sort is a bitonic
 // sort in registers, the prefix moments stay in shared memory.
@@ -1818,8 +1794,7 @@ template <int R>
 __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *frames, GpuParams prm, const uint8_t *qim,
                                                           const uint64_t *pts, const uint32_t *cstart,
                                                           const int32_t *cframe, int64_t nclusters, int64_t npoints,
-                                                          const uint32_t *list, const uint32_t *count,
-                                                          uint32_t *next, GpuQuad *quads, uint32_t *quad_ok, int mm,
+                                                          int top, GpuQuad *quads, uint32_t *quad_ok, int mm,
                                                           FitScratch scr) {
     kernel_begin();
     constexpr int CAP = 32 * R;
@@ -1843,13 +1818,12 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
 
     // one resident wave of warps, each taking the class's next cluster
     // from a shared counter as it finishes one (no static share to wait on)
-    const uint32_t ncl = *count;
     for (;;) {
         uint32_t li = 0;
-        if (lane == 0) li = atomicAdd(next, 1u);
+        if (lane == 0) li = fit_next(scr, nclusters, top, top);
         li = __shfl_sync(FULL, li, 0);
-        if (li >= ncl) break;
-        const int64_t c = list[li];
+        if (li == 0xffffffffu) break;
+        const int64_t c = li;
         const int64_t s0 = cstart[c];
         const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - s0;
         const FrameDesc f = frames[cframe[c]];
@@ -3391,9 +3365,8 @@ static void launch_fit_warp(cudaStream_t s, const FrameDesc *frames, const GpuPa
         per_sm = 1;
     const int64_t full = 148 * (int64_t)per_sm;
     const int64_t wb = (nclusters + FIT_WPB - 1) / FIT_WPB;
-    launch(k_fit_warp<R>, (unsigned)(wb < full ? wb : full), FIT_WPB * 32, wsm, s, 
-        frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr.lists + (int64_t)q * nclusters,
-        scr.counts + q, scr.counts + FIT_NCLASS + q, quads, quad_ok, mm, scr);
+    launch(k_fit_warp<R>, (unsigned)(wb < full ? wb : full), FIT_WPB * 32, wsm, s, frames, prm, qim, pts, cstart,
+           cframe, nclusters, npoints, q, quads, quad_ok, mm, scr);
 }
 
 int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frames, const GpuParams &prm,
@@ -3405,45 +3378,37 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
                  large = fit_smem_bytes(FIT_LARGE_SORT, FIT_CHUNK_LARGE, FIT_LARGE_NT / 32);
     cudaFuncSetAttribute(k_fit_quads<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)small);
     cudaFuncSetAttribute(k_fit_quads<FIT_LARGE_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)large);
-    cudaFuncSetAttribute(k_fit_order, cudaFuncAttributeMaxDynamicSharedMemorySize, FIT_ORDER_CAP * 8);
     const int mm = prm.max_nmaxima > 4 ? prm.max_nmaxima : 4;
-    // the size classes' lists, the two block classes' largest first
-    cudaMemsetAsync(scr.counts, 0, 2 * FIT_NCLASS * sizeof(uint32_t), s);
+    cudaMemsetAsync(scr.counts, 0, 2 * FIT_NBUCKET * sizeof(uint32_t), s);
     launch(k_fit_classify, flat_blocks(nclusters, 256), 256, 0, s, frames, cstart, cframe, nclusters, npoints,
                                                                 prm.min_cluster_pixels, quad_ok, scr.lists,
                                                                 scr.counts);
     // five streams, one per group of classes: above 6144 points (a block of
     // FIT_HUGE_NT each; only when a frame allows such clusters at all); the
-    // other large clusters (a block of FIT_LARGE_NT each, two an SM);
-    // 513-1024 points (a block of 128); 257-512 (a warp each); up to 256 (a
-    // warp each). Only the block classes are put largest first, each on its
-    // own stream, so the warp classes start at once (unsorted, the 513-1024
-    // class measured slower: 175 vs 159 us, a long cluster last).
+    // other large clusters (a block of FIT_LARGE_NT each, two an SM: one
+    // cluster's serial steps overlap the other's); 513-1024 points (a block of
+    // 128); 257-512 (a warp each); up to 256 (a warp each). The streams of the
+    // larger clusters have the higher priorities, so that their few long
+    // blocks start before the warp classes' resident waves fill the SMs (165
+    // instead of 173 us for eight 1280 x 720 frames; no difference for 32
+    // frames of 1920 x 1080).
     const bool huge = max_px > FIT_LARGE_SORT;
-    auto list = [&](int q) { return scr.lists + q * nclusters; };
     cudaEventRecord(S.fork, s);
     for (int k = 0; k < (huge ? 4 : 3); k++) cudaStreamWaitEvent(S.side[k], S.fork, 0);
     if (huge) {
         const size_t hsm = fit_smem_bytes(FIT_HUGE_SORT, FIT_CHUNK_LARGE, FIT_HUGE_NT / 32);
         cudaFuncSetAttribute(k_fit_quads<FIT_HUGE_NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm);
-        launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[3], cstart, nclusters, npoints, scr.lists, scr.counts, 5);
-        launch(k_fit_quads<FIT_HUGE_NT>, (unsigned)(nclusters < 148 ? nclusters : 148), FIT_HUGE_NT, hsm, S.side[3], 
-            frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(5),
-            scr.counts + 5, scr.counts + FIT_NCLASS + 5, FIT_HUGE_SORT, FIT_CHUNK_LARGE);
+        launch(k_fit_quads<FIT_HUGE_NT>, (unsigned)(nclusters < 148 ? nclusters : 148), FIT_HUGE_NT, hsm, S.side[3],
+               frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, 15, 12,
+               FIT_HUGE_SORT, FIT_CHUNK_LARGE);
         cudaEventRecord(S.join[3], S.side[3]);
     }
-    launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[0], cstart, nclusters, npoints, scr.lists, scr.counts, 4);
-    launch(k_fit_order, 1, 1024, FIT_ORDER_CAP * 8, S.side[1], cstart, nclusters, npoints, scr.lists, scr.counts, 3);
-    // two blocks an SM: one cluster's serial steps overlap the other's
-    const unsigned nbig = (unsigned)(nclusters < 2 * 148 ? nclusters : 2 * 148);
-    launch(k_fit_quads<FIT_LARGE_NT>, nbig, FIT_LARGE_NT, large, S.side[0], 
-        frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, list(4), scr.counts + 4,
-        scr.counts + FIT_NCLASS + 4, FIT_LARGE_SORT, FIT_CHUNK_LARGE);
+    launch(k_fit_quads<FIT_LARGE_NT>, (unsigned)(nclusters < 2 * 148 ? nclusters : 2 * 148), FIT_LARGE_NT, large,
+           S.side[0], frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, 11, 7,
+           FIT_LARGE_SORT, FIT_CHUNK_LARGE);
     cudaEventRecord(S.join[0], S.side[0]);
-    const unsigned mid = (unsigned)(nclusters < 148 * 4 ? nclusters : 148 * 4);
-    launch(k_fit_quads<128>, mid, 128, small, S.side[1], frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr,
-                                                     quads, quad_ok, err, list(3), scr.counts + 3,
-                                                     scr.counts + FIT_NCLASS + 3, FIT_SMALL, FIT_CHUNK_SMALL);
+    launch(k_fit_quads<128>, (unsigned)(nclusters < 148 * 4 ? nclusters : 148 * 4), 128, small, S.side[1], frames, prm,
+           qim, pts, cstart, cframe, nclusters, npoints, scr, quads, quad_ok, err, 6, 3, FIT_SMALL, FIT_CHUNK_SMALL);
     cudaEventRecord(S.join[1], S.side[1]);
     launch_fit_warp<16>(S.side[2], frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 2, quads, quad_ok,
                         mm);
@@ -3451,7 +3416,7 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
     launch_fit_warp<4>(s, frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 0, quads, quad_ok, mm);
     launch_fit_warp<8>(s, frames, prm, qim, pts, cstart, cframe, nclusters, npoints, scr, 1, quads, quad_ok, mm);
     for (int k = 0; k < (huge ? 4 : 3); k++) cudaStreamWaitEvent(s, S.join[k], 0);
-    return huge ? 10 : 8;
+    return huge ? 7 : 6;
 }
 
 void launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,

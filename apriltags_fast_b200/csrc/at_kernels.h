@@ -13,6 +13,7 @@ struct RunArrays {
     uint32_t *lab;     // each node's label, or AT_NOK
 };
 
+#define FIT_NBUCKET 16
 // Per-point scratch of the quad fit, indexed by point position.
 struct FitScratch {
     uint64_t *keys, *skey;
@@ -21,8 +22,8 @@ struct FitScratch {
     double *mx, *my, *mxx, *mxy, *myy, *mw;
     double *errs, *filt, *mxe;
     int32_t *mxi;
-    uint32_t *lists;   // one list of cluster ids per size class, nclusters apart
-    uint32_t *counts;  // per class: list length, then the next list index to take
+    uint32_t *lists;   // one list of cluster ids per size bucket, nclusters apart
+    uint32_t *counts;  // per bucket: list length, then the clusters taken
 };
 
 struct BlurTaps {
