@@ -77,11 +77,28 @@ constexpr int JMAX_RUNS = 48;
 
 // One Huffman table: runs of equal-length codes over the 16-bit code
 // space, in order (run r ends at rend[r]; position w of it decodes as
-// symbol pool[rsym[r] + ((w - rorigin[r]) >> (16 - rlen[r]))]), and a
-// lookup of the codes of up to 9 bits by the window's first 9 bits.
+// symbol pool[rsym[r] + ((w - rorigin[r]) >> (16 - rlen[r]))]), and what
+// the next 9 bits of the stream decode as (lut): a symbol entry (JENT_*),
+// or JENT_SUB | the place in the job's lut2 of the 128 entries of the next 7
+// bits, or 0 (the runs tell; only in tables with more than JMAX_SUB such
+// prefixes). An entry holds all that a decode step needs, so that the lanes
+// of a warp, each at its own place in the stream, follow one path whatever
+// their codes: with 9-bit entries of (length, symbol) and the runs searched
+// for longer codes, some lane searched in nearly every step.
+constexpr uint32_t JENT_SUB = 0x80000000u;
+constexpr uint32_t JENT_OK = 1u << 22;  // always set in a symbol entry
+__host__ __device__ __forceinline__ uint32_t jent(int len, int sym, bool ac) {
+    const uint32_t sz = sym & 15, dz = !ac ? 1 : sym == 0 ? 64 : (sym >> 4) + 1;
+    return JENT_OK | (len + sz) | (uint32_t)len << 6 | sz << 11 | dz << 15;
+}
+__host__ __device__ __forceinline__ int jent_bits(uint32_t e) { return e & 63; }          // code and value bits
+__host__ __device__ __forceinline__ int jent_len(uint32_t e) { return (e >> 6) & 31; }    // code bits (0: no code)
+__host__ __device__ __forceinline__ int jent_size(uint32_t e) { return (e >> 11) & 15; }  // value bits
+__host__ __device__ __forceinline__ int jent_step(uint32_t e) { return (e >> 15) & 127; } // coefficients passed (64: rest of the block)
+constexpr int JMAX_SUB = 64;
 struct JTab {
-    uint16_t lut[512];    // (bits << 8) | symbol, 0 if the prefix needs the runs
-    uint32_t nrun, r0;    // runs; the first run a lookup miss can land in
+    uint32_t lut[512];
+    uint32_t nrun, r0, ac;  // runs; the first run a lookup miss can land in; whether AC codes
     uint32_t rend[JMAX_RUNS], rorigin[JMAX_RUNS], rsym[JMAX_RUNS];
     uint8_t rlen[JMAX_RUNS];
 };
@@ -121,6 +138,7 @@ struct JPlaneDev {
 struct JJob {
     const uint32_t *stream;      // big-endian bit stream, word aligned
     const JTab *tabs;
+    const uint32_t *lut2;
     const uint8_t *syms;
     const JScanDev *scans;
     const JSegDev *segs;
@@ -193,27 +211,23 @@ struct JReader {
     }
 };
 
-// One code of table t at the window `win` (the next 32 bits): its length
-// in bits (0 when nothing matches) and symbol.
-__host__ __device__ __forceinline__ int jdecode(const JTab *__restrict__ t, const uint8_t *__restrict__ syms, uint32_t win,
-                                       int &sym) {
+// The entry of the code at the window `win` (the next 32 bits) in table t;
+// no code: length 0, symbol 0.
+__host__ __device__ __forceinline__ uint32_t jdecode(const JJob &J, const JTab *__restrict__ t, uint32_t win) {
     const uint32_t e = JLDG(&t->lut[win >> 23]);
-    if (e) {
-        sym = e & 255;
-        return (int)(e >> 8);
-    }
+    if (e & JENT_OK) return e;
     const uint32_t w16 = win >> 16;
+    if (e) return JLDG(&J.lut2[(e & ~JENT_SUB) + (w16 & 127)]);
     const uint32_t nr = JLDG(&t->nrun);
 #pragma unroll 1
     for (uint32_t r = JLDG(&t->r0); r < nr; r++) {
         if (w16 < JLDG(&t->rend[r])) {
             const int l = JLDG(&t->rlen[r]);
-            sym = JLDG(&syms[JLDG(&t->rsym[r]) + ((w16 - JLDG(&t->rorigin[r])) >> (16 - l))]);
-            return l;
+            return jent(l, JLDG(&J.syms[JLDG(&t->rsym[r]) + ((w16 - JLDG(&t->rorigin[r])) >> (16 - l))]),
+                        JLDG(&t->ac) != 0);
         }
     }
-    sym = 0;
-    return 0;
+    return jent(0, 0, JLDG(&t->ac) != 0);
 }
 
 __host__ __device__ __forceinline__ int32_t jextend(uint32_t v, int s) {
@@ -273,10 +287,8 @@ __host__ __device__ unsigned long long jrun_sync(const JJob &J, const JScanDev &
             break;
         }
         const uint32_t win = R.peek(s.p);
-        int sym;
-        const int nb = jdecode(s.z == 0 ? s.dc : s.ac, J.syms, win, sym);
-        const int sz = sym & 15;
-        if (nb == 0) {
+        const uint32_t e = jdecode(J, s.z == 0 ? s.dc : s.ac, win);
+        if (jent_len(e) == 0) {
             if (++stall > stall_max) {
                 out = jpack(JSTUCK, 0, 0);
                 if (!counting) *entry = out;
@@ -285,19 +297,15 @@ __host__ __device__ unsigned long long jrun_sync(const JJob &J, const JScanDev &
         } else {
             stall = 0;
         }
-        if (s.z == 0) {
-            const uint32_t v = sz ? (win << nb) >> (32 - sz) : 0;
-            const uint32_t d = counting ? (uint32_t)jextend(v, sz) : 0u;
+        if (s.z == 0 && counting) {
+            const int sz = jent_size(e);
+            const uint32_t d = (uint32_t)jextend(sz ? (win << jent_len(e)) >> (32 - sz) : 0, sz);
             if (s.comp == 0) dc0 += d;
             else if (s.comp == 1) dc1 += d;
             else dc2 += d;
-            s.z = 1;
-        } else if (sym == 0) {
-            s.z = 64;
-        } else {
-            s.z += (sym >> 4) + 1;
         }
-        s.p += nb + sz;
+        s.z += jent_step(e);
+        s.p += jent_bits(e);
         if (s.z >= 64) {
             s.z = 0;
             if (++s.b == (int)S.bpm) s.b = 0;
@@ -507,28 +515,20 @@ __constant__ uint8_t c_zig[64] = {0,  1,  8,  16, 9,  2,  3,  10, 17, 24, 32, 25
 // it; rotation constants 2048 * sqrt(2) * cos(k * pi / 16).
 constexpr int JC1 = 2841, JC2 = 2676, JC3 = 2408, JC5 = 1609, JC6 = 1108, JC7 = 565;
 
-// One 8-point pass over v[0], v[st], ..., v[7 st] (shared memory). Row
-// pass: in place, DC << 11 with bias 128, results >> 8. Column pass: DC
-// << 8 with bias 8192, rotations rounded (+4) >> 3, results >> 14 + 128,
-// clamped to bytes in pix[0..7]; the column is left zeroed.
+// One 8-point pass over v[0 .. 7]. Row pass: DC << 11 with bias 128,
+// results >> 8, in v. Column pass: DC << 8 with bias 8192, rotations
+// rounded (+4) >> 3, results >> 14 + 128, clamped to bytes, in v.
 template <bool COL>
-__host__ __device__ __forceinline__ void jidct_pass(int32_t *v, int st, uint8_t *pix) {
+__host__ __device__ __forceinline__ void jidct_pass(int32_t v[8]) {
     constexpr int sh = COL ? 8 : 11;
-    const int32_t x1 = (int32_t)((uint32_t)v[4 * st] << sh);
-    const int32_t a2 = v[6 * st], a3 = v[2 * st], a4 = v[1 * st], a5 = v[7 * st], a6 = v[5 * st],
-                  a7 = v[3 * st];
+    const int32_t x1 = (int32_t)((uint32_t)v[4] << sh);
+    const int32_t a2 = v[6], a3 = v[2], a4 = v[1], a5 = v[7], a6 = v[5], a7 = v[3];
     const int32_t v0 = v[0];
+    auto clamp = [](int32_t d) { return d < 0 ? 0 : d > 255 ? 255 : d; };
     if (!(x1 | a2 | a3 | a4 | a5 | a6 | a7)) {
-        if (!COL) {
+        const int32_t d = COL ? clamp(((v0 + 32) >> 6) + 128) : v0 * 8;
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k * st] = v0 * 8;
-        } else {
-            const int32_t d = ((v0 + 32) >> 6) + 128;
-            const uint8_t b = d < 0 ? 0 : d > 255 ? 255 : (uint8_t)d;
-#pragma unroll
-            for (int k = 0; k < 8; k++) pix[k] = b;
-            v[0] = 0;
-        }
+        for (int k = 0; k < 8; k++) v[k] = d;
         return;
     }
     constexpr int32_t rb = COL ? 4 : 0;
@@ -551,17 +551,8 @@ __host__ __device__ __forceinline__ void jidct_pass(int32_t *v, int st, uint8_t 
     const int32_t f7 = e8 + e3, f8 = e8 - e3, f3 = e0 + e2, f0 = e0 - e2;
     const int32_t g2 = (181 * (d4 + d5) + 128) >> 8, g4 = (181 * (d4 - d5) + 128) >> 8;
     const int32_t r[8] = {f7 + s1, f3 + g2, f0 + g4, f8 + s6, f8 - s6, f0 - g4, f3 - g2, f7 - s1};
-    if (!COL) {
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[k * st] = r[k] >> 8;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            const int32_t d = (r[k] >> 14) + 128;
-            pix[k] = d < 0 ? 0 : d > 255 ? 255 : (uint8_t)d;
-            v[k * st] = 0;
-        }
-    }
+    for (int k = 0; k < 8; k++) v[k] = COL ? clamp((r[k] >> 14) + 128) : r[k] >> 8;
 }
 
 // The write pass of one sub-stream: it decodes from its exact entry and
@@ -611,131 +602,148 @@ __host__ __device__ __forceinline__ void jwriter_init(JWriter &w, const JJob &J,
     w.done = false;
 }
 
-// Decodes the sub-stream to its end. Each block it owns and writes is
-// gathered in blk (64 quantised coefficients, natural order; left zeroed)
-// and stored whole to the job's coefficient array, with its DC value.
-__host__ __device__ __forceinline__ void jwriter_run(JWriter &w, const JJob &J, int16_t *blk) {
-    JPos &s = w.s;
-    const JScanDev &S = *w.S;
-    int32_t dcv = 0;
-    while (true) {
-        if (s.z == 0) {
-            if ((!w.last && s.p >= w.end) || w.rel >= w.nblk) break;
-            w.own = true;
-            const int pl = S.plane[s.comp];
-            w.P = pl >= 0 ? J.planes + pl : nullptr;
-        }
-        const uint32_t win = w.R.peek(s.p);
-        int sym;
-        const int nb = jdecode(s.z == 0 ? s.dc : s.ac, J.syms, win, sym);
-        const int sz = sym & 15;
-        const int32_t v = jextend(sz ? (win << nb) >> (32 - sz) : 0, sz);
-        s.p += nb + sz;
-        const bool put = w.own && w.P;
-        if (s.z == 0) {
-            if (w.own) {
-                if (s.comp == 0) dcv = w.pred0 += v;
-                else if (s.comp == 1) dcv = w.pred1 += v;
-                else dcv = w.pred2 += v;
-            }
-            s.z = 1;
-        } else if (sym == 0) {
-            s.z = 64;
-        } else {
-            s.z += sym >> 4;
-            if (put && s.z < 64) {
-#ifdef __CUDA_ARCH__
-                blk[c_zig[s.z]] = (int16_t)v;
-#else
-                blk[H_ZIG[s.z]] = (int16_t)v;
-#endif
-            }
-            s.z += 1;
-        }
-        if (s.z >= 64) {
-            if (put) {
-                const JPlaneDev &P = *w.P;
-                const uint32_t gb = P.blk0 + w.mcu * (P.sx * P.sy) + S.bsy[s.b] * P.sx + S.bsx[s.b];
-                J.dc[gb] = dcv;
-                uint4 *src = (uint4 *)blk, *dst = (uint4 *)(J.coef + (size_t)gb * 64);
-                const uint4 zero = make_uint4(0, 0, 0, 0);
-#pragma unroll
-                for (int k = 0; k < 8; k++) {
-                    dst[k] = src[k];
-                    src[k] = zero;
-                }
-            }
-            s.z = 0;
-            // where the segment's decode ends: the reference looks for the
-            // next restart marker from there
-            if (++w.rel == w.nblk) J.seg_endbit[w.seg] = s.p;
-            if (++s.b == (int)S.bpm) {
-                s.b = 0;
-                w.mcu++;
-            }
-            jset_block(s, S, J.tabs);
-        }
-    }
-}
-
-// One thread per sub-stream, each decoding on its own.
+// One thread per sub-stream, each decoding on its own, a code a turn. Each
+// block it owns and writes is gathered in its 64 quantised coefficients
+// (natural order) in shared memory; when it ends, the whole warp stores it
+// to the job's coefficient array (and clears it), its DC value apart. Lanes
+// storing their own blocks held up the others: some lane's block ends in
+// nearly every turn.
 __global__ void __launch_bounds__(JWRITE_THREADS) k_jpeg_write(JJob J) {
     __shared__ __align__(16) int16_t s_blk[JWRITE_THREADS][64];
     const uint32_t i = blockIdx.x * JWRITE_THREADS + threadIdx.x;
+    const int lane = threadIdx.x & 31, lane0 = threadIdx.x & ~31;
     int16_t *blk = s_blk[threadIdx.x];
     for (int k = 0; k < 8; k++) ((uint4 *)blk)[k] = make_uint4(0, 0, 0, 0);
     JWriter w;
     jwriter_init(w, J, i, i < J.nsub);
-    if (!w.done) jwriter_run(w, J, blk);
+    JPos &s = w.s;
+    int32_t dcv = 0;
+    while (__any_sync(0xffffffffu, !w.done)) {
+        uint32_t full = 0xffffffffu;  // the block that this lane's coefficients now are
+        if (!w.done && s.z == 0) {
+            if ((!w.last && s.p >= w.end) || w.rel >= w.nblk) {
+                w.done = true;
+            } else {
+                w.own = true;
+                const int pl = w.S->plane[s.comp];
+                w.P = pl >= 0 ? J.planes + pl : nullptr;
+            }
+        }
+        if (!w.done) {
+            const uint32_t win = w.R.peek(s.p);
+            const uint32_t e = jdecode(J, s.z == 0 ? s.dc : s.ac, win);
+            const int sz = jent_size(e), step = jent_step(e);
+            const int32_t v = jextend(sz ? (win << jent_len(e)) >> (32 - sz) : 0, sz);
+            s.p += jent_bits(e);
+            const bool put = w.own && w.P;
+            if (s.z == 0) {
+                if (w.own) {
+                    if (s.comp == 0) dcv = w.pred0 += v;
+                    else if (s.comp == 1) dcv = w.pred1 += v;
+                    else dcv = w.pred2 += v;
+                }
+            } else if (put && s.z + step <= 64) {
+                blk[c_zig[s.z + step - 1]] = (int16_t)v;  // (the rest of a block, step 64, never fits)
+            }
+            s.z += step;
+            if (s.z >= 64) {
+                if (put) {
+                    const JPlaneDev &P = *w.P;
+                    full = P.blk0 + w.mcu * (P.sx * P.sy) + w.S->bsy[s.b] * P.sx + w.S->bsx[s.b];
+                    J.dc[full] = dcv;
+                }
+                s.z = 0;
+                // where the segment's decode ends: the reference looks for the
+                // next restart marker from there
+                if (++w.rel == w.nblk) J.seg_endbit[w.seg] = s.p;
+                if (++s.b == (int)w.S->bpm) {
+                    s.b = 0;
+                    w.mcu++;
+                }
+                jset_block(s, *w.S, J.tabs);
+            }
+        }
+        uint32_t m = __ballot_sync(0xffffffffu, full != 0xffffffffu);
+        if (!m) continue;
+        __syncwarp();
+        for (; m; m &= m - 1) {
+            const int l = __ffs(m) - 1;
+            const uint32_t gb = __shfl_sync(0xffffffffu, full, l);
+            uint32_t *src = reinterpret_cast<uint32_t *>(s_blk[lane0 + l]);
+            reinterpret_cast<uint32_t *>(J.coef)[(size_t)gb * 32 + lane] = src[lane];
+            src[lane] = 0;
+        }
+        __syncwarp();
+    }
 }
 
 // The IDCT and pixel stores: 8 lanes per block (lane r: row r, then column
-// r), 4 blocks per warp.
+// r, then row r of the pixels), 4 blocks per warp. The passes are in
+// registers; between them the values cross over in shared memory, rows 9
+// words apart and blocks 72, so that no two lanes meet on a bank (with the
+// passes in place in shared memory, 8 to a bank: 195 us per 32 frames of
+// 1920 x 1080).
 constexpr int JIDCT_THREADS = 256;
 __global__ void __launch_bounds__(JIDCT_THREADS) k_jpeg_idct(JJob J) {
-    __shared__ int32_t s_v[JIDCT_THREADS / 8][64];
-    __shared__ __align__(16) uint8_t s_px[JIDCT_THREADS / 8][64];
+    __shared__ int32_t s_v[JIDCT_THREADS / 8][72];
+    __shared__ uint32_t s_plane;
     const uint32_t g = threadIdx.x >> 3, r = threadIdx.x & 7;
-    const uint32_t gb = blockIdx.x * (JIDCT_THREADS / 8) + g;
+    const uint32_t gb0 = blockIdx.x * (JIDCT_THREADS / 8), gb = gb0 + g;
     const bool live = gb < J.nblocks;
-    // the block's plane (planes in order of blk0)
-    uint32_t lo = 0, hi = J.nplanes;
-    while (live && hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (J.planes[mid].blk0 <= gb) lo = mid;
-        else hi = mid;
+    // the block's plane (planes in order of blk0): the first block's by one
+    // thread, the others' from there
+    if (threadIdx.x == 0) {
+        uint32_t lo = 0, hi = J.nplanes;
+        while (hi - lo > 1) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (J.planes[mid].blk0 <= gb0) lo = mid;
+            else hi = mid;
+        }
+        s_plane = lo;
     }
-    const JPlaneDev &P = J.planes[lo];
+    __syncthreads();
+    uint32_t pl = s_plane;
+    while (pl + 1 < J.nplanes && J.planes[pl + 1].blk0 <= gb) pl++;
+    const JPlaneDev &P = J.planes[pl];
     int32_t *v = s_v[g];
+    int32_t x[8];
     if (live) {
         const uint4 raw = *(const uint4 *)(J.coef + (size_t)gb * 64 + r * 8);
-        const int16_t *c = (const int16_t *)&raw;
+        const uint32_t c[4] = {raw.x, raw.y, raw.z, raw.w};
 #pragma unroll
-        for (int k = 0; k < 8; k++) v[r * 8 + k] = (int32_t)c[k] * P.q[r * 8 + k];
-        if (r == 0) v[0] = J.dc[gb] * P.q[0];
-        jidct_pass<false>(v + r * 8, 1, nullptr);
+        for (int k = 0; k < 8; k++) x[k] = (int32_t)(int16_t)(c[k >> 1] >> (16 * (k & 1))) * P.q[r * 8 + k];
+        if (r == 0) x[0] = J.dc[gb] * P.q[0];
+        jidct_pass<false>(x);
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[r * 9 + k] = x[k];
     }
     __syncwarp();
-    uint8_t pix[8];
     if (live) {
-        jidct_pass<true>(v + r, 8, pix);
 #pragma unroll
-        for (int k = 0; k < 8; k++) s_px[g][k * 8 + r] = pix[k];
+        for (int k = 0; k < 8; k++) x[k] = v[k * 9 + r];
+        jidct_pass<true>(x);
+    }
+    __syncwarp();
+    if (live) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) v[k * 9 + r] = x[k];
     }
     __syncwarp();
     if (!live) return;
+#pragma unroll
+    for (int k = 0; k < 8; k++) x[k] = v[r * 9 + k];
     const uint32_t L = gb - P.blk0, per = P.sx * P.sy;
     const uint32_t mcu = L / per, sub = L - mcu * per;
     const uint32_t px = ((mcu % P.mcus_x) * P.sx + sub % P.sx) * 8;
     const uint32_t py = ((mcu / P.mcus_x) * P.sy + sub / P.sx) * 8 + r;
     if (px >= P.ow || py >= P.oh) return;
     uint8_t *o = P.out + (int64_t)py * P.stride + px;
-    const uint2 row = *(const uint2 *)&s_px[g][r * 8];
     if (px + 8 <= P.ow && !((uintptr_t)o & 7)) {
-        *(uint2 *)o = row;
+        *(uint2 *)o = make_uint2(x[0] | x[1] << 8 | x[2] << 16 | x[3] << 24, x[4] | x[5] << 8 | x[6] << 16 | x[7] << 24);
     } else {
-        const uint32_t nx = min(8u, P.ow - px);
-        for (uint32_t x = 0; x < nx; x++) o[x] = s_px[g][r * 8 + x];
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++)
+            if (px + k < P.ow) o[k] = (uint8_t)x[k];
     }
 }
 
@@ -1219,6 +1227,8 @@ struct HJob {
     int64_t stream_n = 0;                 // stream bytes (at the staging's start, or at stream_src)
     const uint8_t *stream_src = nullptr;  // copied to the staging's start by run_job
     std::vector<JTab> tabs;
+    std::vector<uint32_t> lut2;
+    HTab last_tab[4];  // the tables of tabs' last four
     std::vector<uint8_t> syms;
     std::vector<JScanDev> scans;
     std::vector<JSegDev> segs;
@@ -1252,12 +1262,13 @@ std::vector<char> restart_failures(const HJob &J, const uint8_t *stream, int nim
     return bad;
 }
 
-JTab make_tab(const HTab &t, std::vector<uint8_t> &pool) {
+JTab make_tab(const HTab &t, bool ac, std::vector<uint8_t> &pool, std::vector<uint32_t> &lut2) {
     JTab d;
     memset(&d, 0, sizeof d);
     const uint32_t base = (uint32_t)pool.size();
     pool.insert(pool.end(), t.syms.begin(), t.syms.end());
     d.nrun = (uint32_t)t.runs.size();
+    d.ac = ac;
     for (size_t r = 0; r < t.runs.size(); r++) {
         d.rend[r] = t.runs[r].end;
         d.rorigin[r] = t.runs[r].origin;
@@ -1265,22 +1276,42 @@ JTab make_tab(const HTab &t, std::vector<uint8_t> &pool) {
         d.rlen[r] = (uint8_t)t.runs[r].len;
     }
     d.r0 = d.nrun;
+    // the entry of window w, r the first run that ends past it (runs leave no gaps)
+    auto entry = [&](uint32_t w, size_t r) {
+        if (r >= t.runs.size()) return jent(0, 0, ac);
+        const HRun &u = t.runs[r];
+        return jent(u.len, t.syms[u.sym0 + ((w - u.origin) >> (16 - u.len))], ac);
+    };
     size_t r = 0;
+    int nsub = 0;
     for (uint32_t p = 0; p < 512; p++) {
         const uint32_t lo = p << 7, hi = lo + 127;
         while (r < t.runs.size() && t.runs[r].end <= lo) r++;
-        bool hit = false;
-        if (r < t.runs.size() && t.runs[r].start <= lo && hi < t.runs[r].end && t.runs[r].len <= 9) {
+        bool whole = r >= t.runs.size();  // past all codes
+        if (!whole && hi < t.runs[r].end && t.runs[r].len <= 9) {
             const HRun &u = t.runs[r];
-            const uint32_t k = (lo - u.origin) >> (16 - u.len);
-            if (k == ((hi - u.origin) >> (16 - u.len))) {
-                d.lut[p] = (uint16_t)((u.len << 8) | t.syms[u.sym0 + k]);
-                hit = true;
-            }
+            whole = (lo - u.origin) >> (16 - u.len) == (hi - u.origin) >> (16 - u.len);
         }
-        if (!hit && r < d.r0) d.r0 = (uint32_t)r;
+        if (whole) {
+            d.lut[p] = entry(lo, r);
+        } else if (nsub < JMAX_SUB) {
+            nsub++;
+            d.lut[p] = JENT_SUB | (uint32_t)lut2.size();
+            size_t q = r;
+            for (uint32_t w = lo; w <= hi; w++) {
+                while (q < t.runs.size() && t.runs[q].end <= w) q++;
+                lut2.push_back(entry(w, q));
+            }
+        } else if (r < d.r0) {
+            d.r0 = (uint32_t)r;
+        }
     }
     return d;
+}
+
+bool same_tab(const HTab &a, const HTab &b) {
+    return a.runs.size() == b.runs.size() && a.syms == b.syms &&
+           (a.runs.empty() || !memcmp(a.runs.data(), b.runs.data(), a.runs.size() * sizeof(HRun)));
 }
 
 // Adds the scans of a parsed image to the job. want: which frame
@@ -1320,8 +1351,15 @@ void add_image(HJob &J, const HImage &im, int img, int64_t s_base, uint32_t sub_
         if (nmcu == 0) continue;
         JScanDev D;
         memset(&D, 0, sizeof D);
-        D.tab0 = (uint32_t)J.tabs.size();
-        for (int t = 0; t < 4; t++) J.tabs.push_back(make_tab(sc.tab[t], J.syms));
+        // one camera's files share their tables: those of the scan before, if alike
+        bool same = !J.tabs.empty();
+        for (int t = 0; t < 4 && same; t++) same = same_tab(sc.tab[t], J.last_tab[t]);
+        if (!same)
+            for (int t = 0; t < 4; t++) {
+                J.tabs.push_back(make_tab(sc.tab[t], t >= 2, J.syms, J.lut2));
+                J.last_tab[t] = sc.tab[t];
+            }
+        D.tab0 = (uint32_t)J.tabs.size() - 4;
         D.mcus_x = sc.mx;
         D.nmcu = (uint32_t)nmcu;
         D.restart = sc.restart;
@@ -1492,6 +1530,7 @@ int run_job(at_jpeg *d, HJob &J, double parse_ms) {
     auto put = [&](size_t bytes) { size_t o = off; off = align256(off + bytes); return o; };
     const size_t o_stream = put((size_t)J.stream_n + 32);
     const size_t o_tabs = put(J.tabs.size() * sizeof(JTab));
+    const size_t o_lut2 = put(J.lut2.size() * 4);
     const size_t o_syms = put(J.syms.size() + 16);
     const size_t o_scans = put(J.scans.size() * sizeof(JScanDev));
     const size_t o_segs = put(J.segs.size() * sizeof(JSegDev));
@@ -1533,6 +1572,7 @@ int run_job(at_jpeg *d, HJob &J, double parse_ms) {
     if (J.stream_src) memcpy(H + o_stream, J.stream_src, (size_t)J.stream_n);
     memset(H + o_stream + J.stream_n, 0xff, 32);
     if (!J.tabs.empty()) memcpy(H + o_tabs, J.tabs.data(), J.tabs.size() * sizeof(JTab));
+    if (!J.lut2.empty()) memcpy(H + o_lut2, J.lut2.data(), J.lut2.size() * 4);
     if (!J.syms.empty()) memcpy(H + o_syms, J.syms.data(), J.syms.size());
     if (!J.scans.empty()) memcpy(H + o_scans, J.scans.data(), J.scans.size() * sizeof(JScanDev));
     if (!J.segs.empty()) memcpy(H + o_segs, J.segs.data(), J.segs.size() * sizeof(JSegDev));
@@ -1550,6 +1590,7 @@ int run_job(at_jpeg *d, HJob &J, double parse_ms) {
         JJob JJ;
         JJ.stream = (const uint32_t *)(D + o_stream);
         JJ.tabs = (const JTab *)(D + o_tabs);
+        JJ.lut2 = (const uint32_t *)(D + o_lut2);
         JJ.syms = D + o_syms;
         JJ.scans = (const JScanDev *)(D + o_scans);
         JJ.segs = (const JSegDev *)(D + o_segs);

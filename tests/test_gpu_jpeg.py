@@ -13,6 +13,7 @@ import apriltags_fast_b200 as AT
 from apriltags_fast_b200 import synth
 from oracle import oracle as O
 from tests import helpers as H
+from tests import jpeg_cases as J
 from tests.jpeg_cases import bad_files, encode_matrix
 
 pytestmark = pytest.mark.gpu
@@ -169,3 +170,32 @@ def test_damaged_entropy_data_equals_the_oracle(dec):
                 cases.append((f"base{k} flips{n} #{rep}", _flip_entropy(base, rng, n), 0))
     check_batch(dec, cases)
     check_batch(dec, cases[::5], device=True, pad=3)
+
+
+@pytest.mark.parametrize("counts", [{2: 2, 10: 160}, {2: 3, 9: 60, 12: 99}, {3: 6, 16: 156}, {2: 1, 8: 100, 11: 61},
+                                    {1: 1, 13: 161}])
+@pytest.mark.parametrize("color", [False, True])
+def test_code_lengths(counts, color):
+    """AC tables with other code lengths put into a file (its data then
+    decodes to other pixels; with restart intervals, to an error): codes of up
+    to 9 bits, longer ones under few and under more than 64 prefixes, windows
+    without a code. Pixels and error codes as the oracle's."""
+    g = J._gray(120, 168, 11)
+    buf = bytearray(O.jpeg_encode(J._rgb(120, 168, 12), 95, (2, 2), 5) if color else O.jpeg_encode(g, 95))
+    want, at = bytes(counts.get(i, 0) for i in range(1, 17)), 0
+    assert sum(want) == 162
+    while (at := buf.find(b"\xff\xc4", at)) >= 0:  # each DHT segment: AC tables of 162 symbols
+        o, end = at + 4, at + 2 + int.from_bytes(buf[at + 2:at + 4], "big")
+        while o < end:
+            n = sum(buf[o + 1:o + 17])
+            if buf[o] >> 4 == 1 and n == 162:
+                buf[o + 1:o + 17] = want
+            o += 17 + n
+        at = end
+    e, w, h, planes = O.jpeg_decode(bytes(buf))
+    dec = AT.JpegDecoder()
+    frames, errs = dec.decode([bytes(buf)])
+    dec.close()
+    assert errs == [e]
+    if e == 0:
+        assert np.array_equal(frames[0], O.gray_of(w, h, planes))
