@@ -111,12 +111,21 @@ struct JScanDev {
     uint32_t bpm;         // blocks per MCU
     uint32_t ns;          // scan components
     uint8_t bcomp[JMAX_BPM], bsx[JMAX_BPM], bsy[JMAX_BPM];
+    uint32_t bnx[3];      // blocks of each scan component across the MCU
     // the smallest block of the MCU from which the sequence of Huffman
     // tables continues exactly as from block b: decoders at the same bit
     // and coefficient in blocks b and bcanon[b] stay in step for ever
     uint8_t bcanon[JMAX_BPM];
     uint8_t dc[3], ac[3];
-    int32_t plane[3];     // output plane of each scan component, -1: not written
+    // the same per block for MCUs of up to 16 blocks whose places fit 4 bits
+    // (flat; any file within the standard), so that a decoder has them in
+    // registers: its component (2 bits a block), its place in the
+    // component's MCU blocks (4 bits), its canonical block (4 bits)
+    unsigned long long flat_place, flat_canon;
+    uint32_t flat_comp, flat;
+    // each scan component's output: its first block in the job's coefficient
+    // arrays and blocks per MCU (0: not written)
+    uint32_t out_blk0[3], out_per[3];
 };
 
 struct JSegDev {
@@ -187,25 +196,25 @@ __host__ __device__ __forceinline__ unsigned long long jpack(uint32_t p, int z, 
     return (unsigned long long)p | ((unsigned long long)z << 32) | ((unsigned long long)b << 40);
 }
 
-// Reads the stream 32 bits at a time at any bit position, keeping the two
-// words around the last position in registers.
+// Reads the stream 32 bits at a time at positions that only grow, by less
+// than 32 a step: the two words around the last position and the one after
+// them, which is on its way when the reader gets to it.
 struct JReader {
     const uint32_t *w;
-    uint32_t k, a, b;
-    __host__ __device__ __forceinline__ void init(const uint32_t *words) {
+    uint32_t k, a, b, c;  // c: as loaded
+    __host__ __device__ __forceinline__ void init(const uint32_t *words, uint32_t p) {
         w = words;
-        k = 0xfffffffeu;
+        k = p >> 5;
+        a = jbswap(JLDG(w + k));
+        b = jbswap(JLDG(w + k + 1));
+        c = JLDG(w + k + 2);
     }
     __host__ __device__ __forceinline__ uint32_t peek(uint32_t p) {
-        const uint32_t kk = p >> 5;
-        if (kk != k) {
-            if (kk == k + 1) {
-                a = b;
-            } else {
-                a = jbswap(JLDG(w + kk));
-            }
-            b = jbswap(JLDG(w + kk + 1));
-            k = kk;
+        if (p >> 5 != k) {
+            k++;
+            a = b;
+            b = jbswap(c);
+            c = JLDG(w + k + 2);
         }
         return jfunnel(b, a, p & 31);
     }
@@ -234,6 +243,30 @@ __host__ __device__ __forceinline__ int32_t jextend(uint32_t v, int s) {
     return (s && !(v >> (s - 1))) ? (int32_t)v - ((1 << s) - 1) : (int32_t)v;
 }
 
+// What a decoder keeps of its scan in registers (JScanDev).
+struct JScanRegs {
+    const JScanDev *S;
+    const JTab *tabs;
+    unsigned long long place, canon;
+    uint32_t comp, tab4, bpm;  // tab4: per component, DC and AC table, 4 bits each
+    bool flat;
+    __host__ __device__ __forceinline__ void init(const JScanDev &s, const JTab *t) {
+        S = &s;
+        tabs = t + s.tab0;
+        place = s.flat_place;
+        canon = s.flat_canon;
+        comp = s.flat_comp;
+        flat = s.flat != 0;
+        bpm = s.bpm;
+        tab4 = 0;
+        for (int c = 0; c < 3; c++) tab4 |= (uint32_t)(s.dc[c] | s.ac[c] << 4) << (8 * c);
+    }
+    __host__ __device__ __forceinline__ int comp_of(int b) const { return flat ? (int)(comp >> (2 * b) & 3) : S->bcomp[b]; }
+    __host__ __device__ __forceinline__ int canon_of(int b) const {
+        return flat ? (int)(canon >> (4 * b) & 15) : S->bcanon[b];
+    }
+};
+
 // The decoder's position: bit p, next coefficient z (0: the DC code),
 // block b of the MCU, and the tables of that block's component.
 struct JPos {
@@ -243,11 +276,11 @@ struct JPos {
     int comp;
 };
 
-__host__ __device__ __forceinline__ void jset_block(JPos &s, const JScanDev &S, const JTab *tabs) {
-    const int c = S.bcomp[s.b];
+__host__ __device__ __forceinline__ void jset_block(JPos &s, const JScanRegs &Q) {
+    const int c = Q.comp_of(s.b);
     s.comp = c;
-    s.dc = tabs + S.tab0 + S.dc[c];
-    s.ac = tabs + S.tab0 + S.ac[c];
+    s.dc = Q.tabs + (Q.tab4 >> (8 * c) & 15);
+    s.ac = Q.tabs + (Q.tab4 >> (8 * c + 4) & 15);
 }
 
 // Decodes from the state `in` up to the first code boundary at or past
@@ -271,19 +304,21 @@ __host__ __device__ unsigned long long jrun_sync(const JJob &J, const JScanDev &
     }
     s.z = (int)((in >> 32) & 0xff);
     s.b = (int)((in >> 40) & 0xff);
-    jset_block(s, S, J.tabs);
+    JScanRegs Q;
+    Q.init(S, J.tabs);
+    jset_block(s, Q);
     JReader R;
-    R.init(J.stream);
+    R.init(J.stream, s.p);
     const int stall_max = 2 * (int)S.bpm + 2;
     int stall = 0;
     unsigned long long out = 0;
     while (true) {
         if (!counting && s.p >= from) {
             counting = true;
-            *entry = jpack(s.p, s.z, S.bcanon[s.b]);
+            *entry = jpack(s.p, s.z, Q.canon_of(s.b));
         }
         if (s.p >= end) {
-            out = jpack(s.p, s.z, S.bcanon[s.b]);
+            out = jpack(s.p, s.z, Q.canon_of(s.b));
             break;
         }
         const uint32_t win = R.peek(s.p);
@@ -308,8 +343,8 @@ __host__ __device__ unsigned long long jrun_sync(const JJob &J, const JScanDev &
         s.p += jent_bits(e);
         if (s.z >= 64) {
             s.z = 0;
-            if (++s.b == (int)S.bpm) s.b = 0;
-            jset_block(s, S, J.tabs);
+            if (++s.b == (int)Q.bpm) s.b = 0;
+            jset_block(s, Q);
             nblk += counting;
         }
     }
@@ -460,23 +495,31 @@ __global__ void __launch_bounds__(JSYNC_THREADS, 8) k_jpeg_sync(JJob J, uint32_t
     // exclusive scans of the four counts over all sub-streams
     __shared__ uint32_t s_red[4][JSYNC_THREADS];
     __shared__ uint32_t s_base[4];
+    if (threadIdx.x < 4) s_base[threadIdx.x] = 0;
+    __syncthreads();
+    // adds each thread's four values to s_base
+    auto add_all = [&](const uint32_t v[4]) {
+        for (int k = 0; k < 4; k++) {
+            const uint32_t sum = __reduce_add_sync(0xffffffffu, v[k]);
+            if ((threadIdx.x & 31) == 0) atomicAdd(&s_base[k], sum);
+        }
+        __syncthreads();
+    };
     uint32_t t4[4] = {0, 0, 0, 0};
     for (uint32_t i = lo + threadIdx.x; i < hi; i += blockDim.x)
         for (int k = 0; k < 4; k++) t4[k] += J.cnt[4 * (size_t)i + k];
-    for (int k = 0; k < 4; k++) s_red[k][threadIdx.x] = t4[k];
-    __syncthreads();
+    add_all(t4);
     if (threadIdx.x < 4) {
-        uint32_t a = 0;
-        for (int t = 0; t < JSYNC_THREADS; t++) a += s_red[threadIdx.x][t];
-        J.totals[4 * blockIdx.x + threadIdx.x] = a;
+        J.totals[4 * blockIdx.x + threadIdx.x] = s_base[threadIdx.x];
+        s_base[threadIdx.x] = 0;
     }
     if (!jgrid_sync(J.bar, nb, J.err)) return;
-    if (threadIdx.x < 4) {
-        uint32_t a = 0;
-        for (uint32_t j = 0; j < blockIdx.x; j++) a += *(volatile uint32_t *)&J.totals[4 * j + threadIdx.x];
-        s_base[threadIdx.x] = a;
-    }
-    __syncthreads();
+    // the totals of the CTAs before (all threads: one thread's loads in turn
+    // took 90 us in the last of 900 CTAs)
+    for (int k = 0; k < 4; k++) t4[k] = 0;
+    for (uint32_t j = threadIdx.x; j < blockIdx.x; j += blockDim.x)
+        for (int k = 0; k < 4; k++) t4[k] += *(volatile uint32_t *)&J.totals[4 * j + k];
+    add_all(t4);
     for (uint32_t r = lo; r < hi; r += blockDim.x) {
         const uint32_t i = r + threadIdx.x;
         uint32_t v[4] = {0, 0, 0, 0};
@@ -563,8 +606,8 @@ __host__ __device__ __forceinline__ void jidct_pass(int32_t v[8]) {
 struct JWriter {
     JPos s;
     JReader R;
-    const JScanDev *S;
-    const JPlaneDev *P;   // plane of the block in progress (nullptr: not written)
+    JScanRegs Q;
+    uint32_t blk0[3], per[3];  // per component: its output blocks (JScanDev)
     uint32_t seg, end, rel, nblk, mcu;
     int32_t pred0, pred1, pred2;  // DC predictors of the scan components
     bool last, own, done;
@@ -577,7 +620,11 @@ __host__ __device__ __forceinline__ void jwriter_init(JWriter &w, const JJob &J,
     const JSegDev G = J.segs[seg];
     if (J.seg_stuck[seg] < i) return;  // dead: the segment's decode stopped before it
     const JScanDev &S = J.scans[G.scan];
-    w.S = &S;
+    w.Q.init(S, J.tabs);
+    for (int c = 0; c < 3; c++) {
+        w.blk0[c] = S.out_blk0[c];
+        w.per[c] = S.out_per[c];
+    }
     w.seg = seg;
     const unsigned long long in = i == G.sub0 ? jpack(G.start, 0, 0) : J.exitst[i - 1];
     w.last = i == G.sub0 + G.nsub - 1;
@@ -594,11 +641,10 @@ __host__ __device__ __forceinline__ void jwriter_init(JWriter &w, const JJob &J,
     w.s.p = (uint32_t)in;
     w.s.z = (int)((in >> 32) & 0xff);
     w.s.b = (int)((G.blk0 + w.rel) % S.bpm);
-    jset_block(w.s, S, J.tabs);
+    jset_block(w.s, w.Q);
     w.mcu = (G.blk0 + w.rel) / S.bpm;
     w.own = w.s.z == 0;  // a block begun before the entry belongs to the previous sub-stream
-    w.P = nullptr;
-    w.R.init(J.stream);
+    w.R.init(J.stream, w.s.p);
     w.done = false;
 }
 
@@ -625,8 +671,6 @@ __global__ void __launch_bounds__(JWRITE_THREADS) k_jpeg_write(JJob J) {
                 w.done = true;
             } else {
                 w.own = true;
-                const int pl = w.S->plane[s.comp];
-                w.P = pl >= 0 ? J.planes + pl : nullptr;
             }
         }
         if (!w.done) {
@@ -635,7 +679,8 @@ __global__ void __launch_bounds__(JWRITE_THREADS) k_jpeg_write(JJob J) {
             const int sz = jent_size(e), step = jent_step(e);
             const int32_t v = jextend(sz ? (win << jent_len(e)) >> (32 - sz) : 0, sz);
             s.p += jent_bits(e);
-            const bool put = w.own && w.P;
+            const uint32_t per = s.comp == 0 ? w.per[0] : s.comp == 1 ? w.per[1] : w.per[2];
+            const bool put = w.own && per;
             if (s.z == 0) {
                 if (w.own) {
                     if (s.comp == 0) dcv = w.pred0 += v;
@@ -648,19 +693,22 @@ __global__ void __launch_bounds__(JWRITE_THREADS) k_jpeg_write(JJob J) {
             s.z += step;
             if (s.z >= 64) {
                 if (put) {
-                    const JPlaneDev &P = *w.P;
-                    full = P.blk0 + w.mcu * (P.sx * P.sy) + w.S->bsy[s.b] * P.sx + w.S->bsx[s.b];
+                    const uint32_t b0 = s.comp == 0 ? w.blk0[0] : s.comp == 1 ? w.blk0[1] : w.blk0[2];
+                    const JScanDev &S = *w.Q.S;
+                    const uint32_t at = w.Q.flat ? (uint32_t)(w.Q.place >> (4 * s.b)) & 15u
+                                                 : S.bsy[s.b] * S.bnx[s.comp] + S.bsx[s.b];
+                    full = b0 + w.mcu * per + at;
                     J.dc[full] = dcv;
                 }
                 s.z = 0;
                 // where the segment's decode ends: the reference looks for the
                 // next restart marker from there
                 if (++w.rel == w.nblk) J.seg_endbit[w.seg] = s.p;
-                if (++s.b == (int)w.S->bpm) {
+                if (++s.b == (int)w.Q.bpm) {
                     s.b = 0;
                     w.mcu++;
                 }
-                jset_block(s, *w.S, J.tabs);
+                jset_block(s, w.Q);
             }
         }
         uint32_t m = __ballot_sync(0xffffffffu, full != 0xffffffffu);
@@ -1390,9 +1438,21 @@ void add_image(HJob &J, const HImage &im, int img, int64_t s_base, uint32_t sub_
             if (D.dc[i] > 3) D.dc[i] = 0;
             if (D.ac[i] > 3) D.ac[i] = 2;
             const int c = sc.cidx[i];
-            D.plane[i] = (im.comp[c].scan == (int)s) ? plane_of[c] : -1;
+            D.bnx[i] = im.comp[c].sx;
+            const int pl = im.comp[c].scan == (int)s ? plane_of[c] : -1;
+            if (pl >= 0) {
+                D.out_blk0[i] = J.planes[pl].blk0;
+                D.out_per[i] = J.planes[pl].sx * J.planes[pl].sy;
+            }
         }
-        for (int i = sc.ns; i < 3; i++) D.plane[i] = -1;
+        D.flat = sc.bpm <= 16;
+        for (uint32_t b = 0; b < sc.bpm && D.flat; b++) {
+            const uint32_t at = (uint32_t)sc.bsy[b] * D.bnx[sc.bcomp[b]] + sc.bsx[b];
+            if (at > 15) D.flat = 0;
+            D.flat_comp |= (uint32_t)sc.bcomp[b] << (2 * b);
+            D.flat_place |= (unsigned long long)(at & 15) << (4 * b);
+            D.flat_canon |= (unsigned long long)D.bcanon[b] << (4 * b);
+        }
         const uint32_t scan_id = (uint32_t)J.scans.size();
         J.scans.push_back(D);
         J.scan_image.push_back(img);
