@@ -63,6 +63,12 @@ uint32_t jsub_for(int64_t stream_bytes) {
     while (b < 1024 && (uint64_t)stream_bytes * 8 / b > 65536) b *= 2;
     return b;
 }
+// Bits of run-in: enough for most decodes to fall into step. Long sub-streams
+// (large batches, short of time rather than of threads) take the shorter one
+// and correct a few more: sync pass of 32 1080p gray files 0.24 ms at 256 bits,
+// 0.24 at 512, 0.28 at 1024, of eight 4:2:0 files 0.54, 0.57, 0.63 ms; with
+// sub-streams of 256 bits one file takes 0.08 ms at 128 to 512 bits, 0.09 at 1024.
+uint32_t jback_for(uint32_t sub_bits) { return sub_bits >= 1024 ? 256 : 512; }
 constexpr int JMAX_BPM = 64;        // blocks per MCU (the standard allows 10)
 constexpr int JSYNC_THREADS = 128;
 constexpr int JWRITE_THREADS = 128;
@@ -1845,7 +1851,7 @@ static int decode_group(at_jpeg *dec, int32_t a, int32_t b, const uint8_t *const
     for (int k = 0; k < m; k++)
         if (!errs[k]) total += used[k];
     J.sub_bits = dec->sub_bits ? dec->sub_bits : jsub_for(total);
-    J.back_bits = dec->back_bits ? dec->back_bits : std::max(512u, J.sub_bits);
+    J.back_bits = dec->back_bits ? dec->back_bits : jback_for(J.sub_bits);
     int failed = 0;
     for (int k = 0; k < m; k++) {
         const int32_t i = a + k;

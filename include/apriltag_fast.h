@@ -347,8 +347,8 @@ int at_jpeg_last_stats(const at_jpeg *dec, double *out10);
 int at_jpeg_set_sub_bits(at_jpeg *dec, int32_t bits);
 
 /* Bits a sub-stream's first, speculative decode starts before the
-   sub-stream (by default the larger of 512 and the sub-stream; 0 restores
-   that): longer run-ins fall into step with the true decode more often, at
+   sub-stream (by default 512, or 256 for sub-streams of 1024 bits or more; 0
+   restores that): longer run-ins fall into step with the true decode more often, at
    the cost of decoding them. Returns 0 or 1. */
 int at_jpeg_set_run_in(at_jpeg *dec, int32_t bits);
 
