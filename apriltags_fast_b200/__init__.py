@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as C
 import os
+import sys
 from dataclasses import dataclass
 
 import numpy as np
@@ -207,9 +208,10 @@ class Detection:
         return (self.family, self.id, self.hamming, self.decision_margin, self.H, self.c, self.p)
 
 
-def _detection(d: CDetection) -> Detection:
-    return Detection(int(d.family), int(d.id), int(d.hamming), float(d.decision_margin), tuple(d.H), tuple(d.c),
-                     tuple(tuple(r) for r in d.p))
+def _detections(rec: np.ndarray) -> list[Detection]:
+    """Records (DETECTION_DTYPE) as Detection objects, a field at a time."""
+    return [Detection(f, i, h, m, tuple(H), tuple(c), tuple(map(tuple, p)))
+            for f, i, h, m, H, c, p in zip(*(rec[k].tolist() for k in DETECTION_DTYPE.names))]
 
 
 class Detector:
@@ -254,8 +256,7 @@ class Detector:
         ptr, w, h, s = _image_arg(img, stride)
         self._L.at_detect(self._td, ptr, w, h, s)
         self._check()
-        td = self._td.contents
-        return [_detection(td.detections[i]) for i in range(td.ndetections)]
+        return _detections(self._records())
 
     def detect_batch(self, images, family_masks=None, as_arrays: bool = False):
         """at_detect_batch over images of any sizes. Returns per frame a list
@@ -271,17 +272,19 @@ class Detector:
         res = (FrameResult * max(n, 1))()
         self._L.at_detect_batch(self._td, frames, n, res)
         self._check()
-        td = self._td.contents
         self.last_batch_nquads = [int(res[i].nquads) for i in range(n)]
-        if as_arrays:
-            total = int(td.ndetections)
-            if total:
-                buf = C.cast(td.detections, C.POINTER(C.c_uint8 * (168 * total))).contents
-                allv = np.frombuffer(buf, DETECTION_DTYPE, total).copy()
-            else:
-                allv = np.zeros(0, DETECTION_DTYPE)
-            return [allv[res[i].first:res[i].first + res[i].count] for i in range(n)]
-        return [[_detection(td.detections[res[i].first + k]) for k in range(res[i].count)] for i in range(n)]
+        rec = self._records()
+        allv = rec.copy() if as_arrays else _detections(rec)
+        return [allv[res[i].first:res[i].first + res[i].count] for i in range(n)]
+
+    def _records(self) -> np.ndarray:
+        """The library's detection array of the last call, in place."""
+        td = self._td.contents
+        total = int(td.ndetections)
+        if not total:
+            return np.zeros(0, DETECTION_DTYPE)
+        buf = C.cast(td.detections, C.POINTER(C.c_uint8 * (168 * total))).contents
+        return np.frombuffer(buf, DETECTION_DTYPE, total)
 
     def _check(self):
         msg = C.c_char_p()
@@ -426,10 +429,10 @@ class Server:
 
 
 def _image_arg(img, stride):
-    if hasattr(img, "data_ptr") and getattr(img, "is_cuda", False):
-        assert img.dtype.__str__() == "torch.uint8" and img.dim() == 2
+    if not isinstance(img, np.ndarray) and hasattr(img, "data_ptr") and getattr(img, "is_cuda", False):
+        assert img.dtype is sys.modules["torch"].uint8 and img.dim() == 2
         h, w = img.shape
-        return C.c_void_p(img.data_ptr()), w, h, int(img.stride(0))
+        return C.c_void_p(img.data_ptr()), w, h, img.stride(0)
     a = np.asarray(img)
     if a.dtype != np.uint8 or a.ndim != 2:
         raise TypeError("image must be a 2-D uint8 array")
@@ -531,7 +534,8 @@ class JpegDecoder:
     def decode(self, bufs, flags: int = 0):
         """Host numpy frames (None where an image failed) and error codes."""
         infos = [jpeg_info(b, flags) for b in bufs]
-        outs = [np.zeros((max(h, 1), max(w, 1)), np.uint8) if e == 0 else np.zeros((1, 1), np.uint8)
+        # a decoded frame is written whole, one that failed is not returned
+        outs = [np.empty((max(h, 1), max(w, 1)), np.uint8) if e == 0 else np.empty((1, 1), np.uint8)
                 for e, w, h, _ in infos]
         errs = self._call(bufs, [o.ctypes.data for o in outs], [o.strides[0] for o in outs], False, flags)
         res = [o[:h, :w] if e == 0 else None for o, e, (_, w, h, _) in zip(outs, errs, infos)]
@@ -541,7 +545,7 @@ class JpegDecoder:
         """torch.uint8 CUDA frames (rows padded by `pad` bytes) and error codes."""
         import torch
         infos = [jpeg_info(b, flags) for b in bufs]
-        outs = [torch.zeros((max(h, 1), max(w, 1) + pad), dtype=torch.uint8, device="cuda") for _, w, h, _ in infos]
+        outs = [torch.empty((max(h, 1), max(w, 1) + pad), dtype=torch.uint8, device="cuda") for _, w, h, _ in infos]
         errs = self._call(bufs, [o.data_ptr() for o in outs], [o.stride(0) for o in outs], True, flags)
         return [o[:h, :w] if e == 0 else None for o, e, (_, w, h, _) in zip(outs, errs, infos)], errs
 

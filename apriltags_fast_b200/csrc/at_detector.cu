@@ -26,9 +26,10 @@
 #include "at_kernels.h"
 
 // batch splitting: at most this many pipelines, each given at least
-// AT_SPLIT_MIN_FRAMES frames (measured on 1080p batches: copies from host
-// memory overlap compute, +14% frames/s at 32 frames; below about 20
-// frames one pipeline is as fast)
+// AT_SPLIT_MIN_FRAMES frames, and only for batches with frames to copy from
+// host memory, whose copies overlap another pipeline's kernels. 32 frames of
+// 1920 x 1080 in device memory: one pipeline 2.07 ms, two 2.15, three 2.26;
+// below about 20 host frames one pipeline is as fast.
 #define AT_BATCH_SPLIT_DEFAULT 3
 #define AT_BATCH_SPLIT_MAX 4
 #define AT_SPLIT_MIN_FRAMES 10
@@ -352,6 +353,17 @@ struct CopyTurn {
     ~CopyTurn() { pass(); }
 };
 
+// A frame's pixels as this GPU's kernels read them in place, or null (they
+// are elsewhere and get copied).
+static const uint8_t *device_pixels(const at_internal *in, const uint8_t *pixels) {
+    cudaPointerAttributes pa;
+    if (cudaPointerGetAttributes(&pa, pixels) == cudaSuccess &&
+        (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged) && pa.device == in->device)
+        return static_cast<const uint8_t *>(pa.devicePointer);
+    cudaGetLastError();  // clear the error an unregistered host pointer leaves
+    return nullptr;
+}
+
 static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_frame_result *res,
                       CopyChain *chain = nullptr, int link = 0) {
     at_internal *in = td->in;
@@ -401,16 +413,10 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         f.img = nullptr;
         f.stride = f.w;
         if (live) {
-            cudaPointerAttributes pa;
-            int dev = -1;
-            cudaGetDevice(&dev);
-            if (cudaPointerGetAttributes(&pa, fr.pixels) == cudaSuccess &&
-                (pa.type == cudaMemoryTypeDevice || pa.type == cudaMemoryTypeManaged) && pa.device == dev &&
-                pa.devicePointer != nullptr) {
-                f.img = static_cast<const uint8_t *>(pa.devicePointer);
+            f.img = device_pixels(in, fr.pixels);
+            if (f.img) {
                 f.stride = fr.stride;
             } else {
-                cudaGetLastError();  // clear the error an unregistered host pointer leaves
                 f.img = reinterpret_cast<const uint8_t *>((uintptr_t)img);  // an offset until the arena exists
                 img += (int64_t)f.w * f.h;
                 copied[i] = 1;
@@ -476,15 +482,20 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     memcpy(in->h_frames.p, fd.data(), n * sizeof(FrameDesc));
     const FrameDesc *dfr = B[B_FRAMES].as<FrameDesc>();
 
-    for (int k = 0; k < 12; k++) CK(cudaEventRecord(in->ev[k], st));  // keep all events valid
     CK(cudaEventRecord(in->ev[0], st));
     CK(cudaMemcpyAsync(B[B_FRAMES].p, in->h_frames.p, n * sizeof(FrameDesc), cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(B[B_ERR].p, 0, 4, st));
     turn.wait();
     for (int64_t i = 0; i < n; i++) {
         if (!copied[i]) continue;
-        CK(cudaMemcpy2DAsync(const_cast<uint8_t *>(fd[i].img), fd[i].w, frames[i].pixels, frames[i].stride, fd[i].w,
-                             fd[i].h, cudaMemcpyDefault, st));
+        // rows without gaps go as one block: a pitched copy of pageable rows
+        // of an odd width took 300 us for 1279 x 717
+        if (frames[i].stride == fd[i].w)
+            CK(cudaMemcpyAsync(const_cast<uint8_t *>(fd[i].img), frames[i].pixels, (size_t)fd[i].w * fd[i].h,
+                               cudaMemcpyDefault, st));
+        else
+            CK(cudaMemcpy2DAsync(const_cast<uint8_t *>(fd[i].img), fd[i].w, frames[i].pixels, frames[i].stride,
+                                 fd[i].w, fd[i].h, cudaMemcpyDefault, st));
     }
     turn.pass();
     uint8_t *qim = B[B_QIM].as<uint8_t>(), *thr = B[B_THR].as<uint8_t>();
@@ -1042,6 +1053,11 @@ void at_detect_batch(at_detector *td, const at_frame *frames, int64_t n, at_fram
     td->nquads = 0;
     int P = in->split;
     if (P > n / AT_SPLIT_MIN_FRAMES) P = (int)(n / AT_SPLIT_MIN_FRAMES);
+    if (P > 1) {
+        bool copies = false;
+        for (int64_t i = 0; i < n && !copies; i++) copies = device_pixels(in, frames[i].pixels) == nullptr;
+        if (!copies) P = 1;
+    }
     const bool ok = P > 1 ? run_split(td, frames, n, results, P) : run_batch(td, frames, n, results);
     if (!ok) {
         in->dets.clear();

@@ -1979,7 +1979,7 @@ pjpeg_t *pjpeg_create_from_buffer(uint8_t *buf, int buflen, uint32_t flags, int 
         }
     }
     J.sub_bits = jsub_for(sk.n);
-    J.back_bits = std::max(512u, J.sub_bits);
+    J.back_bits = jback_for(J.sub_bits);
     add_image(J, im, 0, 0, J.sub_bits, 7u, [&](int c, JPlaneDev &P) -> size_t {
         const pjpeg_component_t &o = pj->components[c];
         P.ow = o.width;
