@@ -15,10 +15,9 @@
 //                    pair list.
 //   k_cluster_collect (at_kernels.cu): the distinct pairs.
 //   -- the host reads the pair and point counts (its only wait here) --
-//   k_pair_frame, k_pair_scatter, k_pair_rank: the distinct pairs in order.
-//                    A frame's pairs sort before the next frame's (the
-//                    larger label is a node of the frame), so each frame's
-//                    pairs are ranked among themselves.
+//   k_pair_frame, k_pair_offsets, k_pair_scatter, k_pair_rank: the distinct
+//                    pairs in order. A frame's pairs sort before the next
+//                    frame's (the larger label is a node of the frame).
 //   k_cluster_span   per cluster: count, frame, first row, rows spanned.
 //   scans            each cluster's first point; its row table's offset.
 //   k_seg_fill       a warp per row: its pairs' point counts into the
@@ -249,73 +248,75 @@ __device__ __forceinline__ int frame_of_node(const FrameDesc *frames, int nframe
     return lo;
 }
 
-// Each distinct pair's frame; pairs per frame.
+// The pairs in order: first in buckets, PAIR_BUCKETS per frame by where the
+// larger label lies among the frame's nodes (a monotone function of the
+// pair), then ranked among their bucket's. (Ranked among all pairs of the
+// frame: 210 us for the 24396 pairs of a 4032 x 3024 frame.)
+#define PAIR_BUCKETS 256
 __global__ void k_pair_frame(const uint64_t *okeys, int64_t ncl, int nb, const FrameDesc *frames, int nframes,
-                             uint32_t *kframe, uint32_t *fcount) {
+                             uint32_t *kbucket, uint32_t *bcount) {
     kernel_begin();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < ncl; r += (int64_t)gridDim.x * blockDim.x) {
-        const int fr = frame_of_node(frames, nframes, (int64_t)(okeys[r] >> nb));
-        kframe[r] = (uint32_t)fr;
-        atomicAdd(fcount + fr, 1u);
+        const int64_t hi = (int64_t)(okeys[r] >> nb);
+        const int fr = frame_of_node(frames, nframes, hi);
+        const FrameDesc &f = frames[fr];
+        const uint64_t nodes = (uint64_t)f.qw * f.qh + f.qh;
+        const uint32_t b = (uint32_t)fr * PAIR_BUCKETS + (uint32_t)((uint64_t)(hi - f.node_off) * PAIR_BUCKETS / nodes);
+        kbucket[r] = b;
+        atomicAdd(bcount + b, 1u);
     }
 }
 
-// One block: each frame's first pair (foff, nframes + 1 entries).
-__global__ void __launch_bounds__(1024) k_pair_frame_offsets(const uint32_t *fcount, int nframes, uint32_t *foff,
-                                                             uint32_t *fcur) {
+// One block: each bucket's first pair (boff, nbuckets + 1 entries).
+__global__ void __launch_bounds__(1024) k_pair_offsets(const uint32_t *bcount, int nbuckets, uint32_t *boff,
+                                                       uint32_t *bcur) {
     kernel_begin();
     __shared__ uint32_t sh[32];
     uint32_t base = 0;
-    for (int f0 = 0; f0 < nframes; f0 += blockDim.x) {
-        const int f = f0 + threadIdx.x;
-        const uint32_t c = f < nframes ? fcount[f] : 0u;
+    for (int b0 = 0; b0 < nbuckets; b0 += 4 * blockDim.x) {
+        const int b = b0 + 4 * threadIdx.x;  // nbuckets is a multiple of 4
+        const uint4 c = b < nbuckets ? *reinterpret_cast<const uint4 *>(bcount + b) : make_uint4(0, 0, 0, 0);
         uint32_t total;
-        const uint32_t off = block_excl_scan(c, &total, sh);
-        if (f < nframes) {
-            foff[f] = base + off;
-            fcur[f] = 0;
+        const uint32_t o = base + block_excl_scan(c.x + c.y + c.z + c.w, &total, sh);
+        if (b < nbuckets) {
+            *reinterpret_cast<uint4 *>(boff + b) = make_uint4(o, o + c.x, o + c.x + c.y, o + c.x + c.y + c.z);
+            *reinterpret_cast<uint4 *>(bcur + b) = make_uint4(0, 0, 0, 0);
         }
         base += total;
     }
-    if (threadIdx.x == 0) foff[nframes] = base;
+    if (threadIdx.x == 0) boff[nbuckets] = base;
 }
 
-__global__ void k_pair_scatter(const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, const uint32_t *kframe,
-                               const uint32_t *foff, uint32_t *fcur, uint64_t *gkeys, uint32_t *gslots) {
+__global__ void k_pair_scatter(const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, const uint32_t *kbucket,
+                               const uint32_t *boff, uint32_t *bcur, uint64_t *gkeys, uint32_t *gslots,
+                               uint32_t *gbucket) {
     kernel_begin();
     for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < ncl; r += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t fr = kframe[r];
-        const uint32_t p = foff[fr] + atomicAdd(fcur + fr, 1u);
+        const uint32_t b = kbucket[r];
+        const uint32_t p = boff[b] + atomicAdd(bcur + b, 1u);
         gkeys[p] = okeys[r];
         gslots[p] = oslots[r];
+        gbucket[p] = b;
     }
 }
 
-// A warp per pair: its place = its frame's first place + the number of
-// smaller pairs of the frame (the pairs are distinct).
-__global__ void __launch_bounds__(256) k_pair_rank(const uint64_t *gkeys, const uint32_t *gslots, int64_t ncl,
-                                                   const uint32_t *foff, int nframes, uint64_t *skeys,
-                                                   uint32_t *sslots) {
+// A warp per pair: its place = its bucket's first place + the number of
+// smaller pairs of the bucket (the pairs are distinct).
+__global__ void __launch_bounds__(256) k_pair_rank(const uint64_t *gkeys, const uint32_t *gslots,
+                                                   const uint32_t *gbucket, int64_t ncl, const uint32_t *boff,
+                                                   uint64_t *skeys, uint32_t *sslots) {
     kernel_begin();
     const int lane = threadIdx.x & 31;
     for (int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; p < ncl;
          p += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-        int lo = 0, hi = nframes - 1;  // the frame whose segment holds p
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (foff[mid] <= (uint32_t)p)
-                lo = mid;
-            else
-                hi = mid - 1;
-        }
+        const uint32_t b = gbucket[p], q0 = boff[b], q1 = boff[b + 1];
         const uint64_t k = gkeys[p];
         uint32_t below = 0;
-        for (uint32_t q = foff[lo] + lane; q < foff[lo + 1]; q += 32) below += gkeys[q] < k;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+        for (uint32_t q = q0 + lane; q < q1; q += 32) below += gkeys[q] < k;
+        below = __reduce_add_sync(0xffffffffu, below);
         if (lane == 0) {
-            skeys[foff[lo] + below] = k;
-            sslots[foff[lo] + below] = gslots[p];
+            skeys[q0 + below] = k;
+            sslots[q0 + below] = gslots[p];
         }
     }
 }
@@ -551,12 +552,13 @@ void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *os
                        uint64_t *skeys, uint32_t *sslots, uint32_t *rank_of_slot, uint32_t *ccount, uint32_t *cspan,
                        uint32_t *cy0, int32_t *cframe, uint32_t *cstart, uint32_t *spanoff) {
     if (ncl <= 0) return;
-    cudaMemsetAsync(P.fcount, 0, (size_t)nframes * 4, s);
-    launch(k_pair_frame, flat_grid(ncl, 256), 256, 0, s, okeys, ncl, nb, frames, nframes, P.kframe, P.fcount);
-    launch(k_pair_frame_offsets, 1, 1024, 0, s, P.fcount, nframes, P.foff, P.fcur);
-    launch(k_pair_scatter, flat_grid(ncl, 256), 256, 0, s, okeys, oslots, ncl, P.kframe, P.foff, P.fcur, P.gkeys,
-                                                       P.gslots);
-    launch(k_pair_rank, flat_grid(ncl * 32, 256), 256, 0, s, P.gkeys, P.gslots, ncl, P.foff, nframes, skeys, sslots);
+    const int nbuckets = nframes * PAIR_BUCKETS;
+    cudaMemsetAsync(P.bcount, 0, (size_t)nbuckets * 4, s);
+    launch(k_pair_frame, flat_grid(ncl, 256), 256, 0, s, okeys, ncl, nb, frames, nframes, P.kbucket, P.bcount);
+    launch(k_pair_offsets, 1, 1024, 0, s, P.bcount, nbuckets, P.boff, P.bcur);
+    launch(k_pair_scatter, flat_grid(ncl, 256), 256, 0, s, okeys, oslots, ncl, P.kbucket, P.boff, P.bcur, P.gkeys,
+           P.gslots, P.gbucket);
+    launch(k_pair_rank, flat_grid(ncl * 32, 256), 256, 0, s, P.gkeys, P.gslots, P.gbucket, ncl, P.boff, skeys, sslots);
     launch(k_cluster_span, flat_grid(ncl, 256), 256, 0, s, skeys, sslots, ncl, T, nb, frames, nframes, rank_of_slot,
                                                        ccount, cspan, cy0, cframe);
     const int64_t nblk = (ncl + SCAN_ITEMS - 1) / SCAN_ITEMS;
@@ -566,6 +568,7 @@ void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *os
                                                           spanoff);
 }
 
+int64_t pair_buckets(int nframes) { return (int64_t)nframes * PAIR_BUCKETS; }
 int64_t pair_scan_blocks(int64_t ncl) { return (ncl + SCAN_ITEMS - 1) / SCAN_ITEMS + 1; }
 
 // An exclusive scan of n u32 values into out (n + 1 entries, the total

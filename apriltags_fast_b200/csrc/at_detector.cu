@@ -100,7 +100,7 @@ enum {
     B_KEY, B_VAL, B_KEY2, B_VAL2, B_HEAD, B_HSCAN, B_CSTART, B_CFRAME,
     B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
-    B_HYMIN, B_HYMAX, B_CSPAN, B_CY0, B_SPANOFF, B_PKFRAME, B_PGKEYS, B_PGSLOTS, B_PFRAMES, B_PBSUM, B_SEG,
+    B_HYMIN, B_HYMAX, B_CSPAN, B_CY0, B_SPANOFF, B_PKFRAME, B_PGKEYS, B_PGSLOTS, B_PGBUCKET, B_PFRAMES, B_PBSUM, B_SEG,
     B_QCL, B_CKEY, B_RNEED, B_RNT, B_RTLAB, B_RTPX, B_RTROOT, B_RTLIST, B_RTROW, B_RPRE, B_ROKEY, B_RIDX2,
     B_RPAR, B_RLEN, B_RSUM, B_RSTAMP, B_RTCH, B_RHIST,
     B_PREC, B_PPSLOT, B_PPCNT, B_PPID, B_PINFO, B_QSCR,
@@ -613,14 +613,16 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_PKFRAME].ensure(ncl * 4 + 4));
         CK(B[B_PGKEYS].ensure(ncl * 8 + 8));
         CK(B[B_PGSLOTS].ensure(ncl * 4 + 4));
-        CK(B[B_PFRAMES].ensure((3 * n + 1) * 4));
+        const int64_t nbk = pair_buckets((int)n);
+        CK(B[B_PGBUCKET].ensure(ncl * 4 + 4));
+        CK(B[B_PFRAMES].ensure((3 * nbk + 4) * 4));
         CK(B[B_PBSUM].ensure(2 * pair_scan_blocks(ncl) * 4));
         const int64_t segcap = (int64_t)npts + in->seg_slack * ncl + 4096;
         CK(B[B_SEG].ensure(segcap * 4));
         uint32_t *pf = B[B_PFRAMES].as<uint32_t>();
         uint32_t *bs = B[B_PBSUM].as<uint32_t>();
-        const PairScratch ps{B[B_PKFRAME].as<uint32_t>(), pf, pf + n, pf + 2 * n + 1, B[B_PGKEYS].as<uint64_t>(),
-                             B[B_PGSLOTS].as<uint32_t>(), bs, bs + pair_scan_blocks(ncl)};
+        const PairScratch ps{B[B_PKFRAME].as<uint32_t>(), pf, pf + nbk, pf + 2 * nbk + 4, B[B_PGKEYS].as<uint64_t>(),
+                             B[B_PGSLOTS].as<uint32_t>(), B[B_PGBUCKET].as<uint32_t>(), bs, bs + pair_scan_blocks(ncl)};
         launch_pair_order(st, B[B_HOKEYS].as<uint64_t>(), B[B_HOSLOTS].as<uint32_t>(), ncl, nb, dfr, (int)n, pt, ps,
                           B[B_HSKEYS].as<uint64_t>(), B[B_HSSLOTS].as<uint32_t>(), B[B_HRANK].as<uint32_t>(),
                           B[B_HCCOUNT].as<uint32_t>(), B[B_CSPAN].as<uint32_t>(), B[B_CY0].as<uint32_t>(),

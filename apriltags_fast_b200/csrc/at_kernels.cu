@@ -3032,14 +3032,18 @@ __device__ bool poly_contains(const double (*poly)[2], const double *q) {
     }
     return acc >= 2 || acc <= -2;
 }
+// Whether two quads overlap, by a warp: an edge pair or a containment a lane.
 __device__ bool quads_overlap(const double (*pa)[2], const double (*pb)[2]) {
-    for (int i = 0; i < 4; i++)
-        for (int j = 0; j < 4; j++)
-            if (segments_cross(pa[i], pa[(i + 1) % 4], pb[j], pb[(j + 1) % 4])) return true;
-    double qb[2] = {(pb[0][0] + pb[1][0] + pb[2][0]) / 3.0, (pb[0][1] + pb[1][1] + pb[2][1]) / 3.0};
-    if (poly_contains(pa, qb)) return true;
-    double qa[2] = {(pa[0][0] + pa[1][0] + pa[2][0]) / 3.0, (pa[0][1] + pa[1][1] + pa[2][1]) / 3.0};
-    return poly_contains(pb, qa);
+    const int l = threadIdx.x & 31;
+    bool x = false;
+    if (l < 16) {
+        x = segments_cross(pa[l >> 2], pa[((l >> 2) + 1) & 3], pb[l & 3], pb[((l & 3) + 1) & 3]);
+    } else if (l < 18) {
+        const double(*in)[2] = l == 16 ? pb : pa, (*poly)[2] = l == 16 ? pa : pb;
+        const double q[2] = {(in[0][0] + in[1][0] + in[2][0]) / 3.0, (in[0][1] + in[1][1] + in[2][1]) / 3.0};
+        x = poly_contains(poly, q);
+    }
+    return __any_sync(0xffffffffu, x);
 }
 __device__ __forceinline__ int prefer(int pref, double a, double b) {
     return pref ? pref : a < b ? -1 : b < a ? 1 : 0;
@@ -3125,54 +3129,64 @@ __global__ void k_finalize(int nframes, const int64_t *frame_qstart, int nfam, c
         for (int64_t p = threadIdx.x; p < n; p += blockDim.x) ix[p] = idx2[a + p];
         __syncthreads();
     }
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) rm[i] = 0;
-    __syncthreads();
+    // each place's (family, id), and the group each first place of two or more begins
+    uint32_t *key = idx2 + a;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const GpuDetection &di = dets[ix[i]];
-        bool first = true, more = false;
-        for (int64_t j = 0; j < n && first; j++)
-            if (j != i && dets[ix[j]].id == di.id && dets[ix[j]].family == di.family) {
+        rm[i] = 0;
+        key[i] = (uint32_t)dets[ix[i]].family << 16 | (uint32_t)dets[ix[i]].id;
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    for (int64_t w0 = (threadIdx.x >> 5) * 32; w0 < n; w0 += blockDim.x) {
+        const int64_t i = w0 + lane;
+        bool first = i < n, more = false;
+        for (int64_t j = 0; first && j < n; j++)
+            if (j != i && key[j] == key[i]) {
                 if (j < i) first = false;
                 else more = true;
             }
-        if (!first || !more) continue;
-        // the reference's loop (fast/decode.c:860-891) over this group only
-        int64_t i0 = i;
-        while (i0 < n) {
-            if (rm[i0] || dets[ix[i0]].id != di.id || dets[ix[i0]].family != di.family) {
-                i0++;
-                continue;
-            }
-            for (int64_t i1 = i0 + 1; i1 < n; i1++) {
-                const GpuDetection &d0 = dets[ix[i0]], &d1 = dets[ix[i1]];
-                if (rm[i1] || d1.id != di.id || d1.family != di.family || !quads_overlap(d0.p, d1.p)) continue;
-                int pref = prefer(0, d0.hamming, d1.hamming);
-                pref = prefer(pref, -(double)d0.decision_margin, -(double)d1.decision_margin);
-                for (int k = 0; k < 4; k++) {
-                    pref = prefer(pref, d0.p[k][0], d1.p[k][0]);
-                    pref = prefer(pref, d0.p[k][1], d1.p[k][1]);
+        for (uint32_t bal = __ballot_sync(0xffffffffu, first && more); bal; bal &= bal - 1) {
+            // the reference's loop (fast/decode.c:860-891) over this group only
+            const int64_t g = w0 + __ffs(bal) - 1;
+            const uint32_t k = key[g];
+            // the group's next place from p on that is still there
+            auto next = [&](int64_t p) {
+                for (int64_t q0 = p; q0 < n; q0 += 32) {
+                    const int64_t q = q0 + lane;
+                    const bool in = q < n && key[q] == k && !*(volatile uint8_t *)(rm + q);
+                    const uint32_t m = __ballot_sync(0xffffffffu, in);
+                    if (m) return q0 + __ffs(m) - 1;
                 }
-                if (pref < 0) {
-                    rm[i1] = 1;
-                    continue;
+                return n;
+            };
+            for (int64_t i0 = g; i0 < n; i0 = next(i0 + 1))
+                for (int64_t i1 = next(i0 + 1); i1 < n; i1 = next(i1 + 1)) {
+                    const GpuDetection &d0 = dets[ix[i0]], &d1 = dets[ix[i1]];
+                    if (!quads_overlap(d0.p, d1.p)) continue;
+                    int pref = prefer(0, d0.hamming, d1.hamming);
+                    pref = prefer(pref, -(double)d0.decision_margin, -(double)d1.decision_margin);
+                    for (int c = 0; c < 4; c++) {
+                        pref = prefer(pref, d0.p[c][0], d1.p[c][0]);
+                        pref = prefer(pref, d0.p[c][1], d1.p[c][1]);
+                    }
+                    if (lane == 0) rm[pref < 0 ? i1 : i0] = 1;
+                    __syncwarp();
+                    if (pref >= 0) break;
                 }
-                rm[i0] = 1;
-                break;
-            }
-            i0++;
         }
     }
     __syncthreads();
     // stable sort by id (fast/detector.c:164-179): rank among survivors
+    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) key[i] = rm[i] ? 0xffffffffu : key[i] & 0xffffu;
+    __syncthreads();
     GpuDetection *o = out + out_off[f];
     uint32_t kept = 0;
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) {
-        if (rm[i]) continue;
+        const uint32_t id = key[i];
+        if (id == 0xffffffffu) continue;
         kept++;
-        int32_t id = dets[ix[i]].id;
         int64_t r = 0;
-        for (int64_t j = 0; j < n; j++)
-            if (!rm[j] && (dets[ix[j]].id < id || (dets[ix[j]].id == id && j < i))) r++;
+        for (int64_t j = 0; j < n; j++) r += key[j] < id || (key[j] == id && j < i);
         o[r] = dets[ix[i]];
     }
     uint32_t total;

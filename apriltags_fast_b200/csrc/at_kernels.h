@@ -72,14 +72,16 @@ struct PairTable {
     uint32_t *count, *ymin, *ymax;
     uint32_t mask;
 };
-// Scratch of the pair ordering: per pair its frame, per frame its pair count,
-// first pair (nframes + 1) and a cursor, the pairs grouped by frame, and
-// the block sums of the scans (pair_scan_blocks each).
+// Scratch of the pair ordering: per pair its bucket, per bucket (pair_buckets)
+// its pair count, first pair (one more entry) and a cursor, the pairs grouped
+// by bucket with their buckets, and the block sums of the scans
+// (pair_scan_blocks each). The bucket arrays are 16-byte aligned.
 struct PairScratch {
-    uint32_t *kframe, *fcount, *foff, *fcur;
+    uint32_t *kbucket, *bcount, *boff, *bcur;
     uint64_t *gkeys;
-    uint32_t *gslots, *bsum_a, *bsum_b;
+    uint32_t *gslots, *gbucket, *bsum_a, *bsum_b;
 };
+int64_t pair_buckets(int nframes);
 // The points of each row (rows 1 .. qh-2): records in emission order at
 // rec + 2 (q_off + y qw), at most 2 qw a row (the pair's place in the row's
 // table | neighbour << 12 | pixel is 0 << 14 | x << 15); the row's distinct
