@@ -632,8 +632,10 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
                            B[B_SEG].as<uint32_t>(), segcap, B[B_VAL2].as<uint64_t>(), (int64_t)npts,
                            B[B_ERR].as<uint32_t>());
         in->launches += 13;
-    } else if (npts > 0) {
-        // the pair table overflowed: points in emission order, sorted by pair
+    } else if (!hashed) {
+        // a capacity of the scan was exceeded: points in emission order,
+        // sorted by pair. The scan's count leaves out the rows that it gave
+        // up, so they are counted again.
         uint64_t *row_npts = B[B_ROWPTS].as<uint64_t>(), *row_off = B[B_ROWOFF].as<uint64_t>();
         CK(cudaMemsetAsync(row_npts + rows, 0, 8, st));
         CK(B[B_LAB].ensure(qpx * 4));
@@ -646,6 +648,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
                 return cub::DeviceScan::ExclusiveSum(t, b, row_npts, row_off, rows + 1, st);
             }))
             return false;
+        CK(cudaMemcpyAsync(&npts, row_off + rows, 8, cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
         CK(B[B_KEY].ensure(npts * 8));
         CK(B[B_VAL].ensure(npts * 8));
         CK(B[B_KEY2].ensure(npts * 8));

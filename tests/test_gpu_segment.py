@@ -66,3 +66,21 @@ def test_wide_frames(w):
         r = O.detect(img, fams, [2], O.default_params(quad_decimate=1.0), order=O.ORDER_CANON)
         assert np.array_equal(det.diag("labels"), oracle_pixel_labels(r, 24))
     _check([_blobs(w, 48, 7, w)], 24, 3.0 if w < 12000 else 4.0)
+
+
+@pytest.mark.parametrize("w", [300, 1025])
+def test_rows_above_a_limit(w):
+    """Rows with more points (over two a pixel, below the teeth of a comb) or
+    more pairs of labels (stripes) than the scan has room for, beside a frame
+    without: the sorting path takes every point of the batch."""
+    teeth = np.where(np.arange(w) % 2, 30, 220).astype(np.uint8)[None].repeat(40, 0)
+    comb = teeth.copy()
+    comb[:8], comb[32:] = 220, 30
+    stripes = np.where(np.arange(w) // 2 % 2, 30, 220).astype(np.uint8)[None].repeat(40, 0)
+    _check([comb, stripes, _blobs(w, 40, 3, w)], 24)
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    imgs = [_blobs(w, 40, 3, w), comb, stripes]
+    pts = [O.detect(i, [H.oracle_family("tag36h11")], [2], O.default_params(quad_decimate=1.0), order=O.ORDER_CANON).pts
+           for i in imgs]
+    det.detect_batch(imgs)
+    assert np.array_equal(det.diag("points"), np.concatenate(pts))
