@@ -43,30 +43,43 @@
     for (int64_t y = 1 + blockIdx.x * wpb + (threadIdx.x >> 5); y + 1 < f.qh; y += gridDim.x * wpb) {
 #define ROW_WARPS_END }
 
-// A warp's table of the pairs of its row: open addressing over 2 nd_cap
-// slots (larger label << 32 | smaller, points), then the records of up to
-// 1024 columns before they are copied out, and the pairs' count.
+// What a warp of the scan keeps: its row's pairs, open addressing over 2
+// nd_cap slots (larger label << 32 | smaller, points); (starts, before) of
+// the 32 words it is at in this row and the next, with those beside; up to
+// SCAN_BUF of their points in emission order (column | neighbour << 10 |
+// black << 12); the pairs' count; behind it their slots.
 #define SCAN_BUF 1024
-__host__ __device__ inline size_t row_pairs_bytes(int nd_cap) { return (size_t)24 * nd_cap + 4 * SCAN_BUF + 16; }
+struct ScanPart {
+    uint2 at[2][34];
+    uint16_t pts[SCAN_BUF];
+    uint32_t npair, pad[3];
+};
+__host__ __device__ inline size_t row_pairs_bytes(int nd_cap) { return (size_t)26 * nd_cap + sizeof(ScanPart); }
 
 // Point records: the pair's slot in the row's table | neighbour j << 12 |
 // (pixel is 0) << 14 | x << 15.
 #define PREC_ID 0xfffu
 
+// The run of column c of a word with (starts, before) s.
+__device__ __forceinline__ uint32_t run_in(uint2 s, int c) { return s.y + __popc(s.x & ((2u << (c & 31)) - 1u)) - 1u; }
+
 // Every boundary point, once. The points of 32 columns are bit operations
 // on the masks of the row and the row below (the masks hold labelled pixels
-// only; fast/clusters.c:144-252, as point_mask per pixel). Then a lane goes
-// through its word's points in emission order (x, then neighbour): the
-// labels by run number, the pair looked up in the row's table when it
-// differs from the last one, the record into the warp's buffer. At the
-// row's end each pair goes into the frame's pair table (count, first and
+// only; fast/clusters.c:144-252, as point_mask per pixel), a word a lane.
+// Each lane lists its word's points in emission order (x, then neighbour);
+// then a lane takes a point: the labels by run number, the pair looked up in
+// the row's table by the first of a run of equal ones, the record written. At
+// the row's end each pair goes into the frame's pair table (count, first and
 // last row) and, with its points in the row, into the row's pair list. Any
 // capacity exceeded (pairs of a row, records of a row, probes of the pair
 // table) sets *full and the batch takes the sorting path instead.
 //
-// Bound by instruction issue: about 25 instructions a point, where a lane
-// per pixel with labels per pixel took some 90 a pixel group and 4 bytes a
-// pixel of labels written and read.
+// Bound by instruction issue. For 32 frames of 1920 x 1080 (9.4 million
+// points): a lane per pixel with labels per pixel 313 us; a lane looking up
+// all its word's points, where the fullest of 32 words sets the pace, 180 us
+// (10 of 32 lanes busy, 13 instructions a warp and point); 8 columns a lane
+// from a queue 208 us; this 105 us (228 to 140 for 16 of mixed sizes,
+// 346 to 194 for one 4032 x 3024).
 __global__ void __launch_bounds__(256) k_point_scan(const FrameDesc *frames, const RowWord *words, const uint32_t *lab,
                                                     int nb, PairTable T, PointRows P, uint32_t *full,
                                                     unsigned long long *npoints) {
@@ -74,12 +87,14 @@ __global__ void __launch_bounds__(256) k_point_scan(const FrameDesc *frames, con
     extern __shared__ __align__(16) uint8_t s_mem[];
     const int nd_cap = P.nd_cap, rt = 2 * nd_cap;
     uint64_t *tkey = reinterpret_cast<uint64_t *>(s_mem + (threadIdx.x >> 5) * row_pairs_bytes(nd_cap));
-    uint32_t *tcnt = reinterpret_cast<uint32_t *>(tkey + rt), *buf = tcnt + rt, *npair = buf + SCAN_BUF;
+    uint32_t *tcnt = reinterpret_cast<uint32_t *>(tkey + rt);
+    ScanPart &W = *reinterpret_cast<ScanPart *>(tcnt + rt);
+    uint16_t *used = reinterpret_cast<uint16_t *>(&W + 1);
     for (int i = threadIdx.x & 31; i < rt; i += 32) {
         tkey[i] = CH_EMPTY;
         tcnt[i] = 0;
     }
-    if ((threadIdx.x & 31) == 0) *npair = 0;
+    if ((threadIdx.x & 31) == 0) W.npair = 0;
     __syncwarp();
     const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
     uint64_t pts = 0;
@@ -120,115 +135,125 @@ __global__ void __launch_bounds__(256) k_point_scan(const FrameDesc *frames, con
         const uint32_t cm1 = ((a.white & Kbm) | (a.black & Wbm)) & x1 & ~left11;
         const uint32_t c11 = ((a.white & Kb1) | (a.black & Wb1)) & x1;
         uint32_t total;
-        const uint32_t off = warp_excl_scan(__popc(c10) + __popc(c01) + __popc(cm1) + __popc(c11), &total);
+        const uint32_t own = __popc(c10) + __popc(c01) + __popc(cm1) + __popc(c11);
+        const uint32_t off = warp_excl_scan(own, &total), end = off + own;
         if (total == 0) continue;
         if (nrec + total > rcap) {
             if (lane == 0) atomicOr(full, 1u);
             return;
         }
-        uint32_t *dst = total <= SCAN_BUF ? buf + off : rec + nrec + off;
-        uint32_t any = c10 | c01 | cm1 | c11, jm = 0, rx = 0, la = 0, pla = 0, plb = 0, id = 0, cnt = 0;
-        int c = 0;
-        while (jm | any) {
-            if (jm == 0) {  // the next pixel with points
-                c = __ffs(any) - 1;
-                any &= any - 1;
-                jm = (c10 >> c & 1u) | (c01 >> c & 1u) << 1 | (cm1 >> c & 1u) << 2 | (c11 >> c & 1u) << 3;
-                la = la_of[run_at(a, c)];
-                rx = (uint32_t)(32 * i + c) << 15 | (a.black >> c & 1u) << 14;
-            }
-            const uint32_t j = (uint32_t)__ffs(jm) - 1u;
-            jm &= jm - 1;
-            // the neighbour's label: this row or the next, column c + d
-            const int d = j == 0 || j == 3 ? 1 : j == 2 ? -1 : 0, cc = c + d;
-            uint32_t st = j == 0 ? a.starts : b.starts, be = j == 0 ? a.before : b.before;
-            if (cc > 31) {
-                st = j == 0 ? an.starts : bn.starts;
-                be = j == 0 ? an.before : bn.before;
-            } else if (cc < 0) {
-                st = bp.starts;
-                be = bp.before;
-            }
-            const uint32_t *lp = (j == 0 ? la_of : lb_of) + (be + __popc(st & ((2u << (cc & 31)) - 1u)) - 1u);
-            if (d > 0 && 32 * i + cc == qw - 1) lp = lcol + (j == 0 ? 0 : 1);
-            const uint32_t lb = *lp;
-            if (la != pla || lb != plb || cnt == 0) {
-                if (cnt) atomicAdd(tcnt + id, cnt);
-                cnt = 0;
-                pla = la;
-                plb = lb;
-                const uint32_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
-                const uint64_t k = (uint64_t)hi << 32 | lo;
-                uint32_t h = hi * 0x9e3779b1u + lo * 0x85ebca6bu;
-                h = (h ^ h >> 16) & (uint32_t)(rt - 1);
-                for (int p = 0; p < rt; p++) {  // a table without room has set *full below
-                    uint64_t cur = *(volatile uint64_t *)(tkey + h);
-                    if (cur == CH_EMPTY) {
-                        cur = atomicCAS(reinterpret_cast<unsigned long long *>(tkey + h), CH_EMPTY, k);
-                        if (cur == CH_EMPTY) {
-                            if (atomicAdd(npair, 1u) >= (uint32_t)nd_cap) atomicOr(full, 1u);
-                            break;
-                        }
-                    }
-                    if (cur == k) break;
-                    h = (h + 1) & (uint32_t)(rt - 1);
-                }
-                id = h;
-            }
-            cnt++;
-            *dst++ = id | j << 12 | rx;
+        W.at[0][lane + 1] = make_uint2(a.starts, a.before);
+        W.at[1][lane + 1] = make_uint2(b.starts, b.before);
+        if (lane == 0) W.at[1][0] = make_uint2(bp.starts, bp.before);
+        if (lane == 31) {
+            W.at[0][33] = make_uint2(an.starts, an.before);
+            W.at[1][33] = make_uint2(bn.starts, bn.before);
         }
-        if (cnt) atomicAdd(tcnt + id, cnt);
-        __syncwarp();
-        if (total <= SCAN_BUF)
-            for (uint32_t t = lane; t < total; t += 32) rec[nrec + t] = buf[t];
-        if (*(volatile uint32_t *)npair > (uint32_t)nd_cap) return;  // *full is set
+        for (uint32_t base = 0, lim; base < total; base = lim) {
+            // the words whose points there is room for (a word has 128 at most)
+            const bool fits = end <= base + SCAN_BUF;
+            lim = __reduce_max_sync(0xffffffffu, fits ? end : 0u);
+            const uint32_t n = lim - base;
+            if (fits && off >= base) {
+                uint16_t *to = W.pts + (off - base);
+                for (uint32_t any = c10 | c01 | cm1 | c11; any; any &= any - 1) {
+                    const int c = __ffs(any) - 1;
+                    const uint32_t px = (uint32_t)(32 * lane + c) | (a.black >> c & 1u) << 12;
+                    if (c10 >> c & 1u) *to++ = (uint16_t)px;
+                    if (c01 >> c & 1u) *to++ = (uint16_t)(px | 1u << 10);
+                    if (cm1 >> c & 1u) *to++ = (uint16_t)(px | 2u << 10);
+                    if (c11 >> c & 1u) *to++ = (uint16_t)(px | 3u << 10);
+                }
+            }
+            __syncwarp();
+            for (uint32_t t0 = 0; t0 < n; t0 += 32) {
+                const bool on = t0 + lane < n;
+                uint32_t pt = 0, la = 0, lb = 0;
+                if (on) {
+                    pt = W.pts[t0 + lane];
+                    const int xl = pt & 1023u, j = pt >> 10 & 3u;
+                    la = la_of[run_in(W.at[0][(xl >> 5) + 1], xl)];
+                    // the neighbour's label: this row or the next, a column on, none, or back
+                    const int d = j == 0 || j == 3 ? 1 : j == 2 ? -1 : 0, row = j == 0 ? 0 : 1, cl = xl + d;
+                    const uint32_t *lp = (row ? lb_of : la_of) + run_in(W.at[row][(cl >> 5) + 1], cl);
+                    if (d > 0 && 32 * i0 + cl == qw - 1) lp = lcol + row;
+                    lb = *lp;
+                }
+                // the first of each run of points of one pair finds it
+                const uint32_t ua = __shfl_up_sync(0xffffffffu, la, 1), ub = __shfl_up_sync(0xffffffffu, lb, 1);
+                const bool head = on && (lane == 0 || ua != la || ub != lb);
+                const uint32_t heads = __ballot_sync(0xffffffffu, head), ons = __ballot_sync(0xffffffffu, on);
+                uint32_t id = 0;
+                if (head) {
+                    const uint32_t later = heads & ~lt & ~(1u << lane);
+                    const uint32_t hi = la > lb ? la : lb, lo = la > lb ? lb : la;
+                    const uint64_t k = (uint64_t)hi << 32 | lo;
+                    id = hi * 0x9e3779b1u + lo * 0x85ebca6bu;
+                    id = (id ^ id >> 16) & (uint32_t)(rt - 1);
+                    for (int p = 0; p < rt; p++) {  // a table without room has set *full below
+                        uint64_t cur = *(volatile uint64_t *)(tkey + id);
+                        if (cur == CH_EMPTY) {
+                            cur = atomicCAS(reinterpret_cast<unsigned long long *>(tkey + id), CH_EMPTY, k);
+                            if (cur == CH_EMPTY) {
+                                const uint32_t at = atomicAdd(&W.npair, 1u);
+                                if (at >= (uint32_t)nd_cap)
+                                    atomicOr(full, 1u);
+                                else
+                                    used[at] = (uint16_t)id;
+                                break;
+                            }
+                        }
+                        if (cur == k) break;
+                        id = (id + 1) & (uint32_t)(rt - 1);
+                    }
+                    atomicAdd(tcnt + id, (uint32_t)((later ? __ffs(later) - 1 : __popc(ons)) - lane));
+                }
+                const uint32_t mine = heads & (lt | 1u << lane);
+                id = __shfl_sync(0xffffffffu, id, mine ? 31 - __clz(mine) : 0);
+                if (on) rec[nrec + base + t0 + lane] = id | (pt & 0x1c00u) << 2 | ((uint32_t)(32 * i0) + (pt & 1023u)) << 15;
+            }
+            __syncwarp();
+        }
+        if (*(volatile uint32_t *)&W.npair > (uint32_t)nd_cap) return;  // *full is set
         __syncwarp();
         nrec += total;
     }
     // the row's pairs into the frame's pair table; the table cleared
     uint32_t *ps = P.pslot + (f.row0 + y) * nd_cap, *pc = P.pcnt + (f.row0 + y) * nd_cap;
     uint16_t *pi = P.pid + (f.row0 + y) * nd_cap;
-    uint32_t nd = 0;
-    if (nrec)
-        for (int s = lane; s < rt; s += 32) {
-            const uint64_t kk = tkey[s];
-            const bool occ = kk != CH_EMPTY;
-            const uint32_t bal = __ballot_sync(0xffffffffu, occ);
-            if (occ) {
-                const uint32_t at = nd + __popc(bal & lt), n = tcnt[s];
-                const uint64_t k = (kk >> 32) << nb | (kk & 0xffffffffu);
-                uint32_t slot = ch_hash(k) & T.mask;
-                int p = 0;
-                for (; p < CH_PROBES; p++) {
-                    uint64_t cur = *(volatile uint64_t *)(T.keys + slot);
-                    if (cur == CH_EMPTY) {
-                        const unsigned long long old =
-                            atomicCAS(reinterpret_cast<unsigned long long *>(T.keys + slot), CH_EMPTY, k);
-                        cur = old == CH_EMPTY ? k : old;
-                    }
-                    if (cur == k) break;
-                    slot = (slot + 1) & T.mask;
-                }
-                if (p == CH_PROBES) {
-                    atomicOr(full, 1u);
-                } else {
-                    atomicAdd(T.count + slot, n);
-                    atomicMin(T.ymin + slot, (uint32_t)y);
-                    atomicMax(T.ymax + slot, (uint32_t)y);
-                }
-                ps[at] = slot;
-                pc[at] = n;
-                pi[at] = (uint16_t)s;
-                tkey[s] = CH_EMPTY;
-                tcnt[s] = 0;
+    const uint32_t nd = W.npair;
+    for (uint32_t at = lane; at < nd; at += 32) {
+        const uint32_t id = used[at], n = tcnt[id];
+        const uint64_t kk = tkey[id], k = (kk >> 32) << nb | (kk & 0xffffffffu);
+        uint32_t slot = ch_hash(k) & T.mask;
+        int p = 0;
+        for (; p < CH_PROBES; p++) {
+            uint64_t cur = *(volatile uint64_t *)(T.keys + slot);
+            if (cur == CH_EMPTY) {
+                const unsigned long long old =
+                    atomicCAS(reinterpret_cast<unsigned long long *>(T.keys + slot), CH_EMPTY, k);
+                cur = old == CH_EMPTY ? k : old;
             }
-            nd += __popc(bal);
-            __syncwarp();
+            if (cur == k) break;
+            slot = (slot + 1) & T.mask;
         }
+        if (p == CH_PROBES) {
+            atomicOr(full, 1u);
+        } else {
+            atomicAdd(T.count + slot, n);
+            atomicMin(T.ymin + slot, (uint32_t)y);
+            atomicMax(T.ymax + slot, (uint32_t)y);
+        }
+        ps[at] = slot;
+        pc[at] = n;
+        pi[at] = (uint16_t)id;
+        tkey[id] = CH_EMPTY;
+        tcnt[id] = 0;
+    }
+    __syncwarp();
     if (lane == 0) {
         P.info[f.row0 + y] = make_uint2(nrec, nd);
-        *npair = 0;
+        W.npair = 0;
     }
     pts += nrec;
     __syncwarp();

@@ -68,6 +68,19 @@ def test_wide_frames(w):
     _check([_blobs(w, 48, 7, w)], 24, 3.0 if w < 12000 else 4.0)
 
 
+@pytest.mark.parametrize("w", [512, 700, 1024, 1025, 2080])
+@pytest.mark.parametrize("tooth", [1, 2])
+def test_dense_points(w, tooth):
+    """Two combs in one another: up to two points a pixel, so that 1024
+    columns hold more than a warp lists at a time, of one pair of labels."""
+    img = np.where(np.arange(w) // tooth % 2, 30, 220).astype(np.uint8)[None].repeat(40, 0)
+    img[:8], img[32:] = 220, 30
+    _check([img], 24)
+    r = O.detect(img, [H.oracle_family("tag36h11")], [2], O.default_params(quad_decimate=1.0), order=O.ORDER_CANON)
+    per_row = len(r.pts) / 24  # the rows of the teeth
+    assert per_row > (1.9 if tooth == 1 else 0.95) * w, per_row
+
+
 @pytest.mark.parametrize("w", [300, 1025])
 def test_rows_above_a_limit(w):
     """Rows with more points (over two a pixel, below the teeth of a comb) or
