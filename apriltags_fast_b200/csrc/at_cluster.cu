@@ -496,6 +496,9 @@ __global__ void __launch_bounds__(256) k_seg_fill(const FrameDesc *frames, Point
 // pair's cluster (seg, after the scan) plus the pair's points before it in
 // the row; the records are in emission order, so a cluster's points keep
 // the reference's order.
+//
+// Bound by memory latency: the records of the next two steps are on their way
+// during one (32 frames of 1920 x 1080: 72 -> 51 us).
 __global__ void __launch_bounds__(256) k_point_place(const FrameDesc *frames, PointRows P,
                                                      const uint32_t *rank_of_slot, const uint32_t *spanoff,
                                                      const uint32_t *cy0, int64_t ncl, const uint32_t *seg, int64_t cap,
@@ -515,10 +518,13 @@ __global__ void __launch_bounds__(256) k_point_place(const FrameDesc *frames, Po
     }
     __syncwarp();
     const uint32_t *rec = P.rec + 2 * (f.q_off + y * f.qw);
+    uint32_t rc0 = lane < inf.x ? rec[lane] : 0u, rc1 = lane + 32 < inf.x ? rec[lane + 32] : 0u;
     for (uint32_t r0 = 0; r0 < inf.x; r0 += 32) {
         const uint32_t r = r0 + lane;
         const bool valid = r < inf.x;
-        const uint32_t rc = valid ? rec[r] : 0u;
+        const uint32_t rc = rc0;
+        rc0 = rc1;
+        if (r + 64 < inf.x) rc1 = rec[r + 64];
         const uint32_t id = valid ? rc & PREC_ID : 0xffffffffu;
         const uint32_t peers = __match_any_sync(0xffffffffu, id);
         const uint32_t at = valid ? base[id] + __popc(peers & lt) : 0u;
