@@ -769,33 +769,33 @@ __device__ __forceinline__ void moment_terms(uint64_t pt, int32_t g2, double m[6
     m[5] = w;
 }
 
-// The prefix sums of src[0, n) in place, after `run`, one lane: a chain of
-// dependent additions (8.3 cycles each); the next 8 terms are loaded before
-// the additions of these 8, and the stores follow them, so the chain does
-// not wait for shared memory.
+// The prefix sums of src[0, n) in place (16-byte aligned), after `run`, one
+// lane: a chain of dependent additions, 8.4 cycles each. The next 8 terms are
+// loaded, and the sums stored, two at a time between the additions: 9.4
+// cycles a term, where eight loads, eight additions and eight stores in turn
+// took 12.5 (the chain stood still while the loads and stores issued).
 __device__ __forceinline__ void prefix_chain(double *src, int n, double &run) {
     int t = 0;
     if (n >= 8) {
-        double v[8], x[8];
+        double2 *p = reinterpret_cast<double2 *>(src), v[4], r;
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = src[u];
-        for (; t + 16 <= n; t += 8) {
+        for (int u = 0; u < 4; u++) v[u] = p[u];
+        for (; t + 16 <= n; t += 8, p += 4) {
 #pragma unroll
-            for (int u = 0; u < 8; u++) x[u] = src[t + 8 + u];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                run = __dadd_rn(run, v[u]);
-                v[u] = run;
+            for (int u = 0; u < 4; u++) {
+                r.x = __dadd_rn(run, v[u].x);
+                r.y = __dadd_rn(r.x, v[u].y);
+                v[u] = p[4 + u];
+                run = r.y;
+                p[u] = r;
             }
-#pragma unroll
-            for (int u = 0; u < 8; u++) src[t + u] = v[u];
-#pragma unroll
-            for (int u = 0; u < 8; u++) v[u] = x[u];
         }
 #pragma unroll
-        for (int u = 0; u < 8; u++) {
-            run = __dadd_rn(run, v[u]);
-            src[t + u] = run;
+        for (int u = 0; u < 4; u++) {
+            r.x = __dadd_rn(run, v[u].x);
+            r.y = __dadd_rn(r.x, v[u].y);
+            run = r.y;
+            p[u] = r;
         }
         t += 8;
     }
@@ -914,56 +914,59 @@ __device__ __forceinline__ void line_of(const MSum &s, double lp[4], double *mse
     *mse = eig_small;
 }
 
-
-// The largest of a warp's e[first], e[first + stride], ... (below n) after
-// (pv, pi) in the order (value descending, index ascending); -inf if none.
-__device__ __forceinline__ void warp_next_desc(const double *e, int n, int first, int stride, double &pv, int &pi) {
-    double v = -__longlong_as_double(0x7ff0000000000000ll);
-    int at = 0x7fffffff;
-    for (int i = first; i < n; i += stride) {
-        const double x = e[i];
-        if ((x < pv || (x == pv && i > pi)) && x > v) {
-            v = x;
-            at = i;
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const double v2 = __shfl_xor_sync(0xffffffffu, v, o);
-        const int a2 = __shfl_xor_sync(0xffffffffu, at, o);
-        if (v2 > v || (v2 == v && a2 < at)) {
-            v = v2;
-            at = a2;
-        }
-    }
-    pv = v;
-    pi = at;
+// A double's place among doubles (no NaN; both zeros are one).
+__device__ __forceinline__ uint64_t double_order(double x) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x + 0.0);
+    return b >> 63 ? ~b : b | 1ull << 63;
 }
 
-// The (r + 1)-th largest of e[0, n) (r < n, r <= AT_MAX_NMAXIMA), by the
-// whole block: each warp's r + 1 largest (they hold the block's), then those
-// of the warps' lists by warp 0. cand: (r + 1) values per warp. A radix
-// select over the 64 bits (8 passes, three barriers each) took 20k cycles
-// for 700 points and 140k for 21000; this takes r + 1 short rounds.
-__device__ double block_select_desc(const double *e, int n, int r, double *cand, double *res) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    const double inf = __longlong_as_double(0x7ff0000000000000ll);
-    double pv = inf;
-    int pi = -1;
-    __syncthreads();
-    for (int t = 0; t <= r; t++) {
-        warp_next_desc(e, n, threadIdx.x, blockDim.x, pv, pi);
-        if (lane == 0) cand[w * (r + 1) + t] = pv;
+// A v such that what is above the (r + 1)-th largest of e[0, n) (r < n) has
+// a place >= v and the rest has not. By the whole block: the places from the
+// least to the largest are halved, one barrier a step (as many pivots at a
+// time as there are warps took 3000 cycles longer with 8 of them).
+template <int NT>
+__device__ uint64_t block_above(const double *e, int n, int r, uint64_t *part) {
+    constexpr int NW = NT / 32;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    uint64_t lo = ~0ull, hi = 0;
+    for (int i = threadIdx.x; i < n; i += NT) {
+        const uint64_t k = double_order(e[i]);
+        lo = k < lo ? k : lo;
+        hi = k > hi ? k : hi;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t l = __shfl_xor_sync(0xffffffffu, lo, o), h = __shfl_xor_sync(0xffffffffu, hi, o);
+        lo = l < lo ? l : lo;
+        hi = h > hi ? h : hi;
+    }
+    if (lane == 0) {
+        part[w] = lo;
+        part[NW + w] = hi;
     }
     __syncthreads();
-    if (w == 0) {
-        pv = inf;
-        pi = -1;
-        for (int t = 0; t <= r; t++) warp_next_desc(cand, nw * (r + 1), lane, 32, pv, pi);
-        if (lane == 0) *res = pv;
+    for (int v = 0; v < NW; v++) {
+        lo = part[v] < lo ? part[v] : lo;
+        hi = part[NW + v] > hi ? part[NW + v] : hi;
     }
-    __syncthreads();
-    return *res;
+    hi++;  // more than r have a place >= lo, at most r one >= hi
+    for (int step = 0; hi - lo > 1; step++) {
+        const uint64_t mid = lo + (hi - lo) / 2;
+        int c = 0;
+        for (int i = threadIdx.x; i < n; i += NT) c += double_order(e[i]) >= mid;
+        c = __reduce_add_sync(0xffffffffu, c);
+        // two halves in turn: nobody still reads the one before the last
+        int *cnt = reinterpret_cast<int *>(part + 2 * NW) + (step & 1) * NW;
+        if (lane == 0) cnt[w] = c;
+        __syncthreads();
+        c = 0;
+        for (int v = 0; v < NW; v++) c += cnt[v];
+        if (c > r)
+            lo = mid;
+        else
+            hi = mid;
+        if (c == r) break;
+    }
+    return hi;
 }
 
 // Three size classes of clusters, one kernel template: 128 threads for
@@ -978,7 +981,6 @@ __device__ double block_select_desc(const double *e, int n, int r, double *cand,
 #define FIT_LARGE_SORT 6144
 #define FIT_HUGE_SORT 13312
 #define FIT_HUGE_NT 512
-#define FIT_COUNT_MAX 256
 #define FIT_CHUNK_SMALL 256
 #define FIT_CHUNK_LARGE 512
 #define FIT_LARGE_NT 256  // threads of the largest class's blocks (two blocks an SM)
@@ -995,6 +997,130 @@ __host__ __device__ constexpr size_t fit_x_bytes(int sort_cap, int chunk) {
 }
 __host__ __device__ constexpr size_t fit_smem_bytes(int sort_cap, int chunk, int nwarps) {
     return fit_x_bytes(sort_cap, chunk) + (size_t)sort_cap * 6 + (size_t)256 * nwarps * 4;
+}
+
+// The bucket, of NB, of a slope's order bits (angle_key): the slopes of one
+// quadrant are the tangents t in [0, inf) above a multiple of 65536, spread
+// by 1 - 1 / (1 + t) with the reciprocal drawn straight between powers of
+// two. Never falls as the bits rise: a rounded sum, then integers.
+template <int NB>
+__device__ __forceinline__ int slope_bucket(uint32_t bits) {
+    const float s = __uint_as_float(bits >> 31 ? bits ^ 0x80000000u : ~bits);
+    const float q = floorf(__fmul_rn(s, 1.0f / 65536.0f));
+    if (q < -1.0f) return 0;
+    if (q > 2.0f) return NB - 1;
+    const uint32_t x = __float_as_uint(__fadd_rn(1.0f, __fsub_rn(s, __fmul_rn(q, 65536.0f))));  // 1 + t < 2^17
+    const uint32_t v = (0x1000000u - (x & 0x7fffffu)) >> ((x >> 23) - 127u);                    // 2^24 / (1 + t)
+    const uint32_t b = (0x1000000u - v) / (0x4000000u / NB);
+    return ((int)q + 1) * (NB / 4) + (int)b;
+}
+
+// A cluster is sorted by buckets while its points share theirs with at most
+// this many on average (themselves included); a comb of nearly equal angles
+// takes the sort it had before.
+#define FIT_SHARE 16
+
+// The block's sort of n (32-bit slope bits, 16-bit value) pairs in a stable
+// order: counted into 8 NT buckets, listed by bucket (list: slope bits, place
+// before, value), and each pair's place in its bucket found by comparing it
+// with the bucket's others. The values end up in va. False (and the pairs as
+// they were) if the buckets are too uneven. hist: 8 NT counters.
+// Against the radix sort's four passes: 000 instead of 27000 cycles for 700
+// points and 128 threads, 000 instead of 47500 for 3200 and 256.
+template <int NT>
+__device__ __forceinline__ bool block_bucket_sort(const uint32_t *ka, uint16_t *va, uint64_t *list, int n,
+                                                  uint32_t *hist) {
+    constexpr int NB = 8 * NT;
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    __shared__ uint32_t s_sum[NT / 32];
+    __shared__ uint64_t s_share[NT / 32];
+    uint4 *h4 = reinterpret_cast<uint4 *>(hist) + 2 * tid;
+    h4[0] = h4[1] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+#pragma unroll 4
+    for (int i = tid; i < n; i += NT) atomicAdd(hist + slope_bucket<NB>(ka[i]), 1u);
+    __syncthreads();
+    const uint4 a = h4[0], b = h4[1];
+    const uint32_t c[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t o[8], sum = 0;
+    uint64_t share = 0;
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+        o[k] = sum;
+        sum += c[k];
+        share += (uint64_t)c[k] * c[k];
+    }
+    for (int d = 16; d > 0; d >>= 1) share += __shfl_xor_sync(0xffffffffu, share, d);
+    uint32_t incl = sum;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+    }
+    if (lane == 31) {
+        s_sum[w] = incl;
+        s_share[w] = share;
+    }
+    __syncthreads();
+    for (int v = 1; v < NT / 32; v++) share += s_share[(w + v) % (NT / 32)];
+    if (share > (uint64_t)FIT_SHARE * n) return false;
+    uint32_t before = incl - sum;
+    for (int v = 0; v < w; v++) before += s_sum[v];
+    h4[0] = make_uint4(before + o[0], before + o[1], before + o[2], before + o[3]);
+    h4[1] = make_uint4(before + o[4], before + o[5], before + o[6], before + o[7]);
+    __syncthreads();
+    // from here on a bucket's counter runs to its end
+    for (int i = tid; i < n; i += 2 * NT) {
+        const int i2 = i + NT;
+        const uint32_t k = ka[i], k2 = i2 < n ? ka[i2] : 0u;
+        const uint64_t e = (uint64_t)k << 32 | (uint32_t)i << 16 | va[i],
+                       e2 = i2 < n ? (uint64_t)k2 << 32 | (uint32_t)i2 << 16 | va[i2] : 0ull;
+        const int b1 = slope_bucket<NB>(k), b2 = slope_bucket<NB>(k2);
+        const uint32_t j = atomicAdd(hist + b1, 1u), j2 = i2 < n ? atomicAdd(hist + b2, 1u) : 0u;
+        list[j] = e;
+        if (i2 < n) list[j2] = e2;
+    }
+    __syncthreads();
+    for (int j = tid; j < n; j += NT) {
+        const uint64_t e = list[j];
+        const int bk = slope_bucket<NB>((uint32_t)(e >> 32)), s0 = bk ? (int)hist[bk - 1] : 0, s1 = (int)hist[bk];
+        int at = s0;
+        for (int q = s0; q < s1; q++) at += list[q] < e;
+        va[at] = (uint16_t)e;
+    }
+    __syncthreads();
+    return true;
+}
+
+// The exclusive prefix sums of a warp's NB counts, in place. False if the
+// buckets of n are too uneven (the counts as they were).
+template <int NB>
+__device__ bool warp_bucket_scan(uint32_t *hist, int n, int lane) {
+    constexpr int PER = NB / 32;
+    uint32_t o[PER], sum = 0, share = 0;
+#pragma unroll
+    for (int k = 0; k < PER; k += 4) {
+        const uint4 c = reinterpret_cast<const uint4 *>(hist)[lane * (PER / 4) + k / 4];
+        const uint32_t v[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            o[k + j] = sum;
+            sum += v[j];
+            share += v[j] * v[j];
+        }
+    }
+    uint32_t incl = sum;
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += t;
+    }
+    if (__reduce_add_sync(0xffffffffu, share) > (uint32_t)(FIT_SHARE * n)) return false;
+    const uint32_t before = incl - sum;
+#pragma unroll
+    for (int k = 0; k < PER; k += 4)
+        reinterpret_cast<uint4 *>(hist)[lane * (PER / 4) + k / 4] =
+            make_uint4(before + o[k], before + o[k + 1], before + o[k + 2], before + o[k + 3]);
+    __syncwarp();
+    return true;
 }
 
 // Stable sort of n (32-bit key, 16-bit value) pairs by key: four passes of
@@ -1197,7 +1323,8 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
     __shared__ double s_be[NT / 32], s_lines[4][4], s_lmse[4], s_best;
     __shared__ int s_bo[NT / 32];
     __shared__ uint32_t s_next;
-    __shared__ double s_cand[(NT / 32) * (AT_MAX_NMAXIMA + 1)];
+    __shared__ uint64_t s_part[3 * NT / 32];
+    __shared__ int s_kept[AT_MAX_NMAXIMA], s_nkept;
     const int tid = threadIdx.x;
 
     // the class's clusters, its largest sizes first, each to the next free block
@@ -1388,7 +1515,8 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         }
         __syncthreads();
         FIT_PROF(4)
-        block_radix_sort32(ka, va, kb, vb, (int)sz, s_hist);
+        if (!block_bucket_sort<NT>(ka, va, keys, (int)sz, s_hist))
+            block_radix_sort32(ka, va, kb, vb, (int)sz, s_hist);
         FIT_PROF(5)
 
         // cumulative weighted moments in angle order (fast/quads.c:968-1035):
@@ -1450,7 +1578,13 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         const int64_t ksz = dmin(20, sz / 12);
         if (ksz < 2) continue;
         const double nn = (double)(2 * ksz + 1);
-        double *errs = scr.errs + s0, *filt = scr.filt + s0;
+        // errors, filtered errors and maxima in shared memory where they fit:
+        // the errors where the angle keys were, the filtered errors over the
+        // sort's first buffers and histograms, then the maxima (at most one
+        // in two points) over the errors. From global memory the maxima took
+        // 11500 cycles for 700 points and 32000 for 3200, now 000 and 000.
+        double *errs = in_smem ? reinterpret_cast<double *>(s_key) : scr.errs + s0;
+        double *filt = 8 * sz <= 6 * (int64_t)sort_cap + 32 * NT ? reinterpret_cast<double *>(s_ka) : scr.filt + s0;
         // two points a thread at a time: both windows' loads before either
         // store (a store could alias the next loads)
         for (int64_t i = tid; i < sz; i += 2 * NT) {
@@ -1472,9 +1606,10 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // local maxima with wrap-around, compacted in index order: each
         // warp counts those of its own stretch, then writes them after the
         // warps' before it (two reads of filt, but only two barriers)
-        int32_t *mxi = scr.mxi + s0;
-        double *mxe = scr.mxe + s0;
+        double *mxe = in_smem ? reinterpret_cast<double *>(s_key) : scr.mxe + s0;
+        int32_t *mxi = in_smem ? reinterpret_cast<int32_t *>(fit_smem + (size_t)4 * sort_cap) : scr.mxi + s0;
         int nm;
+        if (tid == 0) s_nkept = 0;
         {
             const int n = (int)sz, lane = tid & 31, w = tid >> 5;
             const int per = ((n + NT / 32 - 1) / (NT / 32) + 31) & ~31, i0 = w * per, i1 = min(i0 + per, n);
@@ -1510,41 +1645,18 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         if (nm < 4) continue;
         if (nm > prm.max_nmaxima) {
             // The reference keeps the maxima whose error is above the
-            // (max_nmaxima+1)-th largest T (its quickselect, quads.c:827-862):
-            // e_i > T exactly when at most max_nmaxima errors are >= e_i. Up
-            // to FIT_COUNT_MAX maxima each thread counts for its own; more
-            // find T first (block_select_desc).
-            const int k = prm.max_nmaxima;
-            double *e = nm <= sort_cap ? reinterpret_cast<double *>(s_key) : filt;
-            for (int i = tid; i < nm; i += NT) e[i] = mxe[i];
-            const bool count = nm <= FIT_COUNT_MAX;
-            double T = 0.0;
-            if (count)
-                __syncthreads();
-            else
-                T = block_select_desc(e, nm, k, s_cand, &s_best);
-            int kept = 0;
-            for (int i0 = 0; i0 < nm; i0 += NT) {
-                const int i = i0 + tid;
-                uint32_t keep = 0;
-                if (i < nm) {
-                    if (count) {
-                        int ge = 0;
-                        for (int j = 0; j < nm; j++) ge += e[j] >= e[i];
-                        keep = ge <= k;
-                    } else {
-                        keep = e[i] > T;
-                    }
-                }
-                uint32_t total;
-                const uint32_t off = block_excl_scan(keep, &total, s_scan);
-                const int32_t mi = i < nm ? mxi[i] : 0;
-                __syncthreads();
-                if (keep) mxi[kept + off] = mi;
-                kept += (int)total;
+            // (max_nmaxima+1)-th largest (its quickselect, quads.c:827-862).
+            const uint64_t v = block_above<NT>(mxe, nm, prm.max_nmaxima, s_part);
+            for (int i = tid; i < nm; i += NT)
+                if (double_order(mxe[i]) >= v) s_kept[atomicAdd(&s_nkept, 1)] = mxi[i];
+            __syncthreads();
+            nm = s_nkept;
+            if (tid < nm) {
+                int before = 0;
+                for (int j = 0; j < nm; j++) before += s_kept[j] < s_kept[tid];
+                mxi[before] = s_kept[tid];
             }
             __syncthreads();
-            nm = kept;
         }
         FIT_PROF(8)
         // line fits of pairs of maxima: (a, b), a < b, and the closing pair
@@ -1712,7 +1824,7 @@ __host__ __device__ constexpr size_t fit_warp_x1(int cap, int mm) {
 // gp: the prefix arrays in global scratch (the largest warp class, where
 // 48 B per point of shared memory would leave few warps per SM)
 __host__ __device__ constexpr size_t fit_warp_smem(int cap, int mm, bool gp = false) {
-    return (size_t)8 * cap + (gp ? 0 : 48 * (cap + 1)) + fit_warp_x1(cap, mm);
+    return (size_t)8 * cap + (gp ? 0 : 48 * (cap + 2)) + fit_warp_x1(cap, mm);
 }
 
 
@@ -1799,7 +1911,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
     kernel_begin();
     constexpr int CAP = 32 * R;
     constexpr bool GP = R >= 16;  // prefix arrays in global scratch
-    constexpr int RS = CAP + 1;   // row stride of the prefix arrays (six rows on distinct banks)
+    constexpr int RS = CAP + 2;   // row stride of the prefix arrays (six rows on distinct banks, 16-byte aligned)
     extern __shared__ __align__(16) unsigned char fw_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const unsigned FULL = 0xffffffffu;
@@ -1906,6 +2018,15 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             // t, and (below the order, since the rest is distinct) the index of
             // its point. The keys live in the last prefix array until the moments.
             uint64_t *s_skey = reinterpret_cast<uint64_t *>(pm + 5 * RS);
+            // buckets, as block_bucket_sort: the counts in x1, each key's
+            // bucket and arrival in prefix array 0, the keys by bucket in 1
+            // and the buckets beside them in 2
+            constexpr int NB = CAP;
+            uint32_t *s_hist = reinterpret_cast<uint32_t *>(x1), *s_at = reinterpret_cast<uint32_t *>(pm);
+            uint64_t *s_list = reinterpret_cast<uint64_t *>(pm + RS);
+            uint16_t *s_bk = reinterpret_cast<uint16_t *>(pm + 2 * RS);
+            for (int i = lane; i < NB; i += 32) s_hist[i] = 0;
+            __syncwarp();
             int np = 32;
             while (np < n) np <<= 1;
             for (int i = lane; i < np; i += 32) {
@@ -1929,12 +2050,31 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                     const uint32_t hidx = ~(uint32_t)head;
                     key = (head & 0xffffffff00000000ull) | (uint64_t)(0xffffu - hidx) << 16 | (uint64_t)tp << 13 |
                           (uint64_t)(~(uint32_t)e & 0x1fffu);
+                    const int b = slope_bucket<NB>((uint32_t)(key >> 32));
+                    s_at[i] = (uint32_t)b << 16 | atomicAdd(s_hist + b, 1u);
                 }
                 s_skey[i] = key;
             }
             __syncwarp();
             FITW_PROF(4)
-            warp_bitonic(s_skey, np, lane);
+            if (warp_bucket_scan<NB>(s_hist, n, lane)) {
+                for (int i = lane; i < n; i += 32) {
+                    const uint32_t b = s_at[i] >> 16, j = s_hist[b] + (s_at[i] & 0xffffu);
+                    s_list[j] = s_skey[i];
+                    s_bk[j] = (uint16_t)b;
+                }
+                __syncwarp();
+                for (int j = lane; j < n; j += 32) {
+                    const uint64_t k = s_list[j];
+                    const int b = s_bk[j], q0 = (int)s_hist[b], q1 = b + 1 < NB ? (int)s_hist[b + 1] : n;
+                    int at = q0;
+                    for (int q = q0; q < q1; q++) at += s_list[q] < k;
+                    s_skey[at] = k;
+                }
+                __syncwarp();
+            } else {
+                warp_bitonic(s_skey, np, lane);
+            }
             s_order = nullptr;
         } else {
             // The angle sort (see k_fit_quads): the points laid out in (head
@@ -1987,9 +2127,34 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             }
             __syncwarp();
             FITW_PROF(4)
-            warp_radix_sort32(s_ka, s_va, s_kb, s_vb, n, s_hist, lane);
+            // buckets, as block_bucket_sort: the counts behind s_va, the list in x0
+            constexpr int NB = 256;
+            static_assert(4 * NB <= 2 * CAP, "the counts fit x1");
+            uint32_t *s_cnt = reinterpret_cast<uint32_t *>(x1 + 6 * CAP);
+            uint64_t *s_list = reinterpret_cast<uint64_t *>(x0);
+            for (int i = lane; i < NB; i += 32) s_cnt[i] = 0;
+            __syncwarp();
+#pragma unroll 4
+            for (int i = lane; i < n; i += 32) atomicAdd(s_cnt + slope_bucket<NB>(s_ka[i]), 1u);
             __syncwarp();
             s_order = s_va;
+            if (warp_bucket_scan<NB>(s_cnt, n, lane)) {
+                for (int i = lane; i < n; i += 32) {
+                    const uint32_t k = s_ka[i];
+                    s_list[atomicAdd(s_cnt + slope_bucket<NB>(k), 1u)] = (uint64_t)k << 32 | (uint32_t)i << 16 | s_va[i];
+                }
+                __syncwarp();
+                for (int j = lane; j < n; j += 32) {
+                    const uint64_t e = s_list[j];
+                    const int b = slope_bucket<NB>((uint32_t)(e >> 32)), q0 = b ? (int)s_cnt[b - 1] : 0, q1 = (int)s_cnt[b];
+                    int at = q0;
+                    for (int q = q0; q < q1; q++) at += s_list[q] < e;
+                    s_va[at] = (uint16_t)e;
+                }
+            } else {
+                warp_radix_sort32(s_ka, s_va, s_kb, s_vb, n, s_hist, lane);
+            }
+            __syncwarp();
         }
         FITW_PROF(5)
 
