@@ -982,6 +982,13 @@ __device__ uint64_t block_above(const double *e, int n, int r, uint64_t *part) {
 #define FIT_HUGE_SORT 13312
 #define FIT_HUGE_NT 512
 #define FIT_CHUNK_SMALL 256
+// Clusters of 257-512 points: a warp each when there are more than this many
+// of them, a block of 128 when not. A block is done in half the time (49000
+// instead of 87000 cycles), but keeps four warps for it: 643 of them (eight
+// 1280 x 720 frames) take the fit stage 131 us in blocks and 151 in warps, 25
+// (640 x 480) 79 and 89; 3592 (4032 x 3024) 941 and 849, 4338 (32 frames of
+// 1920 x 1080) 606 and 525. The line is two waves of the blocks (4 an SM).
+#define FIT_FEW (2 * 4 * 148)
 #define FIT_CHUNK_LARGE 512
 #define FIT_LARGE_NT 256  // threads of the largest class's blocks (two blocks an SM)
 
@@ -1025,8 +1032,8 @@ __device__ __forceinline__ int slope_bucket(uint32_t bits) {
 // before, value), and each pair's place in its bucket found by comparing it
 // with the bucket's others. The values end up in va. False (and the pairs as
 // they were) if the buckets are too uneven. hist: 8 NT counters.
-// Against the radix sort's four passes: 000 instead of 27000 cycles for 700
-// points and 128 threads, 000 instead of 47500 for 3200 and 256.
+// Against the radix sort's four passes: 9900 instead of 27400 cycles for 700
+// points and 128 threads, 21000 instead of 47600 for 3200 and 256.
 template <int NT>
 __device__ __forceinline__ bool block_bucket_sort(const uint32_t *ka, uint16_t *va, uint64_t *list, int n,
                                                   uint32_t *hist) {
@@ -1226,7 +1233,7 @@ extern "C" int at_fit_prof_copy(void *dst, int n) {
 
 // ---------------------------------------------------------------------------
 // The fit's size classes: clusters of at most 128, 256, 512 points (a warp
-// each), at most 1024 (a block of 128), at most 6144 (a block of 256), and
+// each; few of the last: see FIT_FEW), at most 1024 (a block of 128), at most 6144 (a block of 256), and
 // larger (a block of 512). A class's clusters are listed by size in a few
 // buckets, and its blocks take those of the largest bucket first, so that a
 // long cluster does not start last (unsorted, the 513-1024 class took 175
@@ -1298,6 +1305,52 @@ static_assert(AT_MAX_NMAXIMA <= 16, "the 4-subset table covers 16 maxima");
 
 __host__ __device__ constexpr int binom4(int n) { return n < 4 ? 0 : n * (n - 1) * (n - 2) * (n - 3) / 24; }
 
+// The quad of four lines (x, y, nx, ny; line i and its fit's error in lane i
+// of the warp, i < 4): its corners (corner i in lane i), and whether it passes
+// the fit, area and convexity gates (fast/quads.c:1079-1125). A lane a corner:
+// one thread for all four took 5000 cycles.
+__device__ __forceinline__ bool quad_of(int lane, const double ln[4], double lmse, const GpuParams &prm, int tag_width,
+                                        float p[2]) {
+    const unsigned FULL = 0xffffffffu;
+    const int nx = (lane + 1) & 3;
+    double lj[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) lj[k] = __shfl_sync(FULL, ln[k], nx);
+    const double a00 = ln[3], a01 = -lj[3], a10 = -ln[2], a11 = lj[2];
+    const double b0 = -ln[0] + lj[0], b1 = -ln[1] + lj[1];
+    const double det = a00 * a11 - a10 * a01;
+    if (__any_sync(FULL, lane < 4 && (lmse > prm.max_mse || fabs(det) < 0.001))) return false;
+    const double w00 = a11 / det, w01 = -a01 / det;
+    const double l0 = w00 * b0 + w01 * b1;
+    p[0] = (float)(ln[0] + l0 * a00);
+    p[1] = (float)(ln[1] + l0 * a10);
+    float q[4][2];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        q[i][0] = __shfl_sync(FULL, p[0], (lane + i) & 3);
+        q[i][1] = __shfl_sync(FULL, p[1], (lane + i) & 3);
+    }
+    // the triangles (0, 1, 2) and (2, 3, 0) by Heron: lane t the one that
+    // starts at corner t (lanes 0 and 2 count)
+    double len[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const int ib = i == 2 ? 0 : i + 1;
+        const double ddx = (double)__fsub_rn(q[ib][0], q[i][0]), ddy = (double)__fsub_rn(q[ib][1], q[i][1]);
+        len[i] = sqrt(ddx * ddx + ddy * ddy);
+    }
+    const double pp = (len[0] + len[1] + len[2]) / 2.0;
+    const double tri = sqrt(pp * (pp - len[0]) * (pp - len[1]) * (pp - len[2]));
+    const double area = __shfl_sync(FULL, tri, 0) + __shfl_sync(FULL, tri, 2);
+    // convexity at corner lane + 1
+    const double dx1 = (double)__fsub_rn(q[1][0], q[0][0]), dy1 = (double)__fsub_rn(q[1][1], q[0][1]);
+    const double dx2 = (double)__fsub_rn(q[2][0], q[1][0]), dy2 = (double)__fsub_rn(q[2][1], q[1][1]);
+    const double den = sqrt((dx1 * dx1 + dy1 * dy1) * (dx2 * dx2 + dy2 * dy2));
+    const double cs = (dx1 * dx2 + dy1 * dy2) / den;
+    const bool bad = den == 0.0 || (cs > prm.max_dot || cs < -prm.max_dot) || dx1 * dy2 < dy1 * dx2;
+    return !__any_sync(FULL, lane < 4 && bad) && !(area < 0.95 * (double)tag_width * (double)tag_width);
+}
+
 template <int NT>
 __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit_quads(const FrameDesc *frames, GpuParams prm, const uint8_t *qim,
                                                    const uint64_t *pts, const uint32_t *cstart,
@@ -1326,11 +1379,12 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
     __shared__ uint64_t s_part[3 * NT / 32];
     __shared__ int s_kept[AT_MAX_NMAXIMA], s_nkept;
     const int tid = threadIdx.x;
+    const int low = NT == 128 && scr.counts[2] <= FIT_FEW ? bottom - 1 : bottom;
 
     // the class's clusters, its largest sizes first, each to the next free block
     for (;;) {
         __syncthreads();
-        if (tid == 0) s_next = fit_next(scr, nclusters, top, bottom);
+        if (tid == 0) s_next = fit_next(scr, nclusters, top, low);
         __syncthreads();
         if (s_next == 0xffffffffu) break;
         const int64_t c = s_next;
@@ -1582,7 +1636,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // the errors where the angle keys were, the filtered errors over the
         // sort's first buffers and histograms, then the maxima (at most one
         // in two points) over the errors. From global memory the maxima took
-        // 11500 cycles for 700 points and 32000 for 3200, now 000 and 000.
+        // 11500 cycles for 700 points and 32000 for 3200, now 10000 and 16000.
         double *errs = in_smem ? reinterpret_cast<double *>(s_key) : scr.errs + s0;
         double *filt = 8 * sz <= 6 * (int64_t)sort_cap + 32 * NT ? reinterpret_cast<double *>(s_ka) : scr.filt + s0;
         // two points a thread at a time: both windows' loads before either
@@ -1741,65 +1795,22 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             __syncthreads();
             if (tid == 0) s_best = be;
         }
-        if (tid == 0) {
+        if (tid < 32) {
             const double inf = __longlong_as_double(0x7ff0000000000000ll);
             const double best = s_best;
-            bool ok = best != inf && best / (double)sz < prm.max_mse;
-            GpuQuad q;
-            q.reversed_border = rev;
-            q.frame = cframe[c];
-            double lines[4][4];
-            for (int i = 0; ok && i < 4; i++) {
-                for (int k = 0; k < 4; k++) lines[i][k] = s_lines[i][k];
-                if (s_lmse[i] > prm.max_mse) ok = false;
-            }
-            for (int i = 0; ok && i < 4; i++) {
-                int j = (i + 1) & 3;
-                double a00 = lines[i][3], a01 = -lines[j][3], a10 = -lines[i][2], a11 = lines[j][2];
-                double b0 = -lines[i][0] + lines[j][0], b1 = -lines[i][1] + lines[j][1];
-                double det = a00 * a11 - a10 * a01;
-                if (fabs(det) < 0.001) {
-                    ok = false;
-                    break;
-                }
-                double w00 = a11 / det, w01 = -a01 / det;
-                double l0 = w00 * b0 + w01 * b1;
-                q.p[i][0] = (float)(lines[i][0] + l0 * a00);
-                q.p[i][1] = (float)(lines[i][1] + l0 * a10);
-            }
-            if (ok) {
-                // area of triangles (0,1,2) and (2,3,0) by Heron (quads.c:1094-1110)
-                const int tri[2][4] = {{0, 1, 2, 0}, {2, 3, 0, 2}};
-                double area = 0.0;
-                for (int t = 0; t < 2; t++) {
-                    double len[3];
-                    for (int i = 0; i < 3; i++) {
-                        int ia = tri[t][i], ib = tri[t][i + 1];
-                        double ddx = (double)__fsub_rn(q.p[ib][0], q.p[ia][0]);
-                        double ddy = (double)__fsub_rn(q.p[ib][1], q.p[ia][1]);
-                        len[i] = sqrt(ddx * ddx + ddy * ddy);
+            if (best != inf && best / (double)sz < prm.max_mse) {
+                const double *l = s_lines[tid & 3];
+                const double ln[4] = {l[0], l[1], l[2], l[3]};
+                float p[2];
+                if (quad_of(tid, ln, s_lmse[tid & 3], prm, f.tag_width, p) && tid < 4) {
+                    quads[c].p[tid][0] = p[0];
+                    quads[c].p[tid][1] = p[1];
+                    if (tid == 0) {
+                        quads[c].reversed_border = rev;
+                        quads[c].frame = cframe[c];
+                        quad_ok[c] = 1;
                     }
-                    double pp = (len[0] + len[1] + len[2]) / 2.0;
-                    area = area + sqrt(pp * (pp - len[0]) * (pp - len[1]) * (pp - len[2]));
                 }
-                if (area < 0.95 * (double)f.tag_width * (double)f.tag_width) ok = false;
-            }
-            for (int i = 0; ok && i < 4; i++) {
-                // convexity (quads.c:1112-1124)
-                int i0 = i, i1 = (i + 1) & 3, i2 = (i + 2) & 3;
-                double dx1 = (double)__fsub_rn(q.p[i1][0], q.p[i0][0]), dy1 = (double)__fsub_rn(q.p[i1][1], q.p[i0][1]);
-                double dx2 = (double)__fsub_rn(q.p[i2][0], q.p[i1][0]), dy2 = (double)__fsub_rn(q.p[i2][1], q.p[i1][1]);
-                double den = sqrt((dx1 * dx1 + dy1 * dy1) * (dx2 * dx2 + dy2 * dy2));
-                if (den == 0.0) {
-                    ok = false;
-                    break;
-                }
-                double cs = (dx1 * dx2 + dy1 * dy2) / den;
-                if ((cs > prm.max_dot || cs < -prm.max_dot) || dx1 * dy2 < dy1 * dx2) ok = false;
-            }
-            if (ok) {
-                quads[c] = q;
-                quad_ok[c] = 1;
             }
             FIT_PROF(10)
 #ifdef AT_FIT_PROF
@@ -1812,8 +1823,8 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
 
 // ---------------------------------------------------------------------------
 // Clusters of at most 32 * R points: one warp each, FIT_WPB per block, no
-// block barriers. The same steps as k_fit_quads; the angle sort is a bitonic
-// sort in registers, the prefix moments stay in shared memory.
+// block barriers. The same steps as k_fit_quads; up to 256 points the prefix
+// moments stay in shared memory.
 #define FIT_WPB 2
 
 // per warp: six prefix arrays, then region x0 (angle keys; errors; the
@@ -1928,6 +1939,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
            *s_pny = s_pnx + mm * mm;
     const double inf = __longlong_as_double(0x7ff0000000000000ll);
 
+    if (R == 16 && scr.counts[2] <= FIT_FEW) return;  // a block of 128 each
     // one resident wave of warps, each taking the class's next cluster
     // from a shared counter as it finishes one (no static share to wait on)
     for (;;) {
@@ -2007,9 +2019,10 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         const int rev = okrev >> 1;
         FITW_PROF(3)
 
-        // The angle sort (see k_fit_quads). Up to 256 points: a bitonic
-        // sort of packed keys; above: the points laid out in (head index,
-        // place) order and a stable radix sort by the head's slope bits.
+        // The angle sort (see k_fit_quads). Up to 256 points: packed keys by
+        // buckets (177 points: 4900 cycles, a bitonic sort 19900); above: the
+        // points laid out in (head index, place) order, then by buckets
+        // (360 points: 22000 cycles, four radix passes 33000).
         const uint16_t *s_order;  // point index of each sorted position
         if constexpr (R <= 8) {
             // The angle sort (see k_fit_quads): position i of leaf (lo, len)
@@ -2091,10 +2104,11 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             uint32_t *s_kb = reinterpret_cast<uint32_t *>(sb);
             uint16_t *s_vb = reinterpret_cast<uint16_t *>(sb + 4 * CAP);
             uint32_t *s_hist = reinterpret_cast<uint32_t *>(sb + (GP ? 6 : 8) * CAP);
-            for (int p = lane; p < n; p += 32) {
-                int lo, len;
-                leaf_of32(n, p, lo, len);
-                if (p != lo) continue;
+            // (the leaves found 32 points at a time, queued behind s_va, and
+            // laid out 32 leaves at a time)
+            uint32_t *lq = reinterpret_cast<uint32_t *>(x1 + 6 * CAP);
+            auto arrange = [&](uint32_t lf) {
+                const int lo = (int)(lf >> 8), len = (int)(lf & 255);
                 uint64_t a[5];
     #pragma unroll
                 for (int t = 0; t < 5; t++) a[t] = t < len ? s_akey[lo + t] : ~0ull;
@@ -2124,7 +2138,23 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                     s_ka[pos] = hkey[t];
                     s_va[pos] = (uint16_t)~(uint32_t)a[t];
                 }
+            };
+            int qn = 0;
+            for (int p0 = 0; p0 < n; p0 += 32) {
+                const int p = p0 + lane;
+                int lo = -1, len = 0;
+                if (p < n) leaf_of32(n, p, lo, len);
+                const uint32_t bal = __ballot_sync(FULL, lo == p);
+                if (lo == p) lq[qn + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)lo << 8 | (uint32_t)len;
+                qn += __popc(bal);
+                __syncwarp();
+                if (qn >= 32) {
+                    qn -= 32;
+                    arrange(lq[qn + lane]);
+                    __syncwarp();
+                }
             }
+            if (lane < qn) arrange(lq[lane]);
             __syncwarp();
             FITW_PROF(4)
             // buckets, as block_bucket_sort: the counts behind s_va, the list in x0
@@ -2357,64 +2387,13 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             const int ma = bo >> (12 - 4 * lane) & 15, mb = bo >> (12 - 4 * ((lane + 1) & 3)) & 15;
             line_of(seg_moments(mo, all, s_mxi[ma], s_mxi[mb]), ln, &lmse);
         }
-        double lines[4][4], lm[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            lm[i] = __shfl_sync(FULL, lmse, i);
-#pragma unroll
-            for (int k = 0; k < 4; k++) lines[i][k] = __shfl_sync(FULL, ln[k], i);
-        }
-        if (lane == 0) {
-            bool ok = true;
-            for (int i = 0; i < 4; i++)
-                if (lm[i] > prm.max_mse) ok = false;
-            GpuQuad q;
-            q.reversed_border = rev;
-            q.frame = cframe[c];
-            for (int i = 0; ok && i < 4; i++) {
-                int j = (i + 1) & 3;
-                double a00 = lines[i][3], a01 = -lines[j][3], a10 = -lines[i][2], a11 = lines[j][2];
-                double b0 = -lines[i][0] + lines[j][0], b1 = -lines[i][1] + lines[j][1];
-                double det = a00 * a11 - a10 * a01;
-                if (fabs(det) < 0.001) {
-                    ok = false;
-                    break;
-                }
-                double w00 = a11 / det, w01 = -a01 / det;
-                double l0 = w00 * b0 + w01 * b1;
-                q.p[i][0] = (float)(lines[i][0] + l0 * a00);
-                q.p[i][1] = (float)(lines[i][1] + l0 * a10);
-            }
-            if (ok) {
-                const int tri[2][4] = {{0, 1, 2, 0}, {2, 3, 0, 2}};
-                double area = 0.0;
-                for (int t = 0; t < 2; t++) {
-                    double len[3];
-                    for (int i = 0; i < 3; i++) {
-                        int ia = tri[t][i], ib = tri[t][i + 1];
-                        double ddx = (double)__fsub_rn(q.p[ib][0], q.p[ia][0]);
-                        double ddy = (double)__fsub_rn(q.p[ib][1], q.p[ia][1]);
-                        len[i] = sqrt(ddx * ddx + ddy * ddy);
-                    }
-                    double pp = (len[0] + len[1] + len[2]) / 2.0;
-                    area = area + sqrt(pp * (pp - len[0]) * (pp - len[1]) * (pp - len[2]));
-                }
-                if (area < 0.95 * (double)f.tag_width * (double)f.tag_width) ok = false;
-            }
-            for (int i = 0; ok && i < 4; i++) {
-                int i0 = i, i1 = (i + 1) & 3, i2 = (i + 2) & 3;
-                double dx1 = (double)__fsub_rn(q.p[i1][0], q.p[i0][0]), dy1 = (double)__fsub_rn(q.p[i1][1], q.p[i0][1]);
-                double dx2 = (double)__fsub_rn(q.p[i2][0], q.p[i1][0]), dy2 = (double)__fsub_rn(q.p[i2][1], q.p[i1][1]);
-                double den = sqrt((dx1 * dx1 + dy1 * dy1) * (dx2 * dx2 + dy2 * dy2));
-                if (den == 0.0) {
-                    ok = false;
-                    break;
-                }
-                double cs = (dx1 * dx2 + dy1 * dy2) / den;
-                if ((cs > prm.max_dot || cs < -prm.max_dot) || dx1 * dy2 < dy1 * dx2) ok = false;
-            }
-            if (ok) {
-                quads[c] = q;
+        float p[2];
+        if (quad_of(lane, ln, lmse, prm, f.tag_width, p) && lane < 4) {
+            quads[c].p[lane][0] = p[0];
+            quads[c].p[lane][1] = p[1];
+            if (lane == 0) {
+                quads[c].reversed_border = rev;
+                quads[c].frame = cframe[c];
                 quad_ok[c] = 1;
             }
         }

@@ -53,3 +53,53 @@ def test_quads_of_large_clusters(name):
         name.split("-")[0]]
     fitted = sizes[[q[2] for q in r.quads]]
     assert ((fitted >= lo) & (fitted <= hi)).any()
+
+
+def _same(img, **params):
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0, **params)
+    got = [d.key() for d in det.detect(img)]
+    r = O.detect(img, [H.oracle_family("tag36h11")], [2], O.default_params(quad_decimate=1.0, **params),
+                 order=O.ORDER_CANON)
+    quads = det.diag("quads")
+    assert len(quads) == len(r.quads)
+    ref = np.array([q[0] for q in r.quads], np.float32).reshape(-1, 4, 2)
+    assert np.array_equal(quads["p"].view(np.uint32), ref.view(np.uint32))
+    assert got == r.dets
+    return r
+
+
+@pytest.mark.parametrize("rows", [33, 36])
+def test_few_and_many_mid_clusters(rows):
+    """Clusters of 257-512 points: a block each up to 1184, a warp each above."""
+    img = np.full((rows * 50 + 16, rows * 50 + 16), 200)
+    for y in range(rows):
+        for x in range(rows):
+            s = 33 + (7 * x + 3 * y) % 10
+            img[8 + 50 * y : 8 + 50 * y + s, 8 + 50 * x : 8 + 50 * x + s] = 40
+    r = _same(img.astype(np.uint8))
+    sizes = np.diff(r.cstart)
+    mid = ((sizes > 256) & (sizes <= 512)).sum()
+    assert len(r.quads) > 900 and (mid <= 1184 if rows == 33 else mid > 1184)
+
+
+def _share(pts, buckets):
+    """Points in a point's bucket on average, by the points' own slopes."""
+    x, y = (pts & 0xFFFF).astype(np.float32), (pts >> 16 & 0xFFFF).astype(np.float32)
+    dx = x - np.float32((float(x.min()) + float(x.max())) * 0.5 + 0.05118)
+    dy = y - np.float32((float(y.min()) + float(y.max())) * 0.5 - 0.028581)
+    turn = (np.arctan2(dy, dx) / (np.pi / 2)) % 4
+    t = np.tan((turn % 1) * (np.pi / 2))
+    n = np.bincount((np.floor(turn) + 1 - 1 / (1 + t)).__mul__(buckets // 4).astype(int))
+    return (n.astype(float) ** 2).sum() / len(pts)
+
+
+@pytest.mark.parametrize("h,w,buckets", [(1, 62, 256), (2, 124, 256), (3, 250, 1024), (4, 250, 1024), (8, 1500, 2048),
+                                         (20, 1500, 2048), (24, 3200, 4096), (30, 3900, 4096)])
+def test_uneven_angles(h, w, buckets):
+    """Bars so long that most points share a few angles: the sort falls back
+    from buckets to the one it replaced, in every class."""
+    img = np.full((h + 60, w + 80), 200.0)
+    img[30 : 30 + h, 40 : 40 + w] = 20
+    img += np.random.default_rng(1).normal(0, 0.4, img.shape)
+    r = _same(np.clip(img, 0, 255).astype(np.uint8))
+    assert max(_share(r.pts[a:b], buckets) for a, b in zip(r.cstart[:-1], r.cstart[1:])) > 17
