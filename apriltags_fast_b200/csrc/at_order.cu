@@ -183,6 +183,11 @@ __global__ void __launch_bounds__(256) k_ref_targets(const FrameDesc *frames, in
 //   trow[row0 + y] = count | (the last-column link joins a target run) << 31
 // and each of them (and each link's last-column node) a root of the forest.
 
+// A row's targets are looked up a run a lane first (its labels lie side by
+// side); a lane that looked up its word's runs one by one waited for each
+// (4032 x 3024: 155 us, so 000 us; 32 frames of 1920 x 1080: 30 and 000).
+#define REF_ROW_RUNS ((REF_PCAP + 32) & ~31)  // runs of a row, at most
+
 #define REF_INF 0xffffffffu  // the time of a root: never joined
 
 __device__ __forceinline__ void ref_node_init(const RefOrder &ref, uint32_t node, uint32_t px) {
@@ -201,17 +206,15 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
     const FrameDesc fd = frames[f];
     for (int i = threadIdx.x; i < REF_HASH; i += blockDim.x) s_key[i] = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        const uint32_t nt = ref.nt[f];
-        for (uint32_t t = 0; t < nt; t++) {
-            const uint32_t label = ref.tlabel[(int64_t)f * AT_REF_MAXT + t];
-            uint32_t h = ref_hash(label) & (REF_HASH - 1);
-            while (s_key[h]) h = (h + 1) & (REF_HASH - 1);
-            s_key[h] = label + 1;
-            s_idx[h] = (uint8_t)t;
-        }
+    for (uint32_t t = threadIdx.x; t < ref.nt[f]; t += blockDim.x) {
+        const uint32_t label = ref.tlabel[(int64_t)f * AT_REF_MAXT + t];
+        uint32_t h = ref_hash(label) & (REF_HASH - 1);
+        while (atomicCAS(s_key + h, 0u, label + 1)) h = (h + 1) & (REF_HASH - 1);  // (the table is half empty)
+        s_idx[h] = (uint8_t)t;
     }
     __syncthreads();
+    extern __shared__ uint8_t s_target[];  // by run of the warp's row
+    uint8_t *mine = s_target + (threadIdx.x >> 5) * REF_ROW_RUNS;
     const int lane = threadIdx.x & 31;
     const int64_t wpb = blockDim.x >> 5;
     const int qw = fd.qw, nw = (qw + 31) / 32;
@@ -219,6 +222,12 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
         const int64_t base = fd.node_off + y * qw;
         const RowWord *row = words + fd.word_off + y * nw;
         uint32_t cnt = 0;
+        // the row's runs, 32 at a time: their targets (a run of no label
+        // looks up what no table holds)
+        const uint32_t nr = row_nruns[fd.row0 + y];
+        __syncwarp();
+        for (uint32_t k = lane; k < nr; k += 32) mine[k] = (uint8_t)ref_lookup(s_key, s_idx, runs.lab[base + k]);
+        __syncwarp();
         for (int i0 = 0; i0 < nw; i0 += 32) {
             // a word a lane: its target runs, then (after the lanes before) their entries
             const int i = i0 + lane;
@@ -228,15 +237,13 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
                 w = row[i];
                 uint32_t k = w.before;
                 for (uint32_t m = w.starts; m; m &= m - 1, k++)
-                    if (((w.white | w.black) & m & (0u - m)) &&
-                        ref_lookup(s_key, s_idx, runs.lab[base + k]) != REF_NONE)
-                        tm |= m & (0u - m);
+                    if (((w.white | w.black) & m & (0u - m)) && mine[k] != REF_NONE) tm |= m & (0u - m);
             }
             uint32_t total;
             uint32_t at = cnt + warp_excl_scan(__popc(tm), &total);
             for (uint32_t m = tm; m; m &= m - 1, at++) {
                 const int c = __ffs(m) - 1;
-                const uint32_t k = run_at(w, c), t = ref_lookup(s_key, s_idx, runs.lab[base + k]);
+                const uint32_t k = run_at(w, c), t = mine[k];
                 const bool white = w.white >> c & 1u;
                 // the run's end: the first later column of another value or the last run column
                 int e = 32 * i + c + 1;
@@ -261,7 +268,7 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
             if (y >= 1) {
                 auto white = [&](const RowWord *r, int x) { return r[x >> 5].white >> (x & 31) & 1u; };
                 link = white(row, qw - 2) && white(row - nw, qw - 1) && !white(row - nw, qw - 2) &&
-                       ref_lookup(s_key, s_idx, runs.lab[base + row_nruns[fd.row0 + y] - 1]) != REF_NONE;
+                       mine[nr - 1] != REF_NONE;
             }
             if (link) ref_node_init(ref, (uint32_t)(fd.node_off + (int64_t)qw * fd.qh + y - 1), 1u);
             ref.trow[fd.row0 + y] = cnt | (link ? 0x80000000u : 0u);
@@ -456,212 +463,212 @@ __global__ void __launch_bounds__(REF_ROOT_THREADS) k_ref_root(const FrameDesc *
     const FrameDesc fd = frames[f];
     const int tid = threadIdx.x, lane = tid & 31;
     for (uint32_t t = blockIdx.x; t < ref.nt[f]; t += gridDim.x) {
-    __syncthreads();
-    const uint32_t off = (uint32_t)fd.node_off, qw = (uint32_t)fd.qw;
-    const uint32_t vbase = off + (uint32_t)((int64_t)fd.qw * fd.qh);
-    uint32_t *gain = ref.hist + fd.row0 * AT_REF_MAXT + (int64_t)t * fd.qh;
-    uint32_t x = ref.tlabel[(int64_t)f * AT_REF_MAXT + t], root = 0xffffffffu;
-    uint32_t Z = ref.tpx[(int64_t)f * AT_REF_MAXT + t];
-    // the prefix sums of gain over rows [y0, y1]
-    auto scan_gain = [&](int y0, int y1) {
-        uint32_t base = 0;
-        for (int r0 = y0; r0 <= y1; r0 += REF_ROOT_THREADS) {
-            const int r = r0 + tid;
-            const uint32_t v = r <= y1 ? gain[r] : 0u;
-            uint32_t total;
-            const uint32_t o = block_excl_scan(v, &total, s_scan);
-            if (r <= y1) gain[r] = base + o + v;
-            base += total;
-        }
         __syncthreads();
-    };
-    if (x >= vbase) {  // a last-column pixel alone
-        root = x;
-    } else {
-        int ymax = fd.qh - 1, y0 = (int)((x - off) / qw);
-        bool part = false;
-        uint32_t lim = REF_INF, gen = 0;
-        uint32_t lx = ref.len[x];
-        scan_gain(y0, ymax);
-        for (int guard = 0; guard < (1 << 16); guard++) {
-            // the first row (y0 - 1: x alone) that leaves more than Z / 2:
-            // each warp narrows [lo, hi) by 32 probes at a time
-            int lo = y0 - 1, hi = ymax + 1;
-            while (lo < hi) {
-                const int step = (hi - lo + 31) / 32;
-                const int r = lo + lane * step;
-                const bool over = r >= hi || 2ull * (lx + (r < y0 ? 0u : gain[r])) > Z;
-                const uint32_t bal = __ballot_sync(0xffffffffu, over);
-                const int k = bal ? __ffs(bal) - 1 : 32;
-                const int nhi = k == 32 ? hi : min(hi, lo + k * step);
-                lo = k == 0 ? lo : lo + (k - 1) * step + 1;
-                hi = nhi;
-            }
-            if (lo == y0 - 1) {
-                root = x;
-                break;
-            }
-            if (lo <= ymax && (lo < ymax || part)) {
-                Z = lx + gain[lo];
-                ymax = lo;
-                part = false;
-                continue;
-            }
-            // row r, event by event: those before lim that end in x's set
-            const int r = part ? ymax + 1 : ymax;
-            const uint32_t L = part ? lim : REF_INF;
-            const uint32_t rb = off + (uint32_t)r * qw, ra = rb - qw;
-            const uint32_t tr = ref.trow[fd.row0 + r], n = tr & 0x7fffffffu;
-            uint32_t base = lx + (r - 1 < y0 ? 0u : gain[r - 1]);
-            __syncthreads();
-            if (tid == 0) s_ev = s_evj = REF_INF;
-            __syncthreads();
-            gen++;
-            for (uint32_t j0 = 0; j0 < n; j0 += REF_ROOT_THREADS) {
-                const uint32_t j = j0 + tid;
-                uint32_t d = 0, i = 0;
-                if (j < n) {
-                    const uint64_t e = ref.tlist[rb + j];
-                    i = rb + ref_col(e);
-                    if (i < L && (uint32_t)(e >> 56) == t && ref.par[i] == ((uint64_t)i << 32 | x)) {
-                        d = ref_len(e);
-                        const uint32_t tc = ref.tch[rb + j];
-                        if (tc != 0xffffffffu)
-                            for (uint32_t k = tc & 0xffffu; k <= tc >> 16; k++) {
-                                const uint64_t b = ref.tlist[ra + k];
-                                if ((b ^ e) >> 48 & 0xff) continue;
-                                const uint32_t c = ref_climb(ref, ra + ref_col(b), i - 1);
-                                // each set once (only this thread meets it)
-                                if (c == x || ref.stamp[c] == gen) continue;
-                                ref.stamp[c] = gen;
-                                d += ref.sum[c];
-                            }
-                    }
-                }
+        const uint32_t off = (uint32_t)fd.node_off, qw = (uint32_t)fd.qw;
+        const uint32_t vbase = off + (uint32_t)((int64_t)fd.qw * fd.qh);
+        uint32_t *gain = ref.hist + fd.row0 * AT_REF_MAXT + (int64_t)t * fd.qh;
+        uint32_t x = ref.tlabel[(int64_t)f * AT_REF_MAXT + t], root = 0xffffffffu;
+        uint32_t Z = ref.tpx[(int64_t)f * AT_REF_MAXT + t];
+        // the prefix sums of gain over rows [y0, y1]
+        auto scan_gain = [&](int y0, int y1) {
+            uint32_t base = 0;
+            for (int r0 = y0; r0 <= y1; r0 += REF_ROOT_THREADS) {
+                const int r = r0 + tid;
+                const uint32_t v = r <= y1 ? gain[r] : 0u;
                 uint32_t total;
-                const uint32_t o = block_excl_scan(d, &total, s_scan);
-                if (d && 2ull * (base + o) <= Z && 2ull * (base + o + d) > Z) {  // one thread at most
-                    s_ev = i;
-                    s_evj = j;
-                    s_before = base + o;
-                }
-                __syncthreads();
-                if (s_ev != REF_INF) break;
+                const uint32_t o = block_excl_scan(v, &total, s_scan);
+                if (r <= y1) gain[r] = base + o + v;
                 base += total;
             }
-            if (s_ev == REF_INF) {
-                // the row's last-column link: one pixel, which takes the
-                // root only from a set of one pixel
-                const uint32_t wl = rb + qw - 1, vn = vbase + (uint32_t)r - 1;
-                if (!(tr >> 31) || wl >= L || ref.par[vn] != ((uint64_t)wl << 32 | x) || 2ull * (base + 1) <= Z) break;
-                if (base <= 1) {
-                    root = vn;
+            __syncthreads();
+        };
+        if (x >= vbase) {  // a last-column pixel alone
+            root = x;
+        } else {
+            int ymax = fd.qh - 1, y0 = (int)((x - off) / qw);
+            bool part = false;
+            uint32_t lim = REF_INF, gen = 0;
+            uint32_t lx = ref.len[x];
+            scan_gain(y0, ymax);
+            for (int guard = 0; guard < (1 << 16); guard++) {
+                // the first row (y0 - 1: x alone) that leaves more than Z / 2:
+                // each warp narrows [lo, hi) by 32 probes at a time
+                int lo = y0 - 1, hi = ymax + 1;
+                while (lo < hi) {
+                    const int step = (hi - lo + 31) / 32;
+                    const int r = lo + lane * step;
+                    const bool over = r >= hi || 2ull * (lx + (r < y0 ? 0u : gain[r])) > Z;
+                    const uint32_t bal = __ballot_sync(0xffffffffu, over);
+                    const int k = bal ? __ffs(bal) - 1 : 32;
+                    const int nhi = k == 32 ? hi : min(hi, lo + k * step);
+                    lo = k == 0 ? lo : lo + (k - 1) * step + 1;
+                    hi = nhi;
+                }
+                if (lo == y0 - 1) {
+                    root = x;
                     break;
                 }
-                Z = base;
+                if (lo <= ymax && (lo < ymax || part)) {
+                    Z = lx + gain[lo];
+                    ymax = lo;
+                    part = false;
+                    continue;
+                }
+                // row r, event by event: those before lim that end in x's set
+                const int r = part ? ymax + 1 : ymax;
+                const uint32_t L = part ? lim : REF_INF;
+                const uint32_t rb = off + (uint32_t)r * qw, ra = rb - qw;
+                const uint32_t tr = ref.trow[fd.row0 + r], n = tr & 0x7fffffffu;
+                uint32_t base = lx + (r - 1 < y0 ? 0u : gain[r - 1]);
+                __syncthreads();
+                if (tid == 0) s_ev = s_evj = REF_INF;
+                __syncthreads();
+                gen++;
+                for (uint32_t j0 = 0; j0 < n; j0 += REF_ROOT_THREADS) {
+                    const uint32_t j = j0 + tid;
+                    uint32_t d = 0, i = 0;
+                    if (j < n) {
+                        const uint64_t e = ref.tlist[rb + j];
+                        i = rb + ref_col(e);
+                        if (i < L && (uint32_t)(e >> 56) == t && ref.par[i] == ((uint64_t)i << 32 | x)) {
+                            d = ref_len(e);
+                            const uint32_t tc = ref.tch[rb + j];
+                            if (tc != 0xffffffffu)
+                                for (uint32_t k = tc & 0xffffu; k <= tc >> 16; k++) {
+                                    const uint64_t b = ref.tlist[ra + k];
+                                    if ((b ^ e) >> 48 & 0xff) continue;
+                                    const uint32_t c = ref_climb(ref, ra + ref_col(b), i - 1);
+                                    // each set once (only this thread meets it)
+                                    if (c == x || ref.stamp[c] == gen) continue;
+                                    ref.stamp[c] = gen;
+                                    d += ref.sum[c];
+                                }
+                        }
+                    }
+                    uint32_t total;
+                    const uint32_t o = block_excl_scan(d, &total, s_scan);
+                    if (d && 2ull * (base + o) <= Z && 2ull * (base + o + d) > Z) {  // one thread at most
+                        s_ev = i;
+                        s_evj = j;
+                        s_before = base + o;
+                    }
+                    __syncthreads();
+                    if (s_ev != REF_INF) break;
+                    base += total;
+                }
+                if (s_ev == REF_INF) {
+                    // the row's last-column link: one pixel, which takes the
+                    // root only from a set of one pixel
+                    const uint32_t wl = rb + qw - 1, vn = vbase + (uint32_t)r - 1;
+                    if (!(tr >> 31) || wl >= L || ref.par[vn] != ((uint64_t)wl << 32 | x) || 2ull * (base + 1) <= Z) break;
+                    if (base <= 1) {
+                        root = vn;
+                        break;
+                    }
+                    Z = base;
+                    ymax = r - 1;
+                    part = true;
+                    lim = wl;
+                    continue;
+                }
+                // the calls of that event, by warp 0: run i's set against each
+                // set it meets, in order; the larger keeps its root, run i's
+                // side only with strictly more
+                const uint32_t i = s_ev, before = s_before;
+                gen++;
+                if (tid < 32) {
+                    const uint64_t e = ref.tlist[rb + s_evj];
+                    const uint32_t tc = ref.tch[rb + s_evj];
+                    uint32_t win = i, winz = ref_len(e), z = winz;
+                    if (tc != 0xffffffffu)
+                        for (uint32_t k0 = tc & 0xffffu; k0 <= tc >> 16; k0 += 32) {
+                            const uint32_t k = k0 + lane;
+                            uint32_t c = REF_INF, zc = 0;
+                            if (k <= tc >> 16) {
+                                const uint64_t b = ref.tlist[ra + k];
+                                if (!((b ^ e) >> 48 & 0xff)) {
+                                    c = ref_climb(ref, ra + ref_col(b), i - 1);
+                                    zc = c == x ? before : ref.sum[c];
+                                    if (*(volatile uint32_t *)(ref.stamp + c) == gen) c = REF_INF;  // met already
+                                }
+                            }
+                            const uint32_t peers = __match_any_sync(0xffffffffu, c);
+                            const bool first = c != REF_INF && lane == __ffs(peers) - 1;
+                            if (first) *(volatile uint32_t *)(ref.stamp + c) = gen;
+                            uint32_t bal = __ballot_sync(0xffffffffu, first);
+                            __syncwarp();
+                            while (bal) {
+                                const int l = __ffs(bal) - 1;
+                                bal &= bal - 1;
+                                const uint32_t cl = __shfl_sync(0xffffffffu, c, l), zl = __shfl_sync(0xffffffffu, zc, l);
+                                if (z <= zl) {
+                                    win = cl;
+                                    winz = zl;
+                                }
+                                z += zl;
+                            }
+                        }
+                    if (lane == 0) {
+                        s_win = win;
+                        s_winz = winz;
+                    }
+                }
+                __syncthreads();
+                const uint32_t win = s_win;
+                if (win == i) {
+                    root = i;
+                    break;
+                }
+                Z = s_winz;
                 ymax = r - 1;
                 part = true;
-                lim = wl;
-                continue;
-            }
-            // the calls of that event, by warp 0: run i's set against each
-            // set it meets, in order; the larger keeps its root, run i's
-            // side only with strictly more
-            const uint32_t i = s_ev, before = s_before;
-            gen++;
-            if (tid < 32) {
-                const uint64_t e = ref.tlist[rb + s_evj];
-                const uint32_t tc = ref.tch[rb + s_evj];
-                uint32_t win = i, winz = ref_len(e), z = winz;
-                if (tc != 0xffffffffu)
-                    for (uint32_t k0 = tc & 0xffffu; k0 <= tc >> 16; k0 += 32) {
-                        const uint32_t k = k0 + lane;
-                        uint32_t c = REF_INF, zc = 0;
-                        if (k <= tc >> 16) {
-                            const uint64_t b = ref.tlist[ra + k];
-                            if (!((b ^ e) >> 48 & 0xff)) {
-                                c = ref_climb(ref, ra + ref_col(b), i - 1);
-                                zc = c == x ? before : ref.sum[c];
-                                if (*(volatile uint32_t *)(ref.stamp + c) == gen) c = REF_INF;  // met already
-                            }
+                lim = i;
+                if (win == x) continue;
+                // another set's root wins: what its top gained per row (its
+                // branches start in its own row at the earliest, and join by row r)
+                x = win;
+                y0 = (int)((x - off) / qw);
+                lx = ref.len[x];
+                for (int y = y0 + tid; y <= r; y += REF_ROOT_THREADS) gain[y] = 0;
+                __syncthreads();
+                for (int y = y0 + (tid >> 5); y <= r; y += REF_ROOT_THREADS / 32) {
+                    const uint32_t try_ = ref.trow[fd.row0 + y], ny = try_ & 0x7fffffffu;
+                    const uint32_t rby = off + (uint32_t)y * qw;
+                    for (uint32_t j0 = lane; j0 < ny; j0 += 128) {
+                        uint32_t u[4];
+                        uint64_t p[4];
+#pragma unroll
+                        for (int q = 0; q < 4; q++) {
+                            const uint32_t j = j0 + 32 * q;
+                            const uint64_t e = j < ny ? ref.tlist[rby + j] : ~0ull;
+                            u[q] = (uint32_t)(e >> 56) == t ? rby + ref_col(e) : x;
                         }
-                        const uint32_t peers = __match_any_sync(0xffffffffu, c);
-                        const bool first = c != REF_INF && lane == __ffs(peers) - 1;
-                        if (first) *(volatile uint32_t *)(ref.stamp + c) = gen;
-                        uint32_t bal = __ballot_sync(0xffffffffu, first);
-                        __syncwarp();
-                        while (bal) {
-                            const int l = __ffs(bal) - 1;
-                            bal &= bal - 1;
-                            const uint32_t cl = __shfl_sync(0xffffffffu, c, l), zl = __shfl_sync(0xffffffffu, zc, l);
-                            if (z <= zl) {
-                                win = cl;
-                                winz = zl;
-                            }
-                            z += zl;
-                        }
+#pragma unroll
+                        for (int q = 0; q < 4; q++) p[q] = u[q] != x ? ref.par[u[q]] : 0ull;
+#pragma unroll
+                        for (int q = 0; q < 4; q++)
+                            if (u[q] != x && (uint32_t)p[q] == x)
+                                atomicAdd(gain + ((uint32_t)(p[q] >> 32) - off) / qw, ref.sum[u[q]]);
                     }
-                if (lane == 0) {
-                    s_win = win;
-                    s_winz = winz;
-                }
-            }
-            __syncthreads();
-            const uint32_t win = s_win;
-            if (win == i) {
-                root = i;
-                break;
-            }
-            Z = s_winz;
-            ymax = r - 1;
-            part = true;
-            lim = i;
-            if (win == x) continue;
-            // another set's root wins: what its top gained per row (its
-            // branches start in its own row at the earliest, and join by row r)
-            x = win;
-            y0 = (int)((x - off) / qw);
-            lx = ref.len[x];
-            for (int y = y0 + tid; y <= r; y += REF_ROOT_THREADS) gain[y] = 0;
-            __syncthreads();
-            for (int y = y0 + (tid >> 5); y <= r; y += REF_ROOT_THREADS / 32) {
-                const uint32_t try_ = ref.trow[fd.row0 + y], ny = try_ & 0x7fffffffu;
-                const uint32_t rby = off + (uint32_t)y * qw;
-                for (uint32_t j0 = lane; j0 < ny; j0 += 128) {
-                    uint32_t u[4];
-                    uint64_t p[4];
-#pragma unroll
-                    for (int q = 0; q < 4; q++) {
-                        const uint32_t j = j0 + 32 * q;
-                        const uint64_t e = j < ny ? ref.tlist[rby + j] : ~0ull;
-                        u[q] = (uint32_t)(e >> 56) == t ? rby + ref_col(e) : x;
+                    if (lane == 0 && (try_ >> 31)) {  // the link's last-column node
+                        const uint64_t p = ref.par[vbase + (uint32_t)y - 1];
+                        if ((uint32_t)p == x) atomicAdd(gain + ((uint32_t)(p >> 32) - off) / qw, 1u);
                     }
-#pragma unroll
-                    for (int q = 0; q < 4; q++) p[q] = u[q] != x ? ref.par[u[q]] : 0ull;
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if (u[q] != x && (uint32_t)p[q] == x)
-                            atomicAdd(gain + ((uint32_t)(p[q] >> 32) - off) / qw, ref.sum[u[q]]);
                 }
-                if (lane == 0 && (try_ >> 31)) {  // the link's last-column node
-                    const uint64_t p = ref.par[vbase + (uint32_t)y - 1];
-                    if ((uint32_t)p == x) atomicAdd(gain + ((uint32_t)(p >> 32) - off) / qw, 1u);
-                }
+                __syncthreads();
+                scan_gain(y0, r);
             }
-            __syncthreads();
-            scan_gain(y0, r);
         }
-    }
-    // GPU node ids -> the reference's packed node numbers
-    if (tid == 0) {
-        if (root == 0xffffffffu) {
-            atomicOr(err, AT_ERR_ORDER);
-        } else {
-            const uint32_t *pre = ref.rpre + fd.row0 + f;
-            root = root < vbase ? pre[(root - off) / qw] + (root - off) % qw : pre[fd.qh] + (root - vbase);
+        // GPU node ids -> the reference's packed node numbers
+        if (tid == 0) {
+            if (root == 0xffffffffu) {
+                atomicOr(err, AT_ERR_ORDER);
+            } else {
+                const uint32_t *pre = ref.rpre + fd.row0 + f;
+                root = root < vbase ? pre[(root - off) / qw] + (root - off) % qw : pre[fd.qh] + (root - vbase);
+            }
+            ref.troot[(int64_t)f * AT_REF_MAXT + t] = root;
         }
-        ref.troot[(int64_t)f * AT_REF_MAXT + t] = root;
-    }
     }
 }
 
@@ -675,8 +682,8 @@ int launch_ref_order(const Launch &L, const FrameDesc *frames, const RowWord *wo
     launch(k_ref_targets, L.nframes, 256, 0, L.stream, frames, nfam, qstart, dets, det_ok, qcl, ckey, nb, runs, row_nruns,
                                                    ref, err);
     const int64_t b = (L.max_qh + 7) / 8;
-    const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 ? b : 148), (unsigned)L.nframes);
-    launch(k_ref_mark, grid, 256, 0, L.stream, frames, words, runs, row_nruns, ref);
+    const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 * 4 ? b : 148 * 4), (unsigned)L.nframes);
+    launch(k_ref_mark, grid, 256, 8 * REF_ROW_RUNS, L.stream, frames, words, runs, row_nruns, ref);
     const dim3 rows((unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16), (unsigned)L.nframes);
     launch(k_ref_link, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
     launch(k_ref_sums, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
