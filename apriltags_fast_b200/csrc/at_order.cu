@@ -184,11 +184,16 @@ __global__ void __launch_bounds__(256) k_ref_targets(const FrameDesc *frames, in
 // and each of them (and each link's last-column node) a root of the forest.
 
 // A row's targets are looked up a run a lane first (its labels lie side by
-// side); a lane that looked up its word's runs one by one waited for each
-// (4032 x 3024: 155 us, so 000 us; 32 frames of 1920 x 1080: 30 and 000).
+// side), and their entries gathered before they are written (4032 x 3024: 155
+// us when a lane looked up and wrote its word's runs one by one, 107 with the
+// look-up alone, 75 so; 16 frames of mixed sizes 57 and 44).
 #define REF_ROW_RUNS ((REF_PCAP + 32) & ~31)  // runs of a row, at most
+#define REF_STAGE 128                         // entries gathered before they are written
 
 #define REF_INF 0xffffffffu  // the time of a root: never joined
+
+__device__ __forceinline__ uint32_t ref_col(uint64_t e) { return (uint32_t)(e >> 32) & 0xffffu; }  // run index in the row
+__device__ __forceinline__ uint32_t ref_len(uint64_t e) { return (uint32_t)(e >> 16 & 0xffff) - (uint32_t)(e & 0xffff) + 1; }
 
 __device__ __forceinline__ void ref_node_init(const RefOrder &ref, uint32_t node, uint32_t px) {
     ref.par[node] = (uint64_t)REF_INF << 32 | node;
@@ -213,8 +218,9 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
         s_idx[h] = (uint8_t)t;
     }
     __syncthreads();
-    extern __shared__ uint8_t s_target[];  // by run of the warp's row
-    uint8_t *mine = s_target + (threadIdx.x >> 5) * REF_ROW_RUNS;
+    extern __shared__ __align__(16) uint8_t s_target[];  // by run of the warp's row
+    uint8_t *mine = s_target + (threadIdx.x >> 5) * (REF_ROW_RUNS + 8 * REF_STAGE);
+    uint64_t *stage = reinterpret_cast<uint64_t *>(mine + REF_ROW_RUNS);
     const int lane = threadIdx.x & 31;
     const int64_t wpb = blockDim.x >> 5;
     const int qw = fd.qw, nw = (qw + 31) / 32;
@@ -240,24 +246,39 @@ __global__ void __launch_bounds__(256) k_ref_mark(const FrameDesc *frames, const
                     if (((w.white | w.black) & m & (0u - m)) && mine[k] != REF_NONE) tm |= m & (0u - m);
             }
             uint32_t total;
-            uint32_t at = cnt + warp_excl_scan(__popc(tm), &total);
-            for (uint32_t m = tm; m; m &= m - 1, at++) {
-                const int c = __ffs(m) - 1;
-                const uint32_t k = run_at(w, c), t = mine[k];
-                const bool white = w.white >> c & 1u;
-                // the run's end: the first later column of another value or the last run column
-                int e = 32 * i + c + 1;
-                for (int j = i; j < nw; j++) {
-                    const uint32_t colour = (white ? row[j].white : row[j].black) & run_columns(j, qw);
-                    const uint32_t stop = ~colour & (j == i ? ~0u << c : ~0u);
-                    e = 32 * j + (stop ? __ffs(stop) - 1 : 32);
-                    if (stop) break;
+            const uint32_t off = warp_excl_scan(__popc(tm), &total), last = off + __popc(tm);
+            // the entries of as many words as there is room for (a word has
+            // 32 at most), then written a run a lane
+            for (uint32_t from = 0, to; from < total; from = to) {
+                const bool fits = last <= from + REF_STAGE;
+                to = __reduce_max_sync(0xffffffffu, fits ? last : 0u);
+                if (fits && off >= from) {
+                    uint64_t *out = stage + (off - from);
+                    for (uint32_t m = tm; m; m &= m - 1) {
+                        const int c = __ffs(m) - 1;
+                        const uint32_t k = run_at(w, c), t = mine[k];
+                        const bool white = w.white >> c & 1u;
+                        // the run's end: the first later column of another value or the last run column
+                        int e = 32 * i + c + 1;
+                        for (int j = i; j < nw; j++) {
+                            const uint32_t colour = (white ? row[j].white : row[j].black) & run_columns(j, qw);
+                            const uint32_t stop = ~colour & (j == i ? ~0u << c : ~0u);
+                            e = 32 * j + (stop ? __ffs(stop) - 1 : 32);
+                            if (stop) break;
+                        }
+                        *out++ = (uint64_t)(uint32_t)(32 * i + c) | (uint64_t)(uint32_t)(e - 1) << 16 | (uint64_t)k << 32 |
+                                 (uint64_t)(white ? 255 : 0) << 48 | (uint64_t)t << 56;
+                    }
                 }
-                const uint32_t start = (uint32_t)(32 * i + c), end = (uint32_t)(e - 1);
-                ref.tlist[base + at] = (uint64_t)start | (uint64_t)end << 16 | (uint64_t)k << 32 |
-                                       (uint64_t)(white ? 255 : 0) << 48 | (uint64_t)t << 56;
-                ref_node_init(ref, (uint32_t)(base + k), end - start + 1);
-                ref.len[base + k] = (uint16_t)(end - start + 1);
+                __syncwarp();
+                for (uint32_t j = from + lane; j < to; j += 32) {
+                    const uint64_t e = stage[j - from];
+                    const int64_t node = base + ref_col(e);
+                    ref.tlist[base + cnt + j] = e;
+                    ref_node_init(ref, (uint32_t)node, ref_len(e));
+                    ref.len[node] = (uint16_t)ref_len(e);
+                }
+                __syncwarp();
             }
             cnt += total;
         }
@@ -317,8 +338,6 @@ __device__ __forceinline__ void ref_insert(const RefOrder &ref, uint32_t u, uint
     }
 }
 
-__device__ __forceinline__ uint32_t ref_len(uint64_t e) { return (uint32_t)(e >> 16 & 0xffff) - (uint32_t)(e & 0xffff) + 1; }
-__device__ __forceinline__ uint32_t ref_col(uint64_t e) { return (uint32_t)(e >> 32) & 0xffffu; }  // run index in the row
 
 // A block per row: each target run's touching runs in the row above (they
 // are target runs too), kept for k_ref_root in tch[rbase + j] (first | last
@@ -683,7 +702,7 @@ int launch_ref_order(const Launch &L, const FrameDesc *frames, const RowWord *wo
                                                    ref, err);
     const int64_t b = (L.max_qh + 7) / 8;
     const dim3 grid((unsigned)(b < 1 ? 1 : b < 148 * 4 ? b : 148 * 4), (unsigned)L.nframes);
-    launch(k_ref_mark, grid, 256, 8 * REF_ROW_RUNS, L.stream, frames, words, runs, row_nruns, ref);
+    launch(k_ref_mark, grid, 256, 8 * (REF_ROW_RUNS + 8 * REF_STAGE), L.stream, frames, words, runs, row_nruns, ref);
     const dim3 rows((unsigned)(L.max_qh < 148 * 16 ? L.max_qh : 148 * 16), (unsigned)L.nframes);
     launch(k_ref_link, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
     launch(k_ref_sums, rows, REF_ROW_THREADS, 0, L.stream, frames, ref);
