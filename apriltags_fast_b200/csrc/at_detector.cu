@@ -623,15 +623,16 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         uint32_t *bs = B[B_PBSUM].as<uint32_t>();
         const PairScratch ps{B[B_PKFRAME].as<uint32_t>(), pf, pf + nbk, pf + 2 * nbk + 4, B[B_PGKEYS].as<uint64_t>(),
                              B[B_PGSLOTS].as<uint32_t>(), B[B_PGBUCKET].as<uint32_t>(), bs, bs + pair_scan_blocks(ncl)};
-        launch_pair_order(st, B[B_HOKEYS].as<uint64_t>(), B[B_HOSLOTS].as<uint32_t>(), ncl, nb, dfr, (int)n, pt, ps,
+        in->launches += launch_pair_order(st, B[B_HOKEYS].as<uint64_t>(), B[B_HOSLOTS].as<uint32_t>(), ncl, nb, dfr, (int)n, pt, ps,
                           B[B_HSKEYS].as<uint64_t>(), B[B_HSSLOTS].as<uint32_t>(), B[B_HRANK].as<uint32_t>(),
                           B[B_HCCOUNT].as<uint32_t>(), B[B_CSPAN].as<uint32_t>(), B[B_CY0].as<uint32_t>(),
-                          B[B_CFRAME].as<int32_t>(), B[B_CSTART].as<uint32_t>(), B[B_SPANOFF].as<uint32_t>());
+                          B[B_CFRAME].as<int32_t>(), B[B_CSTART].as<uint32_t>(), B[B_SPANOFF].as<uint32_t>(),
+                          B[B_SEG].as<uint32_t>(), segcap, B[B_ERR].as<uint32_t>());
         launch_point_place(L, dfr, prow, B[B_HRANK].as<uint32_t>(), B[B_CSTART].as<uint32_t>(),
                            B[B_SPANOFF].as<uint32_t>(), B[B_CSPAN].as<uint32_t>(), B[B_CY0].as<uint32_t>(), ncl,
                            B[B_SEG].as<uint32_t>(), segcap, B[B_VAL2].as<uint64_t>(), (int64_t)npts,
                            B[B_ERR].as<uint32_t>());
-        in->launches += 13;
+        in->launches += 3;
     } else if (!hashed) {
         // a capacity of the scan was exceeded: points in emission order,
         // sorted by pair. The scan's count leaves out the rows that it gave
@@ -715,18 +716,17 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
                                          B[B_CFRAME].as<int32_t>(), ncl, (int64_t)npts, max_px, scr,
                                          B[B_QUADS].as<GpuQuad>(), qok, B[B_ERR].as<uint32_t>());
         CK(cudaGetLastError());
-        launch_scan_u32(st, qok, ncl, qscan, B[B_QSCR].as<uint32_t>());
-        in->launches += 3;
-        // the quads in cluster order (grouped by frame), their count and each
-        // frame's first quad stay on the device: decode is sized by ncl
+        // the quads, their count and each frame's first quad stay on the
+        // device: decode is sized by ncl
         CK(B[B_QUADSC].ensure(ncl * sizeof(GpuQuad)));
         CK(B[B_QNUM].ensure(8));
         CK(B[B_QCL].ensure(ncl * 4));
+        CK(B[B_QSTART].ensure((n + 1) * 8));
+        CK(B[B_OUTOFF].ensure((n + 1) * 8));
         uint32_t *nq_dev = B[B_QNUM].as<uint32_t>();
-        CK(cudaMemsetAsync(nq_dev, 0, 4, st));
-        launch_gather_quads(st, B[B_QUADS].as<GpuQuad>(), qok, qscan, ncl, B[B_QUADSC].as<GpuQuad>(), nq_dev,
-                            B[B_QCL].as<uint32_t>());
-        in->launches += 1;
+        in->launches += launch_gather_quads(st, B[B_QUADS].as<GpuQuad>(), qok, ncl, qscan, B[B_QSCR].as<uint32_t>(), (int)n,
+                                            in->nfam, B[B_QUADSC].as<GpuQuad>(), nq_dev, B[B_QCL].as<uint32_t>(),
+                                            B[B_QSTART].as<int64_t>(), B[B_OUTOFF].as<int64_t>());
         CK(cudaEventRecord(in->ev[6], st));
         // decode
         if (in->fam_dirty) {
@@ -740,12 +740,8 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_OUT].ensure(nd * sizeof(GpuDetection)));
         CK(B[B_DIDX].ensure(nd * 4));
         CK(B[B_DRM].ensure(nd));
-        CK(B[B_QSTART].ensure((n + 1) * 8));
-        CK(B[B_OUTOFF].ensure((n + 1) * 8));
         CK(B[B_OUTN].ensure((n + 1) * 8));
         CK(B[B_FIRST].ensure((n + 1) * 8));
-        launch_frame_bounds(st, B[B_QUADSC].as<GpuQuad>(), nq_dev, (int)n, in->nfam, B[B_QSTART].as<int64_t>(),
-                            B[B_OUTOFF].as<int64_t>());
         CK(B[B_QCORN].ensure(ncl * 8 * sizeof(float)));
         CK(B[B_QH].ensure(ncl * 9 * sizeof(double)));
         CK(B[B_QHOK].ensure(ncl * sizeof(uint32_t)));
@@ -753,7 +749,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         launch_decode(st, dfr, prm, in->dfam.as<GpuFamily>(), B[B_IMG].as<uint8_t>(), qim, B[B_QUADSC].as<GpuQuad>(),
                       ncl, dscr, B[B_DETS].as<GpuDetection>(), B[B_DETOK].as<uint32_t>());
         CK(cudaEventRecord(in->ev[7], st));
-        in->launches += 4;
+        in->launches += 3;
         // the reference's quad order for detections that share an id: the
         // roots its union order picks for their components (at_order.cu)
         CK(B[B_RNEED].ensure(n * 4));

@@ -97,10 +97,11 @@ struct PointRows {
 bool point_scan_set_smem();
 void launch_point_scan(const Launch &L, const FrameDesc *frames, const RowWord *words, const uint32_t *lab, int nb,
                        const PairTable &T, const PointRows &P, uint32_t *full, unsigned long long *npoints);
-void launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, int nb,
-                       const FrameDesc *frames, int nframes, const PairTable &T, const PairScratch &P,
-                       uint64_t *skeys, uint32_t *sslots, uint32_t *rank_of_slot, uint32_t *ccount, uint32_t *cspan,
-                       uint32_t *cy0, int32_t *cframe, uint32_t *cstart, uint32_t *spanoff);
+int launch_pair_order(cudaStream_t s, const uint64_t *okeys, const uint32_t *oslots, int64_t ncl, int nb,
+                      const FrameDesc *frames, int nframes, const PairTable &T, const PairScratch &P,
+                      uint64_t *skeys, uint32_t *sslots, uint32_t *rank_of_slot, uint32_t *ccount, uint32_t *cspan,
+                      uint32_t *cy0, int32_t *cframe, uint32_t *cstart, uint32_t *spanoff, uint32_t *seg, int64_t cap,
+                      uint32_t *err);
 int64_t pair_scan_blocks(int64_t ncl);
 int64_t scan_u32_scratch(int64_t n);
 void launch_scan_u32(cudaStream_t s, const uint32_t *a, int64_t n, uint32_t *out, uint32_t *scratch);
@@ -121,11 +122,12 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
                      const uint8_t *qim, const uint64_t *pts, const uint32_t *cstart, const int32_t *cframe,
                      int64_t nclusters, int64_t npoints, int64_t max_px, const FitScratch &scr, GpuQuad *quads,
                      uint32_t *quad_ok, uint32_t *err);
-// also each gathered quad's cluster index (qcl)
-void launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, const uint32_t *scan, int64_t n,
-                         GpuQuad *out, uint32_t *nq, uint32_t *qcl);
-void launch_frame_bounds(cudaStream_t s, const GpuQuad *quads, const uint32_t *nq, int nframes, int nfam,
-                         int64_t *qstart, int64_t *out_off);
+// The quads in cluster order (grouped by frame), their clusters (qcl) and
+// count; each frame's first quad and first detection slot (nfam a quad).
+// scan: n + 1 values; scratch: scan_u32_scratch(n). Returns the launches.
+int launch_gather_quads(cudaStream_t s, const GpuQuad *quads, const uint32_t *ok, int64_t n, uint32_t *scan,
+                        uint32_t *scratch, int nframes, int nfam, GpuQuad *out, uint32_t *nq, uint32_t *qcl,
+                        int64_t *qstart, int64_t *out_off);
 void launch_output(cudaStream_t s, int nframes, const int64_t *qstart, const GpuDetection *out,
                    const int64_t *out_off, const int64_t *out_n, int64_t *first, GpuDetection *host,
                    int64_t *meta, int64_t max_dets);

@@ -97,3 +97,27 @@ def test_rows_above_a_limit(w):
            for i in imgs]
     det.detect_batch(imgs)
     assert np.array_equal(det.diag("points"), np.concatenate(pts))
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 129, 1022, 1023, 1024, 2049, 4094, 4095, 4096])
+def test_cluster_counts(n):
+    """n clusters or one more (in one block up to 1024, gathered in one up to
+    4096, by several kernels above), n quads: alone, and in a batch."""
+    img = np.full((65 * 15 + 8, 65 * 15 + 8), 210, np.uint8)
+    for k in range(n):
+        y, x = 4 + 15 * (k // 65), 4 + 15 * (k % 65)
+        img[y : y + 9, x : x + 9 + k % 2] = 40
+    _check([img], 24)
+    fams = [H.oracle_family("tag36h11")]
+    prm = O.default_params(quad_decimate=1.0)
+    imgs = [_blobs(97, 60, 5, 1), img, _blobs(97, 60, 5, 2)]
+    ref = [O.detect(i, fams, [2], prm, order=O.ORDER_CANON) for i in imgs]
+    assert len(ref[1].cstart) - 1 in (n, n + 1) and len(ref[1].quads) == n
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    got = det.detect_batch(imgs)
+    assert np.array_equal(det.diag("points"), np.concatenate([r.pts for r in ref]))
+    quads = det.diag("quads")
+    want = np.array([q[0] for r in ref for q in r.quads], np.float32)
+    assert np.array_equal(quads["p"].view(np.uint32), want.view(np.uint32))
+    assert np.array_equal(quads["frame"], np.repeat([0, 1, 2], [len(r.quads) for r in ref]))
+    assert [[d.key() for d in f] for f in got] == [r.dets for r in ref]
