@@ -1264,24 +1264,26 @@ __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, 
                                int64_t nclusters, int64_t npoints, int32_t min_px, uint32_t *quad_ok,
                                uint32_t *lists, uint32_t *counts) {
     kernel_begin();
-    const int lane = threadIdx.x & 31;
+    __shared__ uint32_t s_n[FIT_NBUCKET], s_at[FIT_NBUCKET];
     for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nclusters; c0 += (int64_t)gridDim.x * blockDim.x) {
+        __syncthreads();
+        if (threadIdx.x < FIT_NBUCKET) s_n[threadIdx.x] = 0;
+        __syncthreads();
         const int64_t c = c0 + threadIdx.x;
         int k = -1;
+        uint32_t at = 0;
         if (c < nclusters) {
             quad_ok[c] = 0;
             const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - cstart[c];
             if (sz >= min_px && sz <= frames[cframe[c]].max_px) k = fit_bucket(sz);
+            if (k >= 0) at = atomicAdd(s_n + k, 1u);
         }
-        // (a frame's clusters are few sizes apart: a turn per bucket met)
-        for (uint32_t met = __reduce_or_sync(0xffffffffu, k < 0 ? 0u : 1u << k); met; met &= met - 1) {
-            const int q = __ffs(met) - 1;
-            const uint32_t bal = __ballot_sync(0xffffffffu, k == q);
-            uint32_t at = 0;
-            if (lane == __ffs(bal) - 1) at = atomicAdd(counts + q, (uint32_t)__popc(bal));
-            at = __shfl_sync(0xffffffffu, at, __ffs(bal) - 1);
-            if (k == q) lists[(int64_t)q * nclusters + at + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)c;
-        }
+        __syncthreads();
+        // (all buckets' places at once: one after the other took 9 us for 132 clusters)
+        if (threadIdx.x < FIT_NBUCKET && s_n[threadIdx.x])
+            s_at[threadIdx.x] = atomicAdd(counts + threadIdx.x, s_n[threadIdx.x]);
+        __syncthreads();
+        if (k >= 0) lists[(int64_t)k * nclusters + s_at[k] + at] = (uint32_t)c;
     }
 }
 
@@ -2927,7 +2929,7 @@ __global__ void __launch_bounds__(QH_WARPS * 32) k_quad_homography(const float *
     }
 }
 
-__global__ void __launch_bounds__(AT_DEC_THREADS) k_decode(const FrameDesc *frames, GpuParams prm,
+__global__ void __launch_bounds__(AT_DEC_THREADS, 6) k_decode(const FrameDesc *frames, GpuParams prm,
                                                               const GpuFamily *fams, const uint8_t *img,
                                                               const uint8_t *qim, const GpuQuad *quads,
                                                               const uint32_t *nq, const double *hs, const uint32_t *hok,
@@ -2989,30 +2991,37 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_decode(const FrameDesc *fram
             }
             __syncthreads();
             if (tid < 32) {
-                // lane 0 the white model (even patterns), lane 1 the black one
-                // (odd patterns), each summed in pattern order in registers
-                double a0 = 0.0, a1 = 0.0, a2 = 0.0, a4 = 0.0, a5 = 0.0, a8 = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
-                if (tid < 2) {
-                    for (int pi = tid; pi < 8; pi += 2)
-                        for (int i = 0; i < wab; i++) {
-                            const int t = pi * wab + i;
-                            if (!s_gk[t]) continue;
-                            const double x = s_gx[t], y = s_gy[t], val = s_gv[t];
-                            a0 = a0 + x * x;
-                            a1 = a1 + x * y;
-                            a2 = a2 + x;
-                            a4 = a4 + y * y;
-                            a5 = a5 + y;
-                            a8 = a8 + 1.0;
-                            b0 = b0 + x * val;
-                            b1 = b1 + y * val;
-                            b2 = b2 + val;
+                // the white model (even patterns) in even lanes, the black
+                // one (odd patterns) in odd ones, one of the nine sums a lane,
+                // in pattern order; then lanes 0 and 1 get theirs and solve.
+                // (All nine in one lane took each sample 15 FP64 instructions
+                // with two lanes busy.)
+                const int acc = tid >> 1;
+                const bool ux = acc < 3 || acc == 6, uy = acc == 3 || acc == 4 || acc == 7;
+                const bool vx = acc == 0, vy = acc == 1 || acc == 3, vv = acc == 6 || acc == 7;
+                const double *pu = ux ? s_gx : uy ? s_gy : s_gv, *pv = vx ? s_gx : vy ? s_gy : s_gv;
+                double sum = 0.0;
+                if (tid < 18)
+                    for (int pi = tid & 1; pi < 8; pi += 2)
+                        for (int t = pi * wab; t < (pi + 1) * wab; t++) {
+                            const double u = acc == 5 ? 1.0 : pu[t], v = vx || vy || vv ? pv[t] : 1.0;
+                            const double next = sum + u * v;
+                            sum = s_gk[t] ? next : sum;
                         }
-                }
                 GrayModel gm;
-                gm.a[0] = a0, gm.a[1] = a1, gm.a[2] = a2, gm.a[4] = a4, gm.a[5] = a5, gm.a[8] = a8;
                 gm.a[3] = gm.a[6] = gm.a[7] = 0.0;
-                gm.b[0] = b0, gm.b[1] = b1, gm.b[2] = b2;
+                {
+                    const int m = tid & 1;
+                    gm.a[0] = __shfl_sync(0xffffffffu, sum, m);
+                    gm.a[1] = __shfl_sync(0xffffffffu, sum, m + 2);
+                    gm.a[2] = __shfl_sync(0xffffffffu, sum, m + 4);
+                    gm.a[4] = __shfl_sync(0xffffffffu, sum, m + 6);
+                    gm.a[5] = __shfl_sync(0xffffffffu, sum, m + 8);
+                    gm.a[8] = __shfl_sync(0xffffffffu, sum, m + 10);
+                    gm.b[0] = __shfl_sync(0xffffffffu, sum, m + 12);
+                    gm.b[1] = __shfl_sync(0xffffffffu, sum, m + 14);
+                    gm.b[2] = __shfl_sync(0xffffffffu, sum, m + 16);
+                }
                 if (tid == 0 || (tid == 1 && wab > 1)) {
                     gm_solve(&gm);
                 } else {
@@ -3059,25 +3068,36 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_decode(const FrameDesc *fram
             __syncthreads();
             DEC_PROF(5)
             if (tid < 32) {
-                float bs = 0.0f, ws = 0.0f, bc = 1.0f, wc = 1.0f;
-                uint64_t rcode = 0;
-                if (tid == 0) {
-                for (int64_t i = 0; i < F.nbits; i++) {
-                    rcode <<= 1;
-                    int64_t cell = (F.bit_y[i] - minc) * tw + (F.bit_x[i] - minc);
-                    double vv = s_vals[cell] + prm.decode_sharpening * s_sharp[cell];
-                    if (vv > 0.0) {
-                        ws = (float)((double)ws + vv);
-                        wc = __fadd_rn(wc, 1.0f);
-                        rcode |= 1;
-                    } else {
-                        bs = (float)((double)bs - vv);
-                        bc = __fadd_rn(bc, 1.0f);
+                // the bits a lane each; then lane 0 sums the white ones in
+                // order and lane 1 the black ones (one lane for all of it
+                // took 3 us a quad of 36 bits)
+                uint64_t white = 0;
+                for (int i0 = 0; i0 < F.nbits; i0 += 32) {
+                    const int i = i0 + tid;
+                    double vv = 0.0;
+                    if (i < F.nbits) {
+                        const int64_t cell = (F.bit_y[i] - minc) * tw + (F.bit_x[i] - minc);
+                        vv = s_vals[cell] + prm.decode_sharpening * s_sharp[cell];
+                        s_gx[i] = vv;
+                    }
+                    white |= (uint64_t)__ballot_sync(0xffffffffu, vv > 0.0) << i0;
+                }
+                __syncwarp();
+                const uint64_t all = F.nbits > 0 ? ~0ull >> (64 - F.nbits) : 0ull;
+                const uint64_t rcode = F.nbits > 0 ? __brevll(white) >> (64 - F.nbits) : 0ull;
+                float sum = 0.0f;
+                if (tid < 2) {
+                    uint64_t m = tid == 0 ? white : ~white & all;
+                    double next = m ? s_gx[__ffsll(m) - 1] : 0.0;
+                    while (m) {
+                        const double vv = next;
+                        m &= m - 1;
+                        if (m) next = s_gx[__ffsll(m) - 1];
+                        sum = (float)(tid == 0 ? (double)sum + vv : (double)sum - vv);
                     }
                 }
-                }
-                rcode = (uint64_t)__shfl_sync(0xffffffffu, (uint32_t)(rcode >> 32), 0) << 32 |
-                        __shfl_sync(0xffffffffu, (uint32_t)rcode, 0);
+                const float ws = sum, bs = __shfl_sync(0xffffffffu, sum, 1);
+                const float wc = (float)(1 + __popcll(white)), bc = (float)(1 + F.nbits - __popcll(white));
                 const uint32_t lk = qd_lookup(F, rcode, tid);
                 double x = (double)__fdiv_rn(ws, wc), y = (double)__fdiv_rn(bs, bc);
                 double m = x != x ? y : y != y ? x : x < y ? x : y;  // fmin

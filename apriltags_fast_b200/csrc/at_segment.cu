@@ -491,7 +491,7 @@ __device__ __forceinline__ uint32_t uf_root(const uint32_t *par, uint32_t x) {
 // to its component's root, and from here on points at it. A block gathers
 // its sums by root in shared memory first: the pieces of a frame's background
 // all lie under one node, whose atomics followed one another (4032 x 3024:
-// 160 us with the sums of a warp's lanes gathered, 000 us so).
+// 160 us with the sums of a warp's lanes gathered, 60 us so).
 #define SUM_ROOTS 256
 #define SUM_PROBES 8
 __global__ void __launch_bounds__(128) k_root_sums(const FrameDesc *frames, RunArrays runs, const uint32_t *band_roots) {
