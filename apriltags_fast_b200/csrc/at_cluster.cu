@@ -7,9 +7,10 @@
 // masks and the run labels, as a 4-byte record in its row's region; the
 // records are then placed, each at its place in its cluster:
 //
-//   k_point_scan     a warp per row, a word of 32 columns a lane: the row's
-//                    points, their label pairs gathered in the warp's table
-//                    (shared memory), the records in emission order; at the
+//   k_point_scan     a warp per row: its points, found as bits of 32 columns
+//                    a lane, then looked up a point a lane; their label pairs
+//                    gathered in the warp's table (shared memory), the
+//                    records in emission order; at the
 //                    row's end each pair of the row into the frame's pair
 //                    table (point count, first and last row) and the row's
 //                    pair list.
@@ -20,6 +21,7 @@
 //                    frame's (the larger label is a node of the frame).
 //   k_cluster_span   per cluster: count, frame, first row, rows spanned.
 //   scans            each cluster's first point; its row table's offset.
+//   (all from k_pair_frame to here in k_pair_small when there are few pairs)
 //   k_seg_fill       a warp per row: its pairs' point counts into the
 //                    clusters' row tables.
 //   k_seg_scan       a warp per cluster: the counts of its rows become the

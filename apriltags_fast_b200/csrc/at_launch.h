@@ -4,9 +4,9 @@
 // read or write of global memory: it waits until the one before has ended
 // and its writes are visible, and, in grids that leave room on the GPU (at
 // most 4 blocks an SM), first lets the next kernel be set up. A frame takes
-// some 40 short kernels one after the other; the launch latency between two
-// of them was 1 to 2 us (640 x 480: 437 us of kernels and gaps before, 394 us
-// with it). In larger grids the next kernel's waiting blocks would only take
+// some 30 short kernels one after the other (40 when this was measured); the
+// launch latency between two of them was 1 to 2 us (640 x 480: 437 us of
+// kernels and gaps before, 394 us with it). In larger grids the next kernel's waiting blocks would only take
 // room from running ones, of other streams above all (32 frames of 1920 x
 // 1080 on three pipelines: 2.17 ms without, 2.40 ms with it everywhere).
 #pragma once

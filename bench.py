@@ -9,8 +9,9 @@ exists for this benchmark). A pool of 64 distinct frames (132 MB, larger
 than the 126 MB L2) rotates through the steps, so no step reads inputs that
 a previous step left in L2.
 
-A step is one at_detect_batch over B frames (spread by the library over 3
-pipelines of its own that overlap on the GPU). `value` is frames/s with the
+A step is one at_detect_batch over B frames (host frames are spread by the
+library over 3 pipelines of its own that overlap on the GPU; frames in device
+memory take one). `value` is frames/s with the
 frames already in device memory; `e2e` is the same call on pinned host
 frames (the host-to-device copies and the copy of the detections back are
 inside the timed region). `single_frame` is the plain at_detect path, one
@@ -47,7 +48,7 @@ sys.path.insert(0, ROOT)
 
 METRIC = "1080p frames/s (batched GPU detector, bit-exact detections)"
 WORKLOAD = "1080p tag36h11 decimate 2, 24 tags + 200 distractors, bits 2"
-# pipelines a batched call spreads its frames over (the library's default)
+# pipelines a batched call of host frames is spread over (the library's default)
 PIPELINES = 3
 W, H = 1920, 1080
 POOL = 64
@@ -351,12 +352,12 @@ def run_reference(args):
 # the kernels of each stage (one launch of each per batch)
 STAGE_KERNELS = {
     "threshold": "threshold stage: k_decimate_threshold (decimate 2, tile max/min and threshold fused)",
-    "unionfind": "unionfind stage: k_row_runs, k_band_union, k_band_join, k_row_sums, k_labels_w",
+    "unionfind": "unionfind stage: k_band_union, k_band_join, k_root_sums, k_run_labels",
     "clusters": "clusters stage: k_point_scan, k_cluster_collect, k_pair_*, k_cluster_span, k_scan2_*, "
                 "k_seg_zero/fill/scan, k_point_place",
-    "fit_quads": "fit_quads stage: k_fit_classify, k_fit_order, k_fit_warp<4/8/16>, k_fit_quads<128/512>",
+    "fit_quads": "fit_quads stage: k_fit_classify, k_fit_warp<4/8/16>, k_fit_quads<128/256/512>",
     "decode": "decode stage: k_refine, k_quad_homography, k_decode",
-    "reconcile": "reconcile stage: k_ref_targets/mark/cut/local/frontier/band/resolve, k_finalize, k_output_*",
+    "reconcile": "reconcile stage: k_ref_targets/mark/link/sums/root, k_finalize, k_output_*",
 }
 
 
