@@ -2929,7 +2929,11 @@ __global__ void __launch_bounds__(QH_WARPS * 32) k_quad_homography(const float *
     }
 }
 
-__global__ void __launch_bounds__(AT_DEC_THREADS, 6) k_decode(const FrameDesc *frames, GpuParams prm,
+// A block per quad. Most of its time goes to one warp (gray models, bit sums,
+// lookup), so it has only one more for the 64 border samples and the bits: 42
+// us for 32 frames of 1920 x 1080, with blocks of 128 threads 55.
+#define DECODE_THREADS 64
+__global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *frames, GpuParams prm,
                                                               const GpuFamily *fams, const uint8_t *img,
                                                               const uint8_t *qim, const GpuQuad *quads,
                                                               const uint32_t *nq, const double *hs, const uint32_t *hok,
@@ -3674,7 +3678,7 @@ void launch_decode(cudaStream_t s, const FrameDesc *frames, const GpuParams &prm
     const int64_t hb = (max_quads + QH_WARPS - 1) / QH_WARPS;
     launch(k_quad_homography, (unsigned)(hb < 148 * 16 ? hb : 148 * 16), QH_WARPS * 32, 0, s, scr.corners, scr.nq,
                                                                                         scr.h, scr.hok);
-    launch(k_decode, blocks, AT_DEC_THREADS, 0, s, frames, prm, fams, img, qim, quads, scr.nq, scr.h, scr.hok, dets,
+    launch(k_decode, blocks, DECODE_THREADS, 0, s, frames, prm, fams, img, qim, quads, scr.nq, scr.h, scr.hok, dets,
                                                det_ok);
 }
 
