@@ -48,7 +48,9 @@
 #include <condition_variable>
 #include <functional>
 #include <mutex>
+#include <string>
 #include <thread>
+#include <unordered_map>
 #include <vector>
 
 #include "apriltag_fast.h"
@@ -84,24 +86,25 @@ constexpr int JMAX_RUNS = 48;
 // One Huffman table: runs of equal-length codes over the 16-bit code
 // space, in order (run r ends at rend[r]; position w of it decodes as
 // symbol pool[rsym[r] + ((w - rorigin[r]) >> (16 - rlen[r]))]), and what
-// the next 9 bits of the stream decode as (lut): a symbol entry (JENT_*),
-// or JENT_SUB | the place in the job's lut2 of the 128 entries of the next 7
-// bits, or 0 (the runs tell; only in tables with more than JMAX_SUB such
-// prefixes). An entry holds all that a decode step needs, so that the lanes
+// the next 9 bits of the stream decode as (lut): a symbol entry (jent), or
+// JENT_SUB | the place in the job's lut2 of the 128 entries of the next 7
+// bits, or 0 (the runs tell; for the prefixes above JMAX_SUB of a table, and
+// for all of those that a job's first JMAX_LUT2 entries have no room for).
+// An entry holds all that a decode step needs, so that the lanes
 // of a warp, each at its own place in the stream, follow one path whatever
 // their codes: with 9-bit entries of (length, symbol) and the runs searched
 // for longer codes, some lane searched in nearly every step.
-constexpr uint32_t JENT_SUB = 0x80000000u;
-constexpr uint32_t JENT_OK = 1u << 22;  // always set in a symbol entry
+constexpr uint32_t JENT_SUB = 0x80000000u;  // in no symbol entry; below it the place
 __host__ __device__ __forceinline__ uint32_t jent(int len, int sym, bool ac) {
     const uint32_t sz = sym & 15, dz = !ac ? 1 : sym == 0 ? 64 : (sym >> 4) + 1;
-    return JENT_OK | (len + sz) | (uint32_t)len << 6 | sz << 11 | dz << 15;
+    return (len + sz) | (uint32_t)len << 6 | sz << 11 | dz << 15;  // never 0: dz is not
 }
 __host__ __device__ __forceinline__ int jent_bits(uint32_t e) { return e & 63; }          // code and value bits
 __host__ __device__ __forceinline__ int jent_len(uint32_t e) { return (e >> 6) & 31; }    // code bits (0: no code)
 __host__ __device__ __forceinline__ int jent_size(uint32_t e) { return (e >> 11) & 15; }  // value bits
 __host__ __device__ __forceinline__ int jent_step(uint32_t e) { return (e >> 15) & 127; } // coefficients passed (64: rest of the block)
 constexpr int JMAX_SUB = 64;
+constexpr size_t JMAX_LUT2 = (size_t)1 << 24;  // 64 MB a job: thousands of files with tables of their own
 struct JTab {
     uint32_t lut[512];
     uint32_t nrun, r0, ac;  // runs; the first run a lookup miss can land in; whether AC codes
@@ -230,7 +233,7 @@ struct JReader {
 // no code: length 0, symbol 0.
 __host__ __device__ __forceinline__ uint32_t jdecode(const JJob &J, const JTab *__restrict__ t, uint32_t win) {
     const uint32_t e = JLDG(&t->lut[win >> 23]);
-    if (e & JENT_OK) return e;
+    if ((int32_t)e > 0) return e;
     const uint32_t w16 = win >> 16;
     if (e) return JLDG(&J.lut2[(e & ~JENT_SUB) + (w16 & 127)]);
     const uint32_t nr = JLDG(&t->nrun);
@@ -329,7 +332,7 @@ __host__ __device__ unsigned long long jrun_sync(const JJob &J, const JScanDev &
         }
         const uint32_t win = R.peek(s.p);
         const uint32_t e = jdecode(J, s.z == 0 ? s.dc : s.ac, win);
-        if (jent_len(e) == 0) {
+        if (jent_bits(e) == 0) {
             if (++stall > stall_max) {
                 out = jpack(JSTUCK, 0, 0);
                 if (!counting) *entry = out;
@@ -1282,7 +1285,7 @@ struct HJob {
     const uint8_t *stream_src = nullptr;  // copied to the staging's start by run_job
     std::vector<JTab> tabs;
     std::vector<uint32_t> lut2;
-    HTab last_tab[4];  // the tables of tabs' last four
+    std::unordered_map<std::string, uint32_t> tab_of;  // by tabs_key: the first of the scan's tables
     std::vector<uint8_t> syms;
     std::vector<JScanDev> scans;
     std::vector<JSegDev> segs;
@@ -1348,7 +1351,7 @@ JTab make_tab(const HTab &t, bool ac, std::vector<uint8_t> &pool, std::vector<ui
         }
         if (whole) {
             d.lut[p] = entry(lo, r);
-        } else if (nsub < JMAX_SUB) {
+        } else if (nsub < JMAX_SUB && lut2.size() < JMAX_LUT2) {
             nsub++;
             d.lut[p] = JENT_SUB | (uint32_t)lut2.size();
             size_t q = r;
@@ -1363,9 +1366,16 @@ JTab make_tab(const HTab &t, bool ac, std::vector<uint8_t> &pool, std::vector<ui
     return d;
 }
 
-bool same_tab(const HTab &a, const HTab &b) {
-    return a.runs.size() == b.runs.size() && a.syms == b.syms &&
-           (a.runs.empty() || !memcmp(a.runs.data(), b.runs.data(), a.runs.size() * sizeof(HRun)));
+// A scan's tables as a key: equal for equal tables only.
+std::string tabs_key(const HScan &sc) {
+    std::string k;
+    for (const HTab &t : sc.tab) {
+        const uint32_t n[2] = {(uint32_t)t.runs.size(), (uint32_t)t.syms.size()};
+        k.append((const char *)n, sizeof n);
+        k.append((const char *)t.runs.data(), n[0] * sizeof(HRun));
+        k.append((const char *)t.syms.data(), n[1]);
+    }
+    return k;
 }
 
 // Adds the scans of a parsed image to the job. want: which frame
@@ -1405,15 +1415,11 @@ void add_image(HJob &J, const HImage &im, int img, int64_t s_base, uint32_t sub_
         if (nmcu == 0) continue;
         JScanDev D;
         memset(&D, 0, sizeof D);
-        // one camera's files share their tables: those of the scan before, if alike
-        bool same = !J.tabs.empty();
-        for (int t = 0; t < 4 && same; t++) same = same_tab(sc.tab[t], J.last_tab[t]);
-        if (!same)
-            for (int t = 0; t < 4; t++) {
-                J.tabs.push_back(make_tab(sc.tab[t], t >= 2, J.syms, J.lut2));
-                J.last_tab[t] = sc.tab[t];
-            }
-        D.tab0 = (uint32_t)J.tabs.size() - 4;
+        // a job keeps equal tables once (one camera's files share them)
+        const auto known = J.tab_of.emplace(tabs_key(sc), (uint32_t)J.tabs.size());
+        if (known.second)
+            for (int t = 0; t < 4; t++) J.tabs.push_back(make_tab(sc.tab[t], t >= 2, J.syms, J.lut2));
+        D.tab0 = known.first->second;
         D.mcus_x = sc.mx;
         D.nmcu = (uint32_t)nmcu;
         D.restart = sc.restart;
