@@ -113,7 +113,7 @@ struct JTab {
 };
 
 struct JScanDev {
-    uint32_t tab0;        // this scan's 4 tables (DC 0, DC 1, AC 0, AC 1) in the job's table array
+    uint32_t tab0;        // this scan's tables (DC 0, DC 1, AC 0, AC 1; where it takes them, AC 0 and 1 as DC) in the job's
     uint32_t mcus_x, nmcu;
     uint32_t restart;     // MCUs per segment (0: one segment)
     uint32_t sub0;        // first sub-stream of the scan
@@ -1367,8 +1367,8 @@ JTab make_tab(const HTab &t, bool ac, std::vector<uint8_t> &pool, std::vector<ui
 }
 
 // A scan's tables as a key: equal for equal tables only.
-std::string tabs_key(const HScan &sc) {
-    std::string k;
+std::string tabs_key(const HScan &sc, bool ac_as_dc) {
+    std::string k(1, ac_as_dc ? '1' : '0');
     for (const HTab &t : sc.tab) {
         const uint32_t n[2] = {(uint32_t)t.runs.size(), (uint32_t)t.syms.size()};
         k.append((const char *)n, sizeof n);
@@ -1415,10 +1415,15 @@ void add_image(HJob &J, const HImage &im, int img, int64_t s_base, uint32_t sub_
         if (nmcu == 0) continue;
         JScanDev D;
         memset(&D, 0, sizeof D);
+        // a scan may take the AC tables for its DC codes: they follow once
+        // more as such
+        bool ac_as_dc = false;
+        for (int i = 0; i < sc.ns; i++) ac_as_dc |= sc.tda[i] >> 4 == 2 || sc.tda[i] >> 4 == 3;
         // a job keeps equal tables once (one camera's files share them)
-        const auto known = J.tab_of.emplace(tabs_key(sc), (uint32_t)J.tabs.size());
+        const auto known = J.tab_of.emplace(tabs_key(sc, ac_as_dc), (uint32_t)J.tabs.size());
         if (known.second)
-            for (int t = 0; t < 4; t++) J.tabs.push_back(make_tab(sc.tab[t], t >= 2, J.syms, J.lut2));
+            for (int t = 0; t < (ac_as_dc ? 6 : 4); t++)
+                J.tabs.push_back(make_tab(sc.tab[t < 4 ? t : t - 2], t == 2 || t == 3, J.syms, J.lut2));
         D.tab0 = known.first->second;
         D.mcus_x = sc.mx;
         D.nmcu = (uint32_t)nmcu;
@@ -1448,6 +1453,7 @@ void add_image(HJob &J, const HImage &im, int img, int64_t s_base, uint32_t sub_
             D.ac[i] = (uint8_t)(2 + (sc.tda[i] & 15));
             // a component with no blocks per MCU never looks its tables up
             if (D.dc[i] > 3) D.dc[i] = 0;
+            if (D.dc[i] > 1) D.dc[i] += 2;  // an AC table's form for DC codes
             if (D.ac[i] > 3) D.ac[i] = 2;
             const int c = sc.cidx[i];
             D.bnx[i] = im.comp[c].sx;

@@ -100,3 +100,8 @@ def bad_files():
             out.append((f"{name} truncated {frac}", b[:int(len(b) * frac)], 0, None))
         out.append((f"{name} without EOI", b[:-2], 0, OK))
     return out
+
+
+def dc_selector(buf, sel):
+    """The file with the table selector of its first scan's first component replaced."""
+    return _patch(buf, _find(buf, 0xDA) + 6, [sel])

@@ -199,3 +199,16 @@ def test_code_lengths(counts, color):
     assert errs == [e]
     if e == 0:
         assert np.array_equal(frames[0], O.gray_of(w, h, planes))
+
+
+@pytest.mark.parametrize("sel", [0x20, 0x30])
+def test_scans_that_take_ac_tables_for_dc(dec, sel):
+    """Scan headers that name table 2 or 3 for DC codes (and, for a gray file
+    without AC table 1, the missing table's error), beside ordinary files."""
+    cases = []
+    for k, (rst, fl) in enumerate([(0, 0), (0, O.JPEG_OPTIMIZE), (0, O.JPEG_OPTIMIZE)]):
+        plain = O.jpeg_encode(J._rgb(101, 150, 20 + k), 90, (2, 2) if k < 2 else (1, 1), rst, fl)
+        cases += [(f"plain {k}", plain, 0), (f"color {k}", J.dc_selector(plain, sel), 0)]
+    cases.append(("gray", J.dc_selector(O.jpeg_encode(J._gray(101, 150, 30), 85), sel), 0))
+    check_batch(dec, cases)
+    check_batch(dec, cases, device=True)

@@ -39,3 +39,12 @@ def test_equal_tables_of_a_job_are_kept_once(exe, tmp_path):
         paths.append(str(tmp_path / f"{k}.jpg"))
         open(paths[-1], "wb").write(O.jpeg_encode(J._gray(64, 64, 3 + 40 * k), 95, (1, 1), 0, O.JPEG_OPTIMIZE))
     _run(exe, "shared", *paths)
+
+
+@pytest.mark.parametrize("sel", [0x00, 0x20, 0x30])
+def test_a_scan_that_takes_ac_tables_for_dc(exe, tmp_path, sel):
+    """A scan header may name table 2 or 3 for DC codes: the AC tables 0 and 1,
+    as DC codes (common/pjpeg.c indexes one array of four)."""
+    p = str(tmp_path / "a.jpg")
+    open(p, "wb").write(J.dc_selector(O.jpeg_encode(J._rgb(64, 64, 5), 90, (2, 2), 0, O.JPEG_OPTIMIZE), sel))
+    _run(exe, "scans", p)
