@@ -1375,7 +1375,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
     __shared__ uint32_t s_scan[32];
     __shared__ double s_perr[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA], s_pmse[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA],
         s_pnx[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA], s_pny[AT_MAX_NMAXIMA * AT_MAX_NMAXIMA];
-    __shared__ double s_be[NT / 32], s_lines[4][4], s_lmse[4], s_best;
+    __shared__ double s_be[NT / 32], s_lines[4][4], s_lmse[4];
     __shared__ int s_bo[NT / 32];
     __shared__ uint32_t s_next;
     __shared__ uint64_t s_part[3 * NT / 32];
@@ -1737,10 +1737,10 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // reference keeps the first strictly smaller error in (m0, m1, m2, m3)
         // order, i.e. the smallest error and, among equal ones, the first in
         // that order. Each thread scans some of the 4-subsets (g_quad4); then
-        // a block-wide minimum of (error, order).
+        // a block-wide minimum of (error, order), which every thread then has.
+        const double inf = __longlong_as_double(0x7ff0000000000000ll);
+        double be = inf;
         {
-            const double inf = __longlong_as_double(0x7ff0000000000000ll);
-            double be = inf;
             int bo = 0x10000;
             const int n = nm, nsub = binom4(n);
             for (int t = tid; t < nsub; t += NT) {
@@ -1795,12 +1795,9 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
                 s_lmse[tid] = mse;
             }
             __syncthreads();
-            if (tid == 0) s_best = be;
         }
         if (tid < 32) {
-            const double inf = __longlong_as_double(0x7ff0000000000000ll);
-            const double best = s_best;
-            if (best != inf && best / (double)sz < prm.max_mse) {
+            if (be != inf && be / (double)sz < prm.max_mse) {
                 const double *l = s_lines[tid & 3];
                 const double ln[4] = {l[0], l[1], l[2], l[3]};
                 float p[2];

@@ -103,3 +103,23 @@ def test_uneven_angles(h, w, buckets):
     img += np.random.default_rng(1).normal(0, 0.4, img.shape)
     r = _same(np.clip(img, 0, 255).astype(np.uint8))
     assert max(_share(r.pts[a:b], buckets) for a, b in zip(r.cstart[:-1], r.cstart[1:])) > 17
+
+
+@pytest.mark.parametrize("side,pitch,lo,hi", [(100, 112, 513, 1024), (146, 160, 1025, 6144)])
+def test_clusters_with_and_without_a_quad_in_turn(side, pitch, lo, hi):
+    """More clusters of a block class than it has blocks, squares beside discs
+    and bars: each cluster is judged by its own best four corners."""
+    nx, ny = 4100 // pitch, 3000 // pitch
+    img = np.full((ny * pitch + 16, nx * pitch + 16), 200.0)
+    yy, xx = np.mgrid[0:side, 0:side] - (side - 1) / 2
+    discs = yy**2 + xx**2 <= side**2 / 4, abs(yy) + 0.9 * abs(xx - yy) < side / 2, np.ones((side, side), bool)
+    rng = np.random.default_rng(8)
+    for k, s in enumerate(rng.integers(0, 4, nx * ny)):
+        y, x = 8 + pitch * (k // nx), 8 + pitch * (k % nx)
+        img[y : y + side, x : x + side][discs[min(s, 2)]] = 40
+    r = _same(np.clip(img + rng.normal(0, 2, img.shape), 0, 255).astype(np.uint8))
+    sizes = np.diff(r.cstart)
+    n = ((sizes >= lo) & (sizes <= hi)).sum()
+    quads = ((sizes >= lo) & (sizes <= hi))[[q[2] for q in r.quads]].sum()
+    print(n, quads)
+    assert n > 148 * (4 if hi == 1024 else 2) and 0.2 * n < quads < 0.8 * n
