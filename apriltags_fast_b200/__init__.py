@@ -482,6 +482,7 @@ def _jpeg_lib():
                                           C.POINTER(C.c_int32)]
         L.at_jpeg_decode_gray.restype = C.c_int
         L.at_jpeg_last_stats.argtypes = [C.c_void_p, C.POINTER(C.c_double)]
+        L.at_jpeg_wait_stream.argtypes = [C.c_void_p, C.c_void_p]
         L.at_jpeg_set_sub_bits.argtypes = [C.c_void_p, C.c_int32]
         L.at_jpeg_set_threads.argtypes = [C.c_void_p, C.c_int32]
         L.at_jpeg_set_run_in.argtypes = [C.c_void_p, C.c_int32]
@@ -542,10 +543,15 @@ class JpegDecoder:
         return res, errs
 
     def decode_device(self, bufs, flags: int = 0, pad: int = 0):
-        """torch.uint8 CUDA frames (rows padded by `pad` bytes) and error codes."""
+        """torch.uint8 CUDA frames (rows padded by `pad` bytes) and error codes.
+        The frames' memory comes from torch's allocator: it is written after
+        the work queued on torch's current stream, which may still use what
+        lay there before."""
         import torch
         infos = [jpeg_info(b, flags) for b in bufs]
         outs = [torch.empty((max(h, 1), max(w, 1) + pad), dtype=torch.uint8, device="cuda") for _, w, h, _ in infos]
+        if self._L.at_jpeg_wait_stream(self._d, torch.cuda.current_stream().cuda_stream):
+            raise RuntimeError("at_jpeg_wait_stream: CUDA error")
         errs = self._call(bufs, [o.data_ptr() for o in outs], [o.stride(0) for o in outs], True, flags)
         return [o[:h, :w] if e == 0 else None for o, e, (_, w, h, _) in zip(outs, errs, infos)], errs
 

@@ -1917,6 +1917,17 @@ int at_jpeg_decode_gray(at_jpeg *dec, int32_t n, const uint8_t *const *bufs, con
     return failed;
 }
 
+int at_jpeg_wait_stream(at_jpeg *dec, void *stream) {
+    if (!dec) return 1;
+    std::lock_guard<std::mutex> lk(dec->mu);
+    cudaEvent_t e = nullptr;  // on the current device, as the stream is
+    if (!jcheck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate")) return 1;
+    bool ok = jcheck(cudaEventRecord(e, (cudaStream_t)stream), "event");
+    ok = ok && jcheck(cudaStreamWaitEvent(dec->stream, e, 0), "wait");
+    cudaEventDestroy(e);
+    return !ok;
+}
+
 int at_jpeg_last_stats(const at_jpeg *dec, double *out10) {
     if (!dec || !out10) return 1;
     memcpy(out10, dec->stats, sizeof dec->stats);

@@ -337,6 +337,14 @@ int at_jpeg_info(const uint8_t *buf, int64_t len, uint32_t flags, int32_t *width
 int at_jpeg_decode_gray(at_jpeg *dec, int32_t n, const uint8_t *const *bufs, const int64_t *lens, uint32_t flags,
                         uint8_t *const *dst, const int64_t *strides, int32_t on_device, int32_t *errors);
 
+/* Makes the decoder's work from here on wait for what is queued so far on
+   `stream` (a cudaStream_t of the calling thread's current device; NULL: its
+   default stream). A decode writes device frames on the decoder's own stream,
+   so call this before it when work on the frames' memory may still be under
+   way, such as kernels that read the frames an allocator had there before.
+   Returns 0 or 1 (CUDA error, message on stderr). */
+int at_jpeg_wait_stream(at_jpeg *dec, void *stream);
+
 /* Figures of the last decode: [0] host parse ms, [1] copy in ms, [2] sync
    pass ms, [3] write and IDCT ms, [4] copy out ms (CUDA events), [5] sub-
    streams, [6] sync passes beyond the first, [7] entropy-coded bytes, [8]

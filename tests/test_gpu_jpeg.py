@@ -212,3 +212,23 @@ def test_scans_that_take_ac_tables_for_dc(dec, sel):
     cases.append(("gray", J.dc_selector(O.jpeg_encode(J._gray(101, 150, 30), 85), sel), 0))
     check_batch(dec, cases)
     check_batch(dec, cases, device=True)
+
+
+def test_device_frames_wait_for_the_work_on_their_memory(dec):
+    """Frames decoded into memory that torch has just got back, while work
+    queued on its stream still reads what was there: that work is done first."""
+    import torch
+
+    bufs = [O.jpeg_encode(J._gray(480, 640, k), 90) for k in (1, 2)]
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            (frame,), _ = dec.decode_device(bufs[:1])
+            want, copy, ptr = frame.cpu(), torch.empty_like(frame), frame.data_ptr()
+            torch.cuda._sleep(100_000_000)  # cycles: some 50 ms
+            copy.copy_(frame)
+            del frame
+            (again,), _ = dec.decode_device(bufs[1:])
+            assert again.data_ptr() == ptr
+            assert torch.equal(copy.cpu(), want)
+            assert np.array_equal(again.cpu().numpy(), expected_gray(bufs[1], 0)[1])
+            del again, copy
