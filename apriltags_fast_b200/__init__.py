@@ -302,9 +302,10 @@ class Detector:
         return {n: getattr(t, n) for n, _ in Timing._fields_}
 
     def set_batch_split(self, pipelines: int) -> None:
-        """Spread large batches over this many pipelines (1-4, default 3),
-        each with its own streams, arenas and host thread; the results do
-        not depend on it."""
+        """Spread large batches over this many pipelines (1-4), each with its
+        own streams, arenas and host thread; without this call over 3 when
+        they have frames in host memory, else one. The results do not depend
+        on it."""
         if self._L.at_detector_set_batch_split(self._td, int(pipelines)) != 0:
             raise ValueError("pipelines must be 1 to 4")
 

@@ -26,9 +26,12 @@
 #include "at_kernels.h"
 
 // batch splitting: at most this many pipelines, each given at least
-// AT_SPLIT_MIN_FRAMES frames, and only for batches with frames to copy from
-// host memory, whose copies overlap another pipeline's kernels. 32 frames of
-// 1920 x 1080 in device memory: one pipeline 2.07 ms, two 2.15, three 2.26;
+// AT_SPLIT_MIN_FRAMES frames, and (unless the caller set their number) only
+// for batches with frames to copy from host memory, whose copies overlap
+// another pipeline's kernels. Frames in device memory, over one, two and three
+// pipelines: 32 of 640 x 480 0.57, 0.66, 0.80 ms; 32 of 1920 x 1080 1.38, 1.49,
+// 1.53 ms; 20 of 3840 x 2160 3.55 ms each; 20 of 4032 x 3024 5.04, 4.95, 4.97 ms
+// (one batch in turn varies by 0.03 ms on one pipeline, 0.2 to 0.5 on more);
 // below about 20 host frames one pipeline is as fast.
 #define AT_BATCH_SPLIT_DEFAULT 3
 #define AT_BATCH_SPLIT_MAX 4
@@ -140,7 +143,7 @@ struct at_internal {
     // and split - 1 helpers (each with its own streams and arenas), each
     // driven by its own host thread, so that one pipeline's host
     // synchronisations and latency-bound kernels overlap the others' work.
-    int split = AT_BATCH_SPLIT_DEFAULT;
+    int split = 0;  // as the caller set it, for every batch; 0: batch_pipelines decides
     at_detector *helper[AT_BATCH_SPLIT_MAX - 1] = {};
     uint64_t fam_gen = 0, helper_gen[AT_BATCH_SPLIT_MAX - 1] = {};
     struct CopyChain *chain = nullptr;  // the order of the pipelines' host copies
@@ -1047,19 +1050,31 @@ static bool run_split(at_detector *td, const at_frame *frames, int64_t n, at_fra
     return true;
 }
 
+// The pipelines of a batch: as many as the caller set; else
+// AT_BATCH_SPLIT_DEFAULT, or one for frames that lie in device memory and fit
+// one pipeline (its node ids below 2^31, a grid row a frame).
+static int batch_pipelines(const at_detector *td, const at_frame *frames, int64_t n) {
+    const at_internal *in = td->in;
+    const int P = (int)std::min<int64_t>(in->split ? in->split : AT_BATCH_SPLIT_DEFAULT, n / AT_SPLIT_MIN_FRAMES);
+    if (in->split || P <= 1) return P;
+    int64_t nodes = 0;
+    for (int64_t i = 0; i < n; i++) {
+        if (!device_pixels(in, frames[i].pixels)) return P;
+        int64_t qw = 0, qh = 0;
+        if (frames[i].width >= 8 && frames[i].height >= 8)
+            quad_size(frames[i].width, frames[i].height, td->quad_decimate, &qw, &qh);
+        nodes += (qw + 1) * qh;
+    }
+    return nodes < (int64_t)1 << 31 && n < 65536 ? 1 : P;
+}
+
 void at_detect_batch(at_detector *td, const at_frame *frames, int64_t n, at_frame_result *results) {
     at_internal *in = td->in;
     in->err = 0;
     in->msg.clear();
     td->ndetections = 0;
     td->nquads = 0;
-    int P = in->split;
-    if (P > n / AT_SPLIT_MIN_FRAMES) P = (int)(n / AT_SPLIT_MIN_FRAMES);
-    if (P > 1) {
-        bool copies = false;
-        for (int64_t i = 0; i < n && !copies; i++) copies = device_pixels(in, frames[i].pixels) == nullptr;
-        if (!copies) P = 1;
-    }
+    const int P = batch_pipelines(td, frames, n);
     const bool ok = P > 1 ? run_split(td, frames, n, results, P) : run_batch(td, frames, n, results);
     if (!ok) {
         in->dets.clear();

@@ -171,16 +171,17 @@ void at_detect_batch(at_detector *td, const at_frame *frames, int64_t n, at_fram
 int at_register_host_buffer(void *ptr, size_t bytes);
 int at_unregister_host_buffer(void *ptr);
 
-/* How many pipelines at_detect_batch spreads a large batch of frames in
-   host memory over, at most (1 to 4; 3 by default). Each pipeline takes a
-   run of consecutive frames (at least 10, with about equal pixel counts):
-   the first runs on this detector, the others on helper detectors made like
-   it (their own streams and device arenas, created at first use), each
-   driven by its own host thread, so that one pipeline's copies overlap
-   another's kernels. Frames in device memory alone need no copies and take
-   one pipeline. Results do not depend on the setting; at_timing and the
-   diagnostics describe the first pipeline's part. Returns -1 for a value out
-   of range. */
+/* How many pipelines at_detect_batch spreads a large batch over, at most (1
+   to 4). Without this call: 3 for a batch with frames in host memory; one
+   for frames in device memory alone, which need no copies (3 where one
+   pipeline has no room for them: 2^31 pixels of the quad images, 65536
+   frames). Each pipeline takes a run of consecutive frames (at least 10,
+   with about equal pixel counts): the first runs on this detector, the
+   others on helper detectors made like it (their own streams and device
+   arenas, created at first use), each driven by its own host thread, so that
+   one pipeline's copies overlap another's kernels. Results do not depend on
+   the setting; at_timing and the diagnostics describe the first pipeline's
+   part. Returns -1 for a value out of range. */
 int at_detector_set_batch_split(at_detector *td, int pipelines);
 
 /* Serving (no counterpart in the reference, which detects one frame per

@@ -232,3 +232,35 @@ def test_server_over_a_device_list():
         srv.close()
     with pytest.raises(RuntimeError):
         AT.Server(det, workers=1, devices=[31])
+
+
+def test_batch_split_of_device_frames():
+    """Frames in device memory take one pipeline, or as many as the caller
+    sets: the diagnostics then describe the first part only, the results are
+    the same."""
+    import torch
+
+    frames, _ = synth.uneven_batch(24, 11)
+    dev = [torch.from_numpy(np.ascontiguousarray(f)).cuda() for f in frames]
+    det = AT.Detector(["tag36h11"], 2)
+    ref = [d.tobytes() for d in det.detect_batch(dev, as_arrays=True)]
+    ref_nq, points = list(det.last_batch_nquads), len(det.diag("points"))
+    for pipelines, part in ((2, 0.75), (1, 1.0), (4, 0.75)):
+        det.set_batch_split(pipelines)
+        assert [d.tobytes() for d in det.detect_batch(dev, as_arrays=True)] == ref
+        assert list(det.last_batch_nquads) == ref_nq
+        n = len(det.diag("points"))
+        assert n == points if part == 1.0 else 0 < n < part * points
+
+
+def test_more_device_frames_than_one_pipeline_takes():
+    import torch
+
+    img = synth.make_frame(synth.Config(160, 120, ntags=(1, 1), side=(50, 60), tilt_deg=0.0), 2)[0]
+    small, tag = torch.full((9, 8), 90, dtype=torch.uint8, device="cuda"), torch.from_numpy(img).cuda()
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    alone = det.detect_batch([tag], as_arrays=True)[0].tobytes()
+    at = (0, 30000, 65599)
+    got = det.detect_batch([tag if i in at else small for i in range(65600)], as_arrays=True)
+    assert [got[i].tobytes() for i in at] == [alone] * 3
+    assert sum(len(d) for d in got) == 3 * len(got[0]) > 0
