@@ -1239,7 +1239,9 @@ extern "C" int at_fit_prof_copy(void *dst, int n) {
 // long cluster does not start last (unsorted, the 513-1024 class took 175
 // instead of 159 us; sorting the lists took a kernel of 27 us before each
 // block class). Clusters outside [min_cluster_pixels, max_px] of their frame
-// get no list (fast/quads.c:1180-1190). Every cluster's quad flag starts at 0.
+// get no list (fast/quads.c:1180-1190), and none does when the row tables were
+// too small (AT_ERR_SEGCAP: the points are not placed, the host runs the batch
+// again). Every cluster's quad flag starts at 0.
 __device__ __forceinline__ int fit_bucket(int64_t sz) {
     if (sz <= 512) return sz <= 128 ? 0 : sz <= 256 ? 1 : 2;
     if (sz <= FIT_SMALL) return sz <= 640 ? 3 : sz <= 768 ? 4 : sz <= 896 ? 5 : 6;
@@ -1262,8 +1264,9 @@ __device__ __forceinline__ uint32_t fit_next(const FitScratch &scr, int64_t nclu
 
 __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, const int32_t *cframe,
                                int64_t nclusters, int64_t npoints, int32_t min_px, uint32_t *quad_ok,
-                               uint32_t *lists, uint32_t *counts) {
+                               uint32_t *lists, uint32_t *counts, const uint32_t *err) {
     kernel_begin();
+    const bool placed = !(*err & AT_ERR_SEGCAP);
     __shared__ uint32_t s_n[FIT_NBUCKET], s_at[FIT_NBUCKET];
     for (int64_t c0 = (int64_t)blockIdx.x * blockDim.x; c0 < nclusters; c0 += (int64_t)gridDim.x * blockDim.x) {
         __syncthreads();
@@ -1275,7 +1278,7 @@ __global__ void k_fit_classify(const FrameDesc *frames, const uint32_t *cstart, 
         if (c < nclusters) {
             quad_ok[c] = 0;
             const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - cstart[c];
-            if (sz >= min_px && sz <= frames[cframe[c]].max_px) k = fit_bucket(sz);
+            if (placed && sz >= min_px && sz <= frames[cframe[c]].max_px) k = fit_bucket(sz);
             if (k >= 0) at = atomicAdd(s_n + k, 1u);
         }
         __syncthreads();
@@ -3605,7 +3608,7 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
     cudaMemsetAsync(scr.counts, 0, 2 * FIT_NBUCKET * sizeof(uint32_t), s);
     launch(k_fit_classify, flat_blocks(nclusters, 256), 256, 0, s, frames, cstart, cframe, nclusters, npoints,
                                                                 prm.min_cluster_pixels, quad_ok, scr.lists,
-                                                                scr.counts);
+                                                                scr.counts, err);
     // five streams, one per group of classes: above 6144 points (a block of
     // FIT_HUGE_NT each; only when a frame allows such clusters at all); the
     // other large clusters (a block of FIT_LARGE_NT each, two an SM: one

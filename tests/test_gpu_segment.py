@@ -121,3 +121,59 @@ def test_cluster_counts(n):
     assert np.array_equal(quads["p"].view(np.uint32), want.view(np.uint32))
     assert np.array_equal(quads["frame"], np.repeat([0, 1, 2], [len(r.quads) for r in ref]))
     assert [[d.key() for d in f] for f in got] == [r.dets for r in ref]
+
+
+def _strips(n, h):
+    """n strips side by side, light and dark in turn, with a slow ramp (no
+    contrast) between them but at both ends, where they touch; dots too small
+    for components keep each strip's contrast. So each pair of neighbours has
+    few points, first and last row far apart."""
+    w, gap, end = 12, 44, 16
+    lv = [(134, 122) if k % 2 == 0 else (122, 134) for k in range(n)]
+    img = np.zeros((h, n * (w + gap) + 24))
+    for x in range(img.shape[1]):
+        k, r = divmod(x - w, w + gap)
+        a, b = lv[k % 2]
+        img[:, x] = a + (b - a) * max(r - w, 0) / gap
+    for k in range(n):
+        x0 = w + k * (w + gap)
+        for y in range(4, h - 4, 8):
+            img[y : y + 3, x0 + 4 : x0 + 7] = lv[k][1]
+        if k + 1 == n:
+            break
+        x0 += w
+        m = x0 + gap // 2
+        for y0 in (0, h - end):
+            img[y0 : y0 + end, x0:m], img[y0 : y0 + end, m : x0 + gap] = lv[k]
+            for x in range(x0 + 2, x0 + gap - 3, 8):
+                if abs(x + 1 - m) >= 6:
+                    for y in range(y0 + 4, y0 + end - 3, 8):
+                        img[y : y + 3, x : x + 3] = lv[k][x < m]
+    return np.round(img).astype(np.uint8)
+
+
+@pytest.mark.parametrize("frames,n,h", [(1, 20, 1200), (15, 72, 500)])
+def test_pairs_that_span_many_rows(frames, n, h):
+    """The rows that the pairs span outnumber the row tables' first room
+    (points + 64 a pair + 4096), with few pairs (one block orders them) and
+    more than 1024: the batch runs again with more room, and later calls
+    have it."""
+    img = _strips(n, h)
+    r = O.detect(img, [H.oracle_family("tag36h11")], [2], O.default_params(quad_decimate=1.0), order=O.ORDER_CANON)
+    y = (r.pts >> np.uint64(16) & np.uint64(0xFFFF)).astype(int) // 2
+    spans = sum(y[a:b].max() - y[a:b].min() + 1 for a, b in zip(r.cstart[:-1], r.cstart[1:]))
+    pairs = len(r.cstart) - 1
+    assert frames * spans > frames * (len(r.pts) + 64 * pairs) + 4096
+    assert (frames * pairs > 1024) == (frames > 1)
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    launches = []
+    for rep in range(2):
+        before = int(det.diag("sizes")[5])
+        got = det.detect_batch([img] * frames)
+        launches.append(int(det.diag("sizes")[5]) - before)
+        assert np.array_equal(det.diag("points"), np.tile(r.pts, frames))
+        at = np.arange(frames)[:, None] * len(r.pts) + r.cstart[:-1].astype(int)
+        assert np.array_equal(det.diag("clusters").astype(int), at.ravel())
+        assert [[d.key() for d in f] for f in got] == [r.dets] * frames
+        assert det.last_batch_nquads == [len(r.quads)] * frames
+    assert launches[0] > launches[1] > 0
