@@ -447,6 +447,10 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
     in->last_qh = n > 0 ? fd[0].qh : 0;
     in->last_npts = in->last_ncl = in->last_nq = 0;
     if (qpx == 0) return true;
+    if (band_smem > SEGMENT_SMEM) {
+        set_error(in, 2, "quad image too wide");
+        return false;
+    }
     if (nodes >= ((int64_t)1 << 32)) {
         set_error(in, 2, "batch too large (union-find ids exceed 32 bits)");
         return false;

@@ -52,6 +52,7 @@ int64_t decimate_threshold_blocks(int64_t qw, int64_t qh);
 void launch_deglitch(const Launch &L, const FrameDesc *frames, uint8_t *thr, uint8_t *tmp);
 // Runs, components and labels (at_segment.cu). segment_plan: the most bands
 // of a frame and the shared memory of a band, over the batch's frames.
+#define SEGMENT_SMEM (224 * 1024)  // a band's, at most: quad images up to 425984 columns
 bool segment_set_smem();
 void segment_plan(int qw, int qh, int64_t *max_bands, size_t *smem);
 int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,

@@ -633,9 +633,9 @@ __global__ void __launch_bounds__(256) k_labels(const FrameDesc *frames, RunArra
 // Launchers.
 
 bool segment_set_smem() {
-    // the most a band takes: 8 rows of 2048 columns or one of 16384, or the
-    // words alone of a row of 65536
-    return cudaFuncSetAttribute(k_band_union, cudaFuncAttributeMaxDynamicSharedMemorySize, 80 * 1024) == cudaSuccess;
+    // 80 KB hold 8 rows of 2048 columns or one of 16384; the words alone of a
+    // wider row take 16 bytes per 32 columns
+    return cudaFuncSetAttribute(k_band_union, cudaFuncAttributeMaxDynamicSharedMemorySize, SEGMENT_SMEM) == cudaSuccess;
 }
 
 int launch_segment(const Launch &L, const FrameDesc *frames, int64_t max_bands, size_t smem, const uint8_t *thr,

@@ -177,3 +177,16 @@ def test_pairs_that_span_many_rows(frames, n, h):
         assert [[d.key() for d in f] for f in got] == [r.dets] * frames
         assert det.last_batch_nquads == [len(r.quads)] * frames
     assert launches[0] > launches[1] > 0
+
+
+@pytest.mark.parametrize("w", [131104, 425984, 425985])
+def test_very_wide_blank_frames(w):
+    """Rows whose words alone fill the shared memory of a band."""
+    det = AT.Detector(["tag36h11"], 2, quad_decimate=1.0)
+    blank = np.full((12, w), 90, np.uint8)
+    if w > 425984:
+        with pytest.raises(RuntimeError, match="too wide"):
+            det.detect(blank)
+        return
+    assert det.detect(blank) == [] and det.nquads == 0
+    assert (det.diag("labels") == 0xFFFFFFFF).all()
