@@ -78,6 +78,19 @@ __device__ __forceinline__ uint32_t warp_excl_scan(uint32_t v, uint32_t *total) 
     return incl - v;
 }
 
+// a / b rounded to nearest, from r = 1 / b rounded to nearest (Markstein's
+// division by a fused multiply-add: the second quotient is faithful, the third
+// correct, as long as no step leaves the normal range). The fit divides sums
+// of moments by sums of weights, both differences of prefix sums: b between
+// about 1 and 2^25, a 0 or between 2^-54 (the last place of the smallest
+// terms, where sums cancel) and 2^56, of either sign. Five divisions by one
+// weight take one reciprocal.
+__host__ __device__ __forceinline__ double div_by(double a, double b, double r) {
+    double q = a * r;
+    q = fma(fma(-b, q, a), r, q);
+    return fma(fma(-b, q, a), r, q);
+}
+
 // Words of row masks (RowWord): the columns of word i that runs cover (all
 // but the last column of the image), the run that covers column b of a word
 // (of its row; the column is in a run), and a node's component root (two

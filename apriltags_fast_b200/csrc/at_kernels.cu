@@ -857,17 +857,6 @@ __device__ __forceinline__ double smooth_at(const double *e, I n, I i, const dou
     return acc;
 }
 
-// a / b rounded to nearest, from r = 1 / b rounded to nearest (Markstein's
-// division by a fused multiply-add: the second quotient is faithful, the
-// third correct; a, b and the quotient far from the ends of the range, as
-// sums of weights >= 1 and of coordinates in [1/2, 65536) are). Five
-// divisions by one weight take one reciprocal.
-__device__ __forceinline__ double div_by(double a, double b, double r) {
-    double q = __dmul_rn(a, r);
-    q = __fma_rn(__fma_rn(-b, q, a), r, q);
-    return __fma_rn(__fma_rn(-b, q, a), r, q);
-}
-
 // Centroid and covariance of the moments (fast/quads.c:570-600, 604-653).
 struct MCov {
     double ex, ey, xx, xy, yy;
