@@ -896,11 +896,7 @@ at_detector *at_detector_create(void) {
         abort();
     }
     for (int k = 0; k < 12; k++) cudaEventCreate(&in->ev[k]);
-    // the fit's streams: larger clusters first (launch_fit_quads)
-    int least = 0, greatest = 0;
-    cudaDeviceGetStreamPriorityRange(&least, &greatest);
-    const int prio[4] = {std::max(greatest, least - 2), std::max(greatest, least - 1), least, greatest};
-    for (int k = 0; k < 4; k++) cudaStreamCreateWithPriority(&in->fit.side[k], cudaStreamNonBlocking, prio[k]);
+    for (cudaStream_t &q : in->fit.side) cudaStreamCreateWithFlags(&q, cudaStreamNonBlocking);
     cudaEventCreateWithFlags(&in->fit.fork, cudaEventDisableTiming);
     for (cudaEvent_t &e : in->fit.join) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     return td;

@@ -3602,11 +3602,11 @@ int launch_fit_quads(cudaStream_t s, const FitStreams &S, const FrameDesc *frame
     // FIT_HUGE_NT each; only when a frame allows such clusters at all); the
     // other large clusters (a block of FIT_LARGE_NT each, two an SM: one
     // cluster's serial steps overlap the other's); 513-1024 points (a block of
-    // 128, few of 257-512 too); 257-512 (a warp each); up to 256 (a warp each). The streams of the
-    // larger clusters have the higher priorities, so that their few long
-    // blocks start before the warp classes' resident waves fill the SMs (165
-    // instead of 173 us for eight 1280 x 720 frames; no difference for 32
-    // frames of 1920 x 1080).
+    // 128, few of 257-512 too); 257-512 (a warp each); up to 256 (a warp
+    // each). No stream has a priority: with higher ones for the larger
+    // clusters, so that their few long blocks start first, eight 1280 x 720
+    // frames take 587 instead of 603 us, but 32 of 1920 x 1080 1772 instead of
+    // 1749, and other streams of the process would wait behind them.
     const bool huge = max_px > FIT_LARGE_SORT;
     cudaEventRecord(S.fork, s);
     for (int k = 0; k < (huge ? 4 : 3); k++) cudaStreamWaitEvent(S.side[k], S.fork, 0);
