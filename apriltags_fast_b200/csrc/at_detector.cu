@@ -101,7 +101,7 @@ enum {
     B_FRAMES, B_IMG, B_QIM, B_THR, B_TMPA, B_TMPB, B_TMAX, B_TMIN, B_LAB,
     B_PARENT, B_PX, B_ROWRUNS, B_ROWPTS, B_ROWOFF, B_WORDS, B_RUNLAB, B_BANDN,
     B_KEY, B_VAL, B_KEY2, B_VAL2, B_HEAD, B_HSCAN, B_CSTART, B_CFRAME,
-    B_SKEYS, B_SSKEY, B_SSVAL, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
+    B_SKEYS, B_SSKEY, B_SSVAL, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW, B_SERRS, B_SFILT,
     B_SMXE, B_SMXI, B_QUADS, B_QOK, B_QSCAN, B_QUADSC, B_DETS, B_DETOK, B_OUT, B_QSTART, B_OUTOFF, B_OUTN, B_DIDX, B_DRM, B_MINID, B_FLIST, B_FCNT, B_QCORN, B_QH, B_QHOK, B_QNUM, B_FIRST, B_HKEYS, B_HCOUNT, B_HRANK, B_HOKEYS, B_HOSLOTS, B_HSKEYS, B_HSSLOTS, B_HCCOUNT, B_HMISC,
     B_HYMIN, B_HYMAX, B_CSPAN, B_CY0, B_SPANOFF, B_PKFRAME, B_PGKEYS, B_PGSLOTS, B_PGBUCKET, B_PFRAMES, B_PBSUM, B_SEG,
     B_QCL, B_CKEY, B_RNEED, B_RNT, B_RTLAB, B_RTPX, B_RTROOT, B_RTLIST, B_RTROW, B_RPRE, B_ROKEY, B_RIDX2,
@@ -699,7 +699,7 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         const uint64_t *ckey = hashed ? B[B_HSKEYS].as<uint64_t>() : B[B_CKEY].as<uint64_t>();
 
         // quads
-        const int sc[] = {B_SKEYS, B_SSKEY, B_SW, B_SFX, B_SFY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW,
+        const int sc[] = {B_SKEYS, B_SSKEY, B_SMX, B_SMY, B_SMXX, B_SMXY, B_SMYY, B_SMW,
                           B_SERRS, B_SFILT, B_SMXE};
         for (int b : sc) CK(B[b].ensure(npts * 8));
         CK(B[B_SSVAL].ensure(npts * 4));
@@ -711,7 +711,6 @@ static bool run_batch(at_detector *td, const at_frame *frames, int64_t n, at_fra
         CK(B[B_FLIST].ensure(ncl * 4 * FIT_NBUCKET));
         CK(B[B_FCNT].ensure(2 * FIT_NBUCKET * 4));
         FitScratch scr{B[B_SKEYS].as<uint64_t>(), B[B_SSKEY].as<uint64_t>(), B[B_SSVAL].as<uint32_t>(),
-                       B[B_SW].as<double>(),      B[B_SFX].as<double>(),    B[B_SFY].as<double>(),
                        B[B_SMX].as<double>(),     B[B_SMY].as<double>(),    B[B_SMXX].as<double>(),
                        B[B_SMXY].as<double>(),    B[B_SMYY].as<double>(),   B[B_SMW].as<double>(),
                        B[B_SERRS].as<double>(),   B[B_SFILT].as<double>(),  B[B_SMXE].as<double>(),

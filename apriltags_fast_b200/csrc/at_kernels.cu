@@ -656,41 +656,10 @@ __device__ __forceinline__ uint64_t angle_key(float dx, float dy, uint32_t idx) 
     return (uint64_t)(b ^ (s | 0x80000000u)) << 32 | (uint32_t)~idx;
 }
 
-// The leaf of the reference's angle sort holding position p of n
-// (fast/quads.c:181-237): cut in four while half the range has more than
-// 5 keys, then in two down to 5 or fewer. Returns start << 8 | length.
-__device__ __forceinline__ uint32_t leaf_of(int64_t n, int64_t p) {
-    int64_t lo = 0, sz = n;
-    while (sz / 2 > 5) {
-        int64_t half = sz / 2, q1 = half / 2, q3 = half + (sz - half) / 2;
-        int64_t r = p - lo;
-        if (r < q1) {
-            sz = q1;
-        } else if (r < half) {
-            lo += q1;
-            sz = half - q1;
-        } else if (r < q3) {
-            lo += half;
-            sz = q3 - half;
-        } else {
-            lo += q3;
-            sz = sz - q3;
-        }
-    }
-    while (sz > 5) {
-        int64_t half = sz / 2;
-        if (p - lo >= half) {
-            lo += half;
-            sz -= half;
-        } else {
-            sz = half;
-        }
-    }
-    return (uint32_t)(lo << 8 | sz);
-}
-
-// The leaf of position p of n (see leaf_of), in 32-bit arithmetic.
-__device__ __forceinline__ void leaf_of32(int n, int p, int &lo, int &len) {
+// The leaf [lo, lo + len) of the reference's angle sort that holds position p
+// of n (fast/quads.c:181-237): cut in four while half the range has more than
+// 5 keys, then in two down to 5 or fewer.
+__device__ __forceinline__ void leaf_of(int n, int p, int &lo, int &len) {
     int l = 0, sz = n;
     while (sz / 2 > 5) {
         const int half = sz / 2, q1 = half / 2, q3 = half + (sz - half) / 2;
@@ -1190,36 +1159,6 @@ __device__ void block_radix_sort32(uint32_t *ka, uint16_t *va, uint32_t *kb, uin
     }
 }
 
-
-// Optional phase timers of the fit kernel (a -DAT_FIT_PROF build only).
-#ifdef AT_FIT_PROF
-#define FIT_PROF_N 32768
-__device__ long long g_fitprof[FIT_PROF_N][12];
-#define FIT_PROF(k)                                              \
-    if (tid == 0 && c < FIT_PROF_N) g_fitprof[c][k] = clock64();
-#define FITW_PROF(k)                                             \
-    if (lane == 0 && c < FIT_PROF_N) g_fitprof[c][k] = clock64();
-#define FITW_SIZE(n)                                             \
-    if (lane == 0 && c < FIT_PROF_N) g_fitprof[c][0] = (n);
-#define FITB_SIZE(n)                                             \
-    if (tid == 0 && c < FIT_PROF_N) g_fitprof[c][0] = (n);
-__device__ long long g_decprof[8192][8];
-#define DEC_PROF(k)                                              \
-    if (tid == 0 && qi < 8192) g_decprof[qi][k] = clock64();
-extern "C" int at_dec_prof_copy(void *dst, int n) {
-    return (int)cudaMemcpyFromSymbol(dst, g_decprof, (size_t)n * 8 * 8);
-}
-extern "C" int at_fit_prof_copy(void *dst, int n) {
-    return (int)cudaMemcpyFromSymbol(dst, g_fitprof, (size_t)n * 12 * 8);
-}
-#else
-#define FIT_PROF(k)
-#define FITW_PROF(k)
-#define FITW_SIZE(n)
-#define FITB_SIZE(n)
-#define DEC_PROF(k)
-#endif
-
 // ---------------------------------------------------------------------------
 // The fit's size classes: clusters of at most 128, 256, 512 points (a warp
 // each; few of the last: see FIT_FEW), at most 1024 (a block of 128), at most 6144 (a block of 256), and
@@ -1389,8 +1328,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             if (tid == 0) atomicOr(err, AT_ERR_CLUSTER_TOO_BIG);
             continue;
         }
-        FIT_PROF(1)
-        FITB_SIZE(sz)
         const uint64_t *P = pts + s0;
         // bounding box (fast/quads.c:515-528)
         uint32_t xmin = 0xffff, xmax = 0, ymin = 0xffff, ymax = 0;
@@ -1425,7 +1362,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         const float cx = (float)((double)(xmin + xmax) * 0.5 + 0.05118);
         const float cy = (float)((double)(ymin + ymax) * 0.5 + -0.028581);
 
-        FIT_PROF(2)
         // angle keys, and the dot product of offsets and gradients: 8 lanes
         // over the whole groups of 8, then the rest (fast/quads.c:467-512)
         // clusters that fit keep their keys in shared memory, where the
@@ -1495,7 +1431,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         // block head and its place in the leaf; then one sort by (head,
         // place), packed into 64 bits as head's slope bits, 0xffff - head's
         // index, and the place.
-        FIT_PROF(3)
         // the sort's two pairs of buffers, in shared memory or global scratch
         uint32_t *ka = in_smem ? s_ka : reinterpret_cast<uint32_t *>(scr.skey + s0), *kb = in_smem ? s_kb : ka + sz;
         uint16_t *va = in_smem ? s_val : reinterpret_cast<uint16_t *>(scr.sval + s0), *vb = in_smem ? s_vb : va + sz;
@@ -1546,7 +1481,7 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             for (int64_t p0 = (int64_t)(tid >> 5) * 32; p0 < sz; p0 += NT) {
                 const int64_t p = p0 + lane;
                 int llo = -1, llen = 0;
-                if (p < sz) leaf_of32((int)sz, (int)p, llo, llen);
+                if (p < sz) leaf_of((int)sz, (int)p, llo, llen);
                 const bool lead = llo == (int)p;
                 const uint32_t lf = (uint32_t)llo << 8 | (uint32_t)llen;
                 const uint32_t bal = __ballot_sync(0xffffffffu, lead);
@@ -1562,10 +1497,8 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             if (lane < qn) arrange(lq[lane]);
         }
         __syncthreads();
-        FIT_PROF(4)
         if (!block_bucket_sort<NT>(ka, va, keys, (int)sz, s_hist))
             block_radix_sort32(ka, va, kb, vb, (int)sz, s_hist);
-        FIT_PROF(5)
 
         // cumulative weighted moments in angle order (fast/quads.c:968-1035):
         // Chunks of points get their six terms (moment_terms) staged in
@@ -1620,7 +1553,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
         __syncthreads();
         const Moments mo = {M[0], M[1], M[2], M[3], M[4], M[5]};
         const MSum all = moments_at(mo, sz - 1);
-        FIT_PROF(6)
 
         // corner search (fast/quads.c:788-959)
         const int64_t ksz = dmin(20, sz / 12);
@@ -1650,7 +1582,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             filt[i2] = fb;
         }
         __syncthreads();
-        FIT_PROF(7)
         // local maxima with wrap-around, compacted in index order: each
         // warp counts those of its own stretch, then writes them after the
         // warps' before it (two reads of filt, but only two barriers)
@@ -1706,7 +1637,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             }
             __syncthreads();
         }
-        FIT_PROF(8)
         // line fits of pairs of maxima: (a, b), a < b, and the closing pair
         // (b, a) wrapping around for b >= a + 3
         for (int t = tid; t < nm * nm; t += NT) {
@@ -1724,7 +1654,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
             s_pny[t] = lp[3];
         }
         __syncthreads();
-        FIT_PROF(9)
         // the 4 maxima with the smallest total error (quads.c:931-958): the
         // reference keeps the first strictly smaller error in (m0, m1, m2, m3)
         // order, i.e. the smallest error and, among equal ones, the first in
@@ -1803,10 +1732,6 @@ __global__ void __launch_bounds__(NT, (NT <= 128 ? 4 : NT <= 256 ? 2 : 1)) k_fit
                     }
                 }
             }
-            FIT_PROF(10)
-#ifdef AT_FIT_PROF
-            if (c < 16384) g_fitprof[c][0] = sz;
-#endif
         }
         __syncthreads();
     }
@@ -1943,8 +1868,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         const int64_t sz = (c + 1 < nclusters ? (int64_t)cstart[c + 1] : npoints) - s0;
         const FrameDesc f = frames[cframe[c]];
         const int n = (int)sz;
-        FITW_SIZE(n)
-        FITW_PROF(1)
         const uint64_t *P = pts + s0;
         // bounding box (fast/quads.c:515-528)
         uint32_t xmin = 0xffff, xmax = 0, ymin = 0xffff, ymax = 0;
@@ -1963,7 +1886,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             ymax = max(ymax, __shfl_xor_sync(FULL, ymax, o));
         }
         if ((int64_t)(xmax - xmin) * (int64_t)(ymax - ymin) < f.tag_width) continue;
-        FITW_PROF(2)
         const float cx = (float)((double)(xmin + xmax) * 0.5 + 0.05118);
         const float cy = (float)((double)(ymin + ymax) * 0.5 + -0.028581);
 
@@ -2008,14 +1930,13 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         okrev = __shfl_sync(FULL, okrev, 0);
         if (!(okrev & 1)) continue;
         const int rev = okrev >> 1;
-        FITW_PROF(3)
 
         // The angle sort (see k_fit_quads). Up to 256 points: packed keys by
         // buckets (177 points: 4900 cycles, a bitonic sort 19900); above: the
         // points laid out in (head index, place) order, then by buckets
         // (360 points: 22000 cycles, four radix passes 33000).
-        const uint16_t *s_order;  // point index of each sorted position
-        if constexpr (R <= 8) {
+        const uint16_t *s_order = nullptr;  // GP: point index of each sorted position
+        if constexpr (!GP) {
             // The angle sort (see k_fit_quads): position i of leaf (lo, len)
             // takes place t = i - lo of the leaf's network order; its sort key
             // packs the slope bits of its block head, 0xffff - the head's index,
@@ -2037,7 +1958,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                 uint64_t key = ~0ull;
                 if (i < n) {
                     int lo, len;
-                    leaf_of32(n, i, lo, len);
+                    leaf_of(n, i, lo, len);
                     uint64_t a[5];
     #pragma unroll
                     for (int t = 0; t < 5; t++) a[t] = t < len ? s_akey[lo + t] : ~0ull;
@@ -2060,7 +1981,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                 s_skey[i] = key;
             }
             __syncwarp();
-            FITW_PROF(4)
             if (warp_bucket_scan<NB>(s_hist, n, lane)) {
                 for (int i = lane; i < n; i += 32) {
                     const uint32_t b = s_at[i] >> 16, j = s_hist[b] + (s_at[i] & 0xffffu);
@@ -2079,22 +1999,19 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             } else {
                 warp_bitonic(s_skey, np, lane);
             }
-            s_order = nullptr;
         } else {
             // The angle sort (see k_fit_quads): the points laid out in (head
             // index descending, place) order, a lane per leaf, then a stable
-            // radix sort by the head's slope bits. The sort keys and indices
-            // live in region x1, their second buffers and the histogram in the
-            // prefix arrays (free until the moments).
+            // sort by the head's slope bits. The sort keys and indices live in
+            // region x1.
             uint32_t *s_ka = reinterpret_cast<uint32_t *>(x1);
             uint16_t *s_va = reinterpret_cast<uint16_t *>(x1 + 4 * CAP);
-            // second buffers: in x0 once the angle keys are read (GP: x0
-            // holds 8 B per point of capacity, 4 + 2 for the buffers and
-            // 1 KB for the histogram)
-            unsigned char *sb = GP ? x0 : reinterpret_cast<unsigned char *>(pm);
-            uint32_t *s_kb = reinterpret_cast<uint32_t *>(sb);
-            uint16_t *s_vb = reinterpret_cast<uint16_t *>(sb + 4 * CAP);
-            uint32_t *s_hist = reinterpret_cast<uint32_t *>(sb + (GP ? 6 : 8) * CAP);
+            // second buffers: in x0 once the angle keys are read (x0 holds 8 B
+            // per point of capacity, 4 + 2 for the buffers and 1 KB for the
+            // histogram)
+            uint32_t *s_kb = reinterpret_cast<uint32_t *>(x0);
+            uint16_t *s_vb = reinterpret_cast<uint16_t *>(x0 + 4 * CAP);
+            uint32_t *s_hist = reinterpret_cast<uint32_t *>(x0 + 6 * CAP);
             // (the leaves found 32 points at a time, queued behind s_va, and
             // laid out 32 leaves at a time)
             uint32_t *lq = reinterpret_cast<uint32_t *>(x1 + 6 * CAP);
@@ -2134,7 +2051,7 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             for (int p0 = 0; p0 < n; p0 += 32) {
                 const int p = p0 + lane;
                 int lo = -1, len = 0;
-                if (p < n) leaf_of32(n, p, lo, len);
+                if (p < n) leaf_of(n, p, lo, len);
                 const uint32_t bal = __ballot_sync(FULL, lo == p);
                 if (lo == p) lq[qn + __popc(bal & ((1u << lane) - 1u))] = (uint32_t)lo << 8 | (uint32_t)len;
                 qn += __popc(bal);
@@ -2147,7 +2064,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             }
             if (lane < qn) arrange(lq[lane]);
             __syncwarp();
-            FITW_PROF(4)
             // buckets, as block_bucket_sort: the counts behind s_va, the list in x0
             constexpr int NB = 256;
             static_assert(4 * NB <= 2 * CAP, "the counts fit x1");
@@ -2177,7 +2093,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             }
             __syncwarp();
         }
-        FITW_PROF(5)
 
         // cumulative weighted moments in angle order (fast/quads.c:968-1035):
         // the six terms of each position (moment_terms), then lane q < 6
@@ -2228,16 +2143,8 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
         } else {
             for (int k = lane; k < n; k += 64) {
                 const int k2 = k + 32 < n ? k + 32 : k;
-                uint32_t src, src2;
-                if constexpr (R <= 8) {
-                    const uint64_t *key = reinterpret_cast<const uint64_t *>(M5);
-                    src = (uint32_t)(key[k] & 0x1fffu);
-                    src2 = (uint32_t)(key[k2] & 0x1fffu);
-                } else {
-                    src = s_order[k];
-                    src2 = s_order[k2];
-                }
-                const uint64_t p1 = P[src], p2 = P[src2];
+                const uint64_t *key = reinterpret_cast<const uint64_t *>(M5);
+                const uint64_t p1 = P[key[k] & 0x1fffu], p2 = P[key[k2] & 0x1fffu];
                 const int32_t g1 = point_grad2(im, f.qw, f.qh, p1), g2 = point_grad2(im, f.qw, f.qh, p2);
                 double m1[6], m2[6];
                 moment_terms(p1, g1, m1);
@@ -2255,7 +2162,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             }
         }
         __syncwarp();
-        FITW_PROF(6)
         const Moments mo = {M0, M1, M2, M3, M4, M5};
         const MSum all = moments_at(mo, n - 1);
 
@@ -2278,7 +2184,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             s_filt[i2] = fb;
         }
         __syncwarp();
-        FITW_PROF(7)
         int nm = 0;
         for (int i0 = 0; i0 < n; i0 += 32) {
             const int i = i0 + lane;
@@ -2322,7 +2227,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             __syncwarp();
             nm = kept;
         }
-        FITW_PROF(8)
         // line fits of pairs of maxima
         for (int t = lane; t < nm * nm; t += 32) {
             const int p = t / nm, q = t - p * nm;
@@ -2338,7 +2242,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
             s_pny[t] = lp[3];
         }
         __syncwarp();
-        FITW_PROF(9)
         // the first smallest total error in (m0, m1, m2, m3) order: the
         // smallest (error, m0 m1 m2 m3) over the 4-subsets of the maxima
         double be = inf;
@@ -2370,7 +2273,6 @@ __global__ void __launch_bounds__(FIT_WPB * 32, 12) k_fit_warp(const FrameDesc *
                 bo = o2;
             }
         }
-        FITW_PROF(10)
         if (!(be != inf && be / (double)sz < prm.max_mse)) continue;
         // the 4 line fits, lanes 0-3 (quads.c:1069-1075)
         double ln[4] = {0.0, 0.0, 0.0, 0.0}, lmse = 0.0;
@@ -2404,87 +2306,15 @@ __device__ __forceinline__ double bil_seq(double a, double b, const uint8_t *p, 
     return (1.0 - a) * (1.0 - b) * p[0] + a * (1.0 - b) * p[1] + (1.0 - a) * b * p[s] + a * b * p[s + 1];
 }
 
-// One sample point of edge refinement (fast/decode.c:549-735): the
-// weighted mean step n0 along the normal, or false when no step counts.
-// The first vsteps steps (a multiple of 4) sum into 4 interleaved partial
-// sums. They go 4 at a time, each step's 8 pixels loaded before any is
-// used (a step outside the image loads pixel (0, 0) and counts 0), so the
-// loads of the 4 steps overlap; the rest of the steps follow in order.
 __device__ __forceinline__ double bil_vals(double a, double b, int p00, int p01, int p10, int p11) {
     double na = 1.0 - a, nb = 1.0 - b;
     return ((na * nb) * p00 + (a * nb) * p01) + ((na * b) * p10 + (a * b) * p11);
 }
 
-__device__ bool refine_sample(const DView &v, double x0, double y0, double nx, double ny, int64_t range,
-                              int64_t vsteps, int64_t nsteps, double *n0) {
-    const double wl = (double)(v.w - 1), hl = (double)(v.h - 1);
-    double ln[4] = {0.0, 0.0, 0.0, 0.0}, lc[4] = {0.0, 0.0, 0.0, 0.0};
-    const bool tiny = v.w < 2 || v.h < 2;
-    for (int64_t k0 = 0; k0 < vsteps; k0 += 4) {
-        bool in[4];
-        double fx1[4], fy1[4], fx2[4], fy2[4];
-        int px[4][8];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const double n = (double)-range + 0.25 * (double)(k0 + u);
-            const double x1 = x0 + (n + 1.0) * nx - 0.5, y1 = y0 + (n + 1.0) * ny - 0.5;
-            const double x2 = x0 + (n - 1.0) * nx - 0.5, y2 = y0 + (n - 1.0) * ny - 0.5;
-            in[u] = x1 > -1.0 && x1 < wl && y1 > -1.0 && y1 < hl && x2 > -1.0 && x2 < wl && y2 > -1.0 && y2 < hl;
-            const double tx1 = trunc(x1), ty1 = trunc(y1), tx2 = trunc(x2), ty2 = trunc(y2);
-            fx1[u] = x1 - tx1;
-            fy1[u] = y1 - ty1;
-            fx2[u] = x2 - tx2;
-            fy2[u] = y2 - ty2;
-            const bool safe = in[u] || !tiny;
-            const uint8_t *p1 = v.im + (in[u] ? (int64_t)ty1 * v.s + (int64_t)tx1 : 0);
-            const uint8_t *p2 = v.im + (in[u] ? (int64_t)ty2 * v.s + (int64_t)tx2 : 0);
-            if (safe) {
-                px[u][0] = p1[0], px[u][1] = p1[1], px[u][2] = p1[v.s], px[u][3] = p1[v.s + 1];
-                px[u][4] = p2[0], px[u][5] = p2[1], px[u][6] = p2[v.s], px[u][7] = p2[v.s + 1];
-            } else {
-#pragma unroll
-                for (int t = 0; t < 8; t++) px[u][t] = 0;
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const double n = (double)-range + 0.25 * (double)(k0 + u);
-            double wgt = 0.0;
-            if (in[u]) {
-                const double g1 = bil_vals(fx1[u], fy1[u], px[u][0], px[u][1], px[u][2], px[u][3]);
-                const double g2 = bil_vals(fx2[u], fy2[u], px[u][4], px[u][5], px[u][6], px[u][7]);
-                const double d = g2 - g1;
-                wgt = !(g1 < g2) ? d * d : 0.0;
-            }
-            ln[u] = ln[u] + wgt * n;
-            lc[u] = lc[u] + wgt;
-        }
-    }
-    double mn = 0.0 + ((ln[0] + ln[2]) + (ln[1] + ln[3]));
-    double mc = 0.0 + ((lc[0] + lc[2]) + (lc[1] + lc[3]));
-    for (int64_t k = vsteps; k < nsteps; k++) {
-        double n = (double)-range + 0.25 * (double)k;
-        double x1 = x0 + (n + 1.0) * nx - 0.5, y1 = y0 + (n + 1.0) * ny - 0.5;
-        int64_t x1i = c_int(x1), y1i = c_int(y1);
-        if (x1i < 0 || x1i + 1 >= v.w || y1i < 0 || y1i + 1 >= v.h) continue;
-        double x2 = x0 + (n - 1.0) * nx - 0.5, y2 = y0 + (n - 1.0) * ny - 0.5;
-        int64_t x2i = c_int(x2), y2i = c_int(y2);
-        if (x2i < 0 || x2i + 1 >= v.w || y2i < 0 || y2i + 1 >= v.h) continue;
-        double g1 = bil_seq(x1 - (double)x1i, y1 - (double)y1i, v.im + y1i * v.s + x1i, v.s);
-        double g2 = bil_seq(x2 - (double)x2i, y2 - (double)y2i, v.im + y2i * v.s + x2i, v.s);
-        if (g1 < g2) continue;
-        double wgt = (g2 - g1) * (g2 - g1);
-        mn = mn + wgt * n;
-        mc = mc + wgt;
-    }
-    if (mc == 0.0) return false;
-    *n0 = mn / mc;
-    return true;
-}
-
-// Lane u's share of one sample's first vsteps steps (a multiple of 4): the
-// steps k = u, u + 4, ..., summed in that order into (ln, lc), which is
-// partial sum u of refine_sample, so four lanes give its four sums.
+// One sample point of edge refinement (fast/decode.c:549-735) gives the
+// weighted mean of its steps along the normal. The reference sums the first
+// vsteps steps (a multiple of 4) into 4 interleaved partial sums: lane u's
+// share, the steps k = u, u + 4, ..., in that order into (ln, lc).
 __device__ __forceinline__ void refine_part(const DView &v, double x0, double y0, double nx, double ny, int64_t range,
                                             int64_t vsteps, int u, double *ln, double *lc) {
     const double wl = (double)(v.w - 1), hl = (double)(v.h - 1);
@@ -2518,7 +2348,7 @@ __device__ __forceinline__ void refine_part(const DView &v, double x0, double y0
 }
 
 // The steps after the first vsteps of one sample, in order, added to the
-// sums (mn, mc) (the tail of refine_sample).
+// sums (mn, mc).
 __device__ __forceinline__ void refine_tail(const DView &v, double x0, double y0, double nx, double ny, int64_t range,
                                             int64_t vsteps, int64_t nsteps, double *mn, double *mc) {
     for (int64_t k = vsteps; k < nsteps; k++) {
@@ -2767,7 +2597,6 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_refine(const FrameDesc *fram
     const int tid = threadIdx.x;
     for (int64_t qi = blockIdx.x; qi < nquads; qi += gridDim.x) {
         const GpuQuad q = quads[qi];
-        DEC_PROF(0)
         const FrameDesc f = frames[q.frame];
         DView v;
         if (prm.decode_blurred)
@@ -2861,7 +2690,6 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_refine(const FrameDesc *fram
                 }
                 __syncthreads();
             }
-            DEC_PROF(1)
             if (tid < 4) {
                 double ex = mx / cnt, ey = my / cnt;
                 double cxx = mxx / cnt - ex * ex, cxy = mxy / cnt - ex * ey, cyy = myy / cnt - ey * ey;
@@ -2887,7 +2715,6 @@ __global__ void __launch_bounds__(AT_DEC_THREADS) k_refine(const FrameDesc *fram
                 }
             }
             __syncthreads();
-            DEC_PROF(2)
         }
         if (tid < 8) corners[qi * 8 + tid] = s_p[tid >> 1][tid & 1];
         __syncthreads();
@@ -2948,7 +2775,6 @@ __global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *
         __syncthreads();
         if (tid < 9) s_H[tid] = hs[qi * 9 + tid];
         __syncthreads();
-        DEC_PROF(3)
         for (int fi = 0; fi < prm.nfam; fi++) {
             const GpuFamily &F = fams[fi];
             if (F.reversed_border != q.reversed_border) continue;
@@ -3030,7 +2856,6 @@ __global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *
             }
             __syncthreads();
             if (!s_pol) continue;
-            DEC_PROF(4)
             // bit values less the local threshold, sharpened (decode.c:340-377)
             const int64_t tw = F.tw;
             const int64_t minc = (wab - tw) / 2;
@@ -3059,7 +2884,6 @@ __global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *
                 s_sharp[t] = acc;
             }
             __syncthreads();
-            DEC_PROF(5)
             if (tid < 32) {
                 // the bits a lane each; then lane 0 sums the white ones in
                 // order and lane 1 the black ones (one lane for all of it
@@ -3122,7 +2946,6 @@ __global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *
                 }
             }
             __syncthreads();
-            DEC_PROF(6)
         }
         __syncthreads();
     }
@@ -3131,7 +2954,7 @@ __global__ void __launch_bounds__(DECODE_THREADS, 12) k_decode(const FrameDesc *
 // ---------------------------------------------------------------------------
 // 10. Per frame: gather the detections in (quad, family) order, remove
 // overlapping detections of one tag (fast/decode.c:766-891), stable sort by
-// id (fast/detector.c:164-179). One thread per frame.
+// id (fast/detector.c:164-179). A block per frame.
 
 struct GLine {
     double p[2], u[2];
@@ -3206,11 +3029,6 @@ __device__ __forceinline__ int prefer(int pref, double a, double b) {
     return pref ? pref : a < b ? -1 : b < a ? 1 : 0;
 }
 
-// One block per frame. Overlap removal only ever drops a detection in favour
-// of another with the same (family, id), and its outcome for one such
-// group depends only on that group's detections in quad order; so the
-// groups are resolved independently (one thread each, the rare groups of
-// two or more), and the survivors are placed by their stable rank by id.
 // The bucket count of the reference's cluster table for a quad image of
 // w x h at one thread (fast/clusters.c:97-103, fast/detector.c:223).
 __device__ __forceinline__ uint64_t ref_buckets(int64_t w, int64_t h) {
@@ -3220,6 +3038,11 @@ __device__ __forceinline__ uint64_t ref_buckets(int64_t w, int64_t h) {
     return (uint64_t)n;
 }
 
+// One block per frame. Overlap removal only ever drops a detection in favour
+// of another with the same (family, id), and its outcome for one such
+// group depends only on that group's detections in quad order; so the
+// groups are resolved independently (a warp each, the rare groups of
+// two or more), and the survivors are placed by their stable rank by id.
 __global__ void k_finalize(int nframes, const int64_t *frame_qstart, int nfam, const GpuDetection *dets,
                            const uint32_t *det_ok, uint32_t *idx, uint8_t *removed, GpuDetection *out,
                            const int64_t *out_off, int64_t *out_n, const FrameDesc *frames, RefOrder ref,

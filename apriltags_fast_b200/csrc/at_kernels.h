@@ -18,7 +18,6 @@ struct RunArrays {
 struct FitScratch {
     uint64_t *keys, *skey;
     uint32_t *sval;
-    double *w, *fx, *fy;
     double *mx, *my, *mxx, *mxy, *myy, *mw;
     double *errs, *filt, *mxe;
     int32_t *mxi;
