@@ -105,3 +105,33 @@ def bad_files():
 def dc_selector(buf, sel):
     """The file with the table selector of its first scan's first component replaced."""
     return _patch(buf, _find(buf, 0xDA) + 6, [sel])
+
+
+def many_tables(nscans, seed, h=64, w=72):
+    """A gray file of nscans scans of its one component, each with four Huffman
+    tables of its own (codes of 1 and 10 bits, so that most are found by a
+    second look-up) and random blocks coded with two of them."""
+    rng = np.random.default_rng(seed)
+    out = bytearray(b"\xff\xd8\xff\xdb\x00\x43\x00" + bytes(rng.integers(1, 9, 64, dtype=np.uint8)))
+    out += b"\xff\xc0\x00\x0b\x08" + bytes([h >> 8, h & 255, w >> 8, w & 255]) + b"\x01\x01\x11\x00"
+    for _ in range(nscans):
+        tabs = [rng.permutation(255) for _ in range(4)]  # (no FF: FF 00 reads as FF in headers too)
+        out += b"\xff\xc4" + (2 + 4 * (17 + 255)).to_bytes(2, "big")
+        for cls, t in zip((0x00, 0x01, 0x10, 0x11), tabs):
+            out += bytes([cls]) + bytes({1: 1, 10: 254}.get(n, 0) for n in range(1, 17)) + t.astype(np.uint8).tobytes()
+        out += b"\xff\xda\x00\x08\x01\x01\x00\x00\x3f\x00"
+        bits = []
+        for _ in range(((h + 7) // 8) * ((w + 7) // 8)):
+            z = 0
+            while z < 64:
+                t = tabs[0 if z == 0 else 2]
+                k = int(rng.choice(np.flatnonzero((t & 15) <= 8)))  # values of up to 8 bits
+                sym = int(t[k])
+                bits.append("0" if k == 0 else format((1 << 9) + k - 1, "010b"))
+                if sym & 15:
+                    bits.append(format(int(rng.integers(0, 1 << (sym & 15))), f"0{sym & 15}b"))
+                z += 1 if z == 0 else 64 if sym == 0 else (sym >> 4) + 1
+        data = "".join(bits)
+        data += "1" * (-len(data) % 8)
+        out += int(data, 2).to_bytes(len(data) // 8, "big").replace(b"\xff", b"\xff\x00")
+    return bytes(out) + b"\xff\xd9"

@@ -232,3 +232,12 @@ def test_device_frames_wait_for_the_work_on_their_memory(dec):
             assert torch.equal(copy.cpu(), want)
             assert np.array_equal(again.cpu().numpy(), expected_gray(bufs[1], 0)[1])
             del again, copy
+
+
+def test_a_job_whose_tables_pass_2_22_entries(dec):
+    """Files of many scans with tables of their own: alone, and after one
+    another in a call, so that a later file's tables lie high."""
+    cases = [(f"{n} scans", J.many_tables(n, n), 0) for n in (1, 132, 2)]
+    check_batch(dec, cases[1:2])
+    check_batch(dec, cases)
+    check_batch(dec, cases, device=True)

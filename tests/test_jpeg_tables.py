@@ -48,3 +48,12 @@ def test_a_scan_that_takes_ac_tables_for_dc(exe, tmp_path, sel):
     p = str(tmp_path / "a.jpg")
     open(p, "wb").write(J.dc_selector(O.jpeg_encode(J._rgb(64, 64, 5), 90, (2, 2), 0, O.JPEG_OPTIMIZE), sel))
     _run(exe, "scans", p)
+
+
+def test_a_file_whose_tables_pass_2_22_entries(exe, tmp_path):
+    """132 scans of four tables with 64 second levels each."""
+    p = str(tmp_path / "a.jpg")
+    buf = J.many_tables(132, 5)
+    assert O.jpeg_decode(buf)[0] == 0
+    open(p, "wb").write(buf)
+    _run(exe, "scans", p)
